@@ -316,6 +316,25 @@ static int reduce_core(Context *ctx, int algo, Work &w, const Outputs &o, oph_in
     return OPH_OK;
 }
 
+// The reduction without the column store, where it applies (complex2.cu).
+static int complex2_core(Context *ctx, int algo, C2Job &job, const Outputs &o, oph_info *info, bool *taken) {
+    *taken = false;
+    if (!complex2_applies(ctx, algo) || job.m < 1) return OPH_OK;
+    job.low = o.low;
+    job.ess = o.ess;
+    job.one_based = o.one_based;
+    oph_info local{};
+    int rc = reduce_complex2(ctx, job, &local, taken);
+    if (rc || !*taken) return rc;
+    if (o.arglow) {
+        k_fill_i32<<<grid_for(ctx, job.m), 256, 0, ctx->stream>>>(o.arglow, job.m, -1);
+        k_finalize2<<<grid_for(ctx, job.m), 256, 0, ctx->stream>>>(o.low, job.m, nullptr, 0, nullptr, o.arglow);
+        OPH_CUDA_TRY(cudaGetLastError());
+    }
+    if (info) *info = local;
+    return OPH_OK;
+}
+
 static int check_algo(int algo) { return algo >= OPH_ALGO_STANDARD && algo <= OPH_ALGO_PMS ? OPH_OK : OPH_ERR_ALGO; }
 
 }  // namespace oph
@@ -359,7 +378,7 @@ __attribute__((visibility("default"))) int oph_context_create(int device, oph_co
     ctx->device = device;
     cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMallocHost((void **)&ctx->h_status, sizeof(DevStatus)) != cudaSuccess) {
+        cudaMallocHost((void **)&ctx->h_status, 2 * sizeof(DevStatus)) != cudaSuccess) {
         delete ctx;
         return OPH_ERR_CUDA;
     }
@@ -422,20 +441,29 @@ __attribute__((visibility("default"))) int oph_reduce_device(oph_context *ctx, i
     if (!ctx || m < 0 || m >= (1ll << 29) || !d_colptr || (m > 0 && !d_low)) return OPH_ERR_BAD_INPUT;
     if (check_algo(algo)) return OPH_ERR_ALGO;
     OPH_CUDA_TRY(cudaSetDevice(ctx->device));
-    int64_t nnz = 0;
-    OPH_CUDA_TRY(cudaMemcpyAsync(&nnz, d_colptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-    OPH_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (nnz < 0 || (nnz > 0 && !d_rows)) return OPH_ERR_BAD_INPUT;
-    Work w;
-    int rc = alloc_work(ctx, w, m);
-    if (rc) return rc;
-    w.nnz = nnz;
-    w.colptr = d_colptr;
-    w.rows = d_rows;
     Outputs o;
     o.low = d_low;
     o.ess = d_ess;
     o.arglow = d_arglow;
+    C2Job job;
+    job.m = m;
+    job.colptr = d_colptr;
+    job.rows = d_rows;
+    bool taken = false;
+    int rc = complex2_core(ctx, algo, job, o, info, &taken);
+    if (rc || taken) return rc;
+    int64_t nnz = job.nnz;
+    if (!job.nnz_read) {
+        OPH_CUDA_TRY(cudaMemcpyAsync(&nnz, d_colptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+        OPH_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    }
+    if (nnz < 0 || (nnz > 0 && !d_rows)) return OPH_ERR_BAD_INPUT;
+    Work w;
+    rc = alloc_work(ctx, w, m);
+    if (rc) return rc;
+    w.nnz = nnz;
+    w.colptr = d_colptr;
+    w.rows = d_rows;
     rc = reduce_core(ctx, algo, w, o, info);
     if (rc) return rc;
     return OPH_OK;
@@ -456,18 +484,26 @@ __attribute__((visibility("default"))) int oph_reduce(oph_context *ctx, int algo
     if (!d_colptr || !d_rows || !d_out) return OPH_ERR_OOM;
     OPH_CUDA_TRY(cudaMemcpyAsync(d_colptr, colptr, sizeof(int64_t) * (m + 1), cudaMemcpyHostToDevice, s));
     if (nnz > 0) OPH_CUDA_TRY(cudaMemcpyAsync(d_rows, rows, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, s));
-    Work w;
-    int rc = alloc_work(ctx, w, m);
-    if (rc) return rc;
-    w.nnz = nnz;
-    w.colptr = d_colptr;
-    w.rows = d_rows;
     Outputs o;
     o.low = d_out;
     o.ess = ess ? d_out + m : nullptr;
     o.arglow = arglow ? d_out + 2 * m : nullptr;
-    rc = reduce_core(ctx, algo, w, o, info);
+    C2Job job;
+    job.m = m;
+    job.colptr = d_colptr;
+    job.rows = nnz > 0 ? d_rows : nullptr;
+    job.want_nnz = nnz;
+    bool taken = false;
+    int rc = complex2_core(ctx, algo, job, o, info, &taken);
     if (rc) return rc;
+    if (!taken) {
+        Work w;
+        if ((rc = alloc_work(ctx, w, m))) return rc;
+        w.nnz = nnz;
+        w.colptr = d_colptr;
+        w.rows = d_rows;
+        if ((rc = reduce_core(ctx, algo, w, o, info))) return rc;
+    }
     if (m > 0) {
         OPH_CUDA_TRY(cudaMemcpyAsync(low, d_out, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, s));
         if (ess) OPH_CUDA_TRY(cudaMemcpyAsync(ess, d_out + m, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, s));
@@ -480,14 +516,28 @@ __attribute__((visibility("default"))) int oph_reduce(oph_context *ctx, int algo
 static int batch_core(oph_context *ctx, int algo, int32_t count, const int64_t *d_col_off, const int64_t *d_colptr,
                       const int32_t *d_rows_local, int64_t total_m, int64_t total_nnz, int32_t *d_low, int32_t *d_ess,
                       oph_info *info) {
-    cudaStream_t s = ctx->stream;
+    Outputs o;
+    o.low = d_low;
+    o.ess = d_ess;
+    o.inst_off = d_col_off;
+    o.count = count;
+    C2Job job;
+    job.m = total_m;
+    job.colptr = d_colptr;
+    job.rows = d_rows_local;
+    job.inst_off = d_col_off;
+    job.count = count;
+    job.want_nnz = total_nnz;
+    bool taken = false;
+    int rc = complex2_core(ctx, algo, job, o, info, &taken);
+    if (rc || taken) return rc;
     ctx->launches = 0;
     // instance offsets, colptr and local rows checked, and the rows shifted
     // into their instances' column ranges, in one pass (a checked entry is
     // the only one written)
     int32_t *d_rows_g = (int32_t *)ctx_alloc(ctx, S_COO_R, sizeof(int32_t) * (total_nnz > 0 ? total_nnz : 1));
     if (!d_rows_g) return OPH_ERR_OOM;
-    int rc = check_csc(ctx, d_colptr, d_rows_local, total_m, total_nnz, d_col_off, count, d_rows_g);
+    rc = check_csc(ctx, d_colptr, d_rows_local, total_m, total_nnz, d_col_off, count, d_rows_g);
     if (rc) return rc;
     Work w;
     rc = alloc_work(ctx, w, total_m);
@@ -498,11 +548,6 @@ static int batch_core(oph_context *ctx, int algo, int32_t count, const int64_t *
     w.checked = true;
     w.inst_off = d_col_off;
     w.inst_count = count;
-    Outputs o;
-    o.low = d_low;
-    o.ess = d_ess;
-    o.inst_off = d_col_off;
-    o.count = count;
     return reduce_core(ctx, algo, w, o, info);
 }
 
@@ -803,14 +848,32 @@ __attribute__((visibility("default"))) int oph_openph(const char *algstr, const 
     OPH_CUDA_TRY(cudaMemsetAsync(w.st, 0, sizeof(DevStatus), s));
     rc = coo1_to_csc(ctx, d_r1, d_c1, nnz, m, d_colptr, d_rows);
     if (rc) return rc;
-    DevStatus hs;
-    if ((rc = ctx_sync_status(ctx, w, &hs))) return rc;
-    if (hs.error) return OPH_ERR_BAD_INPUT;
+    const bool track = h_low_true && (err_linf || err_lone || err_redu || err_ess);
+    Outputs o;
+    o.low = d_out;
+    o.one_based = 1;
+    o.ess = d_out + mm;
+    oph_info info{};
+    bool taken = false;
+    C2Job job;
+    if (!track) {
+        job.m = m;
+        job.colptr = d_colptr;
+        job.rows = nnz > 0 ? d_rows : nullptr;
+        job.want_nnz = nnz;
+        job.before = w.st;  // the conversion's check comes back with the first read of the status
+        if ((rc = complex2_core(ctx, algo, job, o, &info, &taken))) return rc;
+        if (job.before_error) return OPH_ERR_BAD_INPUT;
+    }
+    if (!job.nnz_read) {
+        DevStatus hs;
+        if ((rc = ctx_sync_status(ctx, w, &hs))) return rc;
+        if (hs.error) return OPH_ERR_BAD_INPUT;
+    }
     w.nnz = nnz;
     w.colptr = d_colptr;
     w.rows = d_rows;
     w.checked = true;  // the COO conversion validated every entry
-    const bool track = h_low_true && (err_linf || err_lone || err_redu || err_ess);
     int32_t *lt0 = d_lt, *esst = d_lt + mm;
     if (track && m > 0) {
         // low_true arrives 1-based and is compared 0-based like the
@@ -842,12 +905,7 @@ __attribute__((visibility("default"))) int oph_openph(const char *algstr, const 
     SeqTracking stk;
     const bool per_col = track && m > 0 && algo != OPH_ALGO_PMS;
     if (per_col) ctx->seq_track = &stk;
-    Outputs o;
-    o.low = d_out;
-    o.one_based = 1;
-    o.ess = d_out + mm;
-    oph_info info{};
-    rc = reduce_core(ctx, algo, w, o, &info);
+    if (!taken) rc = reduce_core(ctx, algo, w, o, &info);
     ctx->track = nullptr;
     ctx->seq_track = nullptr;
     if (rc) return rc;

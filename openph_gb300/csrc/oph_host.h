@@ -75,6 +75,27 @@ int grow_pool(Context *ctx, Work &w);
 // pms.cu
 int run_pms(Context *ctx, Work &w, oph_info *info);
 
+// complex2.cu: pms on a simplicial complex of dimension <= 2 without the
+// column store.  *taken false: the matrix is not one it accepts (or there is
+// no room), nothing of the outputs is settled and the general path decides.
+struct C2Job {
+    int64_t m = 0;
+    const int64_t *colptr = nullptr;    // device, m + 1
+    const int32_t *rows = nullptr;      // device; local to each instance
+    const int64_t *inst_off = nullptr;  // device, count + 1 (nullptr: one matrix)
+    int count = 1;
+    int64_t want_nnz = -1;              // colptr[m] the caller expects (-1: any)
+    const DevStatus *before = nullptr;  // a status block earlier work reported into, read along
+    int32_t *low = nullptr, *ess = nullptr;  // device outputs (ess may be nullptr)
+    int one_based = 0;
+    // out: colptr[m], and before->error, once the first read-back happened
+    int64_t nnz = 0;
+    bool nnz_read = false;
+    int before_error = 0;
+};
+bool complex2_applies(const Context *ctx, int algo);
+int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken);
+
 // variants.cu
 int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *info);
 
@@ -172,7 +193,7 @@ struct Context {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[8] = {};
     DevBuf bufs[48];  // indexed by Slot
-    DevStatus *h_status = nullptr;  // pinned mirror
+    DevStatus *h_status = nullptr;  // pinned mirrors (two)
     int max_sweeps = 0;             // 0 = default
     int64_t initial_pool_bytes = 0; // 0 = default
     int64_t budget = 0;
@@ -204,7 +225,7 @@ struct Context {
 enum Slot {
     S_STATUS, S_COLPTR, S_ROWS, S_LOW, S_CLASSES, S_CLEAR, S_DIM, S_FIRST, S_LEFT, S_BETA, S_WORK, S_WIDE, S_SEG,
     S_ROWPIV, S_AGG, S_POOL, S_POOL2, S_ESS, S_ARGLOW, S_COO_R, S_COO_C, S_LOWTRUE, S_TRACK, S_INSTOFF, S_TMP,
-    S_ULIST, S_KAGG, S_ESSHAT, S_SLIST, S_DGRADE, S_DCOLPTR, S_DSORT, S_DTEMP, S_DLOW, S_BITMAP, S_CHECK, S_IASC, S_IBUCKET, S_IOPEN, S_RANGES, S_SEQNS, S_PRECLEAR, S_NSLOTS
+    S_ULIST, S_KAGG, S_ESSHAT, S_SLIST, S_DGRADE, S_DCOLPTR, S_DSORT, S_DTEMP, S_DLOW, S_BITMAP, S_CHECK, S_IASC, S_IBUCKET, S_IOPEN, S_RANGES, S_SEQNS, S_PRECLEAR, S_C2_TAB, S_C2_WORK, S_NSLOTS
 };
 
 }  // namespace oph

@@ -1,0 +1,109 @@
+"""pms without the column store (csrc/complex2.cu) against the oracle's twist,
+at the sizes and forms where its kernels take another branch, and the inputs
+it must leave to the general path."""
+import numpy as np
+import pytest
+
+import oracle
+from cases import lower_star_volume, random_complex, simplex_skeleton, triangle
+from openph_gb300 import complexes as cx
+from openph_gb300.complexes import BoundaryMatrix
+
+pytestmark = pytest.mark.gpu
+
+
+def check(ctx, bm, **kw):
+    want, want_ess, _ = oracle.twist(bm)
+    low, ess, arg, info = ctx.reduce(bm, "pms", with_arglow=True)
+    np.testing.assert_array_equal(low, want)
+    np.testing.assert_array_equal(ess, want_ess)
+    want_arg = np.full(bm.m, -1, np.int32)
+    want_arg[want[want >= 0]] = np.flatnonzero(want >= 0)
+    np.testing.assert_array_equal(arg, want_arg)
+    return info
+
+
+def shuffled(bm, seed):
+    """The same complex in another filtration order: a random value per
+    simplex, at least its faces' (kinds of columns interleave freely)."""
+    rng = np.random.default_rng(seed)
+    val = rng.random(bm.m)
+    for j in range(bm.m):
+        col = bm.column(j)
+        if len(col):
+            val[j] = max(val[j], val[col].max() + 1e-9)
+    order = np.argsort(val, kind="stable")
+    pos = np.empty(bm.m, np.int64)
+    pos[order] = np.arange(bm.m)
+    return BoundaryMatrix.from_columns([sorted(pos[bm.column(j)].tolist()) for j in order])
+
+
+def graph(n_vertices, edges):
+    return BoundaryMatrix.from_columns([[] for _ in range(n_vertices)] + [sorted(e) for e in edges])
+
+
+# one tile of columns is 2048; 24 x 14 is 1,909 columns, 21 x 17 is 2,029, 18 x 20 is 2,047, 19 x 19 2,053
+@pytest.mark.parametrize("h,w,sigma", [(2, 2, 0.5), (2, 40, 1.0), (18, 20, 1.0), (19, 19, 0.5), (63, 65, 3.0),
+                                       (97, 203, 4.0), (150, 160, 0.3)])
+def test_images(ctx, h, w, sigma):
+    assert check(ctx, cx.lower_star_image(h, w, seed=h + w, sigma=sigma))["sweeps"] >= 1
+
+
+@pytest.mark.parametrize("kind", ["flat", "ties", "stairs", "bowl"])
+def test_images_of_special_order(ctx, kind):
+    y, x = np.mgrid[0:40, 0:37]
+    img = {"flat": 0 * x, "ties": (7 * x * x + 5 * y) % 4, "stairs": (x % 2) * 100 - x,
+           "bowl": (x - 15.2) ** 2 + 0.5 * (y - 20.1) ** 2}[kind]
+    check(ctx, cx.lower_star(img.astype(np.float32)))
+
+
+@pytest.mark.parametrize("seed", range(3))
+def test_kinds_interleaved(ctx, seed):
+    check(ctx, shuffled(cx.lower_star_image(20, 15, seed=seed, sigma=1.0), seed))
+
+
+def test_graphs(ctx):
+    rng = np.random.default_rng(5)
+    path = [(i, i + 1) for i in range(299)]
+    check(ctx, graph(300, path))
+    check(ctx, graph(300, path[::-1]))  # every edge but the first joins a younger singleton
+    check(ctx, graph(40, [(0, i) for i in range(1, 40)]))
+    multi = [tuple(sorted(rng.choice(30, 2, replace=False).tolist())) for _ in range(200)]  # parallel edges
+    check(ctx, graph(34, multi))
+    check(ctx, graph(2, [(0, 1)]))
+
+
+def test_batch_of_images_and_graphs(ctx):
+    mats = [cx.lower_star_image(9, 12, seed=1, sigma=1.0), BoundaryMatrix.from_columns([]), graph(5, [(0, 4), (1, 2)]),
+            BoundaryMatrix.from_columns([[]] * 3), cx.lower_star_image(31, 22, seed=2, sigma=1.0), triangle()]
+    lows, esss, _ = ctx.reduce_batch(mats, "pms")
+    for bm, low, ess in zip(mats, lows, esss):
+        if bm.m:
+            want, want_ess, _ = oracle.twist(bm)
+            np.testing.assert_array_equal(low, want)
+            np.testing.assert_array_equal(ess, want_ess)
+
+
+def test_left_to_the_general_path(ctx):
+    """Matrices that are no such complex give what 'never' (the sweeps on D)
+    gives: a column of one row, of four rows, rows of the wrong kind, three
+    edges that bound nothing, and larger complexes."""
+    path3 = BoundaryMatrix.from_columns([[], [], [], [], [0, 1], [1, 2], [2, 3], [4, 5, 6]])
+    one_row = BoundaryMatrix.from_columns([[], [], [0], [0, 1]])
+    squares = BoundaryMatrix.from_columns([[], [], [], [], [0, 1], [1, 2], [2, 3], [0, 3], [4, 5, 6, 7]])
+    mixed = BoundaryMatrix.from_columns([[], [], [], [0, 1], [0, 2], [1, 2], [3, 4, 5], [0, 1, 2]])
+    edge_on_edge = BoundaryMatrix.from_columns([[], [], [0, 1], [0, 2]])
+    for bm in (path3, one_row, squares, mixed, edge_on_edge, simplex_skeleton(7, seed=3), lower_star_volume(4, seed=1)):
+        ctx.set_dual("never")
+        low_n, ess_n, _ = ctx.reduce(bm, "pms")
+        ctx.set_dual("auto")
+        low, ess, _ = ctx.reduce(bm, "pms")
+        np.testing.assert_array_equal(low, low_n)
+        np.testing.assert_array_equal(ess, ess_n)
+
+
+@pytest.mark.parametrize("p_tri", [0.1, 0.5])
+def test_crowded_edges(ctx, p_tri):
+    """Sparse 2-complexes, some of whose edges have more than two triangles."""
+    for seed in range(4):
+        check(ctx, random_complex(16, 0.4, p_tri, seed))
