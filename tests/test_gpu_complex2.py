@@ -107,3 +107,53 @@ def test_crowded_edges(ctx, p_tri):
     """Sparse 2-complexes, some of whose edges have more than two triangles."""
     for seed in range(4):
         check(ctx, random_complex(16, 0.4, p_tri, seed))
+
+
+@pytest.mark.parametrize("n", [3, 4, 5, 31, 32, 33, 50, 65, 100])
+def test_rips_full(ctx, n):
+    check(ctx, cx.rips_cube(n, seed=n))
+    check(ctx, cx.rips(cx.points_circle(n, seed=n)))
+
+
+@pytest.mark.parametrize("target", [3_000, 40_000, 200_000, 700_000])
+def test_rips_thresholds(ctx, target):
+    """Torus complexes cut off early: essential classes, several components,
+    windows of triangles left behind."""
+    check(ctx, cx.rips_torus(300, target, seed=target))
+
+
+def test_rips_ties(ctx):
+    """Equal distances (a grid, repeated points): few apparent pairs."""
+    g = np.stack(np.meshgrid(*[np.arange(3.0)] * 3), -1).reshape(-1, 3)
+    check(ctx, cx.rips(g))
+    check(ctx, cx.rips(g, threshold=1.5))
+    check(ctx, cx.rips(np.repeat(g[:12], 3, axis=0)))
+
+
+@pytest.mark.parametrize("n,seed", [(12, 0), (20, 1), (28, 2)])
+def test_rips_in_any_order(ctx, n, seed):
+    """Random filtration orders: most edges are residual, their columns sums
+    of many, claimed and taken over by CTAs at the same time."""
+    check(ctx, shuffled(cx.rips_cube(n, seed=seed), seed))
+
+
+def test_doubled_simplices(ctx):
+    """Two triangles on the same edges, two edges on the same vertices: no
+    simplicial complex, and too many triangles for a graph."""
+    tri = [[0, 1], [0, 2], [1, 2]]
+    cols = [[], [], []] + tri + [[3, 4, 5]] * 4
+    check(ctx, BoundaryMatrix.from_columns(cols))
+    cols = [[], [], []] + tri + [[1, 2]] + [[3, 4, 5], [3, 4, 6], [3, 4, 5], [3, 4, 6], [3, 4, 6]]
+    check(ctx, BoundaryMatrix.from_columns(cols))
+
+
+def test_batch_of_rips(ctx):
+    mats = [cx.rips_mixed(n, seed=70 + n) for n in (60, 3, 25, 2, 1, 40)]
+    mats[2:2] = [BoundaryMatrix.from_columns([]), triangle(), cx.lower_star_image(9, 7, seed=5)]
+    mats.append(shuffled(cx.rips_cube(18, seed=9), 4))
+    lows, esss, _ = ctx.reduce_batch(mats, "pms")
+    for bm, low, ess in zip(mats, lows, esss):
+        if bm.m:
+            want, want_ess, _ = oracle.twist(bm)
+            np.testing.assert_array_equal(low, want)
+            np.testing.assert_array_equal(ess, want_ess)
