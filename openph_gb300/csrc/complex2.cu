@@ -56,7 +56,7 @@ struct C2Word {
 struct __align__(16) C2Inst {
     int voff, eoff, nv, ne;
     long long base, cols;
-    long long coff, pad;  // its part of the edge-vertex table
+    long long coff, roff;  // its part of the table (cells) and of the runs' bits
 };
 struct C2Status {
     int bad;         // a column or row that is none of the accepted kinds
@@ -68,9 +68,11 @@ struct C2Status {
     int live[3];     // edges left, by round modulo three
     unsigned long long joins;
     int max_nv;      // the largest instance's vertices
+    int unsorted;    // the triangles do not come in runs
     int nres, cursor, overflow;      // residual edges; the CTAs' queue; a list ran out of room
     long long cells;                 // entries of the edge-vertex table
-    unsigned long long cells_set;    // and those a triangle wrote
+    long long pairs, run_words;      // entries of the edge-id table, words of the runs' bits
+    unsigned long long cells_set;    // entries of the edge-vertex table that a triangle wrote
     unsigned long long arena;        // entries of published lists
     unsigned long long adds, slots;  // additions of the residual columns, entries toggled
 };
@@ -78,8 +80,7 @@ struct C2Status {
 constexpr int C2_THREADS = 256, C2_TILE = 2048;
 constexpr int C2_MAX_ROUNDS = 512;
 constexpr int C2_MAX_NV = 8192;                   // vertices of an instance the dense form takes
-constexpr int RS_THREADS = 256, RS_WORDS = 8192;  // residual columns: a CTA, a window of 2^18 triangles
-constexpr int RS_WAVE = 16;                       //   pivots added at a time
+constexpr int RS_WAVE = 16;                       // residual columns: pivots added at a time,
 constexpr int RS_LIST = 16384;                    //   edges a column under reduction may be the sum of
 constexpr int RS_FLAG = 1 << 30;
 
@@ -107,17 +108,18 @@ struct C2Args {
     int32_t *tlist;           // column of each triangle
     int32_t *low, *ess;       // outputs
     int one_based;
-    // dense form: the edge-vertex table, the vertex that dies at each edge
-    // (-1: none), the owner of each triangle's row (an edge's rank; with
-    // RS_FLAG a residual one, which may still change; -1: none) and which
-    // have one, the residual edges with their first triangles, the triangle
-    // each holds, the list its column is the sum of (offset << 24 | length)
-    int32_t *cells;
+    // dense forms: the vertex that dies at each edge (-1: none) and which
+    // vertices die; the edge-vertex table or, with runs, the edge-id table
+    // (vertices by vertices), its rows in edge order, and the runs (per edge
+    // and 32 vertices: which have a triangle, and the first one's column); which triangles have an
+    // owner (low[] names it), and which for good; the residual edges, and the
+    // list each is the sum of (offset << 24 | length)
     int32_t *neg;
-    int32_t *owner;
-    uint32_t *owned;
-    int2 *res;
-    int32_t *death;
+    uint8_t *dead;
+    int32_t *cells, *adj;
+    uint2 *runs;
+    uint32_t *owned, *fixed;
+    int32_t *res;
     unsigned long long *sum;
     int32_t *arena;
     long long arena_cap;
@@ -195,6 +197,9 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_words(C2Args a) {
     if (bad) a.st->bad = 1;
 }
 
+// The pitch of an instance's rows over its vertices: whole 16-byte loads.
+__host__ __device__ __forceinline__ int c2_pitch(int nv) { return (nv + 3) & ~3; }
+
 // Exclusive prefix over the block of 1024 threads; red holds 33 values.
 __device__ __forceinline__ long long c2_block_excl(long long v, long long *red, long long *total) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -268,12 +273,14 @@ __global__ void __launch_bounds__(1024) k_c2_scan(C2Args a, int64_t ntiles) {
             s.cols = a.m;
             a.inst[0] = s;
             a.st->max_nv = s.nv;
-            a.st->cells = (long long)s.nv * s.ne;
+            a.st->cells = (long long)c2_pitch(s.nv) * s.ne;
+            a.st->pairs = (long long)c2_pitch(s.nv) * s.nv;
+            a.st->run_words = (long long)((s.nv + 31) >> 5) * s.ne;
         }
     }
     __syncthreads();
     if (!a.inst_off) return;
-    long long cells = 0;
+    long long cells = 0, pairs = 0, words = 0;
     for (int b0 = 0; b0 < a.count; b0 += 1024) {
         const int b = b0 + (int)threadIdx.x;
         C2Inst s{};
@@ -292,12 +299,34 @@ __global__ void __launch_bounds__(1024) k_c2_scan(C2Args a, int64_t ntiles) {
                 atomicMax(&a.st->max_nv, s.nv);
             }
         }
+        // coff serves the form tried first (runs); the table's is k_c2_cells'
         long long total;
-        s.coff = cells + c2_block_excl((long long)s.nv * s.ne, red, &total);
+        s.coff = pairs + c2_block_excl((long long)c2_pitch(s.nv) * s.nv, red, &total);
+        pairs += total;
+        s.roff = words + c2_block_excl((long long)((s.nv + 31) >> 5) * s.ne, red, &total);
+        words += total;
+        c2_block_excl((long long)c2_pitch(s.nv) * s.ne, red, &total);
         cells += total;
         if (b < a.count) a.inst[b] = s;
     }
-    if (threadIdx.x == 0) a.st->cells = cells;
+    if (threadIdx.x == 0) {
+        a.st->cells = cells;
+        a.st->pairs = pairs;
+        a.st->run_words = words;
+    }
+}
+
+// The instances' parts of the edge-vertex table (one block).
+__global__ void __launch_bounds__(1024) k_c2_cells(C2Args a) {
+    __shared__ long long red[33];
+    long long cells = 0, total;
+    for (int b0 = 0; b0 < a.count; b0 += 1024) {
+        const int b = b0 + (int)threadIdx.x;
+        const long long n = b < a.count ? (long long)c2_pitch(a.inst[b].nv) * a.inst[b].ne : 0;
+        const long long off = cells + c2_block_excl(n, red, &total);
+        cells += total;
+        if (b < a.count) a.inst[b].coff = off;
+    }
 }
 
 // A thread per word: absolute ranks, the lists of vertices and edges, the
@@ -372,6 +401,16 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_edges(C2Args a) {
         }
         a.erec[k] = make_int4(u, v, b, 0);
         if (a.neg) a.neg[k] = -1;
+        if (a.runs && !bad) {
+            // the edge on two vertices (its rank in the instance), from either side
+            int32_t *t = a.cells + in.coff;
+            const int pitch = c2_pitch(in.nv), x = u - in.voff, y = v - in.voff;
+            const C2Word w = a.words[j >> 5];
+            if (atomicCAS(t + (int64_t)x * pitch + y, -1, k - in.eoff) != -1 ||
+                w.vpre + __popc(w.v & below(j & 31)) != in.voff + in.nv)
+                a.st->unsorted = 1;
+            t[(int64_t)y * pitch + x] = k - in.eoff;
+        }
         if (a.ends) {
             a.ends[k] = make_int2(u, v);
             a.ends[2 * (int64_t)ne - 1 - k] = make_int2(-1, -1);
@@ -576,108 +615,187 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_graph(C2Args a, int max_round
 }
 
 // -------------------------------------------------------------- dense form
-// The edges on vertices of one instance, by the elder rule, a CTA in column
-// order: 1024 edges at a time whose ends carry different labels (most after
-// the first few hundred do not), those joined one by one by a warp, which
-// relabels the younger component.  It stops when one component is left: on
-// the torus after 1,788 of 58,988 edges.  Bound by the latency of its
-// nv - 1 relabellings, and hidden behind the triangles of the same launch.
+// The edges on vertices of one instance, by the elder rule, a CTA: 1024 edges
+// at a time in column order, each lot resolved in the rounds of k_c2_graph
+// before the next, with the components in shared memory (a lot's pairs
+// depend on no later edge).  It stops when one component is left: on the
+// torus after 1,788 of 58,988 edges.  Bound by the latency of its rounds (a
+// few hundred cycles each, some ten to a lot), and hidden behind the
+// triangles of the same launch.
 constexpr int KR_ITEMS = 4, KR_EDGES = KR_ITEMS * C2_THREADS;
-__device__ void c2_kruskal(const C2Args &a, const C2Inst &in, uint16_t *label, uint16_t (*su)[C2_THREADS],
-                           uint16_t (*sv)[C2_THREADS], unsigned (*mask)[C2_THREADS / 32], int *s_parts) {
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int x = tid; x < in.nv; x += C2_THREADS) label[x] = (uint16_t)x;
+__device__ __forceinline__ int kr_find(uint16_t *parent, int x) {
+    for (;;) {
+        const int p = ((volatile uint16_t *)parent)[x];
+        if (p == x) return x;
+        const int g = ((volatile uint16_t *)parent)[p];
+        ((volatile uint16_t *)parent)[x] = (uint16_t)g;
+        x = g;
+    }
+}
+__device__ void c2_kruskal(const C2Args &a, const C2Inst &in, uint32_t *best, uint16_t *parent, int *s_parts) {
+    const int tid = threadIdx.x;
+    for (int x = tid; x < in.nv; x += C2_THREADS) {
+        parent[x] = (uint16_t)x;
+        best[x] = 0xffffffffu;
+    }
     if (tid == 0) *s_parts = in.nv;
     __syncthreads();
+    unsigned tag = 0x3fffff;  // counts down by rounds: nothing in best[] is reset
     for (int c0 = 0; c0 < in.ne && *s_parts > 1; c0 += KR_EDGES) {
-        int4 e[KR_ITEMS];
+        int u[KR_ITEMS], v[KR_ITEMS];
 #pragma unroll
         for (int q = 0; q < KR_ITEMS; q++) {
             const int i = c0 + q * C2_THREADS + tid;
-            e[q] = i < in.ne ? a.erec[in.eoff + i] : make_int4(in.voff, in.voff, 0, 0);
+            const int4 e = i < in.ne ? a.erec[in.eoff + i] : make_int4(in.voff, in.voff, 0, 0);
+            u[q] = e.x - in.voff;
+            v[q] = e.y - in.voff;
         }
+        for (;; tag--) {
+            bool live = false;
 #pragma unroll
-        for (int q = 0; q < KR_ITEMS; q++) {
-            const int u = e[q].x - in.voff, v = e[q].y - in.voff;
-            su[q][tid] = (uint16_t)u;
-            sv[q][tid] = (uint16_t)v;
-            const unsigned b = __ballot_sync(0xffffffffu, label[u] != label[v]);
-            if (lane == 0) mask[q][wid] = b;
-        }
-        __syncthreads();
-        if (wid == 0) {
-            int parts = *s_parts;
-            for (int g = 0; g < KR_ITEMS * (C2_THREADS / 32) && parts > 1; g++) {
-                const int q = g / (C2_THREADS / 32), w = g % (C2_THREADS / 32);
-                if (!mask[q][w]) continue;
-                const int u = su[q][w * 32 + lane], v = sv[q][w * 32 + lane];
-                for (;;) {
-                    const int lu = label[u], lv = label[v];
-                    const unsigned b = __ballot_sync(0xffffffffu, lu != lv);
-                    if (!b) break;
-                    const int first = __ffs(b) - 1;
-                    const int young = __shfl_sync(0xffffffffu, max(lu, lv), first);
-                    const int old = __shfl_sync(0xffffffffu, min(lu, lv), first);
-                    for (int x = lane; x < in.nv; x += 32)
-                        if (label[x] == young) label[x] = (uint16_t)old;
-                    if (lane == 0) a.neg[in.eoff + c0 + g * 32 + first] = young;
-                    parts--;
-                    __syncwarp();
-                }
+            for (int q = 0; q < KR_ITEMS; q++) {
+                if (u[q] == v[q]) continue;
+                u[q] = kr_find(parent, u[q]);
+                v[q] = kr_find(parent, v[q]);
+                if (u[q] == v[q]) continue;
+                live = true;
+                const unsigned key = tag << 10 | (unsigned)(q * C2_THREADS + tid);
+                atomicMin(best + u[q], key);
+                atomicMin(best + v[q], key);
             }
-            if (lane == 0) *s_parts = parts;
+            if (!__syncthreads_or(live)) break;
+#pragma unroll
+            for (int q = 0; q < KR_ITEMS; q++) {
+                const int young = max(u[q], v[q]), old = min(u[q], v[q]);
+                if (young == old || best[young] != (tag << 10 | (unsigned)(q * C2_THREADS + tid))) continue;
+                parent[young] = (uint16_t)old;
+                a.neg[in.eoff + c0 + q * C2_THREADS + tid] = young;
+                a.dead[in.voff + young] = 1;
+                atomicSub(s_parts, 1);
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 }
 
-// The first blocks pair the edges with vertices (an instance each); the rest
-// check the triangles, a thread each, and write each at its three entries of
-// the table.  Bound by the table's scattered 4-byte writes.
-__global__ void __launch_bounds__(C2_THREADS) k_c2_table(C2Args a, int kruskal_blocks) {
-    __shared__ uint16_t label[C2_MAX_NV];
-    __shared__ uint16_t su[KR_ITEMS][C2_THREADS], sv[KR_ITEMS][C2_THREADS];
-    __shared__ unsigned mask[KR_ITEMS][C2_THREADS / 32];
+// One vertex's row of the edge-id table in the order of its edges: each entry
+// written at the number of smaller ones (a warp; `row` holds the row in
+// shared memory, absent edges as the largest id).  An entry is the edge's
+// rank and the other vertex.
+constexpr int ADJ_SHIFT = 10;
+__device__ void c2_sort_row(const int32_t *src, int32_t *dst, int nv, int pitch, int32_t *row) {
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i < pitch; i += 32) {
+        const int x = src[i];
+        row[i] = x < 0 ? INT_MAX : x;
+        dst[i] = INT_MAX;
+    }
+    __syncwarp();
+    for (int i = lane; i < nv; i += 32) {
+        const int x = row[i];
+        if (x == INT_MAX) continue;
+        int at = 0;
+        for (int q = 0; q < pitch; q += 4) {
+            const int4 y = *reinterpret_cast<const int4 *>(row + q);
+            at += (y.x < x) + (y.y < x) + (y.z < x) + (y.w < x);
+        }
+        dst[at] = x << ADJ_SHIFT | i;
+    }
+    __syncwarp();
+}
+
+// The first blocks pair the edges with vertices (an instance each); with
+// RUNS, the next ones sort the vertices' edges (a warp each); the rest check
+// the triangles, a thread each.
+//
+// RUNS: in a Rips filtration every triangle follows its last edge with no
+// other edge between (triangles carry their longest edge's length and come
+// after it), the third vertices of an edge's triangles ascending.  A set of
+// vertices per edge, one bit each, then names all of its run, and with it
+// every triangle: per 32 vertices the bits and the first one's column, so
+// (edge f, vertex z) is that column + the bits below z.  The triangles write
+// nothing else, and the lanes of a warp on one word write together, where the table costs three scattered 4-byte
+// writes each, of which 2% are ever read.  A triangle out of that order, or
+// a second edge on the same two vertices, sets `unsorted`, and the table is
+// built instead.
+template <bool RUNS>
+__global__ void __launch_bounds__(C2_THREADS) k_c2_triangles(C2Args a, int kruskal_blocks, int sort_blocks, int max_nv) {
+    extern __shared__ __align__(16) uint32_t tri_smem[];
     __shared__ int s_parts;
-    if (a.st->bad) return;
+    if (a.st->bad || (RUNS && a.st->unsorted)) return;
+    const int lane = threadIdx.x & 31;
     if ((int)blockIdx.x < kruskal_blocks) {
         for (int b = blockIdx.x; b < a.count; b += kruskal_blocks) {
-            c2_kruskal(a, a.inst[b], label, su, sv, mask, &s_parts);
+            c2_kruskal(a, a.inst[b], tri_smem, reinterpret_cast<uint16_t *>(tri_smem + max_nv), &s_parts);
             __syncthreads();
         }
         return;
     }
-    bool bad = false;
-    const int64_t stride = (int64_t)(gridDim.x - kruskal_blocks) * C2_THREADS;
-    for (int64_t j = (int64_t)(blockIdx.x - kruskal_blocks) * C2_THREADS + threadIdx.x; j < a.m; j += stride) {
-        const C2Word w = a.words[j >> 5];
-        if (((w.v | w.e) >> (j & 31)) & 1u) continue;
-        const C2Inst &in = a.inst[c2_inst_of(a, j)];
+    if (RUNS && (int)blockIdx.x < kruskal_blocks + sort_blocks) {
+        int32_t *row = reinterpret_cast<int32_t *>(tri_smem) + (threadIdx.x >> 5) * c2_pitch(max_nv);
+        const int warps = sort_blocks * (C2_THREADS / 32);
+        for (int v = (blockIdx.x - kruskal_blocks) * (C2_THREADS / 32) + (threadIdx.x >> 5); v < a.st->nv; v += warps) {
+            const C2Inst &in = a.inst[c2_inst_of(a, a.vlist[v])];
+            const int pitch = c2_pitch(in.nv);
+            const int64_t at = in.coff + (int64_t)(v - in.voff) * pitch;
+            c2_sort_row(a.cells + at, a.adj + at, in.nv, pitch, row);
+        }
+        return;
+    }
+    bool bad = false, unsorted = false;
+    const int others = kruskal_blocks + sort_blocks;
+    const int64_t stride = (int64_t)(gridDim.x - others) * C2_THREADS;
+    for (int64_t j0 = (int64_t)(blockIdx.x - others) * C2_THREADS + (threadIdx.x - lane); j0 < a.m; j0 += stride) {
+        const int64_t j = j0 + lane;
+        const C2Word w = a.words[j0 >> 5];
+        const bool tri = j < a.m && !(((w.v | w.e) >> lane) & 1u);
+        const C2Inst &in = a.inst[tri ? c2_inst_of(a, j) : 0];
         int k[3], o[3];
-        if (!c2_triangle(a, j, w, in, k) ||
-            !c2_opposite(a.erec[k[0]], a.erec[k[1]], a.erec[k[2]], o[0], o[1], o[2])) {
-            bad = true;
+        bool ok = tri && c2_triangle(a, j, w, in, k) &&
+                  c2_opposite(a.erec[k[0]], a.erec[k[1]], a.erec[k[2]], o[0], o[1], o[2]);
+        if (tri && !ok) bad = true;
+        if (!RUNS) {
+            if (ok)
+#pragma unroll
+                for (int q = 0; q < 3; q++)
+                    a.cells[in.coff + (int64_t)(k[q] - in.eoff) * c2_pitch(in.nv) + (o[q] - in.voff)] = (int32_t)j;
             continue;
         }
-#pragma unroll
-        for (int q = 0; q < 3; q++)
-            a.cells[in.coff + (int64_t)(k[q] - in.eoff) * in.nv + (o[q] - in.voff)] = (int32_t)j;
+        const unsigned lt = below(lane);
+        const int last = w.epre + __popc(w.e & lt) - 1;  // the last edge before j
+        const int z = ok ? o[2] - in.voff : 0;
+        if (ok && k[2] != last) unsorted = true;
+        // the third vertex of the triangle before it in the run is smaller
+        int zp = __shfl_up_sync(0xffffffffu, z, 1);
+        const bool okp = __shfl_up_sync(0xffffffffu, (int)ok, 1) != 0;
+        bool first = true;  // of its word
+        if (ok && k[2] == last && j - 1 != a.elist[last]) {
+            if (lane == 0) {
+                int kp[3], op[3];
+                zp = c2_triangle(a, j - 1, a.words[(j - 1) >> 5], in, kp) &&
+                             c2_opposite(a.erec[kp[0]], a.erec[kp[1]], a.erec[kp[2]], op[0], op[1], op[2])
+                         ? op[2] - in.voff
+                         : INT_MAX;
+            } else if (!okp) {
+                zp = INT_MAX;
+            }
+            if (zp >= z) unsorted = true;
+            first = (zp >> 5) != (z >> 5);
+        }
+        // the bits of each word by one lane
+        const int nw = (in.nv + 31) >> 5;
+        const unsigned long long at =
+            ok && k[2] == last ? (unsigned long long)in.roff + (unsigned long long)(last - in.eoff) * nw + (z >> 5)
+                               : ~0ull;
+        const unsigned peers = __match_any_sync(0xffffffffu, at);
+        const unsigned v = __reduce_or_sync(peers, 1u << (z & 31));
+        if (at != ~0ull && lane == __ffs(peers) - 1) {
+            atomicOr(&a.runs[at].x, v);
+            if (first) a.runs[at].y = (unsigned)j;
+        }
     }
     if (bad) a.st->bad = 1;
-}
-
-// Outputs and owners before any pair is known.
-__global__ void __launch_bounds__(C2_THREADS) k_c2_dense_init(C2Args a) {
-    if (a.st->bad) return;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x, nwords = ((a.m + 31) >> 5) + 4;
-    const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int none = a.one_based ? 0 : -1;
-    for (int64_t j = i0; j < a.m; j += stride) {
-        a.low[j] = none;
-        if (a.ess) a.ess[j] = 1;
-        a.owner[j] = -1;
-    }
-    for (int64_t w = i0; w < nwords; w += stride) a.owned[w] = 0u;
+    if (unsorted) a.st->unsorted = 1;
 }
 
 // Column `col` has row `row` as its low (columns of the whole batch).
@@ -689,24 +807,80 @@ __device__ __forceinline__ void c2_pair(const C2Args &a, const C2Inst &in, int c
     }
 }
 
-// A warp per edge: its row of the table read once, for the entries set and
-// its first triangle t.  An edge that kills a vertex is paired with it (its
-// column of D' is cleared); one that is the last edge of t is t's low and t
-// the low of its column of D', finally: an apparent pair.  The others are
-// residual.  Bound by reading the table.
-__global__ void __launch_bounds__(C2_THREADS) k_c2_pairs(C2Args a) {
+// RUNS: a thread per column writes its outputs, from the bits alone.  An
+// edge with a run has it start with its first triangle, which no other
+// column holds before: an apparent pair.  An edge that kills a vertex (its
+// column of D' is cleared) has no run.  An edge with neither is residual.
+__global__ void __launch_bounds__(C2_THREADS) k_c2_runs_out(C2Args a) {
+    if (a.st->bad || a.st->unsorted) return;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, nwords = (a.m + 31) >> 5;
+    const int none = a.one_based ? 0 : -1, lane = threadIdx.x & 31;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < a.m; j += stride) {
+        const int64_t wi = j >> 5;
+        const C2Word w = a.words[wi];
+        const unsigned prev = wi > 0 ? a.words[wi - 1].e >> 31 : 0u;  // the column before the word
+        const unsigned open = w.e << 1 | prev, notri = w.v | w.e;
+        const bool edge = (w.e >> lane) & 1u, vertex = (w.v >> lane) & 1u;
+        int low = none, ess = 1;
+        if (edge) {
+            const int k = w.epre + __popc(w.e & below(lane));
+            const C2Inst &in = a.inst[a.erec[k].z];
+            const int y = a.neg[k];
+            bool run;
+            if (lane < 31) run = j + 1 < a.m && !((notri >> (lane + 1)) & 1u);
+            else run = wi + 1 < nwords && !((a.words[wi + 1].v | a.words[wi + 1].e) & 1u) && j + 1 < a.m;
+            // the next instance starts with no triangle: a run stays inside
+            if (y >= 0) low = a.vlist[in.voff + y] - (int)in.base + a.one_based;
+            if (y >= 0 || run) ess = 0;
+            else a.res[atomicAdd(&a.st->nres, 1)] = k;
+        } else if (vertex) {
+            if (a.dead[w.vpre + __popc(w.v & below(lane))]) ess = 0;
+        } else if ((open >> lane) & 1u) {
+            const int k = w.epre + __popc(w.e & below(lane)) - 1;
+            low = (int)(j - 1 - a.inst[a.erec[k].z].base) + a.one_based;
+            ess = 0;
+        }
+        a.low[j] = low;
+        if (a.ess) a.ess[j] = ess;
+        if (lane == 0) {
+            a.owned[wi] = open & ~notri;
+            a.fixed[wi] = open & ~notri;
+        }
+    }
+}
+
+// Table: outputs and owners before any pair is known.
+__global__ void __launch_bounds__(C2_THREADS) k_c2_table_init(C2Args a) {
+    if (a.st->bad) return;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, nwords = ((a.m + 31) >> 5) + 4;
+    const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int none = a.one_based ? 0 : -1;
+    for (int64_t j = i0; j < a.m; j += stride) {
+        a.low[j] = none;
+        if (a.ess) a.ess[j] = 1;
+    }
+    for (int64_t w = i0; w < nwords; w += stride) a.owned[w] = a.fixed[w] = 0u;
+}
+
+// Table: a warp per edge, its row of the table read once, for the entries set
+// and its first triangle t.  An edge that kills a vertex is paired with it
+// (its column of D' is cleared); one that is the last edge of t is t's low
+// and t the low of its column of D', finally: an apparent pair.  The others
+// are residual.  Bound by reading the table.
+__global__ void __launch_bounds__(C2_THREADS) k_c2_table_pairs(C2Args a) {
     if (a.st->bad) return;
     const int lane = threadIdx.x & 31, ne = a.st->ne;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     unsigned long long set = 0;
     for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < ne; k += nw) {
         const C2Inst in = a.inst[a.erec[k].z];
-        const int32_t *row = a.cells + in.coff + (int64_t)(k - in.eoff) * in.nv;
+        const int pitch = c2_pitch(in.nv);
+        const uint4 *row = reinterpret_cast<const uint4 *>(a.cells + in.coff + (int64_t)(k - in.eoff) * pitch);
         unsigned t = 0xffffffffu;  // an empty entry is the largest
-        for (int i = lane; i < in.nv; i += 32) {
-            const unsigned x = (unsigned)row[i];
-            set += x != 0xffffffffu;
-            t = min(t, x);
+        for (int i = lane; i < pitch / 4; i += 32) {
+            const uint4 x = row[i];
+            set += (x.x != 0xffffffffu) + (x.y != 0xffffffffu) + (x.z != 0xffffffffu) + (x.w != 0xffffffffu);
+            t = min(min(min(t, x.x), min(x.y, x.z)), x.w);
         }
         t = __reduce_min_sync(0xffffffffu, t);
         if (lane == 0) {
@@ -716,11 +890,10 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_pairs(C2Args a) {
             } else if (t != 0xffffffffu) {
                 if (a.rows[a.colptr[t] + 2] + in.base == e) {
                     c2_pair(a, in, (int)t, e);
-                    a.owner[t] = k;
                     atomicOr(a.owned + (t >> 5), 1u << (t & 31));
+                    atomicOr(a.fixed + (t >> 5), 1u << (t & 31));
                 } else {
-                    a.res[atomicAdd(&a.st->nres, 1)] = make_int2(k, (int)t);
-                    a.death[k] = -1;
+                    a.res[atomicAdd(&a.st->nres, 1)] = k;
                 }
             }
         }
@@ -729,19 +902,80 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_pairs(C2Args a) {
     if (lane == 0 && set) atomicAdd(&a.st->cells_set, set);
 }
 
-// Toggle an edge's triangles in the window from w0 (a warp); `later` keeps
-// the first one past the window.
-__device__ __forceinline__ void rs_toggle(const int32_t *row, int nv, int w0, uint32_t *bits, int &later) {
-    for (int i = threadIdx.x & 31; i < nv; i += 128) {
-        int t[4];
+// The rank of edge column `col`.
+__device__ __forceinline__ int c2_edge_rank(const C2Args &a, int col) {
+    const C2Word w = a.words[col >> 5];
+    return w.epre + __popc(w.e & below(col & 31));
+}
+
+__device__ __forceinline__ void rs_flip(uint32_t *bits, int r) {
+    asm volatile("red.shared.xor.b32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bits + (r >> 5))),
+                 "r"(1u << (r & 31))
+                 : "memory");
+}
+
+// The triangles on edge k toggled in the window of WORDS words from w0, by a
+// warp.  RUNS: the triangle with vertex w belongs to the run of the last of
+// its three edges; runs from edge `hi` on lie past the window, so the edges of
+// one end are taken in order only that far (a residual column's window is
+// early: a tenth of a row), the other end's ids and the runs are a gather
+// each.  `later` keeps a bound on what lies past the window: an edge whose
+// run may hold a triangle.  Table: the row, `later` the first triangle past.
+template <bool RUNS, int WORDS>
+__device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int k, int w0, int hi, uint32_t *bits,
+                                          int &later) {
+    const int lane = threadIdx.x & 31, pitch = c2_pitch(in.nv);
+    if (RUNS) {
+        const int4 e = __ldg(a.erec + k);
+        const int u = e.x - in.voff, v = e.y - in.voff, nw = (in.nv + 31) >> 5, kl = k - in.eoff;
+        const int32_t *au = a.adj + in.coff + (int64_t)u * pitch, *iv = a.cells + in.coff + (int64_t)v * pitch;
+        const uint2 *runs = a.runs + in.roff;
+        for (int i = lane; i - lane < pitch; i += 64) {
+            int key[2], f[2], z[2];
+            bool ok[2];
+            uint2 r[2];
+            key[0] = i < pitch ? __ldg(au + i) : INT_MAX;
+            key[1] = i + 32 < pitch ? __ldg(au + i + 32) : INT_MAX;
 #pragma unroll
-        for (int q = 0; q < 4; q++) t[q] = i + 32 * q < nv ? __ldg(row + i + 32 * q) : -1;
+            for (int q = 0; q < 2; q++) {
+                const int x = key[q] >> ADJ_SHIFT, w = key[q] & ((1 << ADJ_SHIFT) - 1);
+                ok[q] = x < hi && key[q] != INT_MAX;
+                if (!ok[q] && key[q] != INT_MAX) later = min(later, max(x, kl));
+                const int y = ok[q] ? __ldg(iv + w) : -1;
+                f[q] = max(max(x, y), kl);
+                z[q] = f[q] == kl ? w : f[q] == x ? v : u;
+                ok[q] = y >= 0;
+                if (ok[q] && f[q] >= hi) {
+                    later = min(later, f[q]);
+                    ok[q] = false;
+                }
+            }
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int r = t[q] - w0;  // an empty entry (-1) falls below the window, as rows already cancelled do
-            if (r < 0 || t[q] < 0) continue;
-            if (r < 32 * RS_WORDS) atomicXor(bits + (r >> 5), 1u << (r & 31));
-            else later = min(later, t[q]);
+            for (int q = 0; q < 2; q++)
+                r[q] = ok[q] ? __ldg(runs + (long long)f[q] * nw + (z[q] >> 5)) : make_uint2(0u, 0u);
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (!((r[q].x >> (z[q] & 31)) & 1u)) continue;
+                const int d = (int)r[q].y + __popc(r[q].x & below(z[q] & 31)) - w0;
+                if (d < 0) continue;  // cancelled already
+                if (d < 32 * WORDS) rs_flip(bits, d);
+                else later = min(later, f[q]);
+            }
+            if (__any_sync(0xffffffffu, (key[1] >> ADJ_SHIFT) >= hi)) break;
+        }
+    } else {
+        const int4 *row = reinterpret_cast<const int4 *>(a.cells + in.coff + (int64_t)(k - in.eoff) * pitch);
+        for (int i = lane; i < pitch / 4; i += 64) {
+            const int4 A = __ldg(row + i);
+            const int4 B = i + 32 < pitch / 4 ? __ldg(row + i + 32) : make_int4(-1, -1, -1, -1);
+            const int t[8] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w};
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int d = t[q] - w0;  // below the window: an empty entry, or cancelled already
+                if (t[q] < 0 || d < 0) continue;
+                if (d < 32 * WORDS) rs_flip(bits, d);
+                else later = min(later, t[q]);
+            }
         }
     }
 }
@@ -756,60 +990,75 @@ __device__ __forceinline__ void rs_toggle(const int32_t *row, int nv, int w0, ui
 //   set bits that have one.  Every column added comes before k in D' (a row
 //   of the sum lies in a column of the sum, and its owner is the first column
 //   that can hold it), so this is a reduction like any other, and the two
-//   chains of 557 additions on the torus take 38 waves.  A wave is three
-//   round trips to L2 (which bits have owners, the owners, their rows).
-// * Owners: a residual column claims its low by compare-and-swap once its
-//   list is published.  Found claimed by an earlier column, that column is
-//   added; by a later one, the claim is taken over and this CTA goes on with
-//   the later column plus its own.  No CTA waits for another, and the lows
-//   are those of any complete reduction.
-__global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
-    if (a.st->bad) return;
-    extern __shared__ __align__(16) uint32_t bits[];  // RS_WORDS
-    constexpr int NW = RS_THREADS / 32;
+//   chains of 557 additions on the torus take 36 and 40 waves.
+// * Owners: low[t] names the owner of triangle t.  A residual column claims
+//   its low by compare-and-swap once its list is published.  Found claimed by
+//   an earlier column, that column is added; by a later one, the claim is
+//   taken over and this CTA goes on with the later column plus its own.  No
+//   CTA waits for another, and the lows are those of any complete reduction.
+//
+// Bound by latency: a wave is a search of the window and four dependent trips
+// to L2 (which set bits have owners, the owners, their vertices, their
+// triangles) and of the instructions of one SM, so the columns of a wave are
+// spread over the CTA's warps and no more of each is looked at than the window
+// holds.  Complexes on many
+// vertices, with few long columns, take large CTAs and windows; batches of
+// small ones as many CTAs as fit.
+template <bool RUNS, int THREADS, int WORDS>
+__global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
+    if (a.st->bad || (RUNS && a.st->unsorted)) return;
+    extern __shared__ __align__(16) uint32_t bits[];  // WORDS
+    constexpr int NW = THREADS / 32;
     __shared__ int s_low[NW], s_cnt[NW], s_wave[RS_WAVE];
     __shared__ int s_i, s_first, s_later, s_act, s_other;
     __shared__ unsigned long long s_sum;
     enum { ACT_DONE, ACT_ADD, ACT_STEAL, ACT_FAIL };
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int nres = a.st->nres;
+    const int nres = a.st->nres, none = a.one_based ? 0 : -1;
     int32_t *list = a.lists + (size_t)blockIdx.x * RS_LIST;
     unsigned long long adds = 0, slots = 0;
     for (;;) {
-        if (tid == 0) s_i = atomicAdd(&a.st->cursor, 1);
+        if (tid == 0) {
+            s_i = atomicAdd(&a.st->cursor, 1);
+            s_later = INT_MAX;
+        }
         __syncthreads();
         const int i = s_i;
-        __syncthreads();
         if (i >= nres) break;
-        int k = a.res[i].x, pos = a.res[i].y;
+        int k = a.res[i];
         const C2Inst in = a.inst[a.erec[k].z];
-        const int32_t *cells = a.cells + in.coff;
-        auto row = [&](int e) { return cells + (int64_t)(e - in.eoff) * in.nv; };
-        int n = 1, w0 = pos & ~127, later = INT_MAX;
-        if (tid == 0) list[0] = k;
-        bool refill = true;
+        const int shift = (int)in.base - a.one_based;
+        int n = 1, pos = a.elist[k] + 1, w0 = 0, hi = 0, later = INT_MAX;  // triangles come after their edges
+        if (tid == 0) __stcg(list, k);
+        bool fresh = true;   // a new window, from pos
         for (;;) {
-            if (refill) {
-                for (int q = 4 * tid; q < RS_WORDS; q += 4 * RS_THREADS)
+            if (fresh) {
+                w0 = pos & ~127;
+                if (RUNS)
+                    hi = (w0 + 32ll * WORDS >= in.base + in.cols ? in.eoff + in.ne
+                                                                  : c2_edge_rank(a, w0 + 32 * WORDS)) - in.eoff;
+                for (int q = 4 * tid; q < WORDS; q += 4 * THREADS)
                     *reinterpret_cast<uint4 *>(bits + q) = make_uint4(0u, 0u, 0u, 0u);
                 if (tid == 0) s_later = INT_MAX;
                 later = INT_MAX;
                 __syncthreads();
-                for (int v = wid; v < n; v += NW) rs_toggle(row(__ldcg(list + v)), in.nv, w0, bits, later);
+                for (int x = wid; x < n; x += NW)
+                    rs_toggle<RUNS, WORDS>(a, in, __ldcg(list + x), w0, hi, bits, later);
                 __syncthreads();
-                refill = false;
+                fresh = false;
             }
             // the low, and the set bits with owners, from pos up
             int low = INT_MAX, before = 0, total = 0, mine = 0, at = 0;
-            uint4 c = make_uint4(0u, 0u, 0u, 0u);
-            for (int base = ((pos - w0) >> 5) & ~3; base < RS_WORDS; base += 4 * RS_THREADS) {
+            uint4 c = make_uint4(0u, 0u, 0u, 0u), fx = c;
+            for (int base = ((pos - w0) >> 5) & ~3; base < WORDS; base += 4 * THREADS) {
                 at = base + 4 * tid;
                 uint4 t = make_uint4(0u, 0u, 0u, 0u);
-                if (at < RS_WORDS) t = *reinterpret_cast<const uint4 *>(bits + at);
+                if (at < WORDS) t = *reinterpret_cast<const uint4 *>(bits + at);
                 int fl = INT_MAX;
                 c = make_uint4(0u, 0u, 0u, 0u);
                 if (t.x | t.y | t.z | t.w) {
                     const uint4 p = __ldcg(reinterpret_cast<const uint4 *>(a.owned + (w0 >> 5) + at));
+                    fx = __ldg(reinterpret_cast<const uint4 *>(a.fixed + (w0 >> 5) + at));
                     c = make_uint4(t.x & p.x, t.y & p.y, t.z & p.z, t.w & p.w);
                     fl = w0 + 32 * at +
                          (t.x ? __ffs(t.x) - 1 : t.y ? 31 + __ffs(t.y) : t.z ? 63 + __ffs(t.z) : 95 + __ffs(t.w));
@@ -827,15 +1076,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
                     s_low[wid] = wl;
                 }
                 __syncthreads();
-                before = incl - mine;
-                total = 0;
-                low = INT_MAX;
-#pragma unroll
-                for (int w = 0; w < NW; w++) {
-                    if (w < wid) before += s_cnt[w];
-                    total += s_cnt[w];
-                    low = min(low, s_low[w]);
-                }
+                const int wc = lane < NW ? s_cnt[lane] : 0;
+                before = incl - mine + __reduce_add_sync(0xffffffffu, lane < wid ? wc : 0);
+                total = __reduce_add_sync(0xffffffffu, wc);
+                low = __reduce_min_sync(0xffffffffu, lane < NW ? s_low[lane] : INT_MAX);
                 if (low != INT_MAX) break;
                 __syncthreads();
             }
@@ -845,23 +1089,26 @@ __global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
                 const int next = s_later;
                 __syncthreads();
                 if (next == INT_MAX) {  // the column is zero: edge k is essential
-                    if (tid == 0) a.death[k] = -1;
+                    if (tid == 0 && a.ess) a.ess[a.elist[k]] = 1;
                     break;
                 }
-                pos = next;
-                w0 = next & ~127;
-                refill = true;
+                pos = RUNS ? a.elist[in.eoff + next] + 1 : next;
+                fresh = true;
                 continue;
             }
             if (mine && before < RS_WAVE) {
-                const unsigned cw[4] = {c.x, c.y, c.z, c.w};
+                const unsigned cw[4] = {c.x, c.y, c.z, c.w}, fw[4] = {fx.x, fx.y, fx.z, fx.w};
                 int r = before;
 #pragma unroll
                 for (int q = 0; q < 4; q++)
                     for (unsigned b = cw[q]; b && r < RS_WAVE; b &= b - 1, r++) {
-                        const int t = w0 + 32 * (at + q) + __ffs(b) - 1;
+                        const int bit = __ffs(b) - 1, t = w0 + 32 * (at + q) + bit;
                         if (r == 0) s_first = t;
-                        s_wave[r] = ld_acquire_i32(a.owner + t);
+                        const bool fixed = (fw[q] >> bit) & 1u;
+                        int o;
+                        if (RUNS && fixed) o = c2_edge_rank(a, t) - 1;  // the last edge before t
+                        else o = c2_edge_rank(a, ld_acquire_i32(a.low + t) + shift);
+                        s_wave[r] = fixed ? o : o | RS_FLAG;
                     }
             }
             __syncthreads();
@@ -885,25 +1132,29 @@ __global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
                     if (tid == 0) a.st->overflow = 1;
                     break;
                 }
-                for (int v = tid; v < n; v += RS_THREADS) __stcg(a.arena + off + v, __ldcg(list + v));
+                for (int v = tid; v < n; v += THREADS) __stcg(a.arena + off + v, __ldcg(list + v));
                 __threadfence();
                 __syncthreads();
                 if (tid == 0) {
                     *(volatile unsigned long long *)(a.sum + k) = (off << 24) | (unsigned)n;
-                    a.death[k] = low;
+                    const int e = a.elist[k];
+                    if (a.ess) {
+                        a.ess[low] = 0;
+                        a.ess[e] = 0;
+                    }
                     __threadfence();
-                    int want = p0, act = ACT_FAIL, other = -1;
+                    int want = p0 < 0 ? none : a.elist[p0 & ~RS_FLAG] - shift, act = ACT_FAIL, other = -1;
                     for (int tries = 0; tries < (1 << 20); tries++) {
-                        const int got = atomicCAS(a.owner + low, want, k | RS_FLAG);
+                        const int got = atomicCAS(a.low + low, want, e - shift);
+                        other = want == none ? -1 : c2_edge_rank(a, want + shift);
                         if (got == want) {
                             atomicOr(a.owned + (low >> 5), 1u << (low & 31));
-                            act = want < 0 ? ACT_DONE : ACT_STEAL;
-                            other = want & ~RS_FLAG;
+                            act = want == none ? ACT_DONE : ACT_STEAL;
                             break;
                         }
-                        if (!(got & RS_FLAG) || (got & ~RS_FLAG) > k) {  // an earlier column's by now
+                        other = c2_edge_rank(a, got + shift);
+                        if (other > k) {  // an earlier column's by now
                             act = ACT_ADD;
-                            other = got;
                             break;
                         }
                         want = got;
@@ -924,16 +1175,15 @@ __global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
                         if (tid == 0) a.st->overflow = 1;
                         break;
                     }
-                    for (int v = tid; v < len; v += RS_THREADS) __stcg(list + n + v, __ldcg(a.arena + from + v));
+                    for (int v = tid; v < len; v += THREADS) __stcg(list + n + v, __ldcg(a.arena + from + v));
                     n += len;
                     k = s_other;
                     pos = low;
-                    w0 = low & ~127;
-                    refill = true;
+                    fresh = true;
                     __syncthreads();
                     continue;
                 }
-                if (tid == 0) s_wave[0] = s_other;
+                if (tid == 0) s_wave[0] = s_other | RS_FLAG;
                 cnt = 1;
                 __syncthreads();
             }
@@ -942,7 +1192,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
             const unsigned m_app = __ballot_sync(0xffffffffu, p >= 0 && !(p & RS_FLAG));
             unsigned m_res = __ballot_sync(0xffffffffu, p >= 0 && (p & RS_FLAG) && (p & ~RS_FLAG) > k);
             for (int q = wid; q < cnt; q += NW)
-                if ((m_app >> q) & 1u) rs_toggle(row(s_wave[q]), in.nv, w0, bits, later);
+                if ((m_app >> q) & 1u) rs_toggle<RUNS, WORDS>(a, in, s_wave[q], w0, hi, bits, later);
             if (wid == 0 && ((m_app >> lane) & 1u)) __stcg(list + n + __popc(m_app & below(lane)), p);
             n += __popc(m_app);
             bool full = false;
@@ -959,11 +1209,9 @@ __global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
                     full = true;
                     break;
                 }
-                for (int v = wid; v < len; v += NW) {
-                    const int e = __ldcg(a.arena + from + v);
-                    rs_toggle(row(e), in.nv, w0, bits, later);
-                    if (lane == 0) __stcg(list + n + v, e);
-                }
+                for (int x = wid; x < len; x += NW)
+                    rs_toggle<RUNS, WORDS>(a, in, __ldcg(a.arena + from + x), w0, hi, bits, later);
+                for (int v = tid; v < len; v += THREADS) __stcg(list + n + v, __ldcg(a.arena + from + v));
                 n += len;
                 adds++;
                 slots += (unsigned long long)len * in.nv;
@@ -980,15 +1228,6 @@ __global__ void __launch_bounds__(RS_THREADS) k_c2_residual(C2Args a) {
     if (tid == 0 && adds) {
         atomicAdd(&a.st->adds, adds);
         atomicAdd(&a.st->slots, slots);
-    }
-}
-
-// The pairs of the residual edges.
-__global__ void __launch_bounds__(C2_THREADS) k_c2_residual_pairs(C2Args a) {
-    if (a.st->bad) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.st->nres; i += gridDim.x * blockDim.x) {
-        const int k = a.res[i].x, t = a.death[k];
-        if (t >= 0) c2_pair(a, a.inst[a.erec[k].z], t, a.elist[k]);
     }
 }
 
@@ -1069,27 +1308,48 @@ static int c2_run_graph(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t 
     return rc;
 }
 
-static int c2_run_dense(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t nt, C2Status *hs, bool *done) {
-    // The table costs a write and a read of its cells; past a few times the
-    // matrix itself (sparse complexes on many vertices) it no longer pays.
-    if (hs->max_nv > C2_MAX_NV || hs->cells > (1ll << 24) + 8 * hs->nnz) return OPH_OK;
-    cudaStream_t s = ctx->stream;
+template <bool RUNS, int THREADS, int WORDS>
+static int c2_residual_grid(Context *ctx) {
     static int per_sm[64];
     int &nb = per_sm[ctx->device & 63];
-    constexpr int SMEM = RS_WORDS * (int)sizeof(uint32_t);
-    if (!nb && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_c2_residual, RS_THREADS, SMEM) != cudaSuccess) {
+    constexpr int SMEM = WORDS * (int)sizeof(uint32_t);
+    if (!nb && (cudaFuncSetAttribute(k_c2_residual<RUNS, THREADS, WORDS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     SMEM) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_c2_residual<RUNS, THREADS, WORDS>, THREADS,
+                                                              SMEM) != cudaSuccess)) {
         cudaGetLastError();
         nb = 0;
-        return OPH_OK;
     }
-    const int gr = (int)std::max<int64_t>(1, std::min<int64_t>(ne, (int64_t)ctx->sm_count * nb));
+    return nb * ctx->sm_count;
+}
+
+// Many vertices: long rows and few, long residual columns, so large CTAs and
+// windows; below, more CTAs.
+constexpr int RS_SMALL_NV = 160;
+
+template <bool RUNS>
+static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status *hs, bool *done) {
+    // what a form's tables may cost, in entries: a few times the matrix itself
+    // (sparse complexes on many vertices are left to the general path)
+    const long long room = (1ll << 24) + 8 * hs->nnz;
+    const long long cells = RUNS ? hs->pairs : hs->cells, run_words = RUNS ? hs->run_words : 0;
+    if (hs->max_nv > (RUNS ? 1 << ADJ_SHIFT : C2_MAX_NV) || 2 * cells > room || 2 * run_words > room) return OPH_OK;
+    cudaStream_t s = ctx->stream;
+    const bool small = hs->max_nv <= RS_SMALL_NV;
+    int gr = small ? c2_residual_grid<RUNS, 256, 8192>(ctx) : c2_residual_grid<RUNS, 1024, 32768>(ctx);
+    if (gr == 0) return OPH_OK;
+    gr = (int)std::min<int64_t>(ne, gr);
+    const int nv = hs->nv;
     a.arena_cap = (1 << 22) + 16 * ne;
+    size_t head = 0;
     for (char *p = nullptr;;) {
         Carve c{p};
-        a.owner = c.take<int32_t>(a.m);
+        a.runs = c.take<uint2>(run_words);
+        a.dead = c.take<uint8_t>(nv + 1);
+        head = c.off;  // zeroed
         a.owned = c.take<uint32_t>((a.m + 31) / 32 + 4);
-        a.res = c.take<int2>(ne);
-        a.death = c.take<int32_t>(ne);
+        a.fixed = c.take<uint32_t>((a.m + 31) / 32 + 4);
+        a.res = c.take<int32_t>(ne);
         a.sum = c.take<unsigned long long>(ne);
         a.arena = c.take<int32_t>(a.arena_cap);
         a.lists = c.take<int32_t>((size_t)gr * RS_LIST);
@@ -1097,26 +1357,37 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t 
         p = (char *)ctx_alloc(ctx, S_C2_MODE, c.off);
         if (!p) return OPH_OK;
     }
-    const size_t cell_bytes = sizeof(int32_t) * (size_t)std::max<long long>(hs->cells, 1);
-    a.cells = (int32_t *)ctx_alloc(ctx, S_C2_CELLS, cell_bytes);
+    if (!RUNS) a.runs = nullptr;
+    const size_t cell_bytes = sizeof(int32_t) * (size_t)std::max<long long>(cells, 1);
+    a.cells = (int32_t *)ctx_alloc(ctx, S_C2_CELLS, (RUNS ? 2 : 1) * cell_bytes);
     if (!a.cells) return OPH_OK;
+    a.adj = RUNS ? a.cells + cells : nullptr;  // cells is a multiple of 4: whole 16-byte loads
     a.ends = nullptr;
     const int kb = std::min(a.count, ctx->sm_count * 4);
     OPH_CUDA_TRY(cudaMemsetAsync(a.cells, 0xff, cell_bytes, s));
+    OPH_CUDA_TRY(cudaMemsetAsync(ctx->bufs[S_C2_MODE].ptr, 0, head, s));
+    if (!RUNS) k_c2_cells<<<1, 1024, 0, s>>>(a);
     k_c2_edges<<<c2_grid(ctx, ne, 8), C2_THREADS, 0, s>>>(a);
-    k_c2_table<<<kb + c2_grid(ctx, a.m, 16), C2_THREADS, 0, s>>>(a, kb);
-    k_c2_dense_init<<<c2_grid(ctx, a.m, 16), C2_THREADS, 0, s>>>(a);
-    k_c2_pairs<<<c2_grid(ctx, 32 * ne, 8), C2_THREADS, 0, s>>>(a);
+    // rows of vertices in shared memory (sorted a warp each), or the components
+    const int smem = std::max(6 * hs->max_nv, RUNS ? 4 * (C2_THREADS / 32) * c2_pitch(hs->max_nv) : 0);
+    const int sb = RUNS ? c2_grid(ctx, 32 * (int64_t)nv, 4) : 0;
+    k_c2_triangles<RUNS><<<kb + sb + c2_grid(ctx, a.m, 16), C2_THREADS, smem, s>>>(a, kb, sb, hs->max_nv);
+    if (RUNS) {
+        k_c2_runs_out<<<c2_grid(ctx, a.m, 16), C2_THREADS, 0, s>>>(a);
+    } else {
+        k_c2_table_init<<<c2_grid(ctx, a.m, 16), C2_THREADS, 0, s>>>(a);
+        k_c2_table_pairs<<<c2_grid(ctx, 32 * ne, 8), C2_THREADS, 0, s>>>(a);
+    }
     if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
-    k_c2_residual<<<gr, RS_THREADS, SMEM, s>>>(a);
-    k_c2_residual_pairs<<<c2_grid(ctx, ne, 1), C2_THREADS, 0, s>>>(a);
-    ctx->launches += 6;
+    if (small) k_c2_residual<RUNS, 256, 8192><<<gr, 256, 8192 * sizeof(uint32_t), s>>>(a);
+    else k_c2_residual<RUNS, 1024, 32768><<<gr, 1024, 32768 * sizeof(uint32_t), s>>>(a);
+    ctx->launches += RUNS ? 4 : 6;
     cudaEventRecord(ctx->ev[1], s);
     int rc = c2_read_status(ctx, a, hs);
     // a table entry written twice (two triangles on the same edge and vertex,
     // which no simplicial complex has) shows in the count of those set
-    *done = !rc && !hs->bad && !hs->overflow && hs->cells_set == 3ull * (unsigned long long)nt;
-    (void)nv;
+    *done = !rc && !hs->bad && !hs->overflow && (!RUNS || !hs->unsorted) &&
+            (RUNS || hs->cells_set == 3ull * (unsigned long long)nt);
     return rc;
 }
 
@@ -1196,7 +1467,14 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
     // every edge with at most two triangles: a graph (an edge found to have
     // more leaves it to the dense form)
     if (3 * nt <= 2 * ne && (rc = c2_run_graph(ctx, a, nv, ne, nt, hs, &done))) return rc;
-    if (!done && !hs->bad && (rc = c2_run_dense(ctx, a, nv, ne, nt, hs, &done))) return rc;
+    if (!done && !hs->bad && (rc = c2_run_dense<true>(ctx, a, ne, nt, hs, &done))) return rc;
+    if (!done && !hs->bad && !hs->overflow) {
+        // not in runs: the same with the table (the status as before the try)
+        if (hs->unsorted) {
+            OPH_CUDA_TRY(cudaMemsetAsync(&a.st->unsorted, 0, sizeof(int), s));
+        }
+        if ((rc = c2_run_dense<false>(ctx, a, ne, nt, hs, &done))) return rc;
+    }
     if (!done) return OPH_OK;
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);

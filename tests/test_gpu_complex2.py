@@ -157,3 +157,24 @@ def test_batch_of_rips(ctx):
             want, want_ess, _ = oracle.twist(bm)
             np.testing.assert_array_equal(low, want)
             np.testing.assert_array_equal(ess, want_ess)
+
+
+def test_runs_and_not(ctx):
+    """Orders next to a Rips filtration's that the run form must refuse: a
+    vertex between an edge and its triangle, the third vertices of an edge's
+    triangles descending, an edge between an edge and its triangles."""
+    tri = [[0, 1], [0, 2], [1, 2]]
+    late = BoundaryMatrix.from_columns([[], [], []] + tri + [[], [3, 4, 5]])
+    check(ctx, late)
+    # edge (0, 1) last, with third vertices 2, 3 and 4
+    cols = [[] for _ in range(5)] + [[0, v] for v in (2, 3, 4)] + [[1, v] for v in (2, 3, 4)] + [[0, 1]]
+    runs = [[5, 8, 11], [6, 9, 11], [7, 10, 11]]
+    for order in (runs, runs[::-1], [runs[1], runs[0], runs[2]]):
+        check(ctx, BoundaryMatrix.from_columns(cols + order))
+    check(ctx, BoundaryMatrix.from_columns(cols + [runs[0], [2, 3], runs[1], runs[2]]))
+
+
+@pytest.mark.parametrize("n", [159, 160, 161, 164])
+def test_rips_cta_sizes(ctx, n):
+    """Either side of the residual columns' CTA and window sizes."""
+    check(ctx, cx.rips(cx.points_circle(n, seed=n), threshold=1.2))
