@@ -57,6 +57,9 @@ struct __align__(16) C2Inst {
     int voff, eoff, nv, ne;
     long long base, cols;
     long long coff, roff;  // its part of the table (cells) and of the runs' bits
+    // words, lists and bitmaps hold its columns relative to wbase, its words
+    // from woff on (0 where the words run through the whole batch)
+    long long wbase, woff;
 };
 struct C2Status {
     int bad;         // a column or row that is none of the accepted kinds
@@ -80,7 +83,7 @@ struct C2Status {
 constexpr int C2_THREADS = 256, C2_TILE = 2048;
 constexpr int C2_MAX_ROUNDS = 512;
 constexpr int C2_MAX_NV = 8192;                   // vertices of an instance the dense form takes
-constexpr int RS_WAVE = 16;                       // residual columns: pivots added at a time,
+constexpr int RS_WAVE = 32;                       // residual columns: pivots added at a time,
 constexpr int RS_LIST = 16384;                    //   edges a column under reduction may be the sum of
 constexpr int RS_FLAG = 1 << 30;
 
@@ -902,9 +905,10 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_table_pairs(C2Args a) {
     if (lane == 0 && set) atomicAdd(&a.st->cells_set, set);
 }
 
-// The rank of edge column `col`.
-__device__ __forceinline__ int c2_edge_rank(const C2Args &a, int col) {
-    const C2Word w = a.words[col >> 5];
+// The edges before column `col` (relative to the instance's wbase): the rank
+// of an edge.
+__device__ __forceinline__ int c2_edge_rank(const C2Args &a, const C2Inst &in, int col) {
+    const C2Word w = a.words[in.woff + (col >> 5)];
     return w.epre + __popc(w.e & below(col & 31));
 }
 
@@ -930,14 +934,15 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
         const int u = e.x - in.voff, v = e.y - in.voff, nw = (in.nv + 31) >> 5, kl = k - in.eoff;
         const int32_t *au = a.adj + in.coff + (int64_t)u * pitch, *iv = a.cells + in.coff + (int64_t)v * pitch;
         const uint2 *runs = a.runs + in.roff;
-        for (int i = lane; i - lane < pitch; i += 64) {
-            int key[2], f[2], z[2];
-            bool ok[2];
-            uint2 r[2];
-            key[0] = i < pitch ? __ldg(au + i) : INT_MAX;
-            key[1] = i + 32 < pitch ? __ldg(au + i + 32) : INT_MAX;
+        constexpr int U = 4;
+        for (int i = lane; i - lane < pitch; i += 32 * U) {
+            int key[U], f[U], z[U];
+            bool ok[U];
+            uint2 r[U];
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
+            for (int q = 0; q < U; q++) key[q] = i + 32 * q < pitch ? __ldg(au + i + 32 * q) : INT_MAX;
+#pragma unroll
+            for (int q = 0; q < U; q++) {
                 const int x = key[q] >> ADJ_SHIFT, w = key[q] & ((1 << ADJ_SHIFT) - 1);
                 ok[q] = x < hi && key[q] != INT_MAX;
                 if (!ok[q] && key[q] != INT_MAX) later = min(later, max(x, kl));
@@ -951,17 +956,17 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 2; q++)
+            for (int q = 0; q < U; q++)
                 r[q] = ok[q] ? __ldg(runs + (long long)f[q] * nw + (z[q] >> 5)) : make_uint2(0u, 0u);
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
+            for (int q = 0; q < U; q++) {
                 if (!((r[q].x >> (z[q] & 31)) & 1u)) continue;
                 const int d = (int)r[q].y + __popc(r[q].x & below(z[q] & 31)) - w0;
                 if (d < 0) continue;  // cancelled already
                 if (d < 32 * WORDS) rs_flip(bits, d);
                 else later = min(later, f[q]);
             }
-            if (__any_sync(0xffffffffu, (key[1] >> ADJ_SHIFT) >= hi)) break;
+            if (__any_sync(0xffffffffu, (key[U - 1] >> ADJ_SHIFT) >= hi)) break;
         }
     } else {
         const int4 *row = reinterpret_cast<const int4 *>(a.cells + in.coff + (int64_t)(k - in.eoff) * pitch);
@@ -1010,7 +1015,7 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
     extern __shared__ __align__(16) uint32_t bits[];  // WORDS
     constexpr int NW = THREADS / 32;
     __shared__ int s_low[NW], s_cnt[NW], s_wave[RS_WAVE];
-    __shared__ int s_i, s_first, s_later, s_act, s_other;
+    __shared__ int s_i, s_later, s_act, s_other;
     __shared__ unsigned long long s_sum;
     enum { ACT_DONE, ACT_ADD, ACT_STEAL, ACT_FAIL };
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1027,16 +1032,20 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
         if (i >= nres) break;
         int k = a.res[i];
         const C2Inst in = a.inst[a.erec[k].z];
-        const int shift = (int)in.base - a.one_based;
+        // columns here are relative to in.wbase; an owner's value in low[] is col - shift
+        const int shift = (int)(in.base - in.wbase) - a.one_based, cols = (int)(in.base + in.cols - in.wbase);
+        int32_t *const out_low = a.low + in.wbase, *const out_ess = a.ess ? a.ess + in.wbase : nullptr;
+        uint32_t *const owned = a.owned + in.woff;
+        const uint32_t *const fixed = a.fixed + in.woff;
         int n = 1, pos = a.elist[k] + 1, w0 = 0, hi = 0, later = INT_MAX;  // triangles come after their edges
         if (tid == 0) __stcg(list, k);
-        bool fresh = true;   // a new window, from pos
+        bool fresh = true;  // a new window, from pos
+        int wave = 4;       // most columns take a wave or two: long ones get the full width
         for (;;) {
             if (fresh) {
                 w0 = pos & ~127;
                 if (RUNS)
-                    hi = (w0 + 32ll * WORDS >= in.base + in.cols ? in.eoff + in.ne
-                                                                  : c2_edge_rank(a, w0 + 32 * WORDS)) - in.eoff;
+                    hi = (w0 + 32ll * WORDS >= cols ? in.eoff + in.ne : c2_edge_rank(a, in, w0 + 32 * WORDS)) - in.eoff;
                 for (int q = 4 * tid; q < WORDS; q += 4 * THREADS)
                     *reinterpret_cast<uint4 *>(bits + q) = make_uint4(0u, 0u, 0u, 0u);
                 if (tid == 0) s_later = INT_MAX;
@@ -1057,8 +1066,8 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
                 int fl = INT_MAX;
                 c = make_uint4(0u, 0u, 0u, 0u);
                 if (t.x | t.y | t.z | t.w) {
-                    const uint4 p = __ldcg(reinterpret_cast<const uint4 *>(a.owned + (w0 >> 5) + at));
-                    fx = __ldg(reinterpret_cast<const uint4 *>(a.fixed + (w0 >> 5) + at));
+                    const uint4 p = __ldcg(reinterpret_cast<const uint4 *>(owned + (w0 >> 5) + at));
+                    fx = __ldg(reinterpret_cast<const uint4 *>(fixed + (w0 >> 5) + at));
                     c = make_uint4(t.x & p.x, t.y & p.y, t.z & p.z, t.w & p.w);
                     fl = w0 + 32 * at +
                          (t.x ? __ffs(t.x) - 1 : t.y ? 31 + __ffs(t.y) : t.z ? 63 + __ffs(t.z) : 95 + __ffs(t.w));
@@ -1089,31 +1098,36 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
                 const int next = s_later;
                 __syncthreads();
                 if (next == INT_MAX) {  // the column is zero: edge k is essential
-                    if (tid == 0 && a.ess) a.ess[a.elist[k]] = 1;
+                    if (tid == 0 && out_ess) out_ess[a.elist[k]] = 1;
                     break;
                 }
                 pos = RUNS ? a.elist[in.eoff + next] + 1 : next;
                 fresh = true;
                 continue;
             }
-            if (mine && before < RS_WAVE) {
+            if (mine && before < wave) {
                 const unsigned cw[4] = {c.x, c.y, c.z, c.w}, fw[4] = {fx.x, fx.y, fx.z, fx.w};
                 int r = before;
 #pragma unroll
                 for (int q = 0; q < 4; q++)
-                    for (unsigned b = cw[q]; b && r < RS_WAVE; b &= b - 1, r++) {
+                    for (unsigned b = cw[q]; b && r < wave; b &= b - 1, r++) {
                         const int bit = __ffs(b) - 1, t = w0 + 32 * (at + q) + bit;
-                        if (r == 0) s_first = t;
-                        const bool fixed = (fw[q] >> bit) & 1u;
-                        int o;
-                        if (RUNS && fixed) o = c2_edge_rank(a, t) - 1;  // the last edge before t
-                        else o = c2_edge_rank(a, ld_acquire_i32(a.low + t) + shift);
-                        s_wave[r] = fixed ? o : o | RS_FLAG;
+                        s_wave[r] = (fw[q] >> bit) & 1u ? t : t | RS_FLAG;
                     }
             }
             __syncthreads();
-            int cnt = min(total, RS_WAVE);
-            const bool have = cnt > 0 && s_first == low;
+            int cnt = min(total, wave);
+            const bool have = cnt > 0 && (s_wave[0] & ~RS_FLAG) == low;
+            wave = min(2 * wave, RS_WAVE);
+            __syncthreads();
+            if (wid == 0 && lane < cnt) {  // the owners, all at once
+                const int t = s_wave[lane] & ~RS_FLAG, fl = s_wave[lane] & RS_FLAG;
+                int o;
+                if (RUNS && !fl) o = c2_edge_rank(a, in, t) - 1;  // the last edge before t
+                else o = c2_edge_rank(a, in, ld_acquire_i32(out_low + t) + shift);
+                s_wave[lane] = o | fl;
+            }
+            __syncthreads();
             const int p0 = have ? s_wave[0] : -1;
             if (n + RS_WAVE > RS_LIST) {
                 if (tid == 0) a.st->overflow = 1;
@@ -1138,21 +1152,21 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
                 if (tid == 0) {
                     *(volatile unsigned long long *)(a.sum + k) = (off << 24) | (unsigned)n;
                     const int e = a.elist[k];
-                    if (a.ess) {
-                        a.ess[low] = 0;
-                        a.ess[e] = 0;
+                    if (out_ess) {
+                        out_ess[low] = 0;
+                        out_ess[e] = 0;
                     }
                     __threadfence();
                     int want = p0 < 0 ? none : a.elist[p0 & ~RS_FLAG] - shift, act = ACT_FAIL, other = -1;
                     for (int tries = 0; tries < (1 << 20); tries++) {
-                        const int got = atomicCAS(a.low + low, want, e - shift);
-                        other = want == none ? -1 : c2_edge_rank(a, want + shift);
+                        const int got = atomicCAS(out_low + low, want, e - shift);
+                        other = want == none ? -1 : c2_edge_rank(a, in, want + shift);
                         if (got == want) {
-                            atomicOr(a.owned + (low >> 5), 1u << (low & 31));
+                            atomicOr(owned + (low >> 5), 1u << (low & 31));
                             act = want == none ? ACT_DONE : ACT_STEAL;
                             break;
                         }
-                        other = c2_edge_rank(a, got + shift);
+                        other = c2_edge_rank(a, in, got + shift);
                         if (other > k) {  // an earlier column's by now
                             act = ACT_ADD;
                             break;
@@ -1325,7 +1339,7 @@ static int c2_residual_grid(Context *ctx) {
 
 // Many vertices: long rows and few, long residual columns, so large CTAs and
 // windows; below, more CTAs.
-constexpr int RS_SMALL_NV = 160;
+constexpr int RS_SMALL_NV = 160, RS_SMALL = 256, RS_SMALL_WORDS = 4096, RS_LARGE = 1024, RS_LARGE_WORDS = 8192;
 
 template <bool RUNS>
 static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status *hs, bool *done) {
@@ -1336,7 +1350,8 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     if (hs->max_nv > (RUNS ? 1 << ADJ_SHIFT : C2_MAX_NV) || 2 * cells > room || 2 * run_words > room) return OPH_OK;
     cudaStream_t s = ctx->stream;
     const bool small = hs->max_nv <= RS_SMALL_NV;
-    int gr = small ? c2_residual_grid<RUNS, 256, 8192>(ctx) : c2_residual_grid<RUNS, 1024, 32768>(ctx);
+    int gr = small ? c2_residual_grid<RUNS, RS_SMALL, RS_SMALL_WORDS>(ctx)
+                   : c2_residual_grid<RUNS, RS_LARGE, RS_LARGE_WORDS>(ctx);
     if (gr == 0) return OPH_OK;
     gr = (int)std::min<int64_t>(ne, gr);
     const int nv = hs->nv;
@@ -1379,8 +1394,10 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
         k_c2_table_pairs<<<c2_grid(ctx, 32 * ne, 8), C2_THREADS, 0, s>>>(a);
     }
     if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
-    if (small) k_c2_residual<RUNS, 256, 8192><<<gr, 256, 8192 * sizeof(uint32_t), s>>>(a);
-    else k_c2_residual<RUNS, 1024, 32768><<<gr, 1024, 32768 * sizeof(uint32_t), s>>>(a);
+    if (small)
+        k_c2_residual<RUNS, RS_SMALL, RS_SMALL_WORDS><<<gr, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
+    else
+        k_c2_residual<RUNS, RS_LARGE, RS_LARGE_WORDS><<<gr, RS_LARGE, RS_LARGE_WORDS * sizeof(uint32_t), s>>>(a);
     ctx->launches += RUNS ? 4 : 6;
     cudaEventRecord(ctx->ev[1], s);
     int rc = c2_read_status(ctx, a, hs);
