@@ -72,6 +72,9 @@ struct C2Status {
     unsigned long long joins;
     int max_nv;      // the largest instance's vertices
     int unsorted;    // the triangles do not come in runs
+    int next;        // whole instances: the CTAs' queue
+    int refused;     //   an instance is too large, or no complex in runs
+    int no_room;     //   the tables' bounds were too small
     int nres, cursor, overflow;      // residual edges; the CTAs' queue; a list ran out of room
     long long cells;                 // entries of the edge-vertex table
     long long pairs, run_words;      // entries of the edge-id table, words of the runs' bits
@@ -113,13 +116,14 @@ struct C2Args {
     int one_based;
     // dense forms: the vertex that dies at each edge (-1: none) and which
     // vertices die; the edge-vertex table or, with runs, the edge-id table
-    // (vertices by vertices), its rows in edge order, and the runs (per edge
-    // and 32 vertices: which have a triangle, and the first one's column); which triangles have an
+    // (vertices by vertices), its rows in edge order, the same table of edge
+    // columns, and the runs (per edge and 32 vertices: which have a triangle,
+    // and the first one's column); which triangles have an
     // owner (low[] names it), and which for good; the residual edges, and the
     // list each is the sum of (offset << 24 | length)
     int32_t *neg;
     uint8_t *dead;
-    int32_t *cells, *adj;
+    int32_t *cells, *adj, *tab;
     uint2 *runs;
     uint32_t *owned, *fixed;
     int32_t *res;
@@ -127,6 +131,9 @@ struct C2Args {
     int32_t *arena;
     long long arena_cap;
     int32_t *lists;           // per CTA: RS_LIST edges
+    // whole instances: what the tables hold (edges, vertices, table entries, run words)
+    long long cap_e, cap_v, cap_c, cap_r;
+    long long nnz;            //   and the entries rows[] holds (-1: colptr[m], one matrix)
 };
 
 __device__ __forceinline__ unsigned below(int bit) { return (1u << bit) - 1u; }
@@ -200,8 +207,8 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_words(C2Args a) {
     if (bad) a.st->bad = 1;
 }
 
-// The pitch of an instance's rows over its vertices: whole 16-byte loads.
-__host__ __device__ __forceinline__ int c2_pitch(int nv) { return (nv + 3) & ~3; }
+// The pitch of an instance's rows over its vertices: whole words of them.
+__host__ __device__ __forceinline__ int c2_pitch(int nv) { return (nv + 31) & ~31; }
 
 // Exclusive prefix over the block of 1024 threads; red holds 33 values.
 __device__ __forceinline__ long long c2_block_excl(long long v, long long *red, long long *total) {
@@ -413,6 +420,8 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_edges(C2Args a) {
                 w.vpre + __popc(w.v & below(j & 31)) != in.voff + in.nv)
                 a.st->unsorted = 1;
             t[(int64_t)y * pitch + x] = k - in.eoff;
+            int32_t *const c = a.tab + in.coff;
+            c[(int64_t)x * pitch + y] = c[(int64_t)y * pitch + x] = j - (int)in.base;
         }
         if (a.ends) {
             a.ends[k] = make_int2(u, v);
@@ -625,7 +634,6 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_graph(C2Args a, int max_round
 // torus after 1,788 of 58,988 edges.  Bound by the latency of its rounds (a
 // few hundred cycles each, some ten to a lot), and hidden behind the
 // triangles of the same launch.
-constexpr int KR_ITEMS = 4, KR_EDGES = KR_ITEMS * C2_THREADS;
 __device__ __forceinline__ int kr_find(uint16_t *parent, int x) {
     for (;;) {
         const int p = ((volatile uint16_t *)parent)[x];
@@ -635,45 +643,44 @@ __device__ __forceinline__ int kr_find(uint16_t *parent, int x) {
         x = g;
     }
 }
-__device__ void c2_kruskal(const C2Args &a, const C2Inst &in, uint32_t *best, uint16_t *parent, int *s_parts) {
+template <int THREADS, class Ends, class Die>
+__device__ void c2_kruskal(int nv, int ne, Ends ends, Die die, uint32_t *best, uint16_t *parent, int *s_parts) {
+    constexpr int ITEMS = 1024 / THREADS;
     const int tid = threadIdx.x;
-    for (int x = tid; x < in.nv; x += C2_THREADS) {
+    for (int x = tid; x < nv; x += THREADS) {
         parent[x] = (uint16_t)x;
         best[x] = 0xffffffffu;
     }
-    if (tid == 0) *s_parts = in.nv;
+    if (tid == 0) *s_parts = nv;
     __syncthreads();
     unsigned tag = 0x3fffff;  // counts down by rounds: nothing in best[] is reset
-    for (int c0 = 0; c0 < in.ne && *s_parts > 1; c0 += KR_EDGES) {
-        int u[KR_ITEMS], v[KR_ITEMS];
+    for (int c0 = 0; c0 < ne && *s_parts > 1; c0 += 1024) {
+        int2 e[ITEMS];
 #pragma unroll
-        for (int q = 0; q < KR_ITEMS; q++) {
-            const int i = c0 + q * C2_THREADS + tid;
-            const int4 e = i < in.ne ? a.erec[in.eoff + i] : make_int4(in.voff, in.voff, 0, 0);
-            u[q] = e.x - in.voff;
-            v[q] = e.y - in.voff;
+        for (int q = 0; q < ITEMS; q++) {
+            const int i = c0 + q * THREADS + tid;
+            e[q] = i < ne ? ends(i) : make_int2(0, 0);
         }
         for (;; tag--) {
             bool live = false;
 #pragma unroll
-            for (int q = 0; q < KR_ITEMS; q++) {
-                if (u[q] == v[q]) continue;
-                u[q] = kr_find(parent, u[q]);
-                v[q] = kr_find(parent, v[q]);
-                if (u[q] == v[q]) continue;
+            for (int q = 0; q < ITEMS; q++) {
+                if (e[q].x == e[q].y) continue;
+                e[q].x = kr_find(parent, e[q].x);
+                e[q].y = kr_find(parent, e[q].y);
+                if (e[q].x == e[q].y) continue;
                 live = true;
-                const unsigned key = tag << 10 | (unsigned)(q * C2_THREADS + tid);
-                atomicMin(best + u[q], key);
-                atomicMin(best + v[q], key);
+                const unsigned key = tag << 10 | (unsigned)(q * THREADS + tid);
+                atomicMin(best + e[q].x, key);
+                atomicMin(best + e[q].y, key);
             }
             if (!__syncthreads_or(live)) break;
 #pragma unroll
-            for (int q = 0; q < KR_ITEMS; q++) {
-                const int young = max(u[q], v[q]), old = min(u[q], v[q]);
-                if (young == old || best[young] != (tag << 10 | (unsigned)(q * C2_THREADS + tid))) continue;
+            for (int q = 0; q < ITEMS; q++) {
+                const int young = max(e[q].x, e[q].y), old = min(e[q].x, e[q].y);
+                if (young == old || best[young] != (tag << 10 | (unsigned)(q * THREADS + tid))) continue;
                 parent[young] = (uint16_t)old;
-                a.neg[in.eoff + c0 + q * C2_THREADS + tid] = young;
-                a.dead[in.voff + young] = 1;
+                die(c0 + q * THREADS + tid, young);
                 atomicSub(s_parts, 1);
             }
             __syncthreads();
@@ -682,19 +689,24 @@ __device__ void c2_kruskal(const C2Args &a, const C2Inst &in, uint32_t *best, ui
 }
 
 // One vertex's row of the edge-id table in the order of its edges: each entry
-// written at the number of smaller ones (a warp; `row` holds the row in
-// shared memory, absent edges as the largest id).  An entry is the edge's
-// rank and the other vertex.
+// written at the number of smaller ones, by THREADS threads (a warp or a
+// CTA; `row` holds the row in shared memory, absent edges as the largest id).
+// An entry is the edge's rank and the other vertex.
 constexpr int ADJ_SHIFT = 10;
+template <int THREADS>
 __device__ void c2_sort_row(const int32_t *src, int32_t *dst, int nv, int pitch, int32_t *row) {
-    const int lane = threadIdx.x & 31;
-    for (int i = lane; i < pitch; i += 32) {
-        const int x = src[i];
+    const int t = threadIdx.x & (THREADS - 1);
+    auto meet = [] {
+        if (THREADS == 32) __syncwarp();
+        else __syncthreads();
+    };
+    for (int i = t; i < pitch; i += THREADS) {
+        const int x = __ldcg(src + i);
         row[i] = x < 0 ? INT_MAX : x;
         dst[i] = INT_MAX;
     }
-    __syncwarp();
-    for (int i = lane; i < nv; i += 32) {
+    meet();
+    for (int i = t; i < nv; i += THREADS) {
         const int x = row[i];
         if (x == INT_MAX) continue;
         int at = 0;
@@ -704,23 +716,72 @@ __device__ void c2_sort_row(const int32_t *src, int32_t *dst, int nv, int pitch,
         }
         dst[at] = x << ADJ_SHIFT | i;
     }
-    __syncwarp();
+    meet();
 }
 
-// The first blocks pair the edges with vertices (an instance each); with
-// RUNS, the next ones sort the vertices' edges (a warp each); the rest check
-// the triangles, a thread each.
+// Runs.  A Rips complex is the flag complex of its edges, and its filtration
+// puts the triangles right after their last edge, third vertices ascending
+// (they carry that edge's length and come after it).  So the run of edge
+// f = (u, v) must be the vertices w joined to u and to v by earlier edges, in
+// order, and the rows of each triangle are those two edges' columns and f's.
+// Nothing is looked up: a warp takes an edge, its lanes the vertices; two
+// rows of the table of edge columns (vertices by vertices) say which have a
+// triangle (a ballot is the run's word), and the triangles' rows are compared
+// with what they must be.  A matrix that passes is a complex in such runs.
 //
-// RUNS: in a Rips filtration every triangle follows its last edge with no
-// other edge between (triangles carry their longest edge's length and come
-// after it), the third vertices of an edge's triangles ascending.  A set of
-// vertices per edge, one bit each, then names all of its run, and with it
-// every triangle: per 32 vertices the bits and the first one's column, so
-// (edge f, vertex z) is that column + the bits below z.  The triangles write
-// nothing else, and the lanes of a warp on one word write together, where the table costs three scattered 4-byte
-// writes each, of which 2% are ever read.  A triangle out of that order, or
-// a second edge on the same two vertices, sets `unsorted`, and the table is
-// built instead.
+// One word of 32 vertices: its set bits, the columns of the two edges.
+// VW > 0: that many words (else vw); four words' rows are in flight at a
+// time, for one word at a time is a trip to HBM each.  Columns are the
+// instance's, `run` holds them plus `shift`.  True where the run is not what
+// it must be; the last edge of an instance may have been cut off inside its
+// run (`cut`).
+constexpr int NO_EDGE = 0x7f7f7f7f;  // past every column, and a byte pattern
+template <int VW, bool GLOBAL>
+__device__ __forceinline__ bool flag_run(const int32_t *tu, const int32_t *tv, int vw, int fc, int len, bool cut,
+                                         const int32_t *src, uint2 *run, int shift) {
+    const int lane = threadIdx.x & 31;
+    constexpr int U = VW > 0 && VW < 4 ? VW : 4;
+    unsigned diff = 0;
+    int n = 0;
+    for (int wb = 0; wb < (VW > 0 ? VW : vw); wb += U) {
+        int x[U], y[U], t[U][3];
+        bool tri[U];
+        uint2 mine = make_uint2(0u, 0u);
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+            const bool on = VW > 0 || wb + q < vw;
+            const int at = 32 * (wb + q) + lane;
+            x[q] = on ? (GLOBAL ? __ldg(tu + at) : tu[at]) : NO_EDGE;
+            y[q] = on ? (GLOBAL ? __ldg(tv + at) : tv[at]) : NO_EDGE;
+        }
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+            tri[q] = max(x[q], y[q]) < fc;
+            unsigned bits = __ballot_sync(0xffffffffu, tri[q]);
+            const int i = n + __popc(bits & below(lane));
+            tri[q] = tri[q] && i < len;
+            if (cut) bits = __ballot_sync(0xffffffffu, tri[q]);
+            if (lane == q) mine = make_uint2(bits, (unsigned)(fc + 1 + n + shift));
+            n += __popc(bits);
+            const int32_t *p = src + 3 * i;
+#pragma unroll
+            for (int c = 0; c < 3; c++) t[q][c] = tri[q] ? __ldg(p + c) : 0;
+        }
+        if (lane < U && (VW > 0 || wb + lane < vw)) run[wb + lane] = mine;
+#pragma unroll
+        for (int q = 0; q < U; q++)
+            if (tri[q])
+                diff |= (unsigned)(t[q][0] ^ min(x[q], y[q])) | (unsigned)(t[q][1] ^ max(x[q], y[q])) |
+                        (unsigned)(t[q][2] ^ fc);
+    }
+    return diff != 0 || n != len;
+}
+
+// The first blocks pair the edges with vertices (an instance each).
+// RUNS: the next ones sort the vertices' edges (a CTA each), the rest check
+// the runs, a warp per edge; what fails sets `unsorted`, and the edge-vertex
+// table is built instead.  Table: the rest check the triangles, a thread
+// each, and write each at its three entries, bound by those scattered writes.
 template <bool RUNS>
 __global__ void __launch_bounds__(C2_THREADS) k_c2_triangles(C2Args a, int kruskal_blocks, int sort_blocks, int max_nv) {
     extern __shared__ __align__(16) uint32_t tri_smem[];
@@ -729,76 +790,69 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_triangles(C2Args a, int krusk
     const int lane = threadIdx.x & 31;
     if ((int)blockIdx.x < kruskal_blocks) {
         for (int b = blockIdx.x; b < a.count; b += kruskal_blocks) {
-            c2_kruskal(a, a.inst[b], tri_smem, reinterpret_cast<uint16_t *>(tri_smem + max_nv), &s_parts);
+            const C2Inst in = a.inst[b];
+            c2_kruskal<C2_THREADS>(
+                in.nv, in.ne,
+                [&](int i) {
+                    const int4 e = a.erec[in.eoff + i];
+                    return make_int2(e.x - in.voff, e.y - in.voff);
+                },
+                [&](int i, int v) {
+                    a.neg[in.eoff + i] = v;
+                    a.dead[in.voff + v] = 1;
+                },
+                tri_smem, reinterpret_cast<uint16_t *>(tri_smem + max_nv), &s_parts);
             __syncthreads();
         }
         return;
     }
     if (RUNS && (int)blockIdx.x < kruskal_blocks + sort_blocks) {
-        int32_t *row = reinterpret_cast<int32_t *>(tri_smem) + (threadIdx.x >> 5) * c2_pitch(max_nv);
-        const int warps = sort_blocks * (C2_THREADS / 32);
-        for (int v = (blockIdx.x - kruskal_blocks) * (C2_THREADS / 32) + (threadIdx.x >> 5); v < a.st->nv; v += warps) {
+        for (int v = blockIdx.x - kruskal_blocks; v < a.st->nv; v += sort_blocks) {
             const C2Inst &in = a.inst[c2_inst_of(a, a.vlist[v])];
             const int pitch = c2_pitch(in.nv);
             const int64_t at = in.coff + (int64_t)(v - in.voff) * pitch;
-            c2_sort_row(a.cells + at, a.adj + at, in.nv, pitch, row);
+            c2_sort_row<C2_THREADS>(a.cells + at, a.adj + at, in.nv, pitch, reinterpret_cast<int32_t *>(tri_smem));
         }
         return;
     }
-    bool bad = false, unsorted = false;
     const int others = kruskal_blocks + sort_blocks;
+    if (RUNS) {
+        bool wrong = false;
+        const int ne = a.st->ne, warps = (gridDim.x - others) * (C2_THREADS / 32);
+        for (int k = (blockIdx.x - others) * (C2_THREADS / 32) + (threadIdx.x >> 5); k < ne; k += warps) {
+            const int4 e = a.erec[k];
+            const C2Inst &in = a.inst[e.z];
+            const int kl = k - in.eoff, fc = a.elist[k];  // columns of the whole batch
+            const bool cut = kl + 1 == in.ne;
+            const int len = (cut ? (int)(in.base + in.cols) : a.elist[k + 1]) - fc - 1;
+            // vertices come first, so the triangles before f are the columns that are neither
+            const int64_t start = a.colptr[fc] + 2;
+            const int pitch = c2_pitch(in.nv), vw = pitch / 32, base = (int)in.base;
+            const int32_t *tab = a.tab + in.coff;
+            wrong |= flag_run<0, true>(tab + (int64_t)(e.x - in.voff) * pitch, tab + (int64_t)(e.y - in.voff) * pitch, vw,
+                                       fc - base, len, cut, a.rows + start, a.runs + in.roff + (long long)kl * vw, base);
+        }
+        if (wrong) a.st->unsorted = 1;
+        return;
+    }
+    bool bad = false;
     const int64_t stride = (int64_t)(gridDim.x - others) * C2_THREADS;
     for (int64_t j0 = (int64_t)(blockIdx.x - others) * C2_THREADS + (threadIdx.x - lane); j0 < a.m; j0 += stride) {
         const int64_t j = j0 + lane;
         const C2Word w = a.words[j0 >> 5];
-        const bool tri = j < a.m && !(((w.v | w.e) >> lane) & 1u);
-        const C2Inst &in = a.inst[tri ? c2_inst_of(a, j) : 0];
+        if (j >= a.m || ((w.v | w.e) >> lane) & 1u) continue;
+        const C2Inst &in = a.inst[c2_inst_of(a, j)];
         int k[3], o[3];
-        bool ok = tri && c2_triangle(a, j, w, in, k) &&
-                  c2_opposite(a.erec[k[0]], a.erec[k[1]], a.erec[k[2]], o[0], o[1], o[2]);
-        if (tri && !ok) bad = true;
-        if (!RUNS) {
-            if (ok)
-#pragma unroll
-                for (int q = 0; q < 3; q++)
-                    a.cells[in.coff + (int64_t)(k[q] - in.eoff) * c2_pitch(in.nv) + (o[q] - in.voff)] = (int32_t)j;
+        if (!c2_triangle(a, j, w, in, k) ||
+            !c2_opposite(a.erec[k[0]], a.erec[k[1]], a.erec[k[2]], o[0], o[1], o[2])) {
+            bad = true;
             continue;
         }
-        const unsigned lt = below(lane);
-        const int last = w.epre + __popc(w.e & lt) - 1;  // the last edge before j
-        const int z = ok ? o[2] - in.voff : 0;
-        if (ok && k[2] != last) unsorted = true;
-        // the third vertex of the triangle before it in the run is smaller
-        int zp = __shfl_up_sync(0xffffffffu, z, 1);
-        const bool okp = __shfl_up_sync(0xffffffffu, (int)ok, 1) != 0;
-        bool first = true;  // of its word
-        if (ok && k[2] == last && j - 1 != a.elist[last]) {
-            if (lane == 0) {
-                int kp[3], op[3];
-                zp = c2_triangle(a, j - 1, a.words[(j - 1) >> 5], in, kp) &&
-                             c2_opposite(a.erec[kp[0]], a.erec[kp[1]], a.erec[kp[2]], op[0], op[1], op[2])
-                         ? op[2] - in.voff
-                         : INT_MAX;
-            } else if (!okp) {
-                zp = INT_MAX;
-            }
-            if (zp >= z) unsorted = true;
-            first = (zp >> 5) != (z >> 5);
-        }
-        // the bits of each word by one lane
-        const int nw = (in.nv + 31) >> 5;
-        const unsigned long long at =
-            ok && k[2] == last ? (unsigned long long)in.roff + (unsigned long long)(last - in.eoff) * nw + (z >> 5)
-                               : ~0ull;
-        const unsigned peers = __match_any_sync(0xffffffffu, at);
-        const unsigned v = __reduce_or_sync(peers, 1u << (z & 31));
-        if (at != ~0ull && lane == __ffs(peers) - 1) {
-            atomicOr(&a.runs[at].x, v);
-            if (first) a.runs[at].y = (unsigned)j;
-        }
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            a.cells[in.coff + (int64_t)(k[q] - in.eoff) * c2_pitch(in.nv) + (o[q] - in.voff)] = (int32_t)j;
     }
     if (bad) a.st->bad = 1;
-    if (unsorted) a.st->unsorted = 1;
 }
 
 // Column `col` has row `row` as its low (columns of the whole batch).
@@ -1011,7 +1065,7 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
 // small ones as many CTAs as fit.
 template <bool RUNS, int THREADS, int WORDS>
 __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
-    if (a.st->bad || (RUNS && a.st->unsorted)) return;
+    if (a.st->bad || (RUNS && (a.st->unsorted || a.st->refused || a.st->no_room))) return;
     extern __shared__ __align__(16) uint32_t bits[];  // WORDS
     constexpr int NW = THREADS / 32;
     __shared__ int s_low[NW], s_cnt[NW], s_wave[RS_WAVE];
@@ -1245,6 +1299,296 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
     }
 }
 
+// ---------------------------------------------------------- whole instances
+// Small Rips complexes (a batch of them, or one): an instance to a CTA, from
+// its colptr to its runs in one launch, with its edges in shared memory.
+//
+// Against a launch per step over all columns this saves the launches, which
+// are all that the smallest complexes cost, and the trips to L2 for tables
+// that fit a CTA: 24 instructions a warp for 32 vertices of an edge are what
+// bounds it.  Whatever is no flag complex in runs, vertices first, or does
+// not fit (`refused`; malformed matrices too) is left to the grid-wide kernels.
+//
+// The tables that the residual columns read later are carved from common
+// arrays by counters; when those turn out too small the host makes them
+// larger and starts again.  The outputs are written (k_c2_inst_out) once
+// every instance has passed.
+constexpr int IN_THREADS = 512;
+constexpr int IN_SMEM = 112 * 1024;  // two CTAs an SM
+constexpr int IN_MAX_NV = 192;       // sorting the vertices' rows takes nv^3 comparisons of one CTA
+// Words of an instance start at a multiple of four (16-byte windows).
+__device__ __forceinline__ long long in_woff(long long o0, int b) { return 4 * ((o0 >> 7) + b); }
+
+// The triangles of an instance, a warp per edge (flag_run); true where a run
+// is not what it must be.
+template <int VW>
+__device__ bool in_triangles(const int32_t *col, const int32_t *tab, const uint16_t *ends, const int32_t *rows,
+                             uint2 *runs, int ne, int nv, int cols) {
+    const int vw = VW > 0 ? VW : (nv + 31) >> 5, idp = 32 * vw;
+    bool wrong = false;
+    for (int k = threadIdx.x >> 5; k < ne; k += IN_THREADS / 32) {
+        const bool cut = k + 1 == ne;
+        const int fc = col[k], len = (cut ? cols : col[k + 1]) - fc - 1, u = ends[k] & 0xff, v = ends[k] >> 8;
+        wrong |= tab[u * idp + v] != fc;  // a second edge on these vertices
+        wrong |= flag_run<VW, false>(tab + u * idp, tab + v * idp, vw, fc, len, cut,
+                                     rows + (2 * (k + 1) + 3 * (fc - nv - k)), runs + (long long)k * vw, 0);
+    }
+    return wrong;
+}
+
+__global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
+    extern __shared__ __align__(16) unsigned char in_smem[];  // IN_SMEM
+    constexpr int NW = IN_THREADS / 32;
+    __shared__ int s_b, s_nv, s_ne, s_no, s_parts, s_wsum[NW];
+    __shared__ C2Inst s_in;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (blockIdx.x == 0 && tid == 0) {
+        a.st->nnz = a.colptr[a.m];
+        if (a.colptr[0] != 0 || (a.nnz >= 0 && a.st->nnz != a.nnz) ||
+            (a.inst_off && (a.inst_off[0] != 0 || a.inst_off[a.count] != a.m)))
+            a.st->refused = 1;
+    }
+    for (;;) {
+        if (tid == 0) {
+            s_b = atomicAdd(&a.st->next, 1);
+            s_nv = s_ne = 0;
+            s_no = 0;
+        }
+        __syncthreads();
+        const int b = s_b;
+        if (b >= a.count) break;
+        const int64_t o0 = a.inst_off ? a.inst_off[b] : 0, o1 = a.inst_off ? a.inst_off[b + 1] : a.m;
+        const int64_t cols64 = o1 - o0;
+        // 6 bytes a word (bits, edges before it), and room for some edges
+        if (o0 < 0 || o1 > a.m || cols64 < 0 || (cols64 + 31) / 32 * 6 > IN_SMEM - 1024) {
+            if (tid == 0) a.st->refused = 1;
+            __syncthreads();
+            continue;
+        }
+        const int cols = (int)cols64, nw = (cols + 31) >> 5, nw2 = (nw + 1) & ~1;
+        uint32_t *ebit = reinterpret_cast<uint32_t *>(in_smem);
+        uint16_t *epre = reinterpret_cast<uint16_t *>(ebit + nw2);
+        const int64_t *cp = a.colptr + o0;
+        const int64_t c_first = cp[0];
+        // no row is read outside [0, nnz): an instance's columns lie between its ends (checked below)
+        const bool outside = c_first < 0 || (a.nnz >= 0 ? cp[cols] > a.nnz : c_first != 0);
+        // the kinds of the columns, eight words a warp in flight
+        bool no = false;
+        int nv = 0, ne = 0;
+        for (int w0 = 8 * wid; w0 < nw; w0 += 8 * NW) {
+            int64_t c0[8], c1[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int j = (w0 + q) * 32 + lane;
+                c0[q] = cp[min(j, cols)];
+                c1[q] = cp[min(j + 1, cols)];
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                if (w0 + q >= nw) break;
+                const bool in = (w0 + q) * 32 + lane < cols;
+                const int64_t n = c1[q] - c0[q];
+                if (in && n != 2 && n != 3 && (n != 0 || c0[q] != c_first)) no = true;  // vertices come first
+                const unsigned e = __ballot_sync(0xffffffffu, in && n == 2);
+                nv += __popc(__ballot_sync(0xffffffffu, in && n == 0));
+                ne += __popc(e);
+                if (lane == 0) ebit[w0 + q] = e;
+            }
+        }
+        if (lane == 0) {
+            atomicAdd(&s_nv, nv);
+            atomicAdd(&s_ne, ne);
+        }
+        if (no) s_no = 1;
+        __syncthreads();
+        nv = s_nv;
+        ne = s_ne;
+        const int pitch = c2_pitch(nv), vw = pitch / 32;
+        // shared memory once the words are written out: in their place the
+        // table of edge columns and the edges' columns; the edges' vertices
+        // (bytes) behind; the rest is scratch
+        const int ends_at = (max(6 * nw2, 4 * pitch * nv + 4 * ne) + 15) & ~15;
+        const int scratch_at = (ends_at + 2 * ne + 15) & ~15, left = IN_SMEM - scratch_at;
+        if (outside || ne > 65535 || nv > IN_MAX_NV || left < max(6 * nv, 4 * pitch)) {
+            if (tid == 0) a.st->refused = 1;
+            s_no = 1;
+        }
+        if (tid == 0) {
+            C2Inst in{};
+            in.nv = nv;
+            in.ne = ne;
+            in.base = in.wbase = o0;
+            in.cols = cols;
+            in.woff = in_woff(o0, b);
+            in.eoff = atomicAdd(&a.st->ne, ne);
+            in.voff = atomicAdd(&a.st->nv, nv);
+            in.coff = (long long)atomicAdd((unsigned long long *)&a.st->pairs, (unsigned long long)pitch * nv);
+            in.roff = (long long)atomicAdd((unsigned long long *)&a.st->run_words, (unsigned long long)ne * vw);
+            atomicMax(&a.st->max_nv, nv);
+            if (in.eoff + ne > a.cap_e || in.voff + nv > a.cap_v || in.coff + (long long)pitch * nv > a.cap_c ||
+                in.roff + (long long)ne * vw > a.cap_r) {
+                a.st->no_room = 1;
+                s_no = 1;
+            }
+            s_in = in;
+            a.inst[b] = in;
+        }
+        __syncthreads();
+        if (s_no) {
+            if (no) a.st->refused = 1;
+            __syncthreads();
+            continue;
+        }
+        const C2Inst in = s_in;
+        {  // edges before each word
+            const int per = (nw + IN_THREADS - 1) / IN_THREADS, w1 = min(tid * per + per, nw);
+            int sum = 0;
+            for (int w = tid * per; w < w1; w++) sum += __popc(ebit[w]);
+            int incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += u;
+            }
+            if (lane == 31) s_wsum[wid] = incl;
+            __syncthreads();
+            int run = incl - sum + __reduce_add_sync(0xffffffffu, lane < wid && lane < NW ? s_wsum[lane] : 0);
+            for (int w = tid * per; w < w1; w++) {
+                epre[w] = (uint16_t)run;
+                run += __popc(ebit[w]);
+            }
+        }
+        int32_t *const elist = a.elist + in.eoff;
+        for (int i = tid; i < nv; i += IN_THREADS) a.dead[in.voff + i] = 0;
+        __syncthreads();
+        for (int w = tid; w < nw; w += IN_THREADS) {
+            const unsigned e = ebit[w];
+            const int k0 = epre[w], v0 = min(nv, 32 * w);
+            *reinterpret_cast<int4 *>(a.words + in.woff + w) =
+                make_int4((int)(nv - v0 >= 32 ? ~0u : below(nv - v0)), (int)e, in.voff + v0, in.eoff + k0);
+            int k = k0;
+            for (unsigned x = e; x; x &= x - 1) elist[k++] = 32 * w + __ffs(x) - 1;
+        }
+        __syncthreads();
+        int32_t *const tab = reinterpret_cast<int32_t *>(in_smem), *const col = tab + pitch * nv;
+        uint16_t *const ends = reinterpret_cast<uint16_t *>(in_smem + ends_at);
+        uint32_t *const scratch = reinterpret_cast<uint32_t *>(in_smem + scratch_at);
+        int32_t *const ids = a.cells + in.coff, *const adj = a.adj + in.coff;
+        for (int i = tid; i < pitch * nv; i += IN_THREADS) {
+            tab[i] = NO_EDGE;
+            ids[i] = -1;
+        }
+        __syncthreads();
+        // the edges: a column starts at 2 (edges before it) + 3 (triangles before it)
+        const int32_t *const rows = a.rows + c_first;
+        for (int k = tid; k < ne; k += IN_THREADS) {
+            const int j = __ldcg(elist + k), s = 2 * k + 3 * (j - nv - k);
+            int r0 = rows[s], r1 = rows[s + 1];
+            if (r0 < 0 || r1 <= r0 || r1 >= nv) {
+                s_no = 1;
+                r0 = r1 = 0;
+            } else {
+                tab[r0 * pitch + r1] = tab[r1 * pitch + r0] = j;
+                ids[r0 * pitch + r1] = ids[r1 * pitch + r0] = k;
+            }
+            col[k] = j;
+            ends[k] = (uint16_t)(r0 | r1 << 8);
+            a.erec[in.eoff + k] = make_int4(in.voff + r0, in.voff + r1, b, 0);
+            a.neg[in.eoff + k] = -1;
+        }
+        __syncthreads();
+        c2_kruskal<IN_THREADS>(
+            nv, ne, [&](int i) { return make_int2(ends[i] & 0xff, ends[i] >> 8); },
+            [&](int i, int v) {
+                a.neg[in.eoff + i] = v;
+                a.dead[in.voff + v] = 1;
+            },
+            scratch, reinterpret_cast<uint16_t *>(scratch + nv), &s_parts);
+        __syncthreads();
+        // the vertices' edges in order, for the residual columns (as many
+        // warps as the scratch has rows for)
+        const int warps = min(NW, left / (4 * pitch));
+        if (wid < warps)
+            for (int v = wid; v < nv; v += warps)
+                c2_sort_row<32>(ids + v * pitch, adj + v * pitch, nv, pitch,
+                            reinterpret_cast<int32_t *>(scratch) + wid * pitch);
+        uint2 *const runs = a.runs + in.roff;
+        bool wrong;
+        switch (vw) {
+            case 1: wrong = in_triangles<1>(col, tab, ends, rows, runs, ne, nv, cols); break;
+            case 2: wrong = in_triangles<2>(col, tab, ends, rows, runs, ne, nv, cols); break;
+            case 3: wrong = in_triangles<3>(col, tab, ends, rows, runs, ne, nv, cols); break;
+            case 4: wrong = in_triangles<4>(col, tab, ends, rows, runs, ne, nv, cols); break;
+            default: wrong = in_triangles<0>(col, tab, ends, rows, runs, ne, nv, cols); break;
+        }
+        if (wrong) s_no = 1;
+        __syncthreads();
+        if (tid == 0 && s_no) a.st->refused = 1;
+        __syncthreads();
+    }
+}
+
+// The outputs of whole instances, as k_c2_runs_out writes them: IO_COLS
+// columns a block are filled with what a positive triangle gets, 16 bytes a
+// store, then a thread per word corrects the few vertices, edges and paired
+// triangles.  Bound by the writes.
+constexpr int IO_THREADS = 256, IO_COLS = 32 * IO_THREADS;
+__global__ void __launch_bounds__(IO_THREADS) k_c2_inst_out(C2Args a, int parts) {
+    if (a.st->refused || a.st->no_room) return;
+    const int none = a.one_based ? 0 : -1, tid = threadIdx.x;
+    auto fill = [&](int32_t *p, int n, int value) {
+        const int head = min(n, (int)((16 - ((uintptr_t)p & 15)) & 15) / 4), body = (n - head) / 4;
+        if (tid < head) p[tid] = value;
+        int4 *q = reinterpret_cast<int4 *>(p + head);
+        for (int i = tid; i < body; i += IO_THREADS) q[i] = make_int4(value, value, value, value);
+        const int at = head + 4 * body + tid;
+        if (at < n) p[at] = value;
+    };
+    for (int b = blockIdx.x / parts; b < a.count; b += gridDim.x / parts) {
+        const C2Inst in = a.inst[b];
+        const C2Word *const words = a.words + in.woff;
+        const int nw = (int)((in.cols + 31) >> 5);
+        int32_t *const low = a.low + in.base, *const ess = a.ess ? a.ess + in.base : nullptr;
+        for (int c0 = (blockIdx.x % parts) * IO_COLS; c0 < in.cols; c0 += parts * IO_COLS) {
+            const int n = min(IO_COLS, (int)in.cols - c0);
+            fill(low + c0, n, none);
+            if (ess) fill(ess + c0, n, 1);
+            __syncthreads();
+            const int wi = (c0 >> 5) + tid;
+            if (wi < nw) {
+                const C2Word w = words[wi];
+                const unsigned prev = wi > 0 ? words[wi - 1].e >> 31 : 0u, notri = w.v | w.e;
+                const int end = min(32, (int)in.cols - 32 * wi);
+                const unsigned here = end == 32 ? ~0u : below(end);
+                const unsigned open = (w.e << 1 | prev) & ~notri & here;  // first triangles: paired with the edge before
+                a.owned[in.woff + wi] = open;
+                a.fixed[in.woff + wi] = open;
+                for (unsigned x = open; x; x &= x - 1) {
+                    const int j = 32 * wi + __ffs(x) - 1;
+                    low[j] = j - 1 + a.one_based;
+                    if (ess) ess[j] = 0;
+                }
+                if (ess)
+                    for (unsigned x = w.v; x; x &= x - 1) {
+                        const int j = 32 * wi + __ffs(x) - 1;
+                        if (a.dead[in.voff + j]) ess[j] = 0;
+                    }
+                // bit x: the column after x is no triangle, or past the instance's end
+                const unsigned next = notri >> 1 | (wi + 1 < nw ? (words[wi + 1].v | words[wi + 1].e) << 31 : ~(here >> 1));
+                int k = w.epre;
+                for (unsigned x = w.e; x; x &= x - 1, k++) {
+                    const int bit = __ffs(x) - 1, j = 32 * wi + bit, y = a.neg[k];
+                    const bool run = !((next >> bit) & 1u);
+                    if (y >= 0) low[j] = y + a.one_based;
+                    if (y < 0 && !run) a.res[atomicAdd(&a.st->nres, 1)] = k;
+                    else if (ess) ess[j] = 0;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
 // ------------------------------------------------------------------ driver
 namespace {
 struct Carve {
@@ -1347,7 +1691,7 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     // (sparse complexes on many vertices are left to the general path)
     const long long room = (1ll << 24) + 8 * hs->nnz;
     const long long cells = RUNS ? hs->pairs : hs->cells, run_words = RUNS ? hs->run_words : 0;
-    if (hs->max_nv > (RUNS ? 1 << ADJ_SHIFT : C2_MAX_NV) || 2 * cells > room || 2 * run_words > room) return OPH_OK;
+    if (hs->max_nv > (RUNS ? 1 << ADJ_SHIFT : C2_MAX_NV) || 3 * cells > room || 2 * run_words > room) return OPH_OK;
     cudaStream_t s = ctx->stream;
     const bool small = hs->max_nv <= RS_SMALL_NV;
     int gr = small ? c2_residual_grid<RUNS, RS_SMALL, RS_SMALL_WORDS>(ctx)
@@ -1359,9 +1703,9 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     size_t head = 0;
     for (char *p = nullptr;;) {
         Carve c{p};
-        a.runs = c.take<uint2>(run_words);
         a.dead = c.take<uint8_t>(nv + 1);
         head = c.off;  // zeroed
+        a.runs = c.take<uint2>(run_words);
         a.owned = c.take<uint32_t>((a.m + 31) / 32 + 4);
         a.fixed = c.take<uint32_t>((a.m + 31) / 32 + 4);
         a.res = c.take<int32_t>(ne);
@@ -1374,19 +1718,21 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     }
     if (!RUNS) a.runs = nullptr;
     const size_t cell_bytes = sizeof(int32_t) * (size_t)std::max<long long>(cells, 1);
-    a.cells = (int32_t *)ctx_alloc(ctx, S_C2_CELLS, (RUNS ? 2 : 1) * cell_bytes);
+    a.cells = (int32_t *)ctx_alloc(ctx, S_C2_CELLS, (RUNS ? 3 : 1) * cell_bytes);
     if (!a.cells) return OPH_OK;
-    a.adj = RUNS ? a.cells + cells : nullptr;  // cells is a multiple of 4: whole 16-byte loads
+    a.adj = RUNS ? a.cells + cells : nullptr;  // cells is a multiple of 32
+    a.tab = RUNS ? a.adj + cells : nullptr;
     a.ends = nullptr;
     const int kb = std::min(a.count, ctx->sm_count * 4);
     OPH_CUDA_TRY(cudaMemsetAsync(a.cells, 0xff, cell_bytes, s));
+    if (RUNS) OPH_CUDA_TRY(cudaMemsetAsync(a.tab, NO_EDGE & 0xff, cell_bytes, s));
     OPH_CUDA_TRY(cudaMemsetAsync(ctx->bufs[S_C2_MODE].ptr, 0, head, s));
     if (!RUNS) k_c2_cells<<<1, 1024, 0, s>>>(a);
     k_c2_edges<<<c2_grid(ctx, ne, 8), C2_THREADS, 0, s>>>(a);
-    // rows of vertices in shared memory (sorted a warp each), or the components
-    const int smem = std::max(6 * hs->max_nv, RUNS ? 4 * (C2_THREADS / 32) * c2_pitch(hs->max_nv) : 0);
-    const int sb = RUNS ? c2_grid(ctx, 32 * (int64_t)nv, 4) : 0;
-    k_c2_triangles<RUNS><<<kb + sb + c2_grid(ctx, a.m, 16), C2_THREADS, smem, s>>>(a, kb, sb, hs->max_nv);
+    // the components, or a row of vertices to sort
+    const int smem = std::max(6 * hs->max_nv, RUNS ? 4 * c2_pitch(hs->max_nv) : 0);
+    const int sb = RUNS ? std::min(nv, ctx->sm_count * 4) : 0;
+    k_c2_triangles<RUNS><<<kb + sb + c2_grid(ctx, RUNS ? 32 * ne : a.m, 16), C2_THREADS, smem, s>>>(a, kb, sb, hs->max_nv);
     if (RUNS) {
         k_c2_runs_out<<<c2_grid(ctx, a.m, 16), C2_THREADS, 0, s>>>(a);
     } else {
@@ -1406,6 +1752,95 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     *done = !rc && !hs->bad && !hs->overflow && (!RUNS || !hs->unsorted) &&
             (RUNS || hs->cells_set == 3ull * (unsigned long long)nt);
     return rc;
+}
+
+// Which calls try whole instances first: a CTA each pays while the CTAs have
+// instances enough (batches of at least a hundred or so), or while one is not
+// much longer alone than the grid-wide kernels' launches.
+constexpr int64_t IN_MAX_COLS = 1 << 15;
+constexpr int IN_MIN_COUNT = 128;
+
+static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
+    *done = false;
+    cudaStream_t s = ctx->stream;
+    static int ready[64];
+    int &ok = ready[ctx->device & 63];
+    if (!ok) {
+        if (cudaFuncSetAttribute(k_c2_inst, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess) {
+            cudaGetLastError();
+            return OPH_OK;
+        }
+        ok = 1;
+    }
+    int gr = c2_residual_grid<true, RS_SMALL, RS_SMALL_WORDS>(ctx);
+    if (gr == 0) return OPH_OK;
+    // bounds for the tables: guesses from the columns, or what an earlier call needed
+    const int64_t m = a.m;
+    long long need[4] = {std::min<long long>(m, m / 6 + 1024), std::min<long long>(m, m / 16 + 1024), m / 2 + 65536,
+                         m / 4 + 65536};
+    for (int q = 0; q < 4; q++) need[q] = std::max(need[q], ctx->c2_need[q]);
+    const long long nwords = 4 * (m / 128 + a.count + 1);
+    for (int tries = 0; tries < 2; tries++) {
+        a.cap_e = need[0];
+        a.cap_v = need[1];
+        a.cap_c = (need[2] + 3) & ~3ll;
+        a.cap_r = need[3];
+        a.arena_cap = (1 << 20) + 16 * a.cap_e;
+        for (char *p = nullptr;;) {
+            Carve c{p};
+            a.st = c.take<C2Status>(1);
+            a.inst = c.take<C2Inst>(a.count);
+            a.words = c.take<C2Word>(nwords);
+            if (p) break;
+            p = (char *)ctx_alloc(ctx, S_C2_TAB, c.off);
+            if (!p) return OPH_OK;
+        }
+        for (char *p = nullptr;;) {
+            Carve c{p};
+            a.elist = c.take<int32_t>(a.cap_e);
+            a.erec = c.take<int4>(a.cap_e);
+            a.neg = c.take<int32_t>(a.cap_e);
+            a.res = c.take<int32_t>(a.cap_e);
+            a.sum = c.take<unsigned long long>(a.cap_e);
+            a.dead = c.take<uint8_t>(a.cap_v);
+            if (p) break;
+            p = (char *)ctx_alloc(ctx, S_C2_WORK, c.off);
+            if (!p) return OPH_OK;
+        }
+        for (char *p = nullptr;;) {
+            Carve c{p};
+            a.runs = c.take<uint2>(a.cap_r);
+            a.owned = c.take<uint32_t>(nwords);
+            a.fixed = c.take<uint32_t>(nwords);
+            a.arena = c.take<int32_t>(a.arena_cap);
+            a.lists = c.take<int32_t>((size_t)gr * RS_LIST);
+            if (p) break;
+            p = (char *)ctx_alloc(ctx, S_C2_MODE, c.off);
+            if (!p) return OPH_OK;
+        }
+        a.cells = (int32_t *)ctx_alloc(ctx, S_C2_CELLS, 2 * sizeof(int32_t) * (size_t)a.cap_c);
+        if (!a.cells) return OPH_OK;
+        a.adj = a.cells + a.cap_c;
+        OPH_CUDA_TRY(cudaMemsetAsync(a.st, 0, sizeof(C2Status), s));
+        k_c2_inst<<<std::min(a.count, 2 * ctx->sm_count), IN_THREADS, IN_SMEM, s>>>(a);
+        // enough blocks for the outputs of one instance as of many
+        const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(16, (m / a.count + IO_COLS - 1) / IO_COLS));
+        k_c2_inst_out<<<parts * std::min(a.count, 65535), IO_THREADS, 0, s>>>(a, parts);
+        if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
+        // a residual edge or so per vertex
+        const int rg = (int)std::min<int64_t>(gr, std::max<int64_t>(1, a.cap_e));
+        k_c2_residual<true, RS_SMALL, RS_SMALL_WORDS><<<rg, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
+        ctx->launches += 3;
+        cudaEventRecord(ctx->ev[1], s);
+        int rc = c2_read_status(ctx, a, hs);
+        if (rc) return rc;
+        if (hs->refused || !hs->no_room) break;
+        const long long used[4] = {hs->ne, hs->nv, hs->pairs, hs->run_words};
+        for (int q = 0; q < 4; q++)
+            if (used[q] > need[q]) need[q] = ctx->c2_need[q] = used[q] + used[q] / 8;
+    }
+    *done = !hs->refused && !hs->no_room && !hs->overflow;
+    return OPH_OK;
 }
 
 // Contexts that ask for something of the sweeps keep them: trackers, a forced
@@ -1438,6 +1873,26 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
     a.low = job.low;
     a.ess = job.ess;
     a.one_based = job.one_based;
+    a.nnz = job.want_nnz;
+    static_assert(sizeof(C2Status) <= sizeof(DevStatus), "read back through the context's pinned status block");
+    C2Status *hs = reinterpret_cast<C2Status *>(ctx->h_status);
+    DevStatus *hb = ctx->h_status + 1;
+    int rc;
+    bool done = false;
+    int64_t nv, ne, nt;
+    cudaEventRecord(ctx->ev[0], s);
+    if (job.rows && (!batch || job.want_nnz >= 0) && (batch ? a.count >= IN_MIN_COUNT || m / a.count <= IN_MAX_COLS : m <= IN_MAX_COLS)) {
+        if (job.before) OPH_CUDA_TRY(cudaMemcpyAsync(hb, job.before, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
+        if ((rc = c2_run_inst(ctx, a, hs, &done))) return rc;
+        if (done) {
+            job.nnz = hs->nnz;
+            job.nnz_read = true;
+            job.before_error = job.before ? hb->error : 0;
+            if (job.before_error) return OPH_OK;
+            done = job.want_nnz < 0 || hs->nnz == job.want_nnz;
+        }
+    }
+    if (!done) {
     for (char *p = nullptr;;) {
         Carve c{p};
         a.st = c.take<C2Status>(1);
@@ -1449,23 +1904,20 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
         p = (char *)ctx_alloc(ctx, S_C2_TAB, c.off);
         if (!p) return OPH_OK;  // no room: the general path decides
     }
-    static_assert(sizeof(C2Status) <= sizeof(DevStatus), "read back through the context's pinned status block");
-    C2Status *hs = reinterpret_cast<C2Status *>(ctx->h_status);
-    int rc;
-    cudaEventRecord(ctx->ev[0], s);
     OPH_CUDA_TRY(cudaMemsetAsync(a.st, 0, sizeof(C2Status), s));
     k_c2_words<<<(int)std::min<int64_t>(ntiles, (int64_t)ctx->sm_count * 8), C2_THREADS, 0, s>>>(a);
     k_c2_scan<<<1, 1024, 0, s>>>(a, ntiles);
     OPH_CUDA_TRY(cudaGetLastError());
     ctx->launches += 2;
-    DevStatus *hb = ctx->h_status + 1;
     if (job.before) OPH_CUDA_TRY(cudaMemcpyAsync(hb, job.before, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
     if ((rc = c2_read_status(ctx, a, hs))) return rc;
     job.nnz = hs->nnz;
     job.nnz_read = true;
     job.before_error = job.before ? hb->error : 0;
     if (job.before_error) return OPH_OK;
-    const int64_t nv = hs->nv, ne = hs->ne, nt = m - nv - ne;
+    nv = hs->nv;
+    ne = hs->ne;
+    nt = m - nv - ne;
     if (hs->bad || hs->nnz != 2 * ne + 3 * nt || (job.want_nnz >= 0 && hs->nnz != job.want_nnz)) return OPH_OK;
     if (ne == 0 || ne >= (1 << 29) || !job.rows) return OPH_OK;
     for (char *p = nullptr;;) {
@@ -1480,7 +1932,6 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
     }
     k_c2_lists<<<c2_grid(ctx, nwords, 8), C2_THREADS, 0, s>>>(a);
     ctx->launches++;
-    bool done = false;
     // every edge with at most two triangles: a graph (an edge found to have
     // more leaves it to the dense form)
     if (3 * nt <= 2 * ne && (rc = c2_run_graph(ctx, a, nv, ne, nt, hs, &done))) return rc;
@@ -1493,6 +1944,10 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
         if ((rc = c2_run_dense<false>(ctx, a, ne, nt, hs, &done))) return rc;
     }
     if (!done) return OPH_OK;
+    }
+    nv = hs->nv;
+    ne = hs->ne;
+    nt = m - nv - ne;
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (ctx->profile) {

@@ -206,6 +206,7 @@ struct Context {
     int launches = 0;               // kernels launched by the current reduction
     int tier0 = 0;                  // Phase II tier-0 candidate (autotuned)
     int dual = OPH_DUAL_AUTO;       // which matrix pms reduces
+    long long c2_need[4] = {};      // complex2.cu: the largest tables a call needed (entries)
     Tracking *track = nullptr;      // per-sweep trackers for the current reduction
     SeqTracking *seq_track = nullptr;  // per-iteration trackers of a standard / twist walk
     // two pms sweeps (the list ping-pong's two parities) captured as one CUDA

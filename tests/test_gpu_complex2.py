@@ -178,3 +178,44 @@ def test_runs_and_not(ctx):
 def test_rips_cta_sizes(ctx, n):
     """Either side of the residual columns' CTA and window sizes."""
     check(ctx, cx.rips(cx.points_circle(n, seed=n), threshold=1.2))
+
+
+@pytest.mark.parametrize("n_max", [100, 121, 125, 140])
+def test_batch_of_whole_instances(ctx, n_max):
+    """130 instances: a CTA each while every one fits its shared memory, the
+    grid-wide kernels for the whole batch where one does not."""
+    sizes = np.full(130, 6, np.int32)
+    sizes[[3, 77]] = n_max, 65
+    sizes[[8, 9]] = 1, 2
+    seeds = np.arange(130, dtype=np.uint64) + np.uint64(5)
+    col_off, colptr, rows = cx.rips_mixed_instances(sizes, seeds)
+    low, ess, _ = ctx.reduce_batch_packed(col_off, colptr, rows)
+    for b in range(130):
+        bm = cx.batch_instance(col_off, colptr, rows, b)
+        want, want_ess, _ = oracle.twist(bm)
+        np.testing.assert_array_equal(low[col_off[b]:col_off[b + 1]], want, err_msg=str(b))
+        np.testing.assert_array_equal(ess[col_off[b]:col_off[b + 1]], want_ess, err_msg=str(b))
+
+
+@pytest.mark.parametrize("cut", [1, 2, 3, 40, 300, 2000, 2300])
+def test_first_simplices_of_a_rips_complex(ctx, cut):
+    """A filtration cut off anywhere: inside the last edge's run, right after
+    an edge, among the vertices."""
+    bm = cx.rips_cube(24, seed=6)
+    check(ctx, BoundaryMatrix(bm.colptr[:cut + 1], bm.rows[:bm.colptr[cut]]))
+    big = cx.rips_cube(80, seed=6)
+    cut = cut * 30
+    check(ctx, BoundaryMatrix(big.colptr[:cut + 1], big.rows[:big.colptr[cut]]))
+
+
+def test_missing_triangle(ctx):
+    """Rips complexes less one triangle each: no flag complexes."""
+    for n in (12, 70):
+        bm = cx.rips_cube(n, seed=3)
+        size = np.diff(bm.colptr)
+        drop = np.flatnonzero(size == 3)[::max(1, bm.m // 7)]
+        for t in drop:
+            cols = np.delete(np.arange(bm.m), t)
+            colptr = np.concatenate([[0], np.cumsum(size[cols])])
+            rows = np.concatenate([bm.rows[:bm.colptr[t]], bm.rows[bm.colptr[t + 1]:]])
+            check(ctx, BoundaryMatrix(colptr, rows - (rows > t)))
