@@ -69,6 +69,7 @@ struct C2Status {
     long long nnz;
     int nv, ne;
     int live[3];     // edges left, by round modulo three
+    unsigned arrived;  // blocks at the graph's meetings
     unsigned long long joins;
     int max_nv;      // the largest instance's vertices
     int unsorted;    // the triangles do not come in runs
@@ -85,6 +86,7 @@ struct C2Status {
 
 constexpr int C2_THREADS = 256, C2_TILE = 2048;
 constexpr int C2_MAX_ROUNDS = 512;
+constexpr unsigned long long C2_FIRST_ROUND = 0xffffffffull << 32;  // the round in a key's upper half, counting down
 constexpr int C2_MAX_NV = 8192;                   // vertices of an instance the dense form takes
 constexpr int RS_WAVE = 32;                       // residual columns: pivots added at a time,
 constexpr int RS_LIST = 16384;                    //   edges a column under reduction may be the sum of
@@ -426,6 +428,10 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_edges(C2Args a) {
         if (a.ends) {
             a.ends[k] = make_int2(u, v);
             a.ends[2 * (int64_t)ne - 1 - k] = make_int2(-1, -1);
+            // a vertex's first edge (the reads spare most of the atomics)
+            const unsigned long long key = C2_FIRST_ROUND | (unsigned)k;
+            if (__ldcg(a.best + u) > key) atomicMin(a.best + u, key);
+            if (__ldcg(a.best + v) > key) atomicMin(a.best + v, key);
         }
     }
     if (bad) a.st->bad = 1;
@@ -458,6 +464,10 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_surface(C2Args a) {
     if (a.st->bad) return;
     const int nv = a.st->nv, ne = a.st->ne, nt = (int)(a.m - nv - ne);
     bool bad = false, crowded = false;
+    // an instance's oldest vertex never dies, and most edges come to lead to
+    // it: nothing is kept for it in best[]
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < a.count; b += gridDim.x * blockDim.x)
+        if (a.inst[b].nv > 0) a.best[a.inst[b].voff] = 0;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < a.m; j += (int64_t)gridDim.x * blockDim.x) {
         const C2Word w = a.words[j >> 5];
         const int bit = (int)(j & 31);
@@ -475,6 +485,7 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_surface(C2Args a) {
         const int t = (int)(j - (w.vpre + __popc(w.v & below(bit))) - (w.epre + __popc(w.e & below(bit))));
         a.tlist[t] = (int32_t)j;
         const int id = nv + 1 + (nt - 1 - t);
+        a.best[id] = C2_FIRST_ROUND | (unsigned)(2 * ne - 1 - k[2]);  // its last edge is its first column of D'
 #pragma unroll
         for (int q = 0; q < 3; q++) {
             int *e = reinterpret_cast<int *>(a.ends + (2 * (int64_t)ne - 1 - k[q]));
@@ -485,56 +496,90 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_surface(C2Args a) {
     if (crowded) a.st->crowded = 1;
 }
 
-// Outputs before any pair is known, and the graph's nodes.
-__global__ void __launch_bounds__(C2_THREADS) k_c2_graph_init(C2Args a) {
-    if (a.st->bad || a.st->crowded) return;
-    const int64_t nodes = a.m - a.st->ne + 1, stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int none = a.one_based ? 0 : -1;
-    for (int64_t j = i0; j < a.m; j += stride) {
-        a.low[j] = none;
-        if (a.ess) a.ess[j] = 1;
-    }
-    for (int64_t i = i0; i < nodes; i += stride) {
-        a.parent[i] = (int)i;
-        a.best[i] = ~0ull;
-    }
-}
-
-// The component of a node: its oldest node.  Parents are always older than
-// their children, and only grow older; the path is halved on the way (racing
-// writers all write ancestors).
-__device__ __forceinline__ int c2_find(int *parent, int x) {
-    int cur = __ldcg(parent + x);
-    if (cur == x) return x;
-    int prev = x;
+// Components are trees: a node's parent is older, its root the component's
+// oldest node.  N nodes' roots at once, so that a step up every path is one
+// trip to memory (x < 0 stands for the ground); the nodes are then hung on
+// them (racing writers all write ancestors).  The way up may go through L1:
+// what it holds of an earlier round is an ancestor too, and half of all paths
+// end at the same few nodes; that the end is a root is read from L2.
+template <int N>
+__device__ __forceinline__ void c2_roots(int *parent, int ground, const int (&x)[N], int (&r)[N]) {
+    int p[N];
+#pragma unroll
+    for (int q = 0; q < N; q++) p[q] = r[q] = x[q] < 0 ? ground : parent[x[q]];
     for (;;) {
-        const int next = __ldcg(parent + cur);
-        if (next == cur) return cur;
-        __stcg(parent + prev, next);
-        prev = cur;
-        cur = next;
+        for (;;) {
+            bool more = false;
+            int up[N];
+#pragma unroll
+            for (int q = 0; q < N; q++) up[q] = parent[r[q]];
+#pragma unroll
+            for (int q = 0; q < N; q++) {
+                more |= up[q] != r[q];
+                r[q] = up[q];
+            }
+            if (!more) break;
+        }
+        bool more = false;
+        int up[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) up[q] = __ldcg(parent + r[q]);
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+            more |= up[q] != r[q];
+            r[q] = up[q];
+        }
+        if (!more) break;
+    }
+#pragma unroll
+    for (int q = 0; q < N; q++)
+        if (x[q] >= 0 && p[q] != r[q]) parent[x[q]] = r[q];
+}
+
+// Every node hung eight steps up (or on its root): three such passes shorten
+// paths of up to 512.
+__device__ __forceinline__ void c2_shorten(int *parent, int nodes, int i0, int stride) {
+    constexpr int N = 4;
+    for (int b = i0; b < nodes; b += N * stride) {
+        int p[N], r[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) p[q] = r[q] = parent[min(b + q * stride, nodes - 1)];
+        bool more = true;
+        for (int h = 1; more && h < 8; h++) {
+            more = false;
+#pragma unroll
+            for (int q = 0; q < N; q++) {
+                const int up = parent[r[q]];
+                more |= up != r[q];
+                r[q] = up;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < N; q++)
+            if (b + q * stride < nodes && r[q] != p[q]) parent[b + q * stride] = r[q];
     }
 }
 
-// A pair: node x dies at slot s.
-__device__ __forceinline__ void c2_die(const C2Args &a, int nv, int ne, int nt, int s, int x) {
-    int lo, col, k;
-    if (s < ne) {  // an edge of D: its low is the vertex
-        k = s;
-        col = a.elist[k];
-        lo = a.vlist[x];
-    } else {  // an edge of D': the triangle's low is the edge
-        k = 2 * ne - 1 - s;
-        lo = a.elist[k];
-        col = a.tlist[nt - 1 - (x - nv - 1)];
+// The blocks of a resident grid meet: the count of arrivals only grows, `goal`
+// is the grid's size times the meetings so far.  False when the others do not
+// come (never, while the grid is resident as a whole; about a second).
+__device__ __forceinline__ bool c2_meet(unsigned *arrived, unsigned goal) {
+    __shared__ int s_late;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_late = 0;
+        __threadfence();
+        atomicAdd(arrived, 1u);
+        int tries = 0;
+        while ((unsigned)ld_acquire_i32(reinterpret_cast<const int *>(arrived)) < goal)
+            if (++tries > (1 << 22)) {
+                s_late = 1;
+                break;
+            }
+        __threadfence();
     }
-    const int base = a.inst_off ? (int)a.inst[a.erec[k].z].base : 0;
-    a.low[col] = lo - base + a.one_based;
-    if (a.ess) {
-        a.ess[col] = 0;
-        a.ess[lo] = 0;
-    }
+    __syncthreads();
+    return !s_late;
 }
 
 // The elder rule on the whole graph, in rounds over the edges that still join
@@ -550,77 +595,139 @@ __device__ __forceinline__ void c2_die(const C2Args &a, int nv, int ne, int nt, 
 // older node; r is the younger, the low of column s.  An edge found inside a
 // component closes a cycle of earlier edges: its column reduces to zero.
 //
-// A round is two passes over the list of such edges, with a grid barrier
-// after each.  Bound by the latency of its dependent loads (parents, best)
-// and the barriers, not by bandwidth: 12 rounds on the 512 x 512 lower-star
-// image (1.57M slots, then 320K, 76K, ...), 19 on white noise of that size.
+// The first round goes over the nodes, whose first edges k_c2_edges and
+// k_c2_surface left in best[]; a node's last best[] is where it died, so the
+// pairs are written at the end, a thread per node.  The paths of the first
+// two rounds are long (on a smooth image they run downhill for a hundred
+// pixels and more), so they are shortened for all nodes at once before roots
+// are looked for edge by edge.  A round is two passes over the live edges,
+// each followed by a meeting of the grid.  Bound by the latency of its
+// dependent loads and the meetings (2-3 us): 10 rounds on the 512 x 512
+// lower-star image (1.57M slots, then 320K, 76K, ...), 19 on white noise of
+// that size.
 __global__ void __launch_bounds__(C2_THREADS) k_c2_graph(C2Args a, int max_rounds) {
     if (a.st->bad || a.st->crowded) return;  // written by earlier kernels: the same for every block
-    cg::grid_group grid = cg::this_grid();
-    const int nv = a.st->nv, ne = a.st->ne, nt = (int)(a.m - nv - ne), ground = nv;
+    const int nv = a.st->nv, ne = a.st->ne, nt = (int)(a.m - nv - ne), ground = nv, nodes = nv + 1 + nt;
     const int stride = gridDim.x * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = 2 * ne;
-    unsigned long long joins = 0;
-    for (int round = 0;; round++) {
+    unsigned goal = 0;
+    auto meet = [&] { return c2_meet(&a.st->arrived, goal += gridDim.x); };
+    // round 0, and the outputs before any pair is known
+    const int none = a.one_based ? 0 : -1;
+    for (int j = i0; j < a.m; j += stride) {
+        a.low[j] = none;
+        if (a.ess) a.ess[j] = 1;
+    }
+    for (int x = i0; x < nodes; x += stride) {
+        const unsigned long long b = __ldcg(a.best + x);
+        int p = x;
+        if (x != ground && b != ~0ull && b != 0) {
+            const int2 e = __ldcg(a.ends + (unsigned)b);
+            int y = e.x == x ? e.y : e.x;
+            if (y < 0) y = ground;
+            p = min(x, y);
+        }
+        a.parent[x] = p;
+    }
+    bool met = meet();
+    for (int q = 0; met && q < 3; q++) {
+        c2_shorten(a.parent, nodes, i0, stride);
+        met = meet();
+    }
+    constexpr int PER = 4, NW = C2_THREADS / 32;
+    __shared__ int s_cnt[NW], s_at;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    int n = 2 * ne, round = 1;
+    for (; met; round++) {
         const unsigned long long tag = (unsigned long long)(~(unsigned)round) << 32;
         const int32_t *in = a.list[(round + 1) & 1];
         int32_t *out = a.list[round & 1];
         int *count = &a.st->live[round % 3];
-        // the warp stays whole for the aggregated append
-        for (int i1 = i0 - (threadIdx.x & 31); i1 < n; i1 += stride) {
-            const int i = i1 + (threadIdx.x & 31);
-            bool live = i < n;
-            int s = 0;
-            if (live) {
-                s = round ? in[i] : i;
-                int2 e = __ldcg(a.ends + s);
-                if (round) {
-                    const int x = c2_find(a.parent, e.x), y = c2_find(a.parent, e.y);
-                    live = x != y;
-                    if (live && (x != e.x || y != e.y)) __stcg(a.ends + s, make_int2(x, y));
-                    e = make_int2(x, y);
-                } else if (s >= ne) {
-                    live = e.x >= 0;  // an edge without triangles: an empty column of D'
-                    if (live && e.y < 0) {
-                        e.y = ground;
-                        a.ends[s] = e;
-                    }
-                }
-                if (live) {
-                    const unsigned long long key = tag | (unsigned)s;
-                    if (e.x != ground && __ldcg(a.best + e.x) > key) atomicMin(a.best + e.x, key);
-                    if (e.y != ground && __ldcg(a.best + e.y) > key) atomicMin(a.best + e.y, key);
-                }
+        // up to four edges a thread, fewer where that fills more blocks; the
+        // block appends those that live together
+        const int per = min(PER, (n + stride - 1) / stride);
+        for (int b0 = blockIdx.x * per * C2_THREADS; b0 < n; b0 += per * stride) {
+            int s[PER], x[2 * PER], r[2 * PER];
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const int i = b0 + q * C2_THREADS + tid;
+                s[q] = i >= n || q >= per ? -1 : round > 1 ? __ldcg(in + i) : i;
             }
-            const unsigned b = __ballot_sync(0xffffffffu, live);
-            if (b) {
-                const int lane = threadIdx.x & 31, leader = __ffs(b) - 1;
-                int at = 0;
-                if (lane == leader) at = atomicAdd(count, __popc(b));
-                at = __shfl_sync(0xffffffffu, at, leader);
-                if (live) out[at + __popc(b & below(lane))] = s;
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const int2 e = s[q] >= 0 ? __ldcg(a.ends + s[q]) : make_int2(-1, -1);
+                if (e.x < 0) s[q] = -1;  // an edge without triangles: an empty column of D'
+                x[2 * q] = e.x;
+                x[2 * q + 1] = e.y;
+            }
+            c2_roots<2 * PER>(a.parent, ground, x, r);
+            unsigned live[PER];
+            int mine = 0;
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const int u = r[2 * q], v = r[2 * q + 1];
+                const bool l = s[q] >= 0 && u != v;
+                if (l) {
+                    if (u != x[2 * q] || v != x[2 * q + 1]) __stcg(a.ends + s[q], make_int2(u, v));
+                    const unsigned long long key = tag | (unsigned)s[q];
+                    // (an old value of best[] only costs the atomic)
+                    if (u != ground && a.best[u] > key) atomicMin(a.best + u, key);
+                    if (v != ground && a.best[v] > key) atomicMin(a.best + v, key);
+                }
+                live[q] = __ballot_sync(0xffffffffu, l);
+                mine += __popc(live[q]);
+            }
+            if (lane == 0) s_cnt[wid] = mine;
+            __syncthreads();
+            const int c = lane < NW ? s_cnt[lane] : 0;
+            const int before = __reduce_add_sync(0xffffffffu, lane < wid ? c : 0);
+            if (tid < 32) {
+                const int total = __reduce_add_sync(0xffffffffu, c);
+                if (lane == 0) s_at = total ? atomicAdd(count, total) : 0;
+            }
+            __syncthreads();
+            int at = s_at + before;
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                if ((live[q] >> lane) & 1u) out[at + __popc(live[q] & below(lane))] = s[q];
+                at += __popc(live[q]);
             }
         }
-        grid.sync();
+        if (!(met = meet())) break;
         n = __ldcg(count);
-        if (i0 == 0) {
-            a.st->live[(round + 1) % 3] = 0;  // last read two rounds ago
-            a.st->rounds = round + 1;
-            if (n > 0 && round + 1 >= max_rounds) a.st->unfinished = 1;
-        }
-        if (n == 0 || round + 1 >= max_rounds) break;
+        if (i0 == 0) a.st->live[(round + 1) % 3] = 0;  // last read two rounds ago
+        if (n == 0 || round >= max_rounds) break;
         for (int i = i0; i < n; i += stride) {
             const int s = __ldcg(out + i);
             const int2 e = __ldcg(a.ends + s);
-            const unsigned long long key = tag | (unsigned)s;
             const int x = max(e.x, e.y), y = min(e.x, e.y);  // only the younger end can die here
-            if (x != ground && __ldcg(a.best + x) == key) {
-                __stcg(a.parent + x, y);
-                c2_die(a, nv, ne, nt, s, x);
-                joins++;
-            }
+            if (x != ground && __ldcg(a.best + x) == (tag | (unsigned)s)) a.parent[x] = y;
         }
-        grid.sync();
+        met = meet();
+        for (int q = 0; round == 1 && met && q < 2; q++) {
+            c2_shorten(a.parent, nodes, i0, stride);
+            met = meet();
+        }
+    }
+    if (i0 == 0) a.st->rounds = round;
+    if (!met || n > 0) {
+        if (threadIdx.x == 0) a.st->unfinished = 1;
+        return;
+    }
+    // the pairs: node x died at the slot in its best[]
+    unsigned long long joins = 0;
+    for (int x = i0; x < nodes; x += stride) {
+        if (x == ground || __ldcg(a.parent + x) == x) continue;
+        const int s = (int)(unsigned)__ldcg(a.best + x), k = s < ne ? s : 2 * ne - 1 - s, e = a.elist[k];
+        const int base = a.inst_off ? (int)a.inst[a.erec[k].z].base : 0;
+        // an edge of D: its low is the vertex; of D': the triangle's low is the edge
+        const int v = x < ground ? a.vlist[x] : a.tlist[nt - 1 - (x - ground - 1)];
+        const int col = x < ground ? e : v, lo = x < ground ? v : e;
+        a.low[col] = lo - base + a.one_based;
+        if (a.ess) {
+            a.ess[col] = 0;
+            a.ess[lo] = 0;
+        }
+        joins++;
     }
     for (int o = 16; o > 0; o >>= 1) joins += __shfl_xor_sync(0xffffffffu, joins, o);
     if ((threadIdx.x & 31) == 0 && joins) atomicAdd(&a.st->joins, joins);
@@ -1650,16 +1757,16 @@ static int c2_run_graph(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t 
         nb = 0;
         return OPH_OK;
     }
-    const int gg = c2_grid(ctx, 2 * ne, std::min(nb, 4));
+    const int gg = c2_grid(ctx, ne, std::min(nb, 4));
     a.neg = nullptr;
+    OPH_CUDA_TRY(cudaMemsetAsync(a.best, 0xff, sizeof(unsigned long long) * nodes, s));
     k_c2_edges<<<c2_grid(ctx, ne, 8), C2_THREADS, 0, s>>>(a);
     k_c2_surface<<<c2_grid(ctx, a.m, 16), C2_THREADS, 0, s>>>(a);
-    k_c2_graph_init<<<c2_grid(ctx, a.m, 16), C2_THREADS, 0, s>>>(a);
     if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
     int max_rounds = C2_MAX_ROUNDS;
     void *params[] = {&a, &max_rounds};
     OPH_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_c2_graph, dim3(gg), dim3(C2_THREADS), params, 0, s));
-    ctx->launches += 4;
+    ctx->launches += 3;
     cudaEventRecord(ctx->ev[1], s);
     int rc = c2_read_status(ctx, a, hs);
     *done = !rc && !hs->bad && !hs->crowded && !hs->unfinished;
