@@ -6,12 +6,23 @@
 // example_factory.m:17-114, stream2cmo.m:1-26) are generated on the host by
 // gen/ophgen.c; these kernels produce the identical matrix (same filtration
 // values, same order, same rows) from the points or the image already in
-// HBM.  The order is (value, dimension, vertex tuple): every simplex gets a
-// 128-bit key, the order-preserving bits of its FP64 value followed by a
-// word holding its dimension and vertex ids, and one radix sort of the keys
-// is the filtration order.  The key alone names the simplex, so the sorted
-// keys are decoded back into columns: a position table per vertex and per
-// edge turns each simplex's facets into row indices.
+// HBM.  The order is (value, dimension, vertex tuple).
+//
+// * Rips: a triangle carries its longest edge's value, so only the edges are
+//   sorted (their 64-bit values; the sort is stable, and they are listed by
+//   vertices).  When no two edges are equally long, the triangles of an edge
+//   (u, v) follow it directly, ascending in the third vertex: the vertices
+//   joined to u and to v by earlier edges.  Counting them per edge, a prefix
+//   sum and one pass over the edges write the matrix.  The whole complex of
+//   the 1M-column torus was sorted by 128-bit keys before, sixteen passes
+//   over 16 bytes a simplex (330 us) after a walk over the triangles by a
+//   warp per vertex (790 us).
+// * Equally long edges mix their triangles: then every simplex gets that
+//   128-bit key, the order-preserving bits of its FP64 value followed by a
+//   word holding its dimension and vertex ids, and one radix sort of the keys
+//   is the filtration order.  The key alone names the simplex.
+// * Lower star: simplices are listed by (dimension, vertices), so a stable
+//   sort of their FP32 values' 32 bits (four passes of 8 bytes) is the order.
 //
 // Distances are summed in the host generator's order with separately
 // rounded multiplies and adds (no FMA) and a correctly rounded square root,
@@ -215,81 +226,219 @@ __global__ void k_rips_rows(const SKey *__restrict__ keys, int64_t m, int n, con
     }
 }
 
-// ------------------------------------------------------------ lower star
-// Vertex (y, x) = y * w + x; edges H(y, x) = (y,x)-(y,x+1), V = (y,x)-(y+1,x),
-// D = (y,x)-(y+1,x+1); triangles per square: upper (y,x),(y,x+1),(y+1,x+1)
-// and lower (y,x),(y+1,x),(y+1,x+1).
-__global__ void k_ls_keys(const float *__restrict__ img, int h, int w, SKey *__restrict__ keys) {
-    const int64_t V = (int64_t)h * w, EH = (int64_t)h * (w - 1), EV = (int64_t)(h - 1) * w,
-                  ED = (int64_t)(h - 1) * (w - 1);
-    const int64_t m = V + EH + EV + ED + 2 * ED;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
-        int64_t t = q;
-        SKey k;
-        if (t < V) {
-            k = SKey{dbits((double)img[t]), lexkey(0, (unsigned)t, 0, 0)};
-        } else if ((t -= V) < EH + EV + ED) {
-            unsigned a, b;
-            if (t < EH) {
-                const int y = (int)(t / (w - 1)), x = (int)(t % (w - 1));
-                a = y * w + x; b = a + 1;
-            } else if ((t -= EH) < EV) {
-                const int y = (int)(t / w), x = (int)(t % w);
-                a = y * w + x; b = a + w;
-            } else {
-                t -= EV;
-                const int y = (int)(t / (w - 1)), x = (int)(t % (w - 1));
-                a = y * w + x; b = a + w + 1;
+// The edges in vertex order: their keys (value bits), their vertices, their
+// place (the sort's payload).  A warp per row, a lane per vertex of a word.
+__global__ void k_rips_edge_list(const unsigned *__restrict__ adj, const double *__restrict__ D, int n, int words,
+                                 const long long *__restrict__ eoff, unsigned long long *__restrict__ key,
+                                 unsigned *__restrict__ place, int2 *__restrict__ ends) {
+    const int lane = threadIdx.x & 31;
+    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int a = wid; a < n; a += nw) {
+        long long e = eoff[a];
+        for (int w = a >> 5; w < words; w++) {
+            const unsigned bits = adj[(int64_t)a * words + w] & above(w, a);
+            if ((bits >> lane) & 1u) {
+                const int b = w * 32 + lane;
+                const long long at = e + __popc(bits & ((1u << lane) - 1u));
+                key[at] = dbits(D[(int64_t)a * n + b]);
+                place[at] = (unsigned)at;
+                ends[at] = make_int2(a, b);
             }
-            const double va = (double)img[a], vb = (double)img[b];
-            k = SKey{dbits(va > vb ? va : vb), lexkey(1, a, b, 0)};
-        } else {
-            t -= EH + EV + ED;
-            const int64_t sq = t >> 1;
-            const int up = (t & 1) == 0;  // the host emits the upper triangle first
-            const int y = (int)(sq / (w - 1)), x = (int)(sq % (w - 1));
-            const unsigned a = y * w + x, b = up ? a + 1 : a + w, c = a + w + 1;
-            double v = (double)img[a];
-            if ((double)img[b] > v) v = (double)img[b];
-            if ((double)img[c] > v) v = (double)img[c];
-            k = SKey{dbits(v), lexkey(2, a, b, c)};
+            e += __popc(bits);
         }
-        keys[q] = k;
     }
 }
 
+// All triangles: common neighbours above the second vertex, a warp per edge.
+__global__ void k_rips_total(const unsigned *__restrict__ adj, int words, const int2 *__restrict__ ends, long long E,
+                             unsigned long long *total) {
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    unsigned long long t = 0;
+    for (long long k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < E; k += nw) {
+        const int2 e = ends[k];
+        for (int w = (e.y >> 5) + lane; w < words; w += 32)
+            t += __popc(adj[(int64_t)e.x * words + w] & adj[(int64_t)e.y * words + w] & above(w, e.y));
+    }
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0 && t) atomicAdd(total, t);
+}
+
+// Sorted edges: the rank of the edge on two vertices, the vertices by rank;
+// *tied when two are equally long.
+__global__ void k_rips_rank(const unsigned long long *__restrict__ key, const unsigned *__restrict__ place,
+                            const int2 *__restrict__ ends, long long E, int n, int32_t *__restrict__ rank,
+                            int2 *__restrict__ by_rank, int *tied) {
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < E; k += (long long)gridDim.x * blockDim.x) {
+        const int2 e = ends[place[k]];
+        by_rank[k] = e;
+        rank[(int64_t)e.x * n + e.y] = rank[(int64_t)e.y * n + e.x] = (int32_t)k;
+        if (k > 0 && key[k] == key[k - 1]) *tied = 1;
+    }
+}
+
+// The triangles whose last edge is k, a warp: `body` gets, word by word of
+// 32 vertices, the mask of third vertices (uniform), and each lane's own
+// edges' ranks.  32 words at a time are looked over first, so that sparse
+// complexes on many vertices skip those without common neighbours.
+template <class Body>
+__device__ __forceinline__ void rips_run(const unsigned *adj, const int32_t *rank, int n, int words, int2 e, int k,
+                                         Body body) {
+    const int lane = threadIdx.x & 31;
+    const unsigned *ra = adj + (int64_t)e.x * words, *rb = adj + (int64_t)e.y * words;
+    for (int w0 = 0; w0 < words; w0 += 32) {
+        const unsigned both = w0 + lane < words ? ra[w0 + lane] & rb[w0 + lane] : 0u;
+        for (unsigned some = __ballot_sync(0xffffffffu, both != 0u); some; some &= some - 1) {
+            const int q = __ffs(some) - 1, c = (w0 + q) * 32 + lane;
+            const unsigned m = __shfl_sync(0xffffffffu, both, q);
+            int x = 0, y = 0;
+            bool on = (m >> lane) & 1u;
+            if (on) {
+                x = rank[(int64_t)e.x * n + c];
+                y = rank[(int64_t)e.y * n + c];
+                on = x < k && y < k;
+            }
+            body(__ballot_sync(0xffffffffu, on), on, x, y);
+        }
+    }
+}
+
+__global__ void k_rips_run_count(const unsigned *__restrict__ adj, const int32_t *__restrict__ rank, int n, int words,
+                                 const int2 *__restrict__ by_rank, long long E, long long *__restrict__ cnt) {
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (long long k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < E; k += nw) {
+        long long c = 0;
+        rips_run(adj, rank, n, words, by_rank[k], (int)k, [&](unsigned mask, bool, int, int) { c += __popc(mask); });
+        if ((threadIdx.x & 31) == 0) cnt[k] = c;
+    }
+}
+
+// The matrix: vertices first, then every edge (column n + k + the triangles
+// before it, toff[k]) with its triangles.
+__global__ void k_rips_write(const unsigned *__restrict__ adj, const int32_t *__restrict__ rank, int n, int words,
+                             const int2 *__restrict__ by_rank, const unsigned long long *__restrict__ key, long long E,
+                             const long long *__restrict__ toff, int64_t *__restrict__ colptr,
+                             int32_t *__restrict__ rows, double *__restrict__ value) {
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        colptr[v] = 0;
+        if (value) value[v] = 0.0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) colptr[n + E + toff[E]] = 2 * E + 3 * toff[E];
+    auto column = [&](int r) { return (int32_t)(n + r + toff[r]); };
+    for (long long k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < E; k += nw) {
+        const int2 e = by_rank[k];
+        const double val = dvalue(key[k]);
+        const int32_t col = column((int)k);
+        const int64_t start = 2 * k + 3 * toff[k];
+        if (lane == 0) {
+            colptr[col] = start;
+            rows[start] = e.x;
+            rows[start + 1] = e.y;
+            if (value) value[col] = val;
+        }
+        int done = 0;
+        rips_run(adj, rank, n, words, e, (int)k, [&](unsigned mask, bool on, int x, int y) {
+            if (on) {
+                const int i = done + __popc(mask & ((1u << lane) - 1u));
+                const int64_t at = start + 2 + 3ll * i;
+                colptr[col + 1 + i] = at;
+                rows[at] = column(min(x, y));
+                rows[at + 1] = column(max(x, y));
+                rows[at + 2] = col;
+                if (value) value[col + 1 + i] = val;
+            }
+            done += __popc(mask);
+        });
+    }
+}
+
+// ------------------------------------------------------------ lower star
+// Vertex (y, x) = y * w + x; the edges of vertex a in the order of their other
+// end: H to a + 1, V to a + w, D to a + w + 1, where the image goes on; per
+// square the triangles upper (a, a+1, a+w+1) and lower (a, a+w, a+w+1).
 __device__ __forceinline__ int64_t ls_edge(unsigned a, unsigned b, int h, int w) {
-    const int64_t V = (int64_t)h * w, EH = (int64_t)h * (w - 1), EV = (int64_t)(h - 1) * w;
     const int y = (int)(a / w), x = (int)(a % w);
-    if (b == a + 1) return V + (int64_t)y * (w - 1) + x;
-    if (b == a + (unsigned)w) return V + EH + (int64_t)y * w + x;
-    return V + EH + EV + (int64_t)y * (w - 1) + x;
+    if (y == h - 1) return (int64_t)y * (3 * w - 2) + x;
+    const int sub = x == w - 1 ? 0 : b == a + 1 ? 0 : b == a + (unsigned)w ? 1 : 2;
+    return (int64_t)y * (3 * w - 2) + 3 * x + sub;
+}
+// The vertices of simplex q (vertices, then edges, then triangles).
+__device__ __forceinline__ int ls_simplex(int64_t q, int h, int w, unsigned &a, unsigned &b, unsigned &c) {
+    const int64_t V = (int64_t)h * w, E = (int64_t)h * (w - 1) + (int64_t)(h - 1) * w + (int64_t)(h - 1) * (w - 1);
+    a = b = c = (unsigned)q;
+    if (q < V) return 0;
+    q -= V;
+    if (q < E) {
+        const int per = 3 * w - 2, y = (int)(q / per), i = (int)(q - (int64_t)y * per);
+        if (y == h - 1) {  // the last row: H only
+            a = y * w + i;
+            b = a + 1;
+        } else {
+            const int x = min(i / 3, w - 1), sub = x == w - 1 ? 1 : i - 3 * x;
+            a = y * w + x;
+            b = sub == 0 ? a + 1 : sub == 1 ? a + w : a + w + 1;
+        }
+        c = b;
+        return 1;
+    }
+    q -= E;
+    const int64_t sq = q >> 1;
+    const int y = (int)(sq / (w - 1)), x = (int)(sq % (w - 1));
+    a = y * w + x;
+    b = (q & 1) ? a + w : a + 1;
+    c = a + w + 1;
+    return 2;
+}
+__device__ __forceinline__ unsigned fbits(float v) {
+    const unsigned u = __float_as_uint(v);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float fvalue(unsigned b) {
+    return __uint_as_float((b & 0x80000000u) ? (b & 0x7fffffffu) : ~b);
 }
 
-__global__ void k_ls_pos(const SKey *__restrict__ keys, int64_t m, int h, int w, int32_t *__restrict__ pos) {
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long L = keys[r].lex;
-        const int dim = (int)(L >> 60);
-        const unsigned a = (unsigned)((L >> 40) & 0xfffff), b = (unsigned)((L >> 20) & 0xfffff);
-        if (dim == 0) pos[a] = (int32_t)r;
-        else if (dim == 1) pos[ls_edge(a, b, h, w)] = (int32_t)r;
+// Every simplex's value (its largest vertex's) and place.
+__global__ void k_ls_keys(const float *__restrict__ img, int h, int w, int64_t m, unsigned *__restrict__ key,
+                          unsigned *__restrict__ place) {
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
+        unsigned a, b, c;
+        const int dim = ls_simplex(q, h, w, a, b, c);
+        float v = img[a];
+        const float vb = img[b], vc = img[c];
+        if (dim == 1) v = v > vb ? v : vb;
+        if (dim == 2) {
+            if (vb > v) v = vb;
+            if (vc > v) v = vc;
+        }
+        key[q] = fbits(v);
+        place[q] = (unsigned)q;
     }
 }
 
-__global__ void k_ls_rows(const SKey *__restrict__ keys, int64_t m, int h, int w, const int32_t *__restrict__ pos,
-                          const int64_t *__restrict__ colptr, int32_t *__restrict__ rows) {
+// Sorted simplices: each one's position, its column's size, its value.
+__global__ void k_ls_pos(const unsigned *__restrict__ key, const unsigned *__restrict__ place, int64_t m, int64_t V,
+                         int64_t VE, int32_t *__restrict__ pos, int64_t *__restrict__ cnt, double *__restrict__ value) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long L = keys[r].lex;
-        const int dim = (int)(L >> 60);
-        const unsigned a = (unsigned)((L >> 40) & 0xfffff), b = (unsigned)((L >> 20) & 0xfffff),
-                       c = (unsigned)(L & 0xfffff);
+        const int64_t q = place[r];
+        if (q < VE) pos[q] = (int32_t)r;
+        cnt[r] = q < V ? 0 : q < VE ? 2 : 3;
+        if (value) value[r] = (double)fvalue(key[r]);
+    }
+}
+
+__global__ void k_ls_rows(const unsigned *__restrict__ place, int64_t m, int h, int w, int64_t V,
+                          const int32_t *__restrict__ pos, const int64_t *__restrict__ colptr,
+                          int32_t *__restrict__ rows) {
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
+        unsigned a, b, c;
+        const int dim = ls_simplex(place[r], h, w, a, b, c);
         const int64_t k = colptr[r];
         if (dim == 1) {
             const int32_t x = pos[a], y = pos[b];
             rows[k] = min(x, y);
             rows[k + 1] = max(x, y);
         } else if (dim == 2) {
-            int32_t x = pos[ls_edge(a, b, h, w)], y = pos[ls_edge(b, c, h, w)], z = pos[ls_edge(a, c, h, w)];
+            int32_t x = pos[V + ls_edge(a, b, h, w)], y = pos[V + ls_edge(b, c, h, w)], z = pos[V + ls_edge(a, c, h, w)];
             sort3(x, y, z);
             rows[k] = x;
             rows[k + 1] = y;
@@ -303,12 +452,30 @@ int grid_of(Context *ctx, int64_t n) {
     return (int)std::max<int64_t>(1, std::min(g, cap));
 }
 
-// Scratch of one generator call, released on every exit.
+// Scratch of one generator call: first from the context's own buffer, kept
+// from call to call (pool allocations are given back to the driver at every
+// synchronisation, and cost more than the kernels on small complexes), then
+// from the stream's memory pool, released on every exit.
 struct Scratch {
     cudaStream_t s;
     std::vector<void *> ptrs;
+    char *kept = nullptr;
+    size_t room = 0, used = 0;
     explicit Scratch(cudaStream_t st) : s(st) {}
+    // the context's buffer `slot`, of at least `bytes` where its budget
+    // allows, for what is taken from here on (S_GEN, and those of the
+    // reduction, which nothing uses now)
+    void keep(Context *ctx, int slot, size_t bytes) {
+        kept = (char *)ctx_alloc(ctx, slot, bytes);
+        room = kept ? ctx->bufs[slot].bytes : 0;
+        used = 0;
+    }
     void *get(size_t bytes) {
+        const size_t want = ((bytes ? bytes : 16) + 255) & ~(size_t)255;
+        if (used + want <= room) {
+            used += want;
+            return kept + used - want;
+        }
         void *p = nullptr;
         if (cudaMallocAsync(&p, bytes ? bytes : 16, s) != cudaSuccess) {
             cudaGetLastError();
@@ -364,12 +531,16 @@ __attribute__((visibility("default"))) int oph_rips_device(oph_context *ctx, con
     cudaStream_t s = ctx->stream;
     Scratch sc(s);
     const int words = (n + 31) / 32;
-    double *D = (double *)sc.get(sizeof(double) * (size_t)n * n);
+    const size_t nn = (size_t)n * n;
+    sc.keep(ctx, S_GEN, 8 * nn + 4 * (size_t)n * words + 16 * (size_t)(n + 1) + (64 << 10));
+    double *D = (double *)sc.get(sizeof(double) * nn);
     unsigned *adj = (unsigned *)sc.get(sizeof(unsigned) * (size_t)n * words);
     long long *deg = (long long *)sc.get(sizeof(long long) * (size_t)(n + 1));
     long long *eoff = (long long *)sc.get(sizeof(long long) * (size_t)(n + 1));
-    if (!D || !adj || !deg || !eoff) return OPH_ERR_OOM;
+    unsigned long long *total = (unsigned long long *)sc.get(2 * sizeof(unsigned long long));
+    if (!D || !adj || !deg || !eoff || !total) return OPH_ERR_OOM;
     OPH_CUDA_TRY(cudaMemsetAsync(adj, 0, sizeof(unsigned) * (size_t)n * words, s));
+    OPH_CUDA_TRY(cudaMemsetAsync(total, 0, 2 * sizeof(unsigned long long), s));
     k_rips_dist<<<grid_of(ctx, (int64_t)n * n), 256, 0, s>>>(d_points, n, d, threshold, D, adj, words);
     k_rips_deg<<<grid_of(ctx, n), 256, 0, s>>>(adj, n, words, deg);
     OPH_CUDA_TRY(cudaMemsetAsync(deg + n, 0, sizeof(long long), s));
@@ -381,36 +552,82 @@ __attribute__((visibility("default"))) int oph_rips_device(oph_context *ctx, con
     long long E = 0;
     OPH_CUDA_TRY(cudaMemcpyAsync(&E, eoff + n, sizeof(long long), cudaMemcpyDeviceToHost, s));
     OPH_CUDA_TRY(cudaStreamSynchronize(s));
-    long long *tcnt = (long long *)sc.get(sizeof(long long) * (size_t)(E + 1));
-    long long *toff = (long long *)sc.get(sizeof(long long) * (size_t)(E + 1));
-    if (!tcnt || !toff) return OPH_ERR_OOM;
-    OPH_CUDA_TRY(cudaMemsetAsync(tcnt, 0, sizeof(long long) * (size_t)(E + 1), s));
     const int wgrid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, (int64_t)ctx->sm_count * 8));
-    if (E > 0) k_rips_tri_count<<<wgrid, 256, 0, s>>>(adj, n, words, eoff, tcnt);
+    const int egrid = (int)std::max<int64_t>(1, std::min<int64_t>((E + 7) / 8, (int64_t)ctx->sm_count * 16));
+    // the edges: keys and places twice (the sort's two buffers), vertices in
+    // both orders, ranks, triangles before each
+    const size_t e1 = (size_t)E + 1;
+    sc.keep(ctx, S_C2_CELLS, (d_colptr ? 4 * nn : 0) + 64 * e1 + (8 << 20));
+    unsigned long long *key[2] = {(unsigned long long *)sc.get(8 * e1), (unsigned long long *)sc.get(8 * e1)};
+    unsigned *place[2] = {(unsigned *)sc.get(4 * e1), (unsigned *)sc.get(4 * e1)};
+    int2 *ends = (int2 *)sc.get(8 * e1);
+    if (!key[0] || !key[1] || !place[0] || !place[1] || !ends) return OPH_ERR_OOM;
+    if (E > 0) k_rips_edge_list<<<wgrid, 256, 0, s>>>(adj, D, n, words, eoff, key[0], place[0], ends);
+    if (!d_colptr) {  // sizes only
+        unsigned long long T = 0;
+        if (E > 0) k_rips_total<<<egrid, 256, 0, s>>>(adj, words, ends, E, total);
+        OPH_CUDA_TRY(cudaGetLastError());
+        OPH_CUDA_TRY(cudaMemcpyAsync(&T, total, sizeof(T), cudaMemcpyDeviceToHost, s));
+        OPH_CUDA_TRY(cudaStreamSynchronize(s));
+        const int64_t m = n + E + (int64_t)T;
+        if (m >= (1ll << 31)) return OPH_ERR_BAD_INPUT;
+        if (m_out) *m_out = m;
+        if (nnz_out) *nnz_out = 2 * E + 3 * (int64_t)T;
+        return OPH_OK;
+    }
+    int2 *by_rank = (int2 *)sc.get(8 * e1);
+    int32_t *rank = (int32_t *)sc.get(4 * nn);
+    long long *tcnt = (long long *)sc.get(8 * e1), *toff = (long long *)sc.get(8 * e1);
+    if (!by_rank || !rank || !tcnt || !toff) return OPH_ERR_OOM;
+    cub::DoubleBuffer<unsigned long long> dk(key[0], key[1]);
+    cub::DoubleBuffer<unsigned> dp(place[0], place[1]);
+    OPH_CUDA_TRY(cudaMemsetAsync(tcnt, 0, 8 * e1, s));
+    if (E > 0) {
+        size_t tb = 0;
+        OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dp, E, 0, 64, s));
+        void *tmp = sc.get(tb);
+        if (!tmp) return OPH_ERR_OOM;
+        OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dp, E, 0, 64, s));
+        k_rips_rank<<<grid_of(ctx, E), 256, 0, s>>>(dk.Current(), dp.Current(), ends, E, n, rank, by_rank,
+                                                    (int *)(total + 1));
+        k_rips_run_count<<<egrid, 256, 0, s>>>(adj, rank, n, words, by_rank, E, tcnt);
+    }
     size_t sb2 = 0;
     OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, sb2, tcnt, toff, E + 1, s));
     void *st2 = sc.get(sb2);
     if (!st2) return OPH_ERR_OOM;
     OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(st2, sb2, tcnt, toff, E + 1, s));
     long long T = 0;
+    int tied = 0;
+    OPH_CUDA_TRY(cudaMemcpyAsync(&tied, total + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
     OPH_CUDA_TRY(cudaMemcpyAsync(&T, toff + E, sizeof(long long), cudaMemcpyDeviceToHost, s));
     OPH_CUDA_TRY(cudaStreamSynchronize(s));
+    // (with equally long edges the triangles by last edge add up to the same)
     const int64_t m = n + E + T, nnz = 2 * E + 3 * T;
     if (m >= (1ll << 31)) return OPH_ERR_BAD_INPUT;
     if (m_out) *m_out = m;
     if (nnz_out) *nnz_out = nnz;
-    if (!d_colptr) return OPH_OK;  // sizes only
     if (!d_rows && nnz > 0) return OPH_ERR_BAD_INPUT;
+    if (!tied) {
+        k_rips_write<<<std::max(egrid, 1), 256, 0, s>>>(adj, rank, n, words, by_rank, dk.Current(), E, toff, d_colptr,
+                                                        d_rows, d_value);
+        OPH_CUDA_TRY(cudaGetLastError());
+        OPH_CUDA_TRY(cudaStreamSynchronize(s));
+        return OPH_OK;
+    }
+    // equally long edges: one sort of every simplex
     SKey *k0 = (SKey *)sc.get(sizeof(SKey) * (size_t)m), *k1 = (SKey *)sc.get(sizeof(SKey) * (size_t)m);
     int32_t *vpos = (int32_t *)sc.get(sizeof(int32_t) * (size_t)n);
-    int32_t *epos = (int32_t *)sc.get(sizeof(int32_t) * (size_t)n * n);
-    if (!k0 || !k1 || !vpos || !epos) return OPH_ERR_OOM;
+    if (!k0 || !k1 || !vpos) return OPH_ERR_OOM;
+    OPH_CUDA_TRY(cudaMemsetAsync(tcnt, 0, 8 * e1, s));
+    k_rips_tri_count<<<wgrid, 256, 0, s>>>(adj, n, words, eoff, tcnt);
+    OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(st2, sb2, tcnt, toff, E + 1, s));
     k_rips_keys<<<wgrid, 256, 0, s>>>(adj, D, n, words, eoff, toff, E, k0);
     SKey *sorted = nullptr;
     int rc = sort_and_colptr(ctx, sc, k0, k1, m, d_colptr, d_value, &sorted);
     if (rc) return rc;
-    k_rips_pos<<<grid_of(ctx, m), 256, 0, s>>>(sorted, m, n, vpos, epos);
-    k_rips_rows<<<grid_of(ctx, m), 256, 0, s>>>(sorted, m, n, vpos, epos, d_colptr, d_rows);
+    k_rips_pos<<<grid_of(ctx, m), 256, 0, s>>>(sorted, m, n, vpos, rank);
+    k_rips_rows<<<grid_of(ctx, m), 256, 0, s>>>(sorted, m, n, vpos, rank, d_colptr, d_rows);
     OPH_CUDA_TRY(cudaGetLastError());
     OPH_CUDA_TRY(cudaStreamSynchronize(s));
     return OPH_OK;
@@ -431,15 +648,24 @@ __attribute__((visibility("default"))) int oph_lower_star_device(oph_context *ct
     OPH_CUDA_TRY(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
     Scratch sc(s);
-    SKey *k0 = (SKey *)sc.get(sizeof(SKey) * (size_t)m), *k1 = (SKey *)sc.get(sizeof(SKey) * (size_t)m);
+    sc.keep(ctx, S_GEN, 16 * (size_t)m + 4 * (size_t)(V + E) + 8 * (size_t)(m + 1) + (4 << 20));
+    unsigned *key[2] = {(unsigned *)sc.get(4 * (size_t)m), (unsigned *)sc.get(4 * (size_t)m)};
+    unsigned *place[2] = {(unsigned *)sc.get(4 * (size_t)m), (unsigned *)sc.get(4 * (size_t)m)};
     int32_t *pos = (int32_t *)sc.get(sizeof(int32_t) * (size_t)(V + E));
-    if (!k0 || !k1 || !pos) return OPH_ERR_OOM;
-    k_ls_keys<<<grid_of(ctx, m), 256, 0, s>>>(d_image, h, w, k0);
-    SKey *sorted = nullptr;
-    int rc = sort_and_colptr(ctx, sc, k0, k1, m, d_colptr, d_value, &sorted);
-    if (rc) return rc;
-    k_ls_pos<<<grid_of(ctx, m), 256, 0, s>>>(sorted, m, h, w, pos);
-    k_ls_rows<<<grid_of(ctx, m), 256, 0, s>>>(sorted, m, h, w, pos, d_colptr, d_rows);
+    int64_t *cnt = (int64_t *)sc.get(sizeof(int64_t) * (size_t)(m + 1));
+    if (!key[0] || !key[1] || !place[0] || !place[1] || !pos || !cnt) return OPH_ERR_OOM;
+    k_ls_keys<<<grid_of(ctx, m), 256, 0, s>>>(d_image, h, w, m, key[0], place[0]);
+    cub::DoubleBuffer<unsigned> dk(key[0], key[1]), dp(place[0], place[1]);
+    size_t tb = 0, sb = 0;
+    OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dp, m, 0, 32, s));
+    OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, sb, cnt, d_colptr, m + 1, s));
+    void *tmp = sc.get(tb), *st = sc.get(sb);
+    if (!tmp || !st) return OPH_ERR_OOM;
+    OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dp, m, 0, 32, s));
+    k_ls_pos<<<grid_of(ctx, m), 256, 0, s>>>(dk.Current(), dp.Current(), m, V, V + E, pos, cnt, d_value);
+    OPH_CUDA_TRY(cudaMemsetAsync(cnt + m, 0, sizeof(int64_t), s));
+    OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(st, sb, cnt, d_colptr, m + 1, s));
+    k_ls_rows<<<grid_of(ctx, m), 256, 0, s>>>(dp.Current(), m, h, w, V, pos, d_colptr, d_rows);
     OPH_CUDA_TRY(cudaGetLastError());
     OPH_CUDA_TRY(cudaStreamSynchronize(s));
     return OPH_OK;

@@ -192,7 +192,7 @@ struct Context {
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[8] = {};
-    DevBuf bufs[48];  // indexed by Slot
+    DevBuf bufs[56];  // indexed by Slot
     DevStatus *h_status = nullptr;  // pinned mirrors (two)
     int max_sweeps = 0;             // 0 = default
     int64_t initial_pool_bytes = 0; // 0 = default
@@ -226,7 +226,7 @@ struct Context {
 enum Slot {
     S_STATUS, S_COLPTR, S_ROWS, S_LOW, S_CLASSES, S_CLEAR, S_DIM, S_FIRST, S_LEFT, S_BETA, S_WORK, S_WIDE, S_SEG,
     S_ROWPIV, S_AGG, S_POOL, S_POOL2, S_ESS, S_ARGLOW, S_COO_R, S_COO_C, S_LOWTRUE, S_TRACK, S_INSTOFF, S_TMP,
-    S_ULIST, S_KAGG, S_ESSHAT, S_SLIST, S_DGRADE, S_DCOLPTR, S_DSORT, S_DTEMP, S_DLOW, S_BITMAP, S_CHECK, S_IASC, S_IBUCKET, S_IOPEN, S_RANGES, S_SEQNS, S_PRECLEAR, S_C2_TAB, S_C2_WORK, S_C2_MODE, S_C2_CELLS, S_NSLOTS
+    S_ULIST, S_KAGG, S_ESSHAT, S_SLIST, S_DGRADE, S_DCOLPTR, S_DSORT, S_DTEMP, S_DLOW, S_BITMAP, S_CHECK, S_IASC, S_IBUCKET, S_IOPEN, S_RANGES, S_SEQNS, S_PRECLEAR, S_C2_TAB, S_C2_WORK, S_C2_MODE, S_C2_CELLS, S_GEN, S_NSLOTS
 };
 
 }  // namespace oph

@@ -72,3 +72,28 @@ def test_generator_input_errors(cuda_lib):
         with pytest.raises(OphError):
             ctx.rips_device(torch.zeros(3, dtype=torch.float64, device="cuda").data_ptr(), 1, 3, float("nan"),
                             lambda m, nnz: (0, 0, 0))
+
+
+@pytest.mark.parametrize("n,thr", [(31, np.inf), (33, 0.7), (65, 0.9), (1030, 0.09), (1500, 0.06)])
+def test_rips_word_edges_equal_host(cuda_lib, n, thr):
+    """Vertex counts around whole words, and sparse complexes on more than 32
+    words of vertices."""
+    pts = cx.points_cube(n, n)
+    assert_same(cx.rips_device(pts, thr), cx.rips(pts, thr))
+
+
+def test_rips_equal_lengths(cuda_lib):
+    """A grid: many equally long edges; two equal lengths among all others."""
+    g = np.stack(np.meshgrid(*[np.arange(3.0)] * 3), -1).reshape(-1, 3)
+    for thr in (1.0, 1.5, np.inf):
+        assert_same(cx.rips_device(g, thr), cx.rips(g, thr))
+    pts = np.concatenate([cx.points_cube(20, 3), [[5.0, 0, 0], [5.0, 1, 0], [5.0, 0, 1]]])
+    assert_same(cx.rips_device(pts), cx.rips(pts))
+
+
+@pytest.mark.parametrize("h,w", [(2, 7), (9, 2), (3, 3), (97, 203)])
+def test_lower_star_odd_sides_equal_host(cuda_lib, h, w):
+    img = cx.image_smoothed(h, w, h * w)
+    img[h // 2:, w // 2:] *= -1
+    img[0, 0], img[1, 1], img[0, 1] = 0.0, -0.0, 0.0
+    assert_same(cx.lower_star_device(img), cx.lower_star(img))
