@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
+#include <mutex>
 
 #include "oph_host.h"
 
@@ -89,7 +90,8 @@ constexpr int C2_MAX_ROUNDS = 512;
 constexpr unsigned long long C2_FIRST_ROUND = 0xffffffffull << 32;  // the round in a key's upper half, counting down
 constexpr int C2_MAX_NV = 8192;                   // vertices of an instance the dense form takes
 constexpr int RS_WAVE = 32;                       // residual columns: pivots added at a time,
-constexpr int RS_LIST = 16384;                    //   edges a column under reduction may be the sum of
+// edges a column under reduction may be the sum of (2,700 on the torus, 600 on 120 points)
+__host__ __device__ constexpr int rs_list(int threads) { return threads >= 1024 ? 16384 : 4096; }
 constexpr int RS_FLAG = 1 << 30;
 
 struct C2Args {
@@ -132,7 +134,7 @@ struct C2Args {
     unsigned long long *sum;
     int32_t *arena;
     long long arena_cap;
-    int32_t *lists;           // per CTA: RS_LIST edges
+    int32_t *lists;           // per CTA: rs_list() edges
     // whole instances: what the tables hold (edges, vertices, table entries, run words)
     long long cap_e, cap_v, cap_c, cap_r;
     long long nnz;            //   and the entries rows[] holds (-1: colptr[m], one matrix)
@@ -1174,7 +1176,7 @@ template <bool RUNS, int THREADS, int WORDS>
 __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
     if (a.st->bad || (RUNS && (a.st->unsorted || a.st->refused || a.st->no_room))) return;
     extern __shared__ __align__(16) uint32_t bits[];  // WORDS
-    constexpr int NW = THREADS / 32;
+    constexpr int NW = THREADS / 32, RS_LIST = rs_list(THREADS);
     __shared__ int s_low[NW], s_cnt[NW], s_wave[RS_WAVE];
     __shared__ int s_i, s_later, s_act, s_other;
     __shared__ unsigned long long s_sum;
@@ -1765,10 +1767,15 @@ static int c2_run_graph(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t 
     if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
     int max_rounds = C2_MAX_ROUNDS;
     void *params[] = {&a, &max_rounds};
+    // one such grid at a time on a device: its blocks wait for one another,
+    // and another thread's context may have half the device's blocks
+    static std::mutex alone[64];
+    std::unique_lock<std::mutex> turn(alone[ctx->device & 63]);
     OPH_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_c2_graph, dim3(gg), dim3(C2_THREADS), params, 0, s));
     ctx->launches += 3;
     cudaEventRecord(ctx->ev[1], s);
     int rc = c2_read_status(ctx, a, hs);
+    turn.unlock();
     *done = !rc && !hs->bad && !hs->crowded && !hs->unfinished;
     return rc;
 }
@@ -1806,7 +1813,7 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     if (gr == 0) return OPH_OK;
     gr = (int)std::min<int64_t>(ne, gr);
     const int nv = hs->nv;
-    a.arena_cap = (1 << 22) + 16 * ne;
+    a.arena_cap = (1 << 20) + 16 * ne;
     size_t head = 0;
     for (char *p = nullptr;;) {
         Carve c{p};
@@ -1818,7 +1825,7 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
         a.res = c.take<int32_t>(ne);
         a.sum = c.take<unsigned long long>(ne);
         a.arena = c.take<int32_t>(a.arena_cap);
-        a.lists = c.take<int32_t>((size_t)gr * RS_LIST);
+        a.lists = c.take<int32_t>((size_t)gr * rs_list(small ? RS_SMALL : RS_LARGE));
         if (p) break;
         p = (char *)ctx_alloc(ctx, S_C2_MODE, c.off);
         if (!p) return OPH_OK;
@@ -1920,7 +1927,7 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
             a.owned = c.take<uint32_t>(nwords);
             a.fixed = c.take<uint32_t>(nwords);
             a.arena = c.take<int32_t>(a.arena_cap);
-            a.lists = c.take<int32_t>((size_t)gr * RS_LIST);
+            a.lists = c.take<int32_t>((size_t)gr * rs_list(RS_SMALL));
             if (p) break;
             p = (char *)ctx_alloc(ctx, S_C2_MODE, c.off);
             if (!p) return OPH_OK;

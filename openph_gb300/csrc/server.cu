@@ -1,8 +1,15 @@
 // Reduction server with continuous batching.
 //
-// Requests (boundary matrices) are queued by oph_server_submit and reduced by
-// one worker thread that owns a CUDA stream and a fixed device arena (the
-// HBM budget).  All active requests live in ONE block-diagonal column space:
+// Requests (boundary matrices) are queued by oph_server_submit.  Simplicial
+// complexes of dimension <= 2 (complex2.cu) need no column store and no
+// sweeps: a few lanes, a thread and a stream each, reduce them as they come,
+// beside one another and beside the sweeps.  A sweep of every active request
+// costs a dozen kernels and a round trip to the host, and such a request took
+// 5 to 58 of them; its own kernels take 50 to 400 us.  Whatever a lane cannot
+// take, for its form or for want of room, goes on to the sweeps:
+//
+// One worker thread owns a CUDA stream and a fixed device arena (the
+// HBM budget).  All its active requests live in ONE block-diagonal column space:
 // request r holds columns [c0, c0 + m) and its rows are shifted by c0, so one
 // pms sweep (pms.cu: Phase I + the Phase II tiers) advances every active
 // request at once.  Between sweeps the worker
@@ -36,6 +43,7 @@
 // columns never add into each other, and the lows of a reduced matrix are
 // unique.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -129,6 +137,7 @@ struct Request {
     int64_t c0 = -1, reg = -1, reg_ints = 0;
     int64_t ring_off = -1;  // low then ess in the pinned result ring (ints), or -1
     bool listed = false;    // in the Phase I list: its sweeps have begun
+    bool in_lane = false;   // queued for a lane, or one is at work on it
 };
 
 // ------------------------------------------------------------------ kernels
@@ -346,8 +355,19 @@ __global__ void k_srv_sweep_reset(DevStatus *st) {
 // the next sweep instead of holding every active request's sweep.
 constexpr int SERVE_CHAIN_CAP = 128;
 
+// Lanes: enough that their kernels, which are small and wait on memory, fill
+// the device beside one another.  Their buffers come out of the share of the
+// budget that the arena leaves free (a sixteenth, half of it for them).
+constexpr int SERVE_LANES = 4;
+
 struct Server {
     Context *ctx = nullptr;  // owns the stream and the device buffers
+    std::vector<std::thread> lanes;
+    std::vector<Context *> lane_ctx;
+    std::deque<Request *> direct;       // requests for the lanes
+    int in_lanes = 0;                   // of them and in a lane
+    std::condition_variable cv_lane;
+    cudaMemPool_t mem = nullptr;        // submitted matrices (kept between requests, up to the rest of that share)
     cudaStream_t sub_stream = nullptr;  // submissions: copy, check, grade
     cudaStream_t adm_stream = nullptr;  // admissions overlapping a sweep
     cudaEvent_t adm_done = nullptr;     //   and their completion
@@ -380,7 +400,8 @@ struct Server {
     bool stop = false;
     int64_t next_ticket = 1;
     // statistics
-    int64_t completed = 0, sweeps = 0, admitted = 0, regrows = 0, dual_admitted = 0;
+    int64_t completed = 0, sweeps = 0, admitted = 0, regrows = 0;
+    std::atomic<int64_t> dual_admitted{0};  // counted by the worker and the lanes
     int error = OPH_OK;
 
     int64_t packed_ints(int64_t m, int64_t nnz) const { return 8 * (m + 1) + 4 * ((nnz + 3) / 4) + 64; }
@@ -624,11 +645,125 @@ struct Server {
         std::lock_guard<std::mutex> lk(mu);
         error = rc;
         for (auto &kv : all)
-            if (!kv.second->done) {
+            if (!kv.second->done && !kv.second->in_lane) {  // the lanes finish or fail theirs
                 kv.second->status = rc;
                 kv.second->done = true;
             }
         cv_done.notify_all();
+    }
+
+    // The matrix the automatic rule chooses for the sweeps, with what a
+    // request split by block keeps; on stream `s`, synchronous.
+    int grade(Request *r, cudaStream_t s) {
+        int choice = DUAL_CHOICE_D;
+        bool bad_g = false;
+        const int64_t *cp = static_cast<const int64_t *>(r->d_buf);
+        const int32_t *rw = reinterpret_cast<const int32_t *>(cp + r->m + 1);
+        void *gtmp = nullptr;
+        int32_t *mapped = nullptr;
+        if (r->m >= DUAL_MIN_M &&
+            cudaMallocFromPoolAsync(&gtmp, dual_grade_tmp_bytes(r->m), mem, s) == cudaSuccess) {
+            if (dual_grade(s, ctx->sm_count, cp, rw, r->m, r->nnz, OPH_DUAL_AUTO, gtmp, &choice, &bad_g, nullptr) !=
+                    OPH_OK ||
+                bad_g)
+                choice = DUAL_CHOICE_D;
+            // a split request keeps its grading, and room for its parts' lows
+            if (choice == DUAL_CHOICE_SPLIT &&
+                cudaMallocFromPoolAsync((void **)&mapped, sizeof(int32_t) * 3 * r->m, mem, s) != cudaSuccess) {
+                cudaGetLastError();
+                choice = DUAL_CHOICE_D;
+            }
+            if (choice != DUAL_CHOICE_SPLIT) {
+                cudaFreeAsync(gtmp, s);
+                gtmp = nullptr;
+            }
+            // the worker uses both on its own streams
+            if (cudaStreamSynchronize(s) != cudaSuccess) {
+                if (gtmp) cudaFreeAsync(gtmp, s);
+                if (mapped) cudaFreeAsync(mapped, s);
+                return OPH_ERR_CUDA;
+            }
+        } else {
+            cudaGetLastError();
+        }
+        r->dual = choice != DUAL_CHOICE_D;
+        r->split = choice == DUAL_CHOICE_SPLIT;
+        r->parts_left = r->split ? 2 : 0;
+        r->d_grade = gtmp;
+        r->d_mapped = mapped;
+        return OPH_OK;
+    }
+
+    // A lane's reduction of one request: OPH_OK with *taken, its results on
+    // their way to the host, or not taken.
+    int reduce_in_lane(Context *c, Request *r, oph_info *info, bool *taken) {
+        *taken = false;
+        int32_t *out = (int32_t *)ctx_alloc(c, S_ESS, sizeof(int32_t) * 2 * r->m);
+        if (!out) return OPH_OK;
+        C2Job job;
+        job.m = r->m;
+        job.colptr = static_cast<const int64_t *>(r->d_buf);
+        job.rows = reinterpret_cast<const int32_t *>(job.colptr + r->m + 1);
+        job.want_nnz = r->nnz;
+        job.low = out;
+        job.ess = out + r->m;
+        int rc = reduce_complex2(c, job, info, taken);
+        if (rc || !*taken) return rc;
+        if (h_ring) {
+            std::lock_guard<std::mutex> lk(mu);
+            r->ring_off = ring.alloc(2 * r->m, 16);
+        }
+        int32_t *dst = r->ring_off >= 0 ? h_ring + r->ring_off : nullptr;
+        if (!dst) {
+            r->low.resize(r->m);
+            r->ess.resize(r->m);
+        }
+        cudaMemcpyAsync(dst ? dst : r->low.data(), out, sizeof(int32_t) * r->m, cudaMemcpyDeviceToHost, c->stream);
+        cudaMemcpyAsync(dst ? dst + r->m : r->ess.data(), out + r->m, sizeof(int32_t) * r->m, cudaMemcpyDeviceToHost,
+                        c->stream);
+        cudaFreeAsync(r->d_buf, c->stream);
+        r->d_buf = nullptr;
+        return cudaStreamSynchronize(c->stream) == cudaSuccess ? OPH_OK : OPH_ERR_CUDA;
+    }
+
+    void run_lane(Context *c) {
+        cudaSetDevice(ctx->device);
+        for (;;) {
+            Request *r = nullptr;
+            {
+                std::unique_lock<std::mutex> lk(mu);
+                cv_lane.wait(lk, [&] { return stop || !direct.empty(); });
+                if (direct.empty()) return;
+                r = direct.front();
+                direct.pop_front();
+                r->t_admit = now_ms();
+            }
+            oph_info info{};
+            bool taken = false;
+            int rc = reduce_in_lane(c, r, &info, &taken);
+            if (rc == OPH_OK && !taken) rc = grade(r, c->stream);
+            {
+                std::lock_guard<std::mutex> lk(mu);
+                in_lanes--;
+                r->in_lane = false;
+                if (error && !taken) rc = error;  // the worker is gone
+                if (rc == OPH_OK && taken) {
+                    r->sweeps = info.sweeps;
+                    r->t_done = now_ms();
+                    r->done = true;
+                    completed++;
+                    dual_admitted += info.dual != 0;
+                } else if (rc == OPH_OK) {
+                    r->t_admit = 0;  // admitted by the worker
+                    pending.push_back(r);
+                } else {
+                    r->status = rc;
+                    r->done = true;
+                }
+            }
+            cv_done.notify_all();
+            cv_work.notify_one();
+        }
     }
 
     // Admits queued requests, first come first served, on `s` while they
@@ -639,7 +774,7 @@ struct Server {
             Request *r = nullptr;
             {
                 std::unique_lock<std::mutex> lk(mu);
-                if (wait_for_work && active == 0) cv_work.wait(lk, [&] { return stop || !pending.empty(); });
+                if (wait_for_work && active == 0) cv_work.wait(lk, [&] { return (stop && in_lanes == 0) || !pending.empty(); });
                 if (pending.empty()) break;
                 r = pending.front();
             }
@@ -680,12 +815,12 @@ struct Server {
                     std::lock_guard<std::mutex> lk(mu);
                     for (auto &rc : retired_cols) cols.release(rc.first, rc.second);
                     retired_cols.clear();
-                    if (stop && pending.empty()) return;
+                    if (stop && in_lanes == 0 && pending.empty()) return;
                 }
                 admit_pending(s, active, true);
                 {
                     std::lock_guard<std::mutex> lk(mu);
-                    if (stop && pending.empty() && active == 0) return;
+                    if (stop && in_lanes == 0 && pending.empty() && active == 0) return;
                 }
                 if (active == 0) {
                     if (!pending.empty()) {
@@ -881,6 +1016,13 @@ __attribute__((visibility("default"))) int oph_server_create(int device, int64_t
     a.cluster_tier = ok && sv->g.g4 > 0;
     // no sweep waits on one long chain of the bitmap tiers
     a.chain_cap = getenv("OPH_SERVE_CHAIN_CAP") ? atoi(getenv("OPH_SERVE_CHAIN_CAP")) : SERVE_CHAIN_CAP;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    unsigned long long keep = (unsigned long long)budget_bytes / 32;
+    if (ok) ok = cudaMemPoolCreate(&sv->mem, &props) == cudaSuccess &&
+                 cudaMemPoolSetAttribute(sv->mem, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess;
     if (ok) ok = cudaStreamCreateWithFlags(&sv->sub_stream, cudaStreamNonBlocking) == cudaSuccess;
     if (ok) ok = cudaStreamCreateWithFlags(&sv->adm_stream, cudaStreamNonBlocking) == cudaSuccess;
     if (ok) ok = cudaEventCreateWithFlags(&sv->adm_done, cudaEventDisableTiming) == cudaSuccess;
@@ -892,6 +1034,7 @@ __attribute__((visibility("default"))) int oph_server_create(int device, int64_t
         if (sv->sub_stream) cudaStreamDestroy(sv->sub_stream);
         if (sv->adm_stream) cudaStreamDestroy(sv->adm_stream);
         if (sv->adm_done) cudaEventDestroy(sv->adm_done);
+        if (sv->mem) cudaMemPoolDestroy(sv->mem);
         oph_context_destroy(raw);
         delete sv;
         return OPH_ERR_OOM;
@@ -913,6 +1056,7 @@ __attribute__((visibility("default"))) int oph_server_create(int device, int64_t
     init.pool_size = (unsigned long long)sv->pool_ints;
     cudaMemcpyAsync(a.st, &init, sizeof(init), cudaMemcpyHostToDevice, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) {
+        cudaMemPoolDestroy(sv->mem);
         oph_context_destroy(raw);
         delete sv;
         return OPH_ERR_CUDA;
@@ -921,6 +1065,15 @@ __attribute__((visibility("default"))) int oph_server_create(int device, int64_t
     sv->pool.init(sv->pool_ints);
     sv->slots.assign(max_active, nullptr);
     sv->worker = std::thread([sv] { sv->run(); });
+    // the chain cap is the sweeps': who sets it means them
+    if (!getenv("OPH_SERVE_CHAIN_CAP"))
+        for (int q = 0; q < SERVE_LANES; q++) {
+            oph_context *c = nullptr;
+            if (oph_context_create(device, &c) != OPH_OK) break;  // the sweeps take every request
+            c->budget = budget_bytes / 32 / SERVE_LANES;
+            sv->lane_ctx.push_back(reinterpret_cast<Context *>(c));
+            sv->lanes.emplace_back([sv, c] { sv->run_lane(reinterpret_cast<Context *>(c)); });
+        }
     *out = sv;
     return OPH_OK;
 }
@@ -930,9 +1083,8 @@ __attribute__((visibility("default"))) int oph_server_create(int device, int64_t
 namespace {
 
 // The server's own device copy of a submitted CSC (from host or device
-// memory; the caller may free its buffers on return), its structural checks
-// and its grading on the device (the matrix a single-matrix pms reduction
-// would choose), then the request queued.  The submitting thread does no
+// memory; the caller may free its buffers on return) and its structural
+// checks on the device, then the request queued.  The submitting thread does no
 // O(nnz) host work beyond the copy; the work runs on the submission stream,
 // beside the worker's sweeps.
 int submit_copy(oph_server *sv, int64_t m, int64_t nnz, const int64_t *colptr, const int32_t *rows,
@@ -944,7 +1096,7 @@ int submit_copy(oph_server *sv, int64_t m, int64_t nnz, const int64_t *colptr, c
     cudaStream_t s = sv->sub_stream;
     const size_t bytes = sizeof(int64_t) * (m + 1) + sizeof(int32_t) * nnz + sizeof(int);
     void *buf = nullptr;
-    if (cudaMallocAsync(&buf, bytes, s) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(&buf, bytes, sv->mem, s) != cudaSuccess) {
         cudaGetLastError();
         return OPH_ERR_OOM;
     }
@@ -963,59 +1115,41 @@ int submit_copy(oph_server *sv, int64_t m, int64_t nnz, const int64_t *colptr, c
         cudaStreamSynchronize(s);
         return e != cudaSuccess ? OPH_ERR_CUDA : OPH_ERR_BAD_INPUT;
     }
-    int choice = DUAL_CHOICE_D;
-    bool bad_g = false;
-    void *gtmp = nullptr;
-    int32_t *mapped = nullptr;
-    if (m >= DUAL_MIN_M && cudaMallocAsync(&gtmp, dual_grade_tmp_bytes(m), s) == cudaSuccess) {
-        if (dual_grade(s, sv->ctx->sm_count, cp, rw, m, nnz, OPH_DUAL_AUTO, gtmp, &choice, &bad_g, nullptr) != OPH_OK ||
-            bad_g)
-            choice = DUAL_CHOICE_D;
-        // a split request keeps its grading, and room for its parts' lows
-        if (choice == DUAL_CHOICE_SPLIT && cudaMallocAsync(&mapped, sizeof(int32_t) * 3 * m, s) != cudaSuccess) {
-            cudaGetLastError();
-            choice = DUAL_CHOICE_D;
-        }
-        if (choice != DUAL_CHOICE_SPLIT) {
-            cudaFreeAsync(gtmp, s);
-            gtmp = nullptr;
-        }
-        // the worker uses both on its own streams
-        if (cudaStreamSynchronize(s) != cudaSuccess) {
-            cudaFreeAsync(buf, s);
-            if (gtmp) cudaFreeAsync(gtmp, s);
-            if (mapped) cudaFreeAsync(mapped, s);
-            cudaStreamSynchronize(s);
-            return OPH_ERR_CUDA;
-        }
-    } else {
-        cudaGetLastError();
-    }
     Request *r = new Request();
     r->m = m;
     r->nnz = nnz;
     r->d_buf = buf;
-    r->dual = choice != DUAL_CHOICE_D;
-    r->split = choice == DUAL_CHOICE_SPLIT;
-    r->parts_left = r->split ? 2 : 0;
-    r->d_grade = gtmp;
-    r->d_mapped = mapped;
     r->t_submit = now_ms();
+    const bool lane = m > 0 && !sv->lanes.empty();
+    if (!lane) {
+        const int rc = sv->grade(r, s);
+        if (rc) {
+            cudaFreeAsync(buf, s);
+            cudaStreamSynchronize(s);
+            delete r;
+            return rc;
+        }
+    }
     {
         std::lock_guard<std::mutex> lk(sv->mu);
         if (sv->error) {
-            cudaFreeAsync(buf, s);
-            if (gtmp) cudaFreeAsync(gtmp, s);
-            if (mapped) cudaFreeAsync(mapped, s);
+            for (void *p : {r->d_buf, r->d_grade, static_cast<void *>(r->d_mapped)})
+                if (p) cudaFreeAsync(p, s);
             delete r;
             return sv->error;
         }
         r->ticket = sv->next_ticket++;
         sv->all[r->ticket] = r;
-        sv->pending.push_back(r);
+        if (lane) {
+            r->in_lane = true;
+            sv->direct.push_back(r);
+            sv->in_lanes++;
+        } else {
+            sv->pending.push_back(r);
+        }
         *ticket = r->ticket;
     }
-    sv->cv_work.notify_one();
+    (lane ? sv->cv_lane : sv->cv_work).notify_one();
     return OPH_OK;
 }
 
@@ -1093,6 +1227,8 @@ __attribute__((visibility("default"))) int oph_server_stats(oph_server *sv, oph_
     int64_t active = 0, pending = 0;
     for (auto *r : sv->slots) active += r != nullptr && (!r->user || r->user->slot < 0);
     for (auto *r : sv->pending) pending += !r->user;
+    pending += (int64_t)sv->direct.size();
+    active += sv->in_lanes - (int64_t)sv->direct.size();
     out->completed = sv->completed;
     out->pending = pending;
     out->active = active;
@@ -1111,9 +1247,12 @@ __attribute__((visibility("default"))) int oph_server_destroy(oph_server *sv) {
         std::lock_guard<std::mutex> lk(sv->mu);
         sv->stop = true;
     }
+    sv->cv_lane.notify_all();
     sv->cv_work.notify_all();
+    for (auto &t : sv->lanes) t.join();  // they finish what is queued for them, or pass it on
     if (sv->worker.joinable()) sv->worker.join();
     cudaSetDevice(sv->ctx->device);
+    for (Context *c : sv->lane_ctx) oph_context_destroy(reinterpret_cast<oph_context *>(c));
     // internal D parts of split requests left by a failure
     for (Request *r : sv->slots)
         if (r && r->user) {
@@ -1137,6 +1276,7 @@ __attribute__((visibility("default"))) int oph_server_destroy(oph_server *sv) {
     if (sv->h_iover) cudaFreeHost(sv->h_iover);
     if (sv->h_rng) cudaFreeHost(sv->h_rng);
     if (sv->h_ring) cudaFreeHost(sv->h_ring);
+    if (sv->mem) cudaMemPoolDestroy(sv->mem);
     oph_context_destroy(reinterpret_cast<oph_context *>(sv->ctx));
     delete sv;
     return OPH_OK;
