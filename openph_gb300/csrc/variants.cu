@@ -1,26 +1,35 @@
 // The standard, twist and row reductions as GPU kernels.
 //
-// These algorithms are sequential by definition (column by column, or row by
-// row), and their results — low, and the ess estimate — follow from that
-// order.  The reference runs them either on the host (standard.cu:1-57,
-// twist.cu:10-87, ph_row.cu:38-121) or as one to five full-grid kernel
-// launches per column/row with a single working thread
+// The reference runs them column by column or row by row, on the host
+// (standard.cu:1-57, twist.cu:10-87, ph_row.cu:38-121) or as one to five
+// full-grid kernel launches per column/row with a single working thread
 // (standard_parallel.cu:1-51, twist_parallel.cu:13-96,
-// ph_row_parallel.cu:20-89).  Here each is ONE persistent launch:
-//   * standard / twist: a single warp walks the columns in the algorithm's
-//     order.  A 32-column window is inspected at once (lows, pivot-table
-//     hits, repeated lows, twist clears landing inside the window) so that
-//     columns needing no addition are retired 32 at a time; a column that
-//     needs additions is reduced by the whole warp with the column kept in
-//     shared memory across its chain of additions.
-//   * row: one CTA walks the rows from the bottom; a warp finds the next row
-//     with two or more columns on it (per-row buckets), and the CTA's 32
-//     warps add the row's pivot into all of that row's other columns in
-//     parallel (mark_neighbours / left_to_right_neighbours,
-//     ph_row_parallel.cu:3-18).
-// Column additions use the same group merge as pms; columns too wide for the
-// shared buffers continue in pool-allocated global buffers.
+// ph_row_parallel.cu:20-89).  Here:
+//   * standard / twist: warps take the columns in the algorithm's order and
+//     reduce them side by side (k_claim), each column by pivots to its left as
+//     the algorithm has it; a column that holds a low which one to its left
+//     comes to as well gives it up and goes on.  The lows of a reduced matrix
+//     are unique, so they are those of the walk, and twist clears, dimension
+//     by dimension, the columns it would.  So is row where only the lows are
+//     asked for.
+//   * standard / twist with trackers, which follow the walk itself, and twist
+//     on matrices whose dimensions do not separate, where the clearing depends
+//     on the order: one launch in which a single warp walks the columns in
+//     the algorithm's order.  A 32-column window is inspected at once (lows,
+//     pivot-table hits, repeated lows, twist clears landing inside the window)
+//     so that columns needing no addition are retired 32 at a time; a column
+//     that needs additions is reduced by the whole warp with the column kept
+//     in shared memory across its chain of additions.
+//   * row with the running essential estimate or trackers: one CTA walks the
+//     rows from the bottom; a warp finds the next row with two or more columns
+//     on it (per-row buckets), and the CTA's 32 warps add the row's pivot into
+//     all of that row's other columns in parallel (mark_neighbours /
+//     left_to_right_neighbours, ph_row_parallel.cu:3-18).
+// Columns too wide for the shared buffers continue in pool-allocated global
+// buffers.
 #include <algorithm>
+#include <climits>
+#include <vector>
 
 #include "oph_host.h"
 
@@ -222,6 +231,403 @@ out:
     }
 }
 
+// ------------------------------------------------- columns side by side
+constexpr int CL_WARPS = 8, CL_THREADS = 32 * CL_WARPS;
+constexpr int CL_CAP = 768;                     // rows of a list that a warp keeps in shared memory
+constexpr int CL_ALONE = 2;                     // additions a column makes one at a time; then 2, 4, ... 32 together
+constexpr int CL_BITS = 3 * CL_CAP;             // words of a warp's bitmap (73,728 rows), at most
+
+// The holder of a low, read and swapped as one 16-byte word: the column (-1: none yet),
+// its segment / 4, and its next two rows down (-1: none), or -2 and its
+// length when it has more than three.
+struct __align__(16) Holder {
+    int col, seg4, b, c;
+};
+// A launch's next column, and how many it gave up.
+struct ClaimCount {
+    unsigned long long next;
+    int failed, pad;
+};
+struct ClaimArgs {
+    int64_t m;
+    int32_t *low;
+    Holder *holder;
+    const int8_t *dim;
+    int64_t *seg;            // a column's segment: what it last published
+    int *pool;
+    DevStatus *st;
+    int want_dim;            // only columns of this dimension (-1: all)
+    int words;               // of a warp's bitmap
+    const int32_t *redo;     // only the columns an earlier launch gave up for want of room, or nullptr
+    int64_t n;               // columns to look at: of redo, or m
+    int32_t *failed;         // columns this launch gives up
+    ClaimCount *count;       // this launch's
+    const ClaimCount *above; // of the dimensions before it, `n_above` of them: nothing to do while one has failed
+    int n_above;
+};
+using Tile32 = cg::thread_block_tile<32>;
+
+__device__ __forceinline__ Holder holder_load(const Holder *h) {
+    long long v0, v1;
+    asm volatile("{ .reg .b128 t; ld.acquire.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(v0), "=l"(v1)
+                 : "l"(h)
+                 : "memory");
+    return Holder{(int)v0, (int)(v0 >> 32), (int)v1, (int)(v1 >> 32)};
+}
+__device__ __forceinline__ Holder holder_of(const Tile32 &tile, const Holder &h, int lane) {
+    return Holder{tile.shfl(h.col, lane), tile.shfl(h.seg4, lane), tile.shfl(h.b, lane), tile.shfl(h.c, lane)};
+}
+__device__ __forceinline__ int holder_rows(const Holder &h) { return h.b == -2 ? h.c : 1 + (h.b >= 0) + (h.c >= 0); }
+__device__ __forceinline__ long long pack2(int lo, int hi) { return (long long)(unsigned)lo | ((long long)hi << 32); }
+// True when `was` stood there and `now` does.
+__device__ __forceinline__ bool holder_swap(const Tile32 &tile, Holder *h, const Holder &was, const Holder &now) {
+    tile.sync();
+    bool ok = false;
+    if (tile.thread_rank() == 0) {
+        const long long w0 = pack2(was.col, was.seg4), w1 = pack2(was.b, was.c);
+        long long g0, g1;
+        asm volatile(
+            "{ .reg .b128 t, w, n; mov.b128 w, {%3, %4}; mov.b128 n, {%5, %6};"
+            " atom.acq_rel.gpu.global.cas.b128 t, [%2], w, n; mov.b128 {%0, %1}, t; }"
+            : "=l"(g0), "=l"(g1)
+            : "l"(h), "l"(w0), "l"(w1), "l"(pack2(now.col, now.seg4)), "l"(pack2(now.b, now.c))
+            : "memory");
+        ok = g0 == w0 && g1 == w1;
+    }
+    ok = tile.shfl((int)ok, 0);
+    tile.sync();
+    return ok;
+}
+
+// A warp's column as a bitmap of all rows: an addition flips bits, the next
+// low is found 1,024 rows at a time.
+struct BitColumn {
+    static constexpr bool WAVES = true;
+    unsigned *bits;
+    int *pick;
+    int n, low, bottom, top;  // rows, the highest, words that may hold bits
+    __device__ void init(const Tile32 &tile, const ClaimArgs &a, int *own, int *own_pick) {
+        bits = reinterpret_cast<unsigned *>(own);
+        pick = own_pick;
+        for (int q = tile.thread_rank(); q < a.words; q += 32) bits[q] = 0;
+        tile.sync();
+    }
+    __device__ void start() { n = 0, low = -1, bottom = 1 << 30, top = -1; }
+    __device__ void end(const Tile32 &tile) {
+        for (int q = bottom + (int)tile.thread_rank(); q <= top; q += 32) bits[q] = 0;
+        tile.sync();
+    }
+    // rows P (np >= 1 ascending, the first 32 also held one a lane in pv)
+    __device__ bool add(const Tile32 &tile, const ClaimArgs &, int pv, const int *P, int np) {
+        const int lane = tile.thread_rank();
+        int both = 0, last = 0;
+        for (int base = 0; base < np; base += 32) {
+            const int q = base + lane;
+            bool was = false;
+            if (q < np) {
+                last = base ? P[q] : pv;
+                was = atomicXor(&bits[last >> 5], 1u << (last & 31)) >> (last & 31) & 1u;
+            }
+            both += __popc(tile.ballot(was));
+        }
+        n += np - 2 * both;
+        bottom = min(bottom, tile.shfl(pv, 0) >> 5);
+        const int high = tile.shfl(last, (np - 1) & 31);
+        top = max(top, high >> 5);
+        tile.sync();
+        find_low(tile, max(low, high) >> 5);
+        return true;
+    }
+    // the highest row, in word w or below
+    __device__ void find_low(const Tile32 &tile, int w) {
+        const int lane = tile.thread_rank();
+        low = -1;
+        for (; w >= bottom; w -= 32) {
+            const unsigned x = w - lane >= bottom ? bits[w - lane] : 0u;
+            const unsigned b = tile.ballot(x != 0);
+            if (b) {
+                const int f = __ffs(b) - 1;
+                low = (w - f) * 32 + 31 - __clz(tile.shfl(x, f));
+                break;
+            }
+        }
+    }
+    // Of its highest rows, a lane each (up to `most`, of 1,024 places): -1
+    // beyond them.  Lane 0 has the low.
+    __device__ int rows_at(const Tile32 &tile, int most) const {
+        const int lane = tile.thread_rank(), w = (low >> 5) - lane;
+        unsigned x = w >= bottom ? bits[w] : 0u;
+        int upto = __popc(x), at = upto;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = tile.shfl_up(upto, o);
+            if (lane >= o) upto += u;
+        }
+        at = upto - at;
+        for (; x && at < most; at++) {
+            const int b = 31 - __clz(x);
+            pick[at] = w * 32 + b;
+            x ^= 1u << b;
+        }
+        tile.sync();
+        const int r = lane < min(most, tile.shfl(upto, 31)) ? pick[lane] : -1;
+        tile.sync();
+        return r;
+    }
+    // Add the columns h of the lanes that `have` one, whose low is row r; all
+    // at once, which no order of additions matters to.
+    __device__ void add_all(const Tile32 &tile, const ClaimArgs &a, const Holder &h, int r, bool have) {
+        const int lane = tile.thread_rank(), np = have ? holder_rows(h) : 0;
+        int both = 0, lowest = 1 << 30;
+        auto flip = [&](int row) {
+            both += atomicXor(&bits[row >> 5], 1u << (row & 31)) >> (row & 31) & 1u;
+            lowest = min(lowest, row);
+        };
+        if (np >= 1 && np <= 3) {
+            flip(r);
+            if (np > 1) flip(h.b);
+            if (np > 2) flip(h.c);
+        }
+        for (unsigned todo = tile.ballot(np > 3); todo;) {
+            // four at a time, their rows loaded together
+            const int *P[4];
+            int pn[4], v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int f = todo ? __ffs(todo) - 1 : 0;
+                pn[u] = todo ? tile.shfl(np, f) : 0;
+                P[u] = a.pool + ((long long)(unsigned)tile.shfl(h.seg4, f) << 2) + SEG_HDR;
+                v[u] = lane < pn[u] ? P[u][lane] : 0;
+                todo &= todo - 1;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (lane < pn[u]) flip(v[u]);
+                for (int q = 32 + lane; q < pn[u]; q += 32) flip(P[u][q]);
+            }
+        }
+        n += __reduce_add_sync(0xffffffffu, np - 2 * both);
+        bottom = min(bottom, __reduce_min_sync(0xffffffffu, lowest) >> 5);
+        tile.sync();
+        find_low(tile, low >> 5);
+    }
+    __device__ void write(const Tile32 &tile, int *out) const {
+        const int lane = tile.thread_rank();
+        int at = 0;
+        for (int w = bottom; w <= (low >> 5); w += 32) {
+            unsigned x = w + lane <= (low >> 5) ? bits[w + lane] : 0u;
+            if (!tile.any(x != 0)) continue;
+            int k = __popc(x), upto = k;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = tile.shfl_up(upto, o);
+                if (lane >= o) upto += u;
+            }
+            int *o = out + at + upto - k;
+            for (; x; x &= x - 1) *o++ = (w + lane) * 32 + __ffs(x) - 1;
+            at += tile.shfl(upto, 31);
+        }
+    }
+};
+
+// A warp's column as an ascending list, in its shared buffers while it fits,
+// else in two halves of a pool allocation; for matrices too large for the
+// bitmaps.
+struct ListColumn {
+    static constexpr bool WAVES = false;
+    int *home, *A, *B, *C;  // rows, the next sum, the staged pivot
+    int n, low, cap;
+    __device__ void init(const Tile32 &, const ClaimArgs &, int *own, int *) { home = own; }
+    __device__ void start() {
+        A = home, B = home + CL_CAP, C = home + 2 * CL_CAP;
+        n = 0, low = -1, cap = CL_CAP;
+    }
+    __device__ void end(const Tile32 &) {}
+    __device__ bool add(const Tile32 &tile, const ClaimArgs &a, int pv, const int *P, int np) {
+        const int lane = tile.thread_rank();
+        if (n + np > cap) {
+            const int ncap = round4(2 * (n + np));
+            long long off = 0;
+            if (lane == 0) off = pool_alloc(a.st, 2ll * ncap);
+            off = tile.shfl(off, 0);
+            if (off < 0) return false;
+            int *N = a.pool + off;
+            group_copy<32>(tile, N, A, n);
+            A = N;
+            B = N + ncap;
+            cap = ncap;
+        }
+        if (np <= 4) {
+            n = merge_xor_seg<32>(tile, A, n, pv, np, B);
+        } else if (np <= 32) {
+            n = merge_xor_thr<32>(tile, A, n, pv, np, B);
+        } else {
+            if (np <= CL_CAP) {  // searched in shared memory
+                group_copy<32>(tile, C, P, np);
+                P = C;
+            }
+            n = merge_xor<32>(tile, A, n, P, np, B);
+        }
+        int *t = A;
+        A = B;
+        B = t;
+        low = n ? A[n - 1] : -1;
+        tile.sync();
+        return true;
+    }
+    __device__ void write(const Tile32 &tile, int *out) const { group_copy<32>(tile, out, A, n); }
+};
+
+// standard and twist, a warp per column, the columns taken in order.  A
+// column adds the holder of its low while that is a column to its left
+// (reduce_col_host, kernels_host.cu:62-75).  Else it publishes its rows and
+// claims the low by compare-and-swap; a low held by a column to the right is
+// taken from it, and the warp goes on with that column, which has the taker
+// to add.  Published rows are never written again (a column that changes gets
+// a new segment), so a reader sees some whole column of an index to its left
+// whatever the others do meanwhile.  No warp waits for another: a swap that
+// fails means that another column has taken the low.
+// Bound by the chain of loads of the columns with the most additions, one
+// after the other: the holder (with the rows of a holder of three) is one
+// load, a longer one's rows a second.  Such a column also adds the holders,
+// where they are columns to its left, of the 2, 4, ... 32 rows below its low
+// in one wave.  Additions, and so the counters, vary with who came first.
+// Device time (setup and reading back included), the walk by one warp first:
+// twist on a 64 x 64 image 8.0 ms -> 0.18 (0.31 without waves), standard on
+// 24 points 17-20 ms -> 0.08; 0.52 and 0.10 with sorted lists and holders of
+// one column index.
+template <class Column>
+__global__ void __launch_bounds__(CL_THREADS) k_claim(ClaimArgs a) {
+    extern __shared__ __align__(16) int smem[];  // a.words a warp
+    const Tile32 tile = cg::tiled_partition<32>(cg::this_thread_block());
+    const int lane = tile.thread_rank();
+    Column c;
+    __shared__ int s_pick[CL_WARPS][32];
+    for (int d = 0; d < a.n_above; d++)
+        if (a.above[d].failed) return;
+    c.init(tile, a, smem + (size_t)(threadIdx.x >> 5) * a.words, s_pick[threadIdx.x >> 5]);
+    long long adds = 0, slots = 0;
+    for (;;) {
+        long long idx = 0;
+        if (lane == 0) idx = (long long)atomicAdd(&a.count->next, 1ull);
+        idx = tile.shfl(idx, 0);
+        if (idx >= a.n) break;
+        int j = (int)idx;
+        if (a.redo) {
+            j = a.redo[idx];
+        } else {
+            const int d = a.dim[j], l0 = a.low[j];
+            if (a.want_dim >= 0 && d != a.want_dim) continue;
+            if (l0 < 0) continue;  // zero, or cleared
+        }
+        // the column as it was last published: header, then rows
+        long long seg = a.seg[j];
+        const int h = a.pool[seg + lane];
+        int n = tile.shfl(h, 0);
+        const int *R = a.pool + seg + SEG_HDR;
+        auto row = [&](int k) { return n <= 32 - SEG_HDR ? tile.shfl(h, SEG_HDR + max(k, 0)) : R[max(k, 0)]; };
+        int l = row(n - 1), rb = row(n - 2), rc = row(n - 3);
+        if (n < 1) l = -1;
+        bool loaded = false, changed = false, room = true;
+        int wave = 0;  // additions so far, and waves of them
+        c.start();
+        while (l >= 0) {
+            // the low's holder, and in a long chain those of the rows below it
+            int r = lane == 0 ? l : -1;
+            if constexpr (Column::WAVES)
+                if (wave > CL_ALONE) r = c.rows_at(tile, 1 << min(wave - CL_ALONE, 5));
+            Holder mine{-1, 0, 0, 0};
+            if (r >= 0) mine = holder_load(a.holder + r);
+            tile.sync();
+            const Holder p = holder_of(tile, mine, 0);
+            if constexpr (Column::WAVES)
+                if (wave > CL_ALONE && p.col >= 0 && p.col < j) {
+                    const bool have = mine.col >= 0 && mine.col < j;
+                    const int before = c.n;
+                    c.add_all(tile, a, mine, r, have);
+                    changed = true;
+                    wave++;
+                    adds += __popc(tile.ballot(have));
+                    slots += before + c.n + __reduce_add_sync(0xffffffffu, have ? holder_rows(mine) : 0);
+                    l = c.low;
+                    continue;
+                }
+            const bool take = p.col < 0 || p.col > j;
+            if (take) {
+                if (changed) {
+                    n = c.n;
+                    if (lane == 0) seg = pool_alloc(a.st, SEG_HDR + round4(n));
+                    seg = tile.shfl(seg, 0);
+                    if (seg < 0) {
+                        room = false;
+                        break;
+                    }
+                    int *out = a.pool + seg + SEG_HDR;
+                    c.write(tile, out);
+                    if (lane == 0) {
+                        a.pool[seg] = n;
+                        a.pool[seg + 1] = round4(n);
+                        a.seg[j] = seg;
+                    }
+                    tile.sync();
+                    if (n <= 3) {
+                        rb = out[max(n - 2, 0)];
+                        rc = out[max(n - 3, 0)];
+                    }
+                    changed = false;
+                }
+                if (lane == 0) a.low[j] = l;
+                const Holder now = n > 3 ? Holder{j, (int)(seg >> 2), -2, n}
+                                         : Holder{j, (int)(seg >> 2), n > 1 ? rb : -1, n > 2 ? rc : -1};
+                if (!holder_swap(tile, a.holder + l, p, now)) continue;  // look again
+                if (p.col < 0) break;  // done, for all that is known
+            }
+            if (!loaded) {
+                loaded = true;
+                const int v = tile.shfl_down(h, SEG_HDR);
+                if (!c.add(tile, a, n <= 32 - SEG_HDR ? v : lane < n ? R[lane] : 0, R, n)) room = false;
+            }
+            // column j += column p; having taken the low, column p += column j
+            const int np = holder_rows(p);
+            const int *P = a.pool + ((long long)(unsigned)p.seg4 << 2) + SEG_HDR;
+            int pv = 0;
+            if (np > 3) {
+                if (lane < np) pv = P[lane];
+            } else {
+                pv = lane == np - 1 ? l : lane == np - 2 ? p.b : p.c;
+            }
+            if (take) j = p.col;
+            const int before = c.n;
+            if (!room || !c.add(tile, a, pv, P, np)) {
+                room = false;  // column j goes on, from what it last published, when there is more
+                break;
+            }
+            changed = true;
+            wave++;
+            adds++;
+            slots += before + np + c.n;
+            l = c.low;
+        }
+        c.end(tile);
+        if (lane == 0) {
+            if (!room) a.failed[atomicAdd(&a.count->failed, 1)] = j;
+            else if (l < 0) a.low[j] = -1;
+        }
+        tile.sync();
+    }
+    if (lane == 0 && adds) {
+        atomicAdd(&a.st->additions, (unsigned long long)adds);
+        atomicAdd(&a.st->slots, (unsigned long long)slots);
+    }
+}
+
+// twist's clearing after a dimension: the columns whose row is a low.
+__global__ void k_claim_clear(ClaimArgs a) {
+    for (int d = 0; d <= a.n_above; d++)
+        if (a.above[d].failed) return;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < a.m; j += (int64_t)gridDim.x * blockDim.x)
+        if (a.dim[j] == a.want_dim && a.low[j] >= 0) a.low[a.low[j]] = -1;
+}
+
 // Row buckets: every column with a low joins the bucket of that row;
 // pivots[r] = the first column holding low r (ph_row.cu:56-59).
 __global__ void k_row_buckets(SeqArgs a) {
@@ -356,12 +762,27 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_walk(SeqArgs a) {
     }
 }
 
-// out[0] = largest dimension, out[1] = columns of dimension >= 1.
-__global__ void k_dim_stats(const int8_t *dim, int64_t m, int *out) {
+// out[0] = largest dimension, out[1] = columns of dimension >= 1,
+// out[2 + d] and -1 - out[2 + 128 + d] = the smallest and largest dimension of
+// a row in a column of dimension d >= 1.
+__global__ void k_dim_stats(const int8_t *dim, const int64_t *colptr, const int32_t *rows, int64_t m, int *out) {
+    __shared__ int s_lo[128], s_hi[128];
+    for (int q = threadIdx.x; q < 128; q += blockDim.x) s_lo[q] = s_hi[q] = INT_MAX;
+    __syncthreads();
     int mx = -1, cnt = 0;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
-        mx = max(mx, (int)dim[j]);
-        cnt += dim[j] >= 1;
+        const int d = dim[j];
+        mx = max(mx, d);
+        if (d < 1) continue;
+        cnt++;
+        int lo = INT_MAX, hi = INT_MAX;
+        for (int64_t k = colptr[j]; k < colptr[j + 1]; k++) {
+            const int r = dim[rows[k]];
+            lo = min(lo, r);
+            hi = min(hi, -1 - r);
+        }
+        if (lo < s_lo[d]) atomicMin(&s_lo[d], lo);
+        if (hi < s_hi[d]) atomicMin(&s_hi[d], hi);
     }
     for (int o = 16; o > 0; o >>= 1) {
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -371,6 +792,91 @@ __global__ void k_dim_stats(const int8_t *dim, int64_t m, int *out) {
         atomicMax(&out[0], mx);
         atomicAdd(&out[1], cnt);
     }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 128; q += blockDim.x)
+        if (s_lo[q] != INT_MAX) {
+            atomicMin(&out[2 + q], s_lo[q]);
+            atomicMin(&out[2 + 128 + q], s_hi[q]);
+        }
+}
+
+// standard (all columns at once) or twist (dimension top down to 1) by
+// k_claim; the store grown and the given-up columns redone when it runs out.
+template <class Column>
+static int claim_columns_as(Context *ctx, Work &w, int words, int top, bool twist, int *regrows) {
+    cudaStream_t s = ctx->stream;
+    const int64_t m = w.m;
+    static bool attr = false;
+    if (!attr) {
+        OPH_CUDA_TRY(cudaFuncSetAttribute(k_claim<Column>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(int) * CL_WARPS * CL_BITS));
+        attr = true;
+    }
+    const size_t smem = sizeof(int) * CL_WARPS * (size_t)words;
+    ClaimArgs a{};
+    a.m = m; a.low = w.low; a.dim = w.dim; a.pool = w.pool; a.st = w.st; a.seg = w.seg; a.words = words;
+    static_assert(sizeof(Holder) <= sizeof(PivRec), "the holders stand in the pivot records' buffer");
+    a.holder = reinterpret_cast<Holder *>(w.rec);
+    OPH_CUDA_TRY(cudaMemsetAsync(a.holder, 0xff, sizeof(Holder) * (size_t)m, s));
+    const int dims = twist ? top : 1;  // launches: one for all columns, or a dimension each from the top
+    if (dims < 1) return OPH_OK;       // twist leaves dimensions 0 and below as they are
+    const size_t head = (sizeof(ClaimCount) * (size_t)dims + 255) & ~(size_t)255;
+    char *tmp = (char *)ctx_alloc(ctx, S_TMP, head + sizeof(int32_t) * 2 * (size_t)m);
+    if (!tmp) return OPH_ERR_OOM;
+    ClaimCount *count = reinterpret_cast<ClaimCount *>(tmp);
+    int32_t *lists[2] = {reinterpret_cast<int32_t *>(tmp + head), reinterpret_cast<int32_t *>(tmp + head) + m};
+    a.above = count;
+    const int64_t per_sm = std::min<int64_t>(2048 / CL_THREADS, (220 << 10) / (smem + 2048));
+    const int grid = (int)std::min<int64_t>((m + CL_WARPS - 1) / CL_WARPS, ctx->sm_count * per_sm);
+    const int grid_m = (int)std::max<int64_t>(1, std::min<int64_t>((m + 255) / 256, (int64_t)ctx->sm_count * 16));
+    std::vector<ClaimCount> seen(dims);
+    int turn = 0, d = 0, redo = 0;
+    for (;;) {
+        OPH_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(ClaimCount) * (size_t)dims, s));
+        for (int e = d; e < dims; e++) {
+            a.want_dim = twist ? top - e : -1;
+            a.redo = e == d && redo ? lists[turn ^ 1] : nullptr;
+            a.n = a.redo ? redo : m;
+            a.failed = lists[turn];
+            a.count = count + e;
+            a.n_above = e;
+            k_claim<Column><<<grid, CL_THREADS, smem, s>>>(a);
+            ctx->launches++;
+            if (twist) {
+                k_claim_clear<<<grid_m, 256, 0, s>>>(a);
+                ctx->launches++;
+            }
+        }
+        OPH_CUDA_TRY(cudaGetLastError());
+        OPH_CUDA_TRY(cudaMemcpyAsync(seen.data(), count, sizeof(ClaimCount) * (size_t)dims, cudaMemcpyDeviceToHost, s));
+        OPH_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, w.st, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
+        OPH_CUDA_TRY(cudaStreamSynchronize(s));
+        while (d < dims && !seen[d].failed) d++;
+        if (d == dims) return OPH_OK;
+        redo = seen[d].failed;
+        const int rc = grow_pool(ctx, w);
+        if (rc != OPH_OK) return rc;
+        a.pool = w.pool;
+        turn ^= 1;
+        (*regrows)++;
+    }
+}
+
+// Bitmaps where a warp's holds every row, else lists.
+static int claim_columns(Context *ctx, Work &w, int top, bool twist, int *regrows) {
+    const int64_t words = ((w.m + 31) / 32 + 31) / 32 * 32;
+    if (words <= CL_BITS) return claim_columns_as<BitColumn>(ctx, w, (int)words, top, twist, regrows);
+    return claim_columns_as<ListColumn>(ctx, w, 3 * CL_CAP, top, twist, regrows);
+}
+
+// The columns as they came, for a walk after columns side by side did not fit.
+static int restart_store(Context *ctx, Work &w, SeqArgs &a) {
+    const int rc = setup_store(ctx, w, false);
+    if (rc) return rc;
+    ctx->launches++;
+    a.low = w.low; a.dim = w.dim; a.seg = w.seg; a.pool = w.pool; a.st = w.st;
+    OPH_CUDA_TRY(cudaMemsetAsync(a.arglow, 0xff, sizeof(int32_t) * w.m, ctx->stream));
+    return OPH_OK;
 }
 
 int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *info) {
@@ -386,10 +892,12 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
     long long iters = m + 1;
     if (!row) {
         a.twist = (algo == OPH_ALGO_TWIST || algo == OPH_ALGO_TWIST_PARALLEL);
-        int *d_stats = (int *)w.agg;
-        int hstats[2] = {-1, 0};
+        int *d_stats = (int *)ctx_alloc(ctx, S_TMP, sizeof(int) * (2 + 2 * 128));
+        if (!d_stats) return OPH_ERR_OOM;
+        int hstats[2 + 2 * 128] = {-1, 0};
+        std::fill(hstats + 2, hstats + 2 + 2 * 128, INT_MAX);
         OPH_CUDA_TRY(cudaMemcpyAsync(d_stats, hstats, sizeof(hstats), cudaMemcpyHostToDevice, s));
-        k_dim_stats<<<grid_m, 256, 0, s>>>(w.dim, m, d_stats);
+        k_dim_stats<<<grid_m, 256, 0, s>>>(w.dim, w.colptr, w.rows, m, d_stats);
         ctx->launches++;
         OPH_CUDA_TRY(cudaMemcpyAsync(hstats, d_stats, sizeof(hstats), cudaMemcpyDeviceToHost, s));
         OPH_CUDA_TRY(cudaMemsetAsync(a.arglow, 0xff, sizeof(int32_t) * m, s));
@@ -404,6 +912,27 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
         if (a.twist) iters = 1 + (long long)hstats[1];
         SeqTracking *tk = ctx->seq_track;
         a.it_base = 1;
+        // side by side, unless the walk itself is asked for, or twist's
+        // clearing could depend on its order
+        bool side_by_side = !tk;
+        if (side_by_side && a.twist) {
+            // every dimension's rows from a lower one, and no two from the same
+            bool from[128] = {};
+            for (int d = 1; d < 128 && side_by_side; d++) {
+                const int lo = hstats[2 + d], hi = -1 - hstats[2 + 128 + d];
+                if (hi < lo) continue;  // no such columns
+                side_by_side = lo == hi && hi < d && !from[hi + 1];
+                from[hi + 1] = true;
+            }
+        }
+        if (side_by_side) {
+            int rc = claim_columns(ctx, w, a.twist ? maxdim : -1, a.twist != 0, &regrows);
+            if (rc == OPH_ERR_OOM || rc == OPH_ERR_OVERFLOW) {  // the walk writes less: it may still fit
+                side_by_side = false;
+                rc = restart_store(ctx, w, a);
+            }
+            if (rc) return rc;
+        }
         if (tk) {
             // the state the host replays from, and a stamp per iteration
             tk->iters = iters;
@@ -422,7 +951,7 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
             OPH_CUDA_TRY(cudaFuncSetAttribute(k_seq_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             attr = true;
         }
-        if (!(a.twist && maxdim < 1)) {
+        if (!side_by_side && !(a.twist && maxdim < 1)) {
             for (;;) {
                 k_seq_walk<<<1, 32, smem, s>>>(a);
                 ctx->launches++;
@@ -457,6 +986,21 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
         a.row_quirk = (algo == OPH_ALGO_PH_ROW) && d_ess != nullptr;
         SeqTracking *tk = ctx->seq_track;
         long long *ev_base = nullptr;
+        // without the running estimate and trackers only the lows are asked
+        // for, which are those of the columns side by side
+        bool side_by_side = !tk && !a.row_quirk;
+        if (side_by_side) {
+            int rc = claim_columns(ctx, w, -1, false, &regrows);
+            if (rc == OPH_ERR_OOM || rc == OPH_ERR_OVERFLOW) {
+                side_by_side = false;
+                rc = restart_store(ctx, w, a);
+                // claim_columns used this slot
+                a.bhead = (int32_t *)ctx_alloc(ctx, S_TMP, sizeof(int32_t) * (3 * m + 1));
+                if (!rc && !a.bhead) rc = OPH_ERR_OOM;
+                a.bnext = a.bhead + m; a.bcnt = a.bnext + m;
+            }
+            if (rc) return rc;
+        }
         if (tk) {
             // the initial lows and a log of the walk's additions for the
             // host's replay: {start ns, length} then the records
@@ -475,7 +1019,7 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
             OPH_CUDA_TRY(cudaFuncSetAttribute(k_row_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             attr = true;
         }
-        for (;;) {
+        while (!side_by_side) {
             OPH_CUDA_TRY(cudaMemsetAsync(a.bhead, 0xff, sizeof(int32_t) * m, s));
             OPH_CUDA_TRY(cudaMemsetAsync(a.bcnt, 0, sizeof(int32_t) * m, s));
             OPH_CUDA_TRY(cudaMemsetAsync(a.arglow, 0x7f, sizeof(int32_t) * m, s));
