@@ -77,6 +77,7 @@ struct C2Status {
     int next;        // whole instances: the CTAs' queue
     int refused;     //   an instance is too large, or no complex in runs
     int no_room;     //   the tables' bounds were too small
+    int items, next_item;  // pieces of theirs, and their queue
     int nres, cursor, overflow;      // residual edges; the CTAs' queue; a list ran out of room
     long long cells;                 // entries of the edge-vertex table
     long long pairs, run_words;      // entries of the edge-id table, words of the runs' bits
@@ -141,6 +142,10 @@ struct C2Args {
     // whole instances: what the tables hold (edges, vertices, table entries, run words)
     long long cap_e, cap_v, cap_c, cap_r;
     long long nnz;            //   and the entries rows[] holds (-1: colptr[m], one matrix)
+    int *order;               //   the order they are taken in (nullptr: as they come)
+    int2 *items;              //   pieces left to k_c2_inst_more: instance, first edge
+    int split_cols;           //   of instances of more columns
+    int chunk;                //   edges of a piece, a multiple of 8 (0: nothing is left to it)
 };
 
 __device__ __forceinline__ unsigned below(int bit) { return (1u << bit) - 1u; }
@@ -1436,25 +1441,63 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
 // every instance has passed.
 constexpr int IN_THREADS = 512;
 constexpr int IN_SMEM = 112 * 1024;  // two CTAs an SM
+// Where the instances have this many columns on average, those with more than
+// three quarters of a CTA's share are split (k_c2_inst_more).  Below, the two
+// launches cost more than they give: 64 complexes of 9 to 20 points took 85 us
+// without and 98 with, one of 30 points 82 and 85, of 36 points 95 and 85.
+constexpr int IN_SPLIT = 6144;
 constexpr int IN_MAX_NV = 192;       // sorting the vertices' rows takes nv^3 comparisons of one CTA
 // Words of an instance start at a multiple of four (16-byte windows).
 __device__ __forceinline__ long long in_woff(long long o0, int b) { return 4 * ((o0 >> 7) + b); }
 
-// The triangles of an instance, a warp per edge (flag_run); true where a run
-// is not what it must be.
+// The triangles of edges k0 ... k0 + own of an instance (col, ends: theirs), a
+// warp per edge (flag_run); true where a run is not what it must be.
 template <int VW>
 __device__ bool in_triangles(const int32_t *col, const int32_t *tab, const uint16_t *ends, const int32_t *rows,
-                             uint2 *runs, int ne, int nv, int cols) {
+                             uint2 *runs, int k0, int own, int ne, int nv, int cols) {
     const int vw = VW > 0 ? VW : (nv + 31) >> 5, idp = 32 * vw;
     bool wrong = false;
-    for (int k = threadIdx.x >> 5; k < ne; k += IN_THREADS / 32) {
+    for (int q = threadIdx.x >> 5; q < own; q += IN_THREADS / 32) {
+        const int k = k0 + q;
         const bool cut = k + 1 == ne;
-        const int fc = col[k], len = (cut ? cols : col[k + 1]) - fc - 1, u = ends[k] & 0xff, v = ends[k] >> 8;
+        const int fc = col[q], len = (cut ? cols : col[q + 1]) - fc - 1, u = ends[q] & 0xff, v = ends[q] >> 8;
         wrong |= tab[u * idp + v] != fc;  // a second edge on these vertices
         wrong |= flag_run<VW, false>(tab + u * idp, tab + v * idp, vw, fc, len, cut,
                                      rows + (2 * (k + 1) + 3 * (fc - nv - k)), runs + (long long)k * vw, 0);
     }
     return wrong;
+}
+
+// The order instances are taken in when there are more than CTAs: the largest
+// first (to 2,048 columns), or the last to start may be one of 300 us when the
+// others are done.  One CTA; its 6 us are those of its chain of steps.
+constexpr int IO_CLASSES = 512;
+__global__ void __launch_bounds__(1024) k_c2_inst_order(C2Args a) {
+    __shared__ int s_at[IO_CLASSES];
+    auto cls = [&](int b) {
+        const int64_t n = a.inst_off[b + 1] - a.inst_off[b];
+        return n <= 0 ? IO_CLASSES - 1 : (int)max((int64_t)0, IO_CLASSES - 1 - (n >> 11));
+    };
+    for (int q = threadIdx.x; q < IO_CLASSES; q += 1024) s_at[q] = 0;
+    __syncthreads();
+    for (int b = threadIdx.x; b < a.count; b += 1024) atomicAdd(&s_at[cls(b)], 1);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int run = 0;
+        for (int q = threadIdx.x; q < IO_CLASSES; q += 32) {
+            const int n = s_at[q];
+            int incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)threadIdx.x >= o) incl += u;
+            }
+            s_at[q] = run + incl - n;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < a.count; b += 1024) a.order[atomicAdd(&s_at[cls(b)], 1)] = b;
 }
 
 __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
@@ -1476,8 +1519,8 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
             s_no = 0;
         }
         __syncthreads();
-        const int b = s_b;
-        if (b >= a.count) break;
+        if (s_b >= a.count) break;
+        const int b = a.order ? a.order[s_b] : s_b;
         const int64_t o0 = a.inst_off ? a.inst_off[b] : 0, o1 = a.inst_off ? a.inst_off[b + 1] : a.m;
         const int64_t cols64 = o1 - o0;
         // 6 bytes a word (bits, edges before it), and room for some edges
@@ -1626,6 +1669,17 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
             },
             scratch, reinterpret_cast<uint16_t *>(scratch + nv), &s_parts);
         __syncthreads();
+        if (a.chunk > 0 && ne > 2 * a.chunk && cols > a.split_cols && !s_no) {
+            // the rest in pieces, to whichever CTAs
+            int4 *const out = reinterpret_cast<int4 *>(a.tab + in.coff);
+            for (int i = tid; i < pitch * nv / 4; i += IN_THREADS) out[i] = reinterpret_cast<const int4 *>(tab)[i];
+            const int pieces = (ne + a.chunk - 1) / a.chunk;
+            if (tid == 0) s_b = atomicAdd(&a.st->items, pieces);
+            __syncthreads();
+            for (int i = tid; i < pieces; i += IN_THREADS) a.items[s_b + i] = make_int2(b, i * a.chunk);
+            __syncthreads();
+            continue;
+        }
         // the vertices' edges in order, for the residual columns (as many
         // warps as the scratch has rows for)
         const int warps = min(NW, left / (4 * pitch));
@@ -1636,15 +1690,79 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         uint2 *const runs = a.runs + in.roff;
         bool wrong;
         switch (vw) {
-            case 1: wrong = in_triangles<1>(col, tab, ends, rows, runs, ne, nv, cols); break;
-            case 2: wrong = in_triangles<2>(col, tab, ends, rows, runs, ne, nv, cols); break;
-            case 3: wrong = in_triangles<3>(col, tab, ends, rows, runs, ne, nv, cols); break;
-            case 4: wrong = in_triangles<4>(col, tab, ends, rows, runs, ne, nv, cols); break;
-            default: wrong = in_triangles<0>(col, tab, ends, rows, runs, ne, nv, cols); break;
+            case 1: wrong = in_triangles<1>(col, tab, ends, rows, runs, 0, ne, ne, nv, cols); break;
+            case 2: wrong = in_triangles<2>(col, tab, ends, rows, runs, 0, ne, ne, nv, cols); break;
+            case 3: wrong = in_triangles<3>(col, tab, ends, rows, runs, 0, ne, ne, nv, cols); break;
+            case 4: wrong = in_triangles<4>(col, tab, ends, rows, runs, 0, ne, ne, nv, cols); break;
+            default: wrong = in_triangles<0>(col, tab, ends, rows, runs, 0, ne, ne, nv, cols); break;
         }
         if (wrong) s_no = 1;
         __syncthreads();
         if (tid == 0 && s_no) a.st->refused = 1;
+        __syncthreads();
+    }
+}
+
+// What k_c2_inst left of larger instances, a CTA a piece: a stretch of edges
+// with their runs, and its share of the vertices' rows.  One CTA takes 330 us
+// over the triangles of 120 points, while the smaller complexes of a batch are
+// long done.  Instructions bound it as in k_c2_inst (47 a word of an edge, 70%
+// of the issue slots); fetching rows to L2 ahead of use, and checking the
+// triangles packed by a list of third vertices, gave nothing or cost 8%.
+// 1,024 complexes of 20 to 120 points 1,909 us -> 1,640 in all, 40 of 20 to 60
+// 182 -> 149, one of 50 points 135 -> 109.
+__global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst_more(C2Args a) {
+    extern __shared__ __align__(16) unsigned char in_smem[];  // IN_SMEM
+    constexpr int NW = IN_THREADS / 32;
+    __shared__ int s_i;
+    const int tid = threadIdx.x, wid = tid >> 5;
+    if (a.st->refused || a.st->no_room) return;
+    const int n_items = a.st->items;
+    for (int i = blockIdx.x; i < n_items; i = s_i) {
+        const int2 item = a.items[i];
+        const C2Inst in = a.inst[item.x];
+        const int nv = in.nv, ne = in.ne, pitch = c2_pitch(nv), vw = pitch / 32;
+        const int k0 = item.y, k1 = min(ne, k0 + a.chunk), own = k1 - k0;
+        const int32_t *const elist = a.elist + in.eoff, *const rows = a.rows + a.colptr[in.base];
+        // the piece's rows of the matrix on their way to L2
+        const int f0 = __ldg(elist + k0), f1 = k1 < ne ? __ldg(elist + k1) : (int)in.cols;
+        const int32_t *const r0 = rows + 2 * (k0 + 1) + 3 * (f0 - nv - k0);
+        for (int q = 32 * tid; q < 2 * (own - 1) + 3 * (f1 - f0 - own); q += 32 * IN_THREADS) prefetch_l2(r0 + q);
+        int32_t *const tab = reinterpret_cast<int32_t *>(in_smem), *const col = tab + pitch * nv;
+        uint16_t *const ends = reinterpret_cast<uint16_t *>(col + a.chunk + 4);
+        const int32_t *const src = a.tab + in.coff;
+        for (int q = tid; q < pitch * nv / 4; q += IN_THREADS)
+            reinterpret_cast<int4 *>(tab)[q] = __ldg(reinterpret_cast<const int4 *>(src) + q);
+        for (int q = tid; q <= own; q += IN_THREADS) {
+            col[q] = k0 + q < ne ? __ldg(elist + k0 + q) : (int)in.cols;
+            if (q < own) {
+                const int4 e = __ldg(a.erec + in.eoff + k0 + q);
+                ends[q] = (uint16_t)((e.x - in.voff) | (e.y - in.voff) << 8);
+            }
+        }
+        __syncthreads();
+        bool wrong = false;
+        uint2 *const runs = a.runs + in.roff;
+        auto check = [&](auto words) {
+            constexpr int VW = decltype(words)::value;
+            wrong = in_triangles<VW>(col, tab, ends, rows, runs, k0, own, ne, nv, (int)in.cols);
+        };
+        switch (vw) {
+            case 1: check(std::integral_constant<int, 1>()); break;
+            case 2: check(std::integral_constant<int, 2>()); break;
+            case 3: check(std::integral_constant<int, 3>()); break;
+            case 4: check(std::integral_constant<int, 4>()); break;
+            default: check(std::integral_constant<int, 0>()); break;
+        }
+        if (wrong) a.st->refused = 1;
+        const int pieces = (ne + a.chunk - 1) / a.chunk;
+        // as many warps as there is room for rows (one at least: k_c2_inst had it beside 6 ne > 12 chunk bytes)
+        int32_t *const row = reinterpret_cast<int32_t *>(ends + a.chunk);
+        const int warps = min(NW, (int)(in_smem + IN_SMEM - reinterpret_cast<unsigned char *>(row)) / (4 * pitch));
+        if (wid < warps)
+            for (int v = k0 / a.chunk + wid * pieces; v < nv; v += warps * pieces)
+                c2_sort_row<32>(a.cells + in.coff + v * pitch, a.adj + in.coff + v * pitch, nv, pitch, row + wid * pitch);
+        if (tid == 0) s_i = gridDim.x + atomicAdd(&a.st->next_item, 1);
         __syncthreads();
     }
 }
@@ -1888,7 +2006,8 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
     static int ready[64];
     int &ok = ready[ctx->device & 63];
     if (!ok) {
-        if (cudaFuncSetAttribute(k_c2_inst, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess) {
+        if (cudaFuncSetAttribute(k_c2_inst, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_c2_inst_more, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess) {
             cudaGetLastError();
             return OPH_OK;
         }
@@ -1902,6 +2021,11 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
                          m / 4 + 65536};
     for (int q = 0; q < 4; q++) need[q] = std::max(need[q], ctx->c2_need[q]);
     const long long nwords = 4 * (m / 128 + a.count + 1);
+    const int slots = 2 * ctx->sm_count;
+    // equal instances fill the CTAs by themselves, and pieces read the tables again: 304 of 60 points
+    // took 394 us whole and 405-420 split, 256 of 20 to 120 points 983 us whole and 690 split
+    a.split_cols = (int)std::min<int64_t>(INT_MAX, m / slots * 3 / 4);
+    a.chunk = m / a.count < IN_SPLIT ? 0 : (int)std::max<int64_t>(64, std::min<int64_t>(512, m / (40 * 2 * slots))) & ~7;
     for (int tries = 0; tries < 2; tries++) {
         a.cap_e = need[0];
         a.cap_v = need[1];
@@ -1925,10 +2049,13 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
             a.res = c.take<int32_t>(a.cap_e);
             a.sum = c.take<unsigned long long>(a.cap_e);
             a.dead = c.take<uint8_t>(a.cap_v);
+            a.order = c.take<int>(a.count);
+            a.items = c.take<int2>(a.chunk ? a.cap_e / a.chunk + a.count : 1);
             if (p) break;
             p = (char *)ctx_alloc(ctx, S_C2_WORK, c.off);
             if (!p) return OPH_OK;
         }
+        if (a.count <= slots || !a.chunk) a.order = nullptr;
         for (char *p = nullptr;;) {
             Carve c{p};
             a.runs = c.take<uint2>(a.cap_r);
@@ -1940,11 +2067,20 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
             p = (char *)ctx_alloc(ctx, S_C2_MODE, c.off);
             if (!p) return OPH_OK;
         }
-        a.cells = (int32_t *)ctx_alloc(ctx, S_C2_CELLS, 2 * sizeof(int32_t) * (size_t)a.cap_c);
+        a.cells = (int32_t *)ctx_alloc(ctx, S_C2_CELLS, (a.chunk ? 3 : 2) * sizeof(int32_t) * (size_t)a.cap_c);
         if (!a.cells) return OPH_OK;
         a.adj = a.cells + a.cap_c;
+        a.tab = a.chunk ? a.adj + a.cap_c : nullptr;
         OPH_CUDA_TRY(cudaMemsetAsync(a.st, 0, sizeof(C2Status), s));
-        k_c2_inst<<<std::min(a.count, 2 * ctx->sm_count), IN_THREADS, IN_SMEM, s>>>(a);
+        if (a.order) {
+            k_c2_inst_order<<<1, 1024, 0, s>>>(a);
+            ctx->launches++;
+        }
+        k_c2_inst<<<std::min(a.count, slots), IN_THREADS, IN_SMEM, s>>>(a);
+        if (a.chunk) {
+            k_c2_inst_more<<<(int)std::min<int64_t>(slots, a.cap_e / a.chunk + 1), IN_THREADS, IN_SMEM, s>>>(a);
+            ctx->launches++;
+        }
         // enough blocks for the outputs of one instance as of many
         const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(16, (m / a.count + IO_COLS - 1) / IO_COLS));
         k_c2_inst_out<<<parts * std::min(a.count, 65535), IO_THREADS, 0, s>>>(a, parts);

@@ -197,6 +197,29 @@ def test_batch_of_whole_instances(ctx, n_max):
         np.testing.assert_array_equal(ess[col_off[b]:col_off[b + 1]], want_ess, err_msg=str(b))
 
 
+@pytest.mark.parametrize("count,n,large,swap", [(1, 34, (34,), False), (1, 57, (57,), True), (9, 20, (48, 61), False),
+                                                (150, 30, (90, 96, 97), False), (400, 34, (64, 65, 90), False),
+                                                (400, 34, (64, 90), True)])
+def test_batch_of_uneven_instances(ctx, count, n, large, swap):
+    """Instances above and below their share of a CTA, fewer and more than
+    CTAs: the larger ones in pieces, the largest first.  With two of the last
+    one's triangles exchanged it is no complex in runs, and the batch goes to
+    the general path."""
+    sizes = np.full(count, n, np.int32)
+    sizes[-len(large):] = large
+    col_off, colptr, rows = cx.rips_mixed_instances(sizes, np.arange(count, dtype=np.uint64) + np.uint64(11))
+    if swap:
+        end = int(colptr[-1])
+        rows = rows.copy()
+        rows[end - 6:] = np.concatenate([rows[end - 3:], rows[end - 6:end - 3]])
+    low, ess, _ = ctx.reduce_batch_packed(col_off, colptr, rows)
+    mats = [cx.batch_instance(col_off, colptr, rows, b) for b in range(count)]
+    for b in sorted({0, count // 3, *range(max(0, count - 5), count)}):
+        want, want_ess, _ = oracle.twist(mats[b])
+        np.testing.assert_array_equal(low[col_off[b]:col_off[b + 1]], want, err_msg=str(b))
+        np.testing.assert_array_equal(ess[col_off[b]:col_off[b + 1]], want_ess, err_msg=str(b))
+
+
 @pytest.mark.parametrize("cut", [1, 2, 3, 40, 300, 2000, 2300])
 def test_first_simplices_of_a_rips_complex(ctx, cut):
     """A filtration cut off anywhere: inside the last edge's run, right after
