@@ -79,6 +79,7 @@ struct C2Status {
     int no_room;     //   the tables' bounds were too small
     int items, next_item;  // pieces of theirs, and their queue
     int nres, cursor, overflow;      // residual edges; the CTAs' queue; a list ran out of room
+    int maps;                        // windows kept of published columns
     long long cells;                 // entries of the edge-vertex table
     long long pairs, run_words;      // entries of the edge-id table, words of the runs' bits
     unsigned long long cells_set;    // entries of the edge-vertex table that a triangle wrote
@@ -90,12 +91,17 @@ constexpr int C2_THREADS = 256, C2_TILE = 2048;
 constexpr int C2_MAX_ROUNDS = 512;
 constexpr unsigned long long C2_FIRST_ROUND = 0xffffffffull << 32;  // the round in a key's upper half, counting down
 constexpr int C2_MAX_NV = 8192;                   // vertices of an instance the dense form takes
-constexpr int RS_WAVE = 32;                       // residual columns: pivots added at a time,
+// residual columns: pivots added at a time, at first and at most; a torus of
+// 200K columns took 279 us with 32 at most, 264 with 64, 252 with 128, batches
+// of 1,024 (columns of 2.6 waves) 1,646 us with 4 at first and 1,607 with 2
+__host__ __device__ constexpr int rs_first(int threads) { return threads >= 1024 ? 4 : 2; }
+__host__ __device__ constexpr int rs_wave(int threads) { return threads >= 1024 ? 128 : 32; }
 // edges a column under reduction may be the sum of (2,700 on the torus, 600 on 120 points)
 __host__ __device__ constexpr int rs_list(int threads) { return threads >= 1024 ? 16384 : 4096; }
 constexpr int RS_FLAG = 1 << 30;
 // Many vertices: long rows and few, long residual columns, so large CTAs and
 // windows; below, more CTAs.
+constexpr int RS_MAPS = 512;  // windows of published columns kept, 16 MB
 constexpr int RS_SMALL_NV = 160, RS_SMALL = 256, RS_SMALL_WORDS = 4096, RS_LARGE = 1024, RS_LARGE_WORDS = 8192;
 
 struct C2Args {
@@ -139,6 +145,8 @@ struct C2Args {
     int32_t *arena;
     long long arena_cap;
     int32_t *lists;           // per CTA: rs_list() edges
+    uint32_t *maps;           // large CTAs: windows of published columns, map_cap of RS_LARGE_WORDS
+    int map_cap;
     // whole instances: what the tables hold (edges, vertices, table entries, run words)
     long long cap_e, cap_v, cap_c, cap_r;
     long long nnz;            //   and the entries rows[] holds (-1: colptr[m], one matrix)
@@ -1089,6 +1097,10 @@ __device__ __forceinline__ void rs_flip(uint32_t *bits, int r) {
                  : "memory");
 }
 
+__device__ __forceinline__ void rs_xor(uint32_t *word, uint32_t x) {
+    asm volatile("red.shared.xor.b32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(word)), "r"(x) : "memory");
+}
+
 // The triangles on edge k toggled in the window of WORDS words from w0, by a
 // warp.  RUNS: the triangle with vertex w belongs to the run of the last of
 // its three edges; runs from edge `hi` on lie past the window, so the edges of
@@ -1162,32 +1174,44 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
 // of triangles; a window left behind is never needed again, a later one is
 // built from the list.  Its low is the first set bit.
 //
-// * Waves: not only the low's pivot is added but those of the first RS_WAVE
+// * Waves: not only the low's pivot is added but those of the first rs_wave()
 //   set bits that have one.  Every column added comes before k in D' (a row
 //   of the sum lies in a column of the sum, and its owner is the first column
-//   that can hold it), so this is a reduction like any other, and the two
-//   chains of 557 additions on the torus take 36 and 40 waves.
+//   that can hold it), so this is a reduction like any other, and the chain
+//   of 970 additions on the torus takes 35 waves of 32.
 // * Owners: low[t] names the owner of triangle t.  A residual column claims
 //   its low by compare-and-swap once its list is published.  Found claimed by
 //   an earlier column, that column is added; by a later one, the claim is
 //   taken over and this CTA goes on with the later column plus its own.  No
 //   CTA waits for another, and the lows are those of any complete reduction.
 //
-// Bound by latency: a wave is a search of the window and four dependent trips
-// to L2 (which set bits have owners, the owners, their vertices, their
-// triangles) and of the instructions of one SM, so the columns of a wave are
-// spread over the CTA's warps and no more of each is looked at than the window
-// holds.  Complexes on many
-// vertices, with few long columns, take large CTAs and windows; batches of
-// small ones as many CTAs as fit.
+// * Published windows: a large CTA publishes its window with its list.  Added
+//   later, the window is xored word by word, where it reaches as far as the
+//   adder's (the windows lie on a common grid, and nothing comes before a
+//   low), instead of the 25 columns or so of the list one by one.
+//
+// Bound by the longest column, on one SM: of 14K cycles a wave on the torus
+// 9.7K went into some 77 columns, 126 cycles each (240 instructions a warp),
+// 2.7K into the search of the window and 1.5K into the owners.  With published
+// windows 28 columns are left to a wave: 250 us -> 190, with wider waves 165
+// (a device call on 200K columns 337 -> 278 -> 252).  Flattening the lists of
+// a wave into one, sharing a column among warps and leaving out the parts of a
+// row past the window cost as much as they saved.  Complexes on many vertices,
+// with few long columns, take large CTAs and windows (4,096 words instead of
+// 8,192: 356 us, 16,384: 272); batches of small ones as many CTAs as fit: six
+// an SM, at 40 registers with some spills, took 1,556-1,581 us for 1,024
+// complexes, five 1,607-1,628, four 1,618-1,644.
 template <bool RUNS, int THREADS, int WORDS>
-__global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
+__global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_residual(C2Args a) {
     if (a.st->bad || (RUNS && (a.st->unsorted || a.st->refused || a.st->no_room))) return;
     extern __shared__ __align__(16) uint32_t bits[];  // WORDS
     constexpr int NW = THREADS / 32, RS_LIST = rs_list(THREADS);
-    __shared__ int s_low[NW], s_cnt[NW], s_wave[RS_WAVE];
+    constexpr bool MAPS = THREADS > RS_SMALL;
+    constexpr int WAVE = rs_wave(THREADS);
+    constexpr int HEAD = MAPS ? 4 : 0;  // of a published list: its window's place (-1: none), start, and what lies past it
+    __shared__ int s_low[NW], s_cnt[NW], s_wave[WAVE];
     __shared__ int s_i, s_later, s_act, s_other;
-    __shared__ unsigned long long s_sum;
+    __shared__ unsigned long long s_sum, s_sums[WAVE];
     enum { ACT_DONE, ACT_ADD, ACT_STEAL, ACT_FAIL };
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nres = a.st->nres, none = a.one_based ? 0 : -1;
@@ -1210,11 +1234,39 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
         const uint32_t *const fixed = a.fixed + in.woff;
         int n = 1, pos = a.elist[k] + 1, w0 = 0, hi = 0, later = INT_MAX;  // triangles come after their edges
         if (tid == 0) __stcg(list, k);
+        // The published column of `sum` added: its edges to the list, its rows to
+        // the window, from the window it was published with where that reaches
+        // as far as this one, else edge by edge.
+        auto add_list = [&](unsigned long long sum, int4 head) {
+            const int len = (int)(sum & 0xffffffu);
+            const int32_t *const from = a.arena + (sum >> 24) + HEAD;
+            if (n + len > RS_LIST) return false;
+            if (MAPS && head.x >= 0 && head.y >= w0) {
+                const uint32_t *const map = a.maps + (size_t)head.x * WORDS;
+                const int off = (head.y - w0) >> 5;
+                for (int q = off + 4 * tid; q < WORDS; q += 4 * THREADS) {
+                    const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(map + (q - off)));
+                    if (x.x) rs_xor(bits + q, x.x);
+                    if (x.y) rs_xor(bits + q + 1, x.y);
+                    if (x.z) rs_xor(bits + q + 2, x.z);
+                    if (x.w) rs_xor(bits + q + 3, x.w);
+                }
+                if (off == 0) later = min(later, head.z);
+                else if (w0 + 32ll * WORDS < cols) later = min(later, RUNS ? max(hi - 1, 0) : w0 + 32 * WORDS);
+            } else {
+                for (int x = wid; x < len; x += NW)
+                    rs_toggle<RUNS, WORDS>(a, in, __ldcg(from + x), w0, hi, bits, later);
+            }
+            for (int v = tid; v < len; v += THREADS) __stcg(list + n + v, __ldcg(from + v));
+            n += len;
+            return true;
+        };
         bool fresh = true;  // a new window, from pos
-        int wave = 4;       // most columns take a wave or two: long ones get the full width
+        int wave = rs_first(THREADS);       // most columns take a wave or two: long ones get the full width
         for (;;) {
             if (fresh) {
-                w0 = pos & ~127;
+                // on a grid of half windows, so that published ones fit each other
+                w0 = MAPS ? pos & ~(16 * WORDS - 1) : pos & ~127;
                 if (RUNS)
                     hi = (w0 + 32ll * WORDS >= cols ? in.eoff + in.ne : c2_edge_rank(a, in, w0 + 32 * WORDS)) - in.eoff;
                 for (int q = 4 * tid; q < WORDS; q += 4 * THREADS)
@@ -1289,35 +1341,46 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
             __syncthreads();
             int cnt = min(total, wave);
             const bool have = cnt > 0 && (s_wave[0] & ~RS_FLAG) == low;
-            wave = min(2 * wave, RS_WAVE);
+            wave = min(2 * wave, WAVE);
             __syncthreads();
-            if (wid == 0 && lane < cnt) {  // the owners, all at once
-                const int t = s_wave[lane] & ~RS_FLAG, fl = s_wave[lane] & RS_FLAG;
+            if (tid < cnt) {  // the owners, all at once
+                const int t = s_wave[tid] & ~RS_FLAG, fl = s_wave[tid] & RS_FLAG;
                 int o;
                 if (RUNS && !fl) o = c2_edge_rank(a, in, t) - 1;  // the last edge before t
                 else o = c2_edge_rank(a, in, ld_acquire_i32(out_low + t) + shift);
-                s_wave[lane] = o | fl;
+                s_wave[tid] = o | fl;
             }
             __syncthreads();
             const int p0 = have ? s_wave[0] : -1;
-            if (n + RS_WAVE > RS_LIST) {
+            if (n + WAVE > RS_LIST) {
                 if (tid == 0) a.st->overflow = 1;
                 break;
             }
             if (!have || ((p0 & RS_FLAG) && (p0 & ~RS_FLAG) < k)) {
                 // claim the low: the list first, then the owner
                 if (tid == 0) {
-                    const unsigned long long off = atomicAdd(&a.st->arena, (unsigned long long)n);
+                    const int room = (HEAD + n + 3) & ~3;
+                    const unsigned long long off = atomicAdd(&a.st->arena, (unsigned long long)room);
                     s_sum = off;
-                    s_act = off + n > (unsigned long long)a.arena_cap ? ACT_FAIL : ACT_DONE;
+                    s_act = off + room > (unsigned long long)a.arena_cap ? ACT_FAIL : ACT_DONE;
+                    if (MAPS) s_other = atomicAdd(&a.st->maps, 1);
                 }
+                if (MAPS && later != INT_MAX) atomicMin(&s_later, later);
                 __syncthreads();
                 const unsigned long long off = s_sum;
                 if (s_act == ACT_FAIL) {
                     if (tid == 0) a.st->overflow = 1;
                     break;
                 }
-                for (int v = tid; v < n; v += THREADS) __stcg(a.arena + off + v, __ldcg(list + v));
+                if (MAPS) {
+                    const int place = s_other < a.map_cap ? s_other : -1;
+                    if (place >= 0)
+                        for (int q = 4 * tid; q < WORDS; q += 4 * THREADS)
+                            __stcg(reinterpret_cast<uint4 *>(a.maps + (size_t)place * WORDS + q),
+                                   *reinterpret_cast<const uint4 *>(bits + q));
+                    if (tid == 0) __stcg(reinterpret_cast<int4 *>(a.arena + off), make_int4(place, w0, s_later, 0));
+                }
+                for (int v = tid; v < n; v += THREADS) __stcg(a.arena + off + HEAD + v, __ldcg(list + v));
                 __threadfence();
                 __syncthreads();
                 if (tid == 0) {
@@ -1354,24 +1417,26 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
                 const int act = s_act;
                 if (act == ACT_DONE || act == ACT_FAIL) break;
                 if (act == ACT_STEAL) {
-                    const int len = (int)(s_sum & 0xffffffu);
-                    const unsigned long long from = s_sum >> 24;
-                    if (n + len > RS_LIST) {
-                        if (tid == 0) a.st->overflow = 1;
-                        break;
-                    }
                     // its rows join those in the window (below their common low both have none left).
                     // Batches of small complexes start the window afresh instead: their lists are short,
                     // and joining cost 1,888 us against 1,843 on 1,024 of them; a torus of 5M columns took
                     // 395-423 us afresh and 378 joining.
-                    if constexpr (THREADS > RS_SMALL) {
-                        for (int x = wid; x < len; x += NW)
-                            rs_toggle<RUNS, WORDS>(a, in, __ldcg(a.arena + from + x), w0, hi, bits, later);
+                    const unsigned long long sum = s_sum;
+                    bool room = true;
+                    if constexpr (MAPS) {
+                        room = add_list(sum, __ldcg(reinterpret_cast<const int4 *>(a.arena + (sum >> 24))));
                     } else {
+                        const int len = (int)(sum & 0xffffffu);
+                        room = n + len <= RS_LIST;
+                        for (int v = tid; room && v < len; v += THREADS)
+                            __stcg(list + n + v, __ldcg(a.arena + (sum >> 24) + v));
+                        n += len;
                         fresh = true;
                     }
-                    for (int v = tid; v < len; v += THREADS) __stcg(list + n + v, __ldcg(a.arena + from + v));
-                    n += len;
+                    if (!room) {
+                        if (tid == 0) a.st->overflow = 1;
+                        break;
+                    }
                     k = s_other;
                     pos = low;
                     __syncthreads();
@@ -1381,34 +1446,43 @@ __global__ void __launch_bounds__(THREADS) k_c2_residual(C2Args a) {
                 cnt = 1;
                 __syncthreads();
             }
-            // the wave
-            const int p = lane < cnt ? s_wave[lane] : -1;
-            const unsigned m_app = __ballot_sync(0xffffffffu, p >= 0 && !(p & RS_FLAG));
-            unsigned m_res = __ballot_sync(0xffffffffu, p >= 0 && (p & RS_FLAG) && (p & ~RS_FLAG) > k);
-            for (int q = wid; q < cnt; q += NW)
-                if ((m_app >> q) & 1u) rs_toggle<RUNS, WORDS>(a, in, s_wave[q], w0, hi, bits, later);
-            if (wid == 0 && ((m_app >> lane) & 1u)) __stcg(list + n + __popc(m_app & below(lane)), p);
-            n += __popc(m_app);
-            bool full = false;
-            adds += __popc(m_app);
-            slots += (unsigned long long)__popc(m_app) * in.nv;
-            for (; m_res; m_res &= m_res - 1) {
-                const int o = s_wave[__ffs(m_res) - 1] & ~RS_FLAG;
-                __syncthreads();
-                if (tid == 0) s_sum = *(volatile unsigned long long *)(a.sum + o);
-                __syncthreads();
-                const int len = (int)(s_sum & 0xffffffu);
-                const unsigned long long from = s_sum >> 24;
-                if (n + len > RS_LIST) {
-                    full = true;
-                    break;
+            // the wave, 32 pivots a lane each (what the residual ones
+            // published is read once for all warps: it may be published anew meanwhile)
+            int app = 0, nres_w = 0;
+#pragma unroll
+            for (int h = 0; h < WAVE; h += 32) {
+                const int p = h + lane < cnt ? s_wave[h + lane] : -1;
+                const bool res = p >= 0 && (p & RS_FLAG) && (p & ~RS_FLAG) > k;
+                const unsigned m_app = __ballot_sync(0xffffffffu, p >= 0 && !(p & RS_FLAG));
+                nres_w += __popc(__ballot_sync(0xffffffffu, res));
+                if (wid == h / 32) {
+                    if ((m_app >> lane) & 1u) __stcg(list + n + app + __popc(m_app & below(lane)), p);
+                    if (res) s_sums[h + lane] = *(volatile unsigned long long *)(a.sum + (p & ~RS_FLAG));
                 }
-                for (int x = wid; x < len; x += NW)
-                    rs_toggle<RUNS, WORDS>(a, in, __ldcg(a.arena + from + x), w0, hi, bits, later);
-                for (int v = tid; v < len; v += THREADS) __stcg(list + n + v, __ldcg(a.arena + from + v));
-                n += len;
-                adds++;
-                slots += (unsigned long long)len * in.nv;
+                app += __popc(m_app);
+            }
+            for (int q = wid; q < cnt; q += NW)
+                if (!(s_wave[q] & RS_FLAG)) rs_toggle<RUNS, WORDS>(a, in, s_wave[q], w0, hi, bits, later);
+            n += app;
+            adds += app + nres_w;
+            slots += (unsigned long long)app * in.nv;
+            bool full = false;
+            if (nres_w) {
+                __syncthreads();
+#pragma unroll
+                for (int h = 0; h < WAVE; h += 32) {
+                    const int p = h + lane < cnt ? s_wave[h + lane] : -1;
+                    const bool res = p >= 0 && (p & RS_FLAG) && (p & ~RS_FLAG) > k;
+                    int4 head = make_int4(-1, 0, 0, 0);
+                    if (MAPS && res) head = __ldcg(reinterpret_cast<const int4 *>(a.arena + (s_sums[h + lane] >> 24)));
+                    for (unsigned m = __ballot_sync(0xffffffffu, res); m && !full; m &= m - 1) {
+                        const int q = __ffs(m) - 1;
+                        const int4 at = make_int4(__shfl_sync(0xffffffffu, head.x, q), __shfl_sync(0xffffffffu, head.y, q),
+                                                  __shfl_sync(0xffffffffu, head.z, q), 0);
+                        full = !add_list(s_sums[h + q], at);
+                        slots += (unsigned long long)(s_sums[h + q] & 0xffffffu) * in.nv;
+                    }
+                }
             }
             if (full) {
                 if (tid == 0) a.st->overflow = 1;
@@ -1952,6 +2026,8 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
         a.sum = c.take<unsigned long long>(ne);
         a.arena = c.take<int32_t>(a.arena_cap);
         a.lists = c.take<int32_t>((size_t)gr * rs_list(small ? RS_SMALL : RS_LARGE));
+        a.map_cap = small ? 0 : (int)std::min<int64_t>(ne, RS_MAPS);
+        a.maps = c.take<uint32_t>((size_t)a.map_cap * RS_LARGE_WORDS);
         if (p) break;
         p = (char *)ctx_alloc(ctx, S_C2_MODE, c.off);
         if (!p) return OPH_OK;

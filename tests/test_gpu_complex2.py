@@ -180,6 +180,14 @@ def test_rips_cta_sizes(ctx, n):
     check(ctx, cx.rips(cx.points_circle(n, seed=n), threshold=1.2))
 
 
+@pytest.mark.parametrize("points,threshold", [(cx.points_circle(165, 2), np.inf), (cx.points_cube(200, 3), np.inf),
+                                              (cx.points_cube(1000, 4), 0.29), (cx.points_circle(190, 5), 1.7)])
+def test_residual_windows(ctx, points, threshold):
+    """Large complexes of several windows of 2^18 triangles: columns published
+    with windows before, at and after those they are added in."""
+    check(ctx, cx.rips(points, threshold))
+
+
 @pytest.mark.parametrize("n_max", [100, 121, 125, 140])
 def test_batch_of_whole_instances(ctx, n_max):
     """130 instances: a CTA each while every one fits its shared memory, the
