@@ -247,7 +247,12 @@ static int reduce_core(Context *ctx, int algo, Work &w, const Outputs &o, oph_in
     // check: here, or in the grading of dual_choose, which makes the same
     // checks (bounds first) whenever it runs
     const bool grades = pms && !ctx->track && ctx->dual != OPH_DUAL_NEVER && m > 0;
-    if (!w.checked && !grades && (rc = check_csc(ctx, w.colptr, w.rows, m, w.nnz, nullptr, 0))) return rc;
+    // (the algorithms that walk D have it within the set-up, and its verdict
+    // with the status)
+    const bool with_setup = !pms && !w.checked && m > 0;
+    if (with_setup && w.nnz < 0) return OPH_ERR_BAD_INPUT;
+    if (!w.checked && !grades && !with_setup && (rc = check_csc(ctx, w.colptr, w.rows, m, w.nnz, nullptr, 0)))
+        return rc;
     int choice = DUAL_CHOICE_D;
     if (pms && !ctx->track) {
         bool bad = false;
@@ -264,8 +269,9 @@ static int reduce_core(Context *ctx, int algo, Work &w, const Outputs &o, oph_in
         // and beta
         if ((rc = dual_setup(ctx, w, wd))) return rc;
     } else {
-        if ((rc = setup_store(ctx, w, pms))) return rc;
+        if ((rc = setup_store(ctx, w, pms, with_setup))) return rc;
         ctx->launches += pms ? 3 : 1;
+        if ((algo == OPH_ALGO_TWIST || algo == OPH_ALGO_TWIST_PARALLEL) && (rc = dim_stats(ctx, w))) return rc;
     }
     Work &wr = dual ? wd : w;
     if (ctx->profile) {

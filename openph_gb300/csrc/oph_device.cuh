@@ -67,6 +67,8 @@ struct DevStatus {
     long long resume_pos;          //   (column or row index; -1 = finished)
     long long resume_iter;         //   and the iteration count reached (trackers)
     int max_dim;                   // largest nnz(col) - 1 seen by the set-up
+    int seq_top, seq_cols;         // twist: largest dimension + 2 (0: no column), columns of dimension >= 1,
+    int seq_separate, seq_blocks;  //   whether the dimensions separate (k_dim_stats); its finished blocks
     int pad;
     int ucount[2];                     // compacted Phase I: list sizes (ping-pong)
     unsigned long long tier_adds[4];   // additions performed by each Phase II tier

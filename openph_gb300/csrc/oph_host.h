@@ -60,9 +60,11 @@ struct Context;
 // setup.cu
 // init_store: the column store (pool) and a fresh status block for w;
 // setup_store: init_store, then the columns of w's CSC into the store, low,
-// dim, and with need_beta the pivot records, left[] and beta.
+// dim, and with need_beta the pivot records, left[] and beta.  With check, the
+// structural check goes before, its verdict in the status (error), and the
+// set-up does nothing on a malformed matrix.
 int init_store(Context *ctx, Work &w);
-int setup_store(Context *ctx, Work &w, bool need_beta);
+int setup_store(Context *ctx, Work &w, bool need_beta, bool check = false);
 int coo1_to_csc(Context *ctx, const int *d_rows1, const int *d_cols1, int64_t nnz, int64_t m, int64_t *d_colptr,
                 int32_t *d_rows0);
 // Structural check of a device CSC (k_check_csc), synchronous: OPH_OK or
@@ -97,6 +99,7 @@ bool complex2_applies(const Context *ctx, int algo);
 int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken);
 
 // variants.cu
+int dim_stats(Context *ctx, const Work &w);
 int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *info);
 
 // dual.cu: pms on the anti-transpose.  dual_choose grades w's buckets and

@@ -91,6 +91,7 @@ __global__ void k_check_csc(const int64_t *__restrict__ colptr, const int32_t *_
 __global__ void k_setup_columns(const int64_t *__restrict__ colptr, const int32_t *__restrict__ rows, int64_t m,
                                 int *__restrict__ pool, int64_t *__restrict__ seg, int32_t *__restrict__ low,
                                 int8_t *__restrict__ dim, DevStatus *st) {
+    if (st->error) return;  // the check before found the columns malformed
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
         int64_t a = colptr[j], b = colptr[j + 1];
         int64_t s = 8 * j + 4 * ((a + 3) >> 2);
@@ -199,7 +200,7 @@ int init_store(Context *ctx, Work &w) {
     return OPH_OK;
 }
 
-int setup_store(Context *ctx, Work &w, bool need_beta) {
+int setup_store(Context *ctx, Work &w, bool need_beta, bool check) {
     const int64_t m = w.m;
     int rc = init_store(ctx, w);
     if (rc) return rc;
@@ -207,6 +208,11 @@ int setup_store(Context *ctx, Work &w, bool need_beta) {
     if (need_beta) {
         OPH_CUDA_TRY(cudaMemsetAsync(w.rec, 0x7f, sizeof(PivRec) * m, ctx->stream));
         OPH_CUDA_TRY(cudaMemsetAsync(w.beta, 0xff, sizeof(int32_t) * m, ctx->stream));
+    }
+    if (check) {
+        k_check_csc<<<grid_for(ctx, m, 256), 256, 0, ctx->stream>>>(w.colptr, w.rows, m, w.nnz, nullptr, 0,
+                                                                    &w.st->error, nullptr);
+        ctx->launches++;
     }
     k_setup_columns<<<grid_for(ctx, m, 256), 256, 0, ctx->stream>>>(w.colptr, w.rows, m, w.pool, w.seg, w.low,
                                                                     w.dim, w.st);

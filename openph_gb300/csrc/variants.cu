@@ -762,12 +762,16 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_walk(SeqArgs a) {
     }
 }
 
-// out[0] = largest dimension, out[1] = columns of dimension >= 1,
-// out[2 + d] and -1 - out[2 + 128 + d] = the smallest and largest dimension of
-// a row in a column of dimension d >= 1.
-__global__ void k_dim_stats(const int8_t *dim, const int64_t *colptr, const int32_t *rows, int64_t m, int *out) {
-    __shared__ int s_lo[128], s_hi[128];
-    for (int q = threadIdx.x; q < 128; q += blockDim.x) s_lo[q] = s_hi[q] = INT_MAX;
+// For twist, into the status: the largest dimension, the columns of dimension
+// >= 1, and whether the dimensions from 1 up separate: each has its rows in
+// one lower dimension, no two in the same.  seen[d], seen[128 + d]: 128 - the
+// smallest and 2 + the largest dimension of a row in a column of dimension d;
+// the last block looks at them.
+__global__ void __launch_bounds__(256) k_dim_stats(const int8_t *dim, const int64_t *colptr, const int32_t *rows,
+                                                   int64_t m, int *seen, DevStatus *st) {
+    __shared__ int s_seen[256], s_last;
+    if (st->error) return;
+    for (int q = threadIdx.x; q < 256; q += blockDim.x) s_seen[q] = 0;
     __syncthreads();
     int mx = -1, cnt = 0;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
@@ -775,29 +779,50 @@ __global__ void k_dim_stats(const int8_t *dim, const int64_t *colptr, const int3
         mx = max(mx, d);
         if (d < 1) continue;
         cnt++;
-        int lo = INT_MAX, hi = INT_MAX;
+        int lo = 126, hi = -1;
         for (int64_t k = colptr[j]; k < colptr[j + 1]; k++) {
             const int r = dim[rows[k]];
             lo = min(lo, r);
-            hi = min(hi, -1 - r);
+            hi = max(hi, r);
         }
-        if (lo < s_lo[d]) atomicMin(&s_lo[d], lo);
-        if (hi < s_hi[d]) atomicMin(&s_hi[d], hi);
+        if (128 - lo > s_seen[d]) atomicMax(&s_seen[d], 128 - lo);
+        if (hi + 2 > s_seen[128 + d]) atomicMax(&s_seen[128 + d], hi + 2);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(&out[0], mx);
-        atomicAdd(&out[1], cnt);
+        atomicMax(&st->seq_top, mx + 2);
+        if (cnt) atomicAdd(&st->seq_cols, cnt);
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < 128; q += blockDim.x)
-        if (s_lo[q] != INT_MAX) {
-            atomicMin(&out[2 + q], s_lo[q]);
-            atomicMin(&out[2 + 128 + q], s_hi[q]);
-        }
+    if (s_seen[threadIdx.x]) atomicMax(&seen[threadIdx.x], s_seen[threadIdx.x]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&st->seq_blocks, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    s_seen[threadIdx.x] = 0;
+    __syncthreads();
+    bool ok = true;
+    const int d = threadIdx.x;
+    if (d >= 1 && d < 128) {
+        const int lo = __ldcg(seen + d), hi = __ldcg(seen + 128 + d);
+        if (hi) ok = 128 - lo == hi - 2 && hi - 2 < d && atomicAdd(&s_seen[hi - 1], 1) == 0;
+    }
+    if (__syncthreads_and(ok) && threadIdx.x == 0) st->seq_separate = 1;
+}
+
+int dim_stats(Context *ctx, const Work &w) {
+    if (w.m == 0) return OPH_OK;
+    int *seen = (int *)ctx_alloc(ctx, S_SEQNS, sizeof(int) * 256);
+    if (!seen) return OPH_ERR_OOM;
+    OPH_CUDA_TRY(cudaMemsetAsync(seen, 0, sizeof(int) * 256, ctx->stream));
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((w.m + 255) / 256, (int64_t)ctx->sm_count * 16));
+    k_dim_stats<<<grid, 256, 0, ctx->stream>>>(w.dim, w.colptr, w.rows, w.m, seen, w.st);
+    ctx->launches++;
+    OPH_CUDA_TRY(cudaGetLastError());
+    return OPH_OK;
 }
 
 // standard (all columns at once) or twist (dimension top down to 1) by
@@ -829,7 +854,9 @@ static int claim_columns_as(Context *ctx, Work &w, int words, int top, bool twis
     const int64_t per_sm = std::min<int64_t>(2048 / CL_THREADS, (220 << 10) / (smem + 2048));
     const int grid = (int)std::min<int64_t>((m + CL_WARPS - 1) / CL_WARPS, ctx->sm_count * per_sm);
     const int grid_m = (int)std::max<int64_t>(1, std::min<int64_t>((m + 255) / 256, (int64_t)ctx->sm_count * 16));
-    std::vector<ClaimCount> seen(dims);
+    // in the context's second pinned status block where it holds them
+    std::vector<ClaimCount> many(sizeof(ClaimCount) * (size_t)dims > sizeof(DevStatus) ? dims : 0);
+    ClaimCount *const seen = many.empty() ? reinterpret_cast<ClaimCount *>(ctx->h_status + 1) : many.data();
     int turn = 0, d = 0, redo = 0;
     for (;;) {
         OPH_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(ClaimCount) * (size_t)dims, s));
@@ -848,7 +875,7 @@ static int claim_columns_as(Context *ctx, Work &w, int words, int top, bool twis
             }
         }
         OPH_CUDA_TRY(cudaGetLastError());
-        OPH_CUDA_TRY(cudaMemcpyAsync(seen.data(), count, sizeof(ClaimCount) * (size_t)dims, cudaMemcpyDeviceToHost, s));
+        OPH_CUDA_TRY(cudaMemcpyAsync(seen, count, sizeof(ClaimCount) * (size_t)dims, cudaMemcpyDeviceToHost, s));
         OPH_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, w.st, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
         OPH_CUDA_TRY(cudaStreamSynchronize(s));
         while (d < dims && !seen[d].failed) d++;
@@ -875,7 +902,6 @@ static int restart_store(Context *ctx, Work &w, SeqArgs &a) {
     if (rc) return rc;
     ctx->launches++;
     a.low = w.low; a.dim = w.dim; a.seg = w.seg; a.pool = w.pool; a.st = w.st;
-    OPH_CUDA_TRY(cudaMemsetAsync(a.arglow, 0xff, sizeof(int32_t) * w.m, ctx->stream));
     return OPH_OK;
 }
 
@@ -892,39 +918,20 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
     long long iters = m + 1;
     if (!row) {
         a.twist = (algo == OPH_ALGO_TWIST || algo == OPH_ALGO_TWIST_PARALLEL);
-        int *d_stats = (int *)ctx_alloc(ctx, S_TMP, sizeof(int) * (2 + 2 * 128));
-        if (!d_stats) return OPH_ERR_OOM;
-        int hstats[2 + 2 * 128] = {-1, 0};
-        std::fill(hstats + 2, hstats + 2 + 2 * 128, INT_MAX);
-        OPH_CUDA_TRY(cudaMemcpyAsync(d_stats, hstats, sizeof(hstats), cudaMemcpyHostToDevice, s));
-        k_dim_stats<<<grid_m, 256, 0, s>>>(w.dim, w.colptr, w.rows, m, d_stats);
-        ctx->launches++;
-        OPH_CUDA_TRY(cudaMemcpyAsync(hstats, d_stats, sizeof(hstats), cudaMemcpyDeviceToHost, s));
-        OPH_CUDA_TRY(cudaMemsetAsync(a.arglow, 0xff, sizeof(int32_t) * m, s));
-        OPH_CUDA_TRY(cudaStreamSynchronize(s));
-        const int maxdim = hstats[0];
+        const DevStatus set_up = *ctx->h_status;  // as the set-up left it (dim_stats)
+        const int maxdim = a.twist ? set_up.seq_top - 2 : 0;
         a.max_dim = maxdim;
         a.start_dim = a.twist ? maxdim : 0;
         a.start_pos = 0;
         if (a.twist && maxdim < 1) a.start_dim = 0;  // nothing to reduce: the loop below runs no dimension
         // the reference counts one iteration per column visited
         // (twist.cu:36-86 visits the columns of dimension >= 1)
-        if (a.twist) iters = 1 + (long long)hstats[1];
+        if (a.twist) iters = 1 + (long long)set_up.seq_cols;
         SeqTracking *tk = ctx->seq_track;
         a.it_base = 1;
         // side by side, unless the walk itself is asked for, or twist's
         // clearing could depend on its order
-        bool side_by_side = !tk;
-        if (side_by_side && a.twist) {
-            // every dimension's rows from a lower one, and no two from the same
-            bool from[128] = {};
-            for (int d = 1; d < 128 && side_by_side; d++) {
-                const int lo = hstats[2 + d], hi = -1 - hstats[2 + 128 + d];
-                if (hi < lo) continue;  // no such columns
-                side_by_side = lo == hi && hi < d && !from[hi + 1];
-                from[hi + 1] = true;
-            }
-        }
+        bool side_by_side = !tk && (!a.twist || set_up.seq_separate);
         if (side_by_side) {
             int rc = claim_columns(ctx, w, a.twist ? maxdim : -1, a.twist != 0, &regrows);
             if (rc == OPH_ERR_OOM || rc == OPH_ERR_OVERFLOW) {  // the walk writes less: it may still fit
@@ -945,6 +952,7 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
             OPH_CUDA_TRY(cudaMemcpyAsync(tk->dim.data(), w.dim, (size_t)m, cudaMemcpyDeviceToHost, s));
             OPH_CUDA_TRY(cudaStreamSynchronize(s));
         }
+        if (!side_by_side) OPH_CUDA_TRY(cudaMemsetAsync(a.arglow, 0xff, sizeof(int32_t) * m, s));
         static bool attr = false;
         const size_t smem = 3 * SEQ_CAP * sizeof(int);
         if (!attr) {
