@@ -62,8 +62,18 @@ __device__ __forceinline__ unsigned long long lexkey(int dim, unsigned a, unsign
 // ------------------------------------------------------------------ Rips
 // Distances of every pair (upper triangle) and the adjacency bitsets: bit c
 // of row a (words of 32) is set when a != c and |p_a - p_c| <= thr.
-__global__ void k_rips_dist(const double *__restrict__ pts, int n, int d, double thr, double *__restrict__ D,
-                            unsigned *__restrict__ adj, int words) {
+// What the host reads of a Rips complex, and the longest edge (its bits).
+struct RipsTotals {
+    unsigned long long edges, triangles, longest;
+    int tied, crowded;  // equally long edges; too many of one coarse length
+};
+__global__ void __launch_bounds__(256) k_rips_dist(const double *__restrict__ pts, int n, int d, double thr,
+                                                   double *__restrict__ D, unsigned *__restrict__ adj, int words,
+                                                   RipsTotals *totals) {
+    __shared__ unsigned long long s_longest;
+    if (threadIdx.x == 0) s_longest = 0;
+    __syncthreads();
+    double longest = 0.0;  // edge; distances are not negative, so their bits compare like them
     const int64_t pairs = (int64_t)n * n;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < pairs; q += (int64_t)gridDim.x * blockDim.x) {
         const int a = (int)(q / n), b = (int)(q % n);
@@ -77,10 +87,15 @@ __global__ void k_rips_dist(const double *__restrict__ pts, int n, int d, double
         D[(int64_t)a * n + b] = v;
         D[(int64_t)b * n + a] = v;
         if (v <= thr) {
+            longest = max(longest, v);
             atomicOr(&adj[(int64_t)a * words + (b >> 5)], 1u << (b & 31));
             atomicOr(&adj[(int64_t)b * words + (a >> 5)], 1u << (a & 31));
         }
     }
+    for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_longest, dbits(longest));
+    __syncthreads();
+    if (threadIdx.x == 0 && s_longest) atomicMax(&totals->longest, s_longest);
 }
 
 // Bits of row r above column c (exclusive), within word w.
@@ -226,13 +241,16 @@ __global__ void k_rips_rows(const SKey *__restrict__ keys, int64_t m, int n, con
     }
 }
 
-// The edges in vertex order: their keys (value bits), their vertices, their
-// place (the sort's payload).  A warp per row, a lane per vertex of a word.
+// The edges in vertex order: their lengths' bits and the first 32 bits of their
+// share of the longest (which order them, but for a few), their vertices,
+// their place (the sort's payload).  A warp per row, a lane per vertex of a word.
 __global__ void k_rips_edge_list(const unsigned *__restrict__ adj, const double *__restrict__ D, int n, int words,
-                                 const long long *__restrict__ eoff, unsigned long long *__restrict__ key,
+                                 const long long *__restrict__ eoff, const RipsTotals *__restrict__ totals,
+                                 unsigned long long *__restrict__ key, unsigned *__restrict__ coarse,
                                  unsigned *__restrict__ place, int2 *__restrict__ ends) {
     const int lane = threadIdx.x & 31;
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const double scale = 4294967040.0 / dvalue(totals->longest);
     for (int a = wid; a < n; a += nw) {
         long long e = eoff[a];
         for (int w = a >> 5; w < words; w++) {
@@ -240,7 +258,9 @@ __global__ void k_rips_edge_list(const unsigned *__restrict__ adj, const double 
             if ((bits >> lane) & 1u) {
                 const int b = w * 32 + lane;
                 const long long at = e + __popc(bits & ((1u << lane) - 1u));
-                key[at] = dbits(D[(int64_t)a * n + b]);
+                const double v = D[(int64_t)a * n + b];
+                key[at] = dbits(v);
+                coarse[at] = __double2uint_rd(v * scale);
                 place[at] = (unsigned)at;
                 ends[at] = make_int2(a, b);
             }
@@ -248,31 +268,65 @@ __global__ void k_rips_edge_list(const unsigned *__restrict__ adj, const double 
         }
     }
 }
-
-// All triangles: common neighbours above the second vertex, a warp per edge.
-__global__ void k_rips_total(const unsigned *__restrict__ adj, int words, const int2 *__restrict__ ends, long long E,
-                             unsigned long long *total) {
+// Edges and triangles, counted by pairs of a vertex and 32 others, a warp each.
+__global__ void __launch_bounds__(256) k_rips_total(const unsigned *__restrict__ adj, int n, int words,
+                                                    RipsTotals *totals) {
     const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
-    unsigned long long t = 0;
-    for (long long k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < E; k += nw) {
-        const int2 e = ends[k];
-        for (int w = (e.y >> 5) + lane; w < words; w += 32)
-            t += __popc(adj[(int64_t)e.x * words + w] & adj[(int64_t)e.y * words + w] & above(w, e.y));
+    unsigned long long t = 0, edges = 0;
+    for (long long q = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; q < (long long)n * words; q += nw) {
+        const int a = (int)(q / words), w0 = (int)(q % words);
+        unsigned bits = w0 >= a >> 5 ? adj[(int64_t)a * words + w0] & above(w0, a) : 0u;
+        if (lane == 0) edges += __popc(bits);
+        for (; bits; bits &= bits - 1) {
+            const int b = w0 * 32 + __ffs(bits) - 1;
+            for (int w = w0 + lane; w < words; w += 32)
+                t += __popc(adj[(int64_t)a * words + w] & adj[(int64_t)b * words + w] & above(w, b));
+        }
     }
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0 && t) atomicAdd(total, t);
+    if (lane == 0) {
+        if (t) atomicAdd(&totals->triangles, t);
+        if (edges) atomicAdd(&totals->edges, edges);
+    }
 }
-
-// Sorted edges: the rank of the edge on two vertices, the vertices by rank;
-// *tied when two are equally long.
-__global__ void k_rips_rank(const unsigned long long *__restrict__ key, const unsigned *__restrict__ place,
-                            const int2 *__restrict__ ends, long long E, int n, int32_t *__restrict__ rank,
-                            int2 *__restrict__ by_rank, int *tied) {
+// The edges' ranks from their order by coarse length (32 bits of the length
+// over the longest, half the passes of a sort by all 64): an edge comes after
+// the shorter ones of its coarse length, of which there are few or none.
+// coarse == nullptr: the order is the exact one.  28K edges of a torus: 8 passes
+// of 10 us by 64 bits, 4 by 32; with the host's reads between the steps (7, now
+// 3) a million columns from points to pairs 659 us -> 554.
+constexpr int RIPS_SAME = 64;  // edges of one coarse length
+__global__ void k_rips_rank(const unsigned *__restrict__ coarse, const unsigned long long *__restrict__ key,
+                            const unsigned *__restrict__ place, const int2 *__restrict__ ends, long long E, int n,
+                            int32_t *__restrict__ rank, int2 *__restrict__ by_rank,
+                            unsigned long long *__restrict__ sorted, RipsTotals *totals) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < E; k += (long long)gridDim.x * blockDim.x) {
-        const int2 e = ends[place[k]];
-        by_rank[k] = e;
-        rank[(int64_t)e.x * n + e.y] = rank[(int64_t)e.y * n + e.x] = (int32_t)k;
-        if (k > 0 && key[k] == key[k - 1]) *tied = 1;
+        const unsigned p = place[k];
+        const int2 e = ends[p];
+        const unsigned long long mine = key[p];
+        long long at = k;
+        if (coarse) {
+            const unsigned c = coarse[k];
+            int same = 0;
+            bool tied = false;
+            for (long long q = k - 1; q >= 0 && coarse[q] == c && same < RIPS_SAME; q--, same++) {
+                const unsigned long long x = key[place[q]];
+                at -= x > mine;
+                tied |= x == mine;
+            }
+            for (long long q = k + 1; q < E && coarse[q] == c && same < RIPS_SAME; q++, same++) {
+                const unsigned long long x = key[place[q]];
+                at += x < mine;
+                tied |= x == mine;
+            }
+            if (tied) totals->tied = 1;
+            if (same == RIPS_SAME) totals->crowded = 1;
+        } else if (k > 0 && key[place[k - 1]] == mine) {
+            totals->tied = 1;
+        }
+        by_rank[at] = e;
+        sorted[at] = mine;
+        rank[(int64_t)e.x * n + e.y] = rank[(int64_t)e.y * n + e.x] = (int32_t)at;
     }
 }
 
@@ -303,8 +357,10 @@ __device__ __forceinline__ void rips_run(const unsigned *adj, const int32_t *ran
 }
 
 __global__ void k_rips_run_count(const unsigned *__restrict__ adj, const int32_t *__restrict__ rank, int n, int words,
-                                 const int2 *__restrict__ by_rank, long long E, long long *__restrict__ cnt) {
+                                 const int2 *__restrict__ by_rank, long long E, const RipsTotals *__restrict__ totals,
+                                 long long *__restrict__ cnt) {
     const int nw = (gridDim.x * blockDim.x) >> 5;
+    if (totals->crowded) return;  // by_rank has gaps
     for (long long k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < E; k += nw) {
         long long c = 0;
         rips_run(adj, rank, n, words, by_rank[k], (int)k, [&](unsigned mask, bool, int, int) { c += __popc(mask); });
@@ -316,9 +372,10 @@ __global__ void k_rips_run_count(const unsigned *__restrict__ adj, const int32_t
 // before it, toff[k]) with its triangles.
 __global__ void k_rips_write(const unsigned *__restrict__ adj, const int32_t *__restrict__ rank, int n, int words,
                              const int2 *__restrict__ by_rank, const unsigned long long *__restrict__ key, long long E,
-                             const long long *__restrict__ toff, int64_t *__restrict__ colptr,
-                             int32_t *__restrict__ rows, double *__restrict__ value) {
+                             const long long *__restrict__ toff, RipsTotals *totals, int64_t *__restrict__ colptr, int32_t *__restrict__ rows, double *__restrict__ value) {
     const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) totals->triangles = (unsigned long long)toff[E];
+    if (totals->tied || totals->crowded || n + E + toff[E] >= 1ll << 31) return;  // the host sees it afterwards
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         colptr[v] = 0;
         if (value) value[v] = 0.0;
@@ -537,11 +594,23 @@ __attribute__((visibility("default"))) int oph_rips_device(oph_context *ctx, con
     unsigned *adj = (unsigned *)sc.get(sizeof(unsigned) * (size_t)n * words);
     long long *deg = (long long *)sc.get(sizeof(long long) * (size_t)(n + 1));
     long long *eoff = (long long *)sc.get(sizeof(long long) * (size_t)(n + 1));
-    unsigned long long *total = (unsigned long long *)sc.get(2 * sizeof(unsigned long long));
-    if (!D || !adj || !deg || !eoff || !total) return OPH_ERR_OOM;
+    RipsTotals *totals = (RipsTotals *)sc.get(sizeof(RipsTotals));
+    if (!D || !adj || !deg || !eoff || !totals) return OPH_ERR_OOM;
     OPH_CUDA_TRY(cudaMemsetAsync(adj, 0, sizeof(unsigned) * (size_t)n * words, s));
-    OPH_CUDA_TRY(cudaMemsetAsync(total, 0, 2 * sizeof(unsigned long long), s));
-    k_rips_dist<<<grid_of(ctx, (int64_t)n * n), 256, 0, s>>>(d_points, n, d, threshold, D, adj, words);
+    OPH_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(RipsTotals), s));
+    k_rips_dist<<<grid_of(ctx, (int64_t)n * n), 256, 0, s>>>(d_points, n, d, threshold, D, adj, words, totals);
+    RipsTotals t{};
+    if (!d_colptr) {  // sizes only
+        k_rips_total<<<grid_of(ctx, 32 * (int64_t)n * words), 256, 0, s>>>(adj, n, words, totals);
+        OPH_CUDA_TRY(cudaGetLastError());
+        OPH_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, s));
+        OPH_CUDA_TRY(cudaStreamSynchronize(s));
+        const int64_t m = n + (int64_t)(t.edges + t.triangles);
+        if (m >= (1ll << 31)) return OPH_ERR_BAD_INPUT;
+        if (m_out) *m_out = m;
+        if (nnz_out) *nnz_out = 2 * (int64_t)t.edges + 3 * (int64_t)t.triangles;
+        return OPH_OK;
+    }
     k_rips_deg<<<grid_of(ctx, n), 256, 0, s>>>(adj, n, words, deg);
     OPH_CUDA_TRY(cudaMemsetAsync(deg + n, 0, sizeof(long long), s));
     size_t sb = 0;
@@ -554,67 +623,79 @@ __attribute__((visibility("default"))) int oph_rips_device(oph_context *ctx, con
     OPH_CUDA_TRY(cudaStreamSynchronize(s));
     const int wgrid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, (int64_t)ctx->sm_count * 8));
     const int egrid = (int)std::max<int64_t>(1, std::min<int64_t>((E + 7) / 8, (int64_t)ctx->sm_count * 16));
-    // the edges: keys and places twice (the sort's two buffers), vertices in
-    // both orders, ranks, triangles before each
+    // the edges: lengths, coarse lengths and places twice (the sort's two
+    // buffers), vertices in both orders, ranks, triangles before each
     const size_t e1 = (size_t)E + 1;
-    sc.keep(ctx, S_C2_CELLS, (d_colptr ? 4 * nn : 0) + 64 * e1 + (8 << 20));
+    sc.keep(ctx, S_C2_CELLS, 4 * nn + 72 * e1 + (8 << 20));
     unsigned long long *key[2] = {(unsigned long long *)sc.get(8 * e1), (unsigned long long *)sc.get(8 * e1)};
+    unsigned *coarse[2] = {(unsigned *)sc.get(4 * e1), (unsigned *)sc.get(4 * e1)};
     unsigned *place[2] = {(unsigned *)sc.get(4 * e1), (unsigned *)sc.get(4 * e1)};
     int2 *ends = (int2 *)sc.get(8 * e1);
-    if (!key[0] || !key[1] || !place[0] || !place[1] || !ends) return OPH_ERR_OOM;
-    if (E > 0) k_rips_edge_list<<<wgrid, 256, 0, s>>>(adj, D, n, words, eoff, key[0], place[0], ends);
-    if (!d_colptr) {  // sizes only
-        unsigned long long T = 0;
-        if (E > 0) k_rips_total<<<egrid, 256, 0, s>>>(adj, words, ends, E, total);
-        OPH_CUDA_TRY(cudaGetLastError());
-        OPH_CUDA_TRY(cudaMemcpyAsync(&T, total, sizeof(T), cudaMemcpyDeviceToHost, s));
-        OPH_CUDA_TRY(cudaStreamSynchronize(s));
-        const int64_t m = n + E + (int64_t)T;
-        if (m >= (1ll << 31)) return OPH_ERR_BAD_INPUT;
-        if (m_out) *m_out = m;
-        if (nnz_out) *nnz_out = 2 * E + 3 * (int64_t)T;
-        return OPH_OK;
-    }
     int2 *by_rank = (int2 *)sc.get(8 * e1);
     int32_t *rank = (int32_t *)sc.get(4 * nn);
     long long *tcnt = (long long *)sc.get(8 * e1), *toff = (long long *)sc.get(8 * e1);
-    if (!by_rank || !rank || !tcnt || !toff) return OPH_ERR_OOM;
-    cub::DoubleBuffer<unsigned long long> dk(key[0], key[1]);
-    cub::DoubleBuffer<unsigned> dp(place[0], place[1]);
-    OPH_CUDA_TRY(cudaMemsetAsync(tcnt, 0, 8 * e1, s));
-    if (E > 0) {
-        size_t tb = 0;
-        OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dp, E, 0, 64, s));
-        void *tmp = sc.get(tb);
-        if (!tmp) return OPH_ERR_OOM;
-        OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dp, E, 0, 64, s));
-        k_rips_rank<<<grid_of(ctx, E), 256, 0, s>>>(dk.Current(), dp.Current(), ends, E, n, rank, by_rank,
-                                                    (int *)(total + 1));
-        k_rips_run_count<<<egrid, 256, 0, s>>>(adj, rank, n, words, by_rank, E, tcnt);
-    }
+    if (!key[0] || !key[1] || !coarse[0] || !coarse[1] || !place[0] || !place[1] || !ends || !by_rank || !rank ||
+        !tcnt || !toff)
+        return OPH_ERR_OOM;
     size_t sb2 = 0;
     OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, sb2, tcnt, toff, E + 1, s));
     void *st2 = sc.get(sb2);
     if (!st2) return OPH_ERR_OOM;
-    OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(st2, sb2, tcnt, toff, E + 1, s));
-    long long T = 0;
-    int tied = 0;
-    OPH_CUDA_TRY(cudaMemcpyAsync(&tied, total + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OPH_CUDA_TRY(cudaMemcpyAsync(&T, toff + E, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    OPH_CUDA_TRY(cudaStreamSynchronize(s));
-    // (with equally long edges the triangles by last edge add up to the same)
-    const int64_t m = n + E + T, nnz = 2 * E + 3 * T;
+    int64_t m = 0, nnz = 0;
+    for (bool exact = false;; exact = true) {
+        OPH_CUDA_TRY(cudaMemsetAsync(tcnt, 0, 8 * e1, s));
+        unsigned long long *sorted = key[1];
+        if (E > 0) {
+            k_rips_edge_list<<<wgrid, 256, 0, s>>>(adj, D, n, words, eoff, totals, key[0], coarse[0], place[0], ends);
+            cub::DoubleBuffer<unsigned> dp(place[0], place[1]);
+            size_t tb = 0;
+            const unsigned *order = nullptr;
+            const unsigned long long *lengths = key[0];
+            if (!exact) {
+                cub::DoubleBuffer<unsigned> dc(coarse[0], coarse[1]);
+                OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, dc, dp, E, 0, 32, s));
+                void *tmp = sc.get(tb);
+                if (!tmp) return OPH_ERR_OOM;
+                OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, dc, dp, E, 0, 32, s));
+                order = dc.Current();
+            } else {
+                // too many edges of one coarse length: by the lengths themselves, beside which they stay by place
+                unsigned long long *const by_place = (unsigned long long *)sc.get(8 * e1);
+                if (!by_place) return OPH_ERR_OOM;
+                OPH_CUDA_TRY(cudaMemcpyAsync(by_place, key[0], 8 * e1, cudaMemcpyDeviceToDevice, s));
+                OPH_CUDA_TRY(cudaMemsetAsync(&totals->tied, 0, 2 * sizeof(int), s));
+                cub::DoubleBuffer<unsigned long long> dk(key[0], key[1]);
+                OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dp, E, 0, 64, s));
+                void *tmp = sc.get(tb);
+                if (!tmp) return OPH_ERR_OOM;
+                OPH_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dp, E, 0, 64, s));
+                lengths = by_place;
+                sorted = dk.Alternate();
+            }
+            k_rips_rank<<<grid_of(ctx, E), 256, 0, s>>>(order, lengths, dp.Current(), ends, E, n, rank, by_rank, sorted,
+                                                        totals);
+            k_rips_run_count<<<egrid, 256, 0, s>>>(adj, rank, n, words, by_rank, E, totals, tcnt);
+        }
+        OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(st2, sb2, tcnt, toff, E + 1, s));
+        if (d_rows || E == 0)
+            k_rips_write<<<std::max(egrid, 1), 256, 0, s>>>(adj, rank, n, words, by_rank, sorted, E, toff, totals,
+                                                            d_colptr, d_rows, d_value);
+        else
+            OPH_CUDA_TRY(cudaMemcpyAsync(&totals->triangles, toff + E, sizeof(long long), cudaMemcpyDeviceToDevice, s));
+        OPH_CUDA_TRY(cudaGetLastError());
+        OPH_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, s));
+        OPH_CUDA_TRY(cudaStreamSynchronize(s));
+        if (t.crowded && !exact) continue;
+        // (with equally long edges the triangles by last edge add up to the same)
+        m = n + E + (int64_t)t.triangles;
+        nnz = 2 * E + 3 * (int64_t)t.triangles;
+        break;
+    }
     if (m >= (1ll << 31)) return OPH_ERR_BAD_INPUT;
     if (m_out) *m_out = m;
     if (nnz_out) *nnz_out = nnz;
     if (!d_rows && nnz > 0) return OPH_ERR_BAD_INPUT;
-    if (!tied) {
-        k_rips_write<<<std::max(egrid, 1), 256, 0, s>>>(adj, rank, n, words, by_rank, dk.Current(), E, toff, d_colptr,
-                                                        d_rows, d_value);
-        OPH_CUDA_TRY(cudaGetLastError());
-        OPH_CUDA_TRY(cudaStreamSynchronize(s));
-        return OPH_OK;
-    }
+    if (!t.tied) return OPH_OK;
     // equally long edges: one sort of every simplex
     SKey *k0 = (SKey *)sc.get(sizeof(SKey) * (size_t)m), *k1 = (SKey *)sc.get(sizeof(SKey) * (size_t)m);
     int32_t *vpos = (int32_t *)sc.get(sizeof(int32_t) * (size_t)n);

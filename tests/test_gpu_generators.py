@@ -91,6 +91,19 @@ def test_rips_equal_lengths(cuda_lib):
     assert_same(cx.rips_device(pts), cx.rips(pts))
 
 
+@pytest.mark.parametrize("near,far,equal", [(9, 1e3, False), (60, 1e3, False), (60, 1e3, True), (200, 1e30, False),
+                                            (40, 1e-3, True)])
+def test_rips_lengths_of_two_scales(cuda_lib, near, far, equal):
+    """A cluster 1e-9 wide and points far off: lengths that 32 bits of the
+    longest do not tell apart, a few or all of the cluster's, with and without
+    equal ones among them."""
+    pts = np.concatenate([cx.points_cube(near, 6) * 1e-9, far * cx.points_cube(3, 7)])
+    if equal:
+        pts = np.concatenate([pts, pts[:2]])
+    for thr in (np.inf, 2e-9):
+        assert_same(cx.rips_device(pts, thr), cx.rips(pts, thr))
+
+
 @pytest.mark.parametrize("h,w", [(2, 7), (9, 2), (3, 3), (97, 203)])
 def test_lower_star_odd_sides_equal_host(cuda_lib, h, w):
     img = cx.image_smoothed(h, w, h * w)
