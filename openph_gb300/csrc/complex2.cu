@@ -1542,6 +1542,63 @@ __device__ bool in_triangles(const int32_t *col, const int32_t *tab, const uint1
     return wrong;
 }
 
+// The outputs of a whole instance, as k_c2_runs_out writes them, by a CTA: a
+// word a thread, from word `first` on and every `step` words, filled with what
+// a positive triangle gets, 16 bytes a store; then the few vertices, edges and
+// paired triangles are corrected.  Bound by the writes.
+template <int THREADS>
+__device__ __forceinline__ void in_out(const C2Args &a, const C2Inst &in, int first, int step) {
+    const int none = a.one_based ? 0 : -1, tid = threadIdx.x;
+    auto fill = [&](int32_t *p, int n, int value) {
+        const int head = min(n, (int)((16 - ((uintptr_t)p & 15)) & 15) / 4), body = (n - head) / 4;
+        if (tid < head) p[tid] = value;
+        int4 *q = reinterpret_cast<int4 *>(p + head);
+        for (int i = tid; i < body; i += THREADS) q[i] = make_int4(value, value, value, value);
+        const int at = head + 4 * body + tid;
+        if (at < n) p[at] = value;
+    };
+    const C2Word *const words = a.words + in.woff;
+    const int nw = (int)((in.cols + 31) >> 5);
+    int32_t *const low = a.low + in.base, *const ess = a.ess ? a.ess + in.base : nullptr;
+    for (int c0 = 32 * first; c0 < in.cols; c0 += 32 * step) {
+        const int n = min(32 * THREADS, (int)in.cols - c0);
+        fill(low + c0, n, none);
+        if (ess) fill(ess + c0, n, 1);
+        __syncthreads();
+        const int wi = (c0 >> 5) + tid;
+        if (wi < nw) {
+            const C2Word w = words[wi];
+            const unsigned prev = wi > 0 ? words[wi - 1].e >> 31 : 0u, notri = w.v | w.e;
+            const int end = min(32, (int)in.cols - 32 * wi);
+            const unsigned here = end == 32 ? ~0u : below(end);
+            const unsigned open = (w.e << 1 | prev) & ~notri & here;  // first triangles: paired with the edge before
+            a.owned[in.woff + wi] = open;
+            a.fixed[in.woff + wi] = open;
+            for (unsigned x = open; x; x &= x - 1) {
+                const int j = 32 * wi + __ffs(x) - 1;
+                low[j] = j - 1 + a.one_based;
+                if (ess) ess[j] = 0;
+            }
+            if (ess)
+                for (unsigned x = w.v; x; x &= x - 1) {
+                    const int j = 32 * wi + __ffs(x) - 1;
+                    if (a.dead[in.voff + j]) ess[j] = 0;
+                }
+            // bit x: the column after x is no triangle, or past the instance's end
+            const unsigned next = notri >> 1 | (wi + 1 < nw ? (words[wi + 1].v | words[wi + 1].e) << 31 : ~(here >> 1));
+            int k = w.epre;
+            for (unsigned x = w.e; x; x &= x - 1, k++) {
+                const int bit = __ffs(x) - 1, j = 32 * wi + bit, y = a.neg[k];
+                const bool run = !((next >> bit) & 1u);
+                if (y >= 0) low[j] = y + a.one_based;
+                if (y < 0 && !run) a.res[atomicAdd(&a.st->nres, 1)] = k;
+                else if (ess) ess[j] = 0;
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // The order instances are taken in when there are more than CTAs: the largest
 // first (to 2,048 columns), or the last to start may be one of 300 us when the
 // others are done.  One CTA; its 6 us are those of its chain of steps.
@@ -1574,6 +1631,7 @@ __global__ void __launch_bounds__(1024) k_c2_inst_order(C2Args a) {
     for (int b = threadIdx.x; b < a.count; b += 1024) a.order[atomicAdd(&s_at[cls(b)], 1)] = b;
 }
 
+template <bool OUT>
 __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
     extern __shared__ __align__(16) unsigned char in_smem[];  // IN_SMEM
     constexpr int NW = IN_THREADS / 32;
@@ -1773,6 +1831,9 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         if (wrong) s_no = 1;
         __syncthreads();
         if (tid == 0 && s_no) a.st->refused = 1;
+        // a single small one's outputs at once: 12 points 54 us -> 46-50 in all
+        if constexpr (OUT)
+            if (!s_no && !a.st->refused) in_out<IN_THREADS>(a, in, 0, IN_THREADS);
         __syncthreads();
     }
 }
@@ -1841,64 +1902,13 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst_more(C2Args a) {
     }
 }
 
-// The outputs of whole instances, as k_c2_runs_out writes them: IO_COLS
-// columns a block are filled with what a positive triangle gets, 16 bytes a
-// store, then a thread per word corrects the few vertices, edges and paired
-// triangles.  Bound by the writes.
+// The outputs, IO_COLS columns a block.
 constexpr int IO_THREADS = 256, IO_COLS = 32 * IO_THREADS;
 __global__ void __launch_bounds__(IO_THREADS) k_c2_inst_out(C2Args a, int parts) {
     if (a.st->refused || a.st->no_room) return;
-    const int none = a.one_based ? 0 : -1, tid = threadIdx.x;
-    auto fill = [&](int32_t *p, int n, int value) {
-        const int head = min(n, (int)((16 - ((uintptr_t)p & 15)) & 15) / 4), body = (n - head) / 4;
-        if (tid < head) p[tid] = value;
-        int4 *q = reinterpret_cast<int4 *>(p + head);
-        for (int i = tid; i < body; i += IO_THREADS) q[i] = make_int4(value, value, value, value);
-        const int at = head + 4 * body + tid;
-        if (at < n) p[at] = value;
-    };
     for (int b = blockIdx.x / parts; b < a.count; b += gridDim.x / parts) {
         const C2Inst in = a.inst[b];
-        const C2Word *const words = a.words + in.woff;
-        const int nw = (int)((in.cols + 31) >> 5);
-        int32_t *const low = a.low + in.base, *const ess = a.ess ? a.ess + in.base : nullptr;
-        for (int c0 = (blockIdx.x % parts) * IO_COLS; c0 < in.cols; c0 += parts * IO_COLS) {
-            const int n = min(IO_COLS, (int)in.cols - c0);
-            fill(low + c0, n, none);
-            if (ess) fill(ess + c0, n, 1);
-            __syncthreads();
-            const int wi = (c0 >> 5) + tid;
-            if (wi < nw) {
-                const C2Word w = words[wi];
-                const unsigned prev = wi > 0 ? words[wi - 1].e >> 31 : 0u, notri = w.v | w.e;
-                const int end = min(32, (int)in.cols - 32 * wi);
-                const unsigned here = end == 32 ? ~0u : below(end);
-                const unsigned open = (w.e << 1 | prev) & ~notri & here;  // first triangles: paired with the edge before
-                a.owned[in.woff + wi] = open;
-                a.fixed[in.woff + wi] = open;
-                for (unsigned x = open; x; x &= x - 1) {
-                    const int j = 32 * wi + __ffs(x) - 1;
-                    low[j] = j - 1 + a.one_based;
-                    if (ess) ess[j] = 0;
-                }
-                if (ess)
-                    for (unsigned x = w.v; x; x &= x - 1) {
-                        const int j = 32 * wi + __ffs(x) - 1;
-                        if (a.dead[in.voff + j]) ess[j] = 0;
-                    }
-                // bit x: the column after x is no triangle, or past the instance's end
-                const unsigned next = notri >> 1 | (wi + 1 < nw ? (words[wi + 1].v | words[wi + 1].e) << 31 : ~(here >> 1));
-                int k = w.epre;
-                for (unsigned x = w.e; x; x &= x - 1, k++) {
-                    const int bit = __ffs(x) - 1, j = 32 * wi + bit, y = a.neg[k];
-                    const bool run = !((next >> bit) & 1u);
-                    if (y >= 0) low[j] = y + a.one_based;
-                    if (y < 0 && !run) a.res[atomicAdd(&a.st->nres, 1)] = k;
-                    else if (ess) ess[j] = 0;
-                }
-            }
-            __syncthreads();
-        }
+        in_out<IO_THREADS>(a, in, (int)(blockIdx.x % parts) * IO_THREADS, parts * IO_THREADS);
     }
 }
 
@@ -2082,7 +2092,8 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
     static int ready[64];
     int &ok = ready[ctx->device & 63];
     if (!ok) {
-        if (cudaFuncSetAttribute(k_c2_inst, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess ||
+        if (cudaFuncSetAttribute(k_c2_inst<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_c2_inst<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess ||
             cudaFuncSetAttribute(k_c2_inst_more, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess) {
             cudaGetLastError();
             return OPH_OK;
@@ -2102,6 +2113,7 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
     // took 394 us whole and 405-420 split, 256 of 20 to 120 points 983 us whole and 690 split
     a.split_cols = (int)std::min<int64_t>(INT_MAX, m / slots * 3 / 4);
     a.chunk = m / a.count < IN_SPLIT ? 0 : (int)std::max<int64_t>(64, std::min<int64_t>(512, m / (40 * 2 * slots))) & ~7;
+    const bool out_here = a.count == 1 && !a.chunk;
     for (int tries = 0; tries < 2; tries++) {
         a.cap_e = need[0];
         a.cap_v = need[1];
@@ -2152,19 +2164,23 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
             k_c2_inst_order<<<1, 1024, 0, s>>>(a);
             ctx->launches++;
         }
-        k_c2_inst<<<std::min(a.count, slots), IN_THREADS, IN_SMEM, s>>>(a);
+        if (out_here) k_c2_inst<true><<<1, IN_THREADS, IN_SMEM, s>>>(a);
+        else k_c2_inst<false><<<std::min(a.count, slots), IN_THREADS, IN_SMEM, s>>>(a);
         if (a.chunk) {
             k_c2_inst_more<<<(int)std::min<int64_t>(slots, a.cap_e / a.chunk + 1), IN_THREADS, IN_SMEM, s>>>(a);
             ctx->launches++;
         }
         // enough blocks for the outputs of one instance as of many
         const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(16, (m / a.count + IO_COLS - 1) / IO_COLS));
-        k_c2_inst_out<<<parts * std::min(a.count, 65535), IO_THREADS, 0, s>>>(a, parts);
+        if (!out_here) {
+            k_c2_inst_out<<<parts * std::min(a.count, 65535), IO_THREADS, 0, s>>>(a, parts);
+            ctx->launches++;
+        }
         if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
         // a residual edge or so per vertex
         const int rg = (int)std::min<int64_t>(gr, std::max<int64_t>(1, a.cap_e));
         k_c2_residual<true, RS_SMALL, RS_SMALL_WORDS><<<rg, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
-        ctx->launches += 3;
+        ctx->launches += 2;
         cudaEventRecord(ctx->ev[1], s);
         int rc = c2_read_status(ctx, a, hs);
         if (rc) return rc;
