@@ -380,6 +380,8 @@ ROOFLINE_NOTES = {
     "tier3": "latency-bound: chains of dependent additions on a few long columns of the anti-transpose "
              "(each addition waits on its low's pivot record, then the pivot's rows, from L2 or HBM); the "
              "merge-equivalent bytes are what a merge would move, far above the kernels' DRAM traffic",
+    "direct": "latency- and issue-bound: half of the time is the longest residual column's waves of additions on "
+              "one SM, the rest the check of every triangle against its run; each input byte is read once",
     "narrow": "instruction-issue-bound (ncu: 60-89% issue active, DRAM 1-2%); T stays on chip per chain",
 }
 
@@ -540,7 +542,7 @@ def run_torus(args, ws, rank, local, bm, dist):
     # each tier on the library's stream): its algorithmic bytes are the
     # per-addition figure 4 (|P| + |T| + |T xor P|) summed over the additions
     # it performed (counted on the device), per launch, over its mean launch
-    # time.  On the anti-transpose that is tier 3's bitmap kernel.
+    # time.
     comps = {"narrow": (narrow_ms, slot_prof["tier_slots"][0],
                         "k_p2_scalar + k_p2_tier<8,128,256> (scalar tier and tier 0, a pair per sweep)"),
              "tier1": (tier_ms[0], slot_prof["tier_slots"][1], "k_p2_tier1<32,512,256> (tier 1)"),
@@ -548,6 +550,13 @@ def run_torus(args, ws, rank, local, bm, dist):
              "tier3": (tier_ms[2], slot_prof["tier_slots"][3],
                        "k_p2_bitmap<1024> + k_p2_cluster<8> (tier 3: bitmap columns in one CTA's shared window, "
                        "wider ones across a cluster's shared memory; one launch of each per sweep)")}
+    # without the column store (simplicial 2-complexes: no sweeps, so no
+    # Phase I) the whole reduction is one component: the matrix read once and
+    # the outputs written once
+    if p1_ms == 0.0 and narrow_ms == 0.0:
+        comps = {"direct": (setup_ms + tier_ms[2], (8 * (m + 1) + 4 * nnz + 8 * m) // 4,
+                            "k_c2_words, k_c2_scan, k_c2_lists, k_c2_edges, k_c2_triangles, k_c2_runs_out, "
+                            "k_c2_residual (the whole reduction)")}
     dom = max(comps, key=lambda k: comps[k][0])
     dom_ms, dom_slots, dom_name = comps[dom]
     per_red_dom_s = dom_ms / 1e3 / args.steps
@@ -583,7 +592,8 @@ def run_torus(args, ws, rank, local, bm, dist):
                                "tier2": tier_ms[1] / args.steps, "tier3": tier_ms[2] / args.steps,
                                "total_launched_one_by_one": profiled_ms,
                                "note": "a second pass of the same steps with events around every phase "
-                                       "(no CUDA graph); the headline pass replays the captured sweeps"},
+                                       "(no CUDA graph; without the column store, setup_and_transpose is all up to "
+                                       "the residual columns and tier3 those)"},
         "matrix_reduced": "anti-transpose D' (OPH_DUAL_AUTO)" if infos[-1]["dual"] else "D",
         "sweeps": infos[-1]["sweeps"], "device_additions": infos[-1]["additions"],
         "device_slots_per_tier": slot_prof["tier_slots"],

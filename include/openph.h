@@ -88,15 +88,20 @@ typedef struct oph_context oph_context;
 
 typedef struct {
     int32_t num_iters;       /* iterations as the reference counts them        */
-    int32_t sweeps;          /* pms sweeps (0 for the sequential variants)     */
-    int64_t additions;       /* column additions performed on the device       */
+    int32_t sweeps;          /* pms sweeps (0 for the sequential variants; of a
+                                2-complex reduced without the column store,
+                                the rounds of its graph, or 1)                */
+    int64_t additions;       /* column additions performed on the device (how
+                                many depends on the order they met in)        */
     int64_t slots_moved;     /* sum over additions of |P| + |T| + |T xor P|    */
-    int64_t pool_bytes;      /* column-store bytes in use at the end           */
+    int64_t pool_bytes;      /* column-store bytes in use at the end (without
+                                the store: bytes of the tables in its place)  */
     int32_t regrows;         /* times the column store had to grow             */
     float device_ms;         /* device time of the reduction (CUDA events)     */
     int32_t dual;            /* 1 when pms reduced the anti-transpose, 2 when
                                 some blocks of D were reduced on D' and the
-                                others on D                                   */
+                                others on D (without the column store: what
+                                OPH_DUAL_AUTO names for the matrix)           */
 } oph_info;
 
 /* A context owns one CUDA stream on one device plus cached device buffers;
@@ -151,7 +156,10 @@ int oph_reduce_batch_device(oph_context *ctx, int algo, int32_t count, const int
  * one block-diagonal column space, admits queued requests between sweeps
  * while they fit in the device arena (budget_bytes of HBM, allocated up
  * front), and releases each request as soon as it has converged.  At most
- * max_active requests are on the device at once.  Each request is reduced on
+ * max_active requests are on the device at once.  Simplicial 2-complexes need
+ * no sweeps: four lanes beside the worker, each with a context of its own,
+ * reduce them as they come; the others, and those the lanes cannot take, join
+ * the sweeps (OPH_SERVE_CHAIN_CAP set: all of them).  There each request is reduced on
  * the matrix a single-matrix pms reduction would choose for it (OPH_DUAL_AUTO
  * below: a Rips-like request through its anti-transpose, built at
  * admission; a request split by block as two parts side by side, the D part

@@ -21,16 +21,27 @@
 // (k_c2_graph), which takes a dozen rounds.
 //
 // Triangles with more on an edge (Rips complexes) are reduced on D' too, but
-// D' is never built column by column.  A table holds, for every edge and
-// vertex, the triangle they span: a triangle writes its three entries with
-// no count, scan, cursor or sort, and an edge's row of it is its column of
-// D'.  The edges that the graph of edges on vertices pairs are cleared
-// (c2_kruskal); an edge whose first triangle has it as its last edge is
-// paired with it at once, as nothing can be added to either (an apparent
+// D' is never built column by column.  A Rips filtration puts the triangles
+// right after their last edge, third vertices ascending, so a bit per edge and
+// vertex names them all (runs; the whole complex is checked against that).
+// Triangles in any other order are found through a table that holds, for
+// every edge and vertex, the triangle they span, written with no count, scan,
+// cursor or sort.  The edges that the graph of edges on vertices pairs are
+// cleared (c2_kruskal); an edge whose first triangle has it as its last edge
+// is paired with it at once, as nothing can be added to either (an apparent
 // pair: 98-99% of a Rips complex's edges).  What is left (107 of 58,988 edges
 // on the 5M-column torus) is reduced a column per CTA (k_c2_residual).
 //
-// What is accepted is checked on the device before anything is written: every
+// Rips complexes that fit a CTA's shared memory go from colptr to runs in one
+// launch, a CTA each (k_c2_inst; the larger ones of a batch in pieces,
+// k_c2_inst_more); others by a launch per step over all columns.
+//
+// Which form (reduce_complex2): a single matrix of at most 2^15 columns, or a
+// batch of at least 128 or of that size on average, as whole instances; else,
+// or where one of them does not fit, the graph when three triangles come to
+// at most two edges, the runs, the table.
+//
+// What is accepted is checked on the device before it is reported: every
 // column has 0, 2 or 3 rows, ascending and in range, the rows of an edge are
 // vertices, the rows of a triangle are the three edges of a triangle (so
 // D D = 0, which clearing relies on).  Anything else, malformed input
@@ -1505,7 +1516,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
 //
 // Against a launch per step over all columns this saves the launches, which
 // are all that the smallest complexes cost, and the trips to L2 for tables
-// that fit a CTA: 24 instructions a warp for 32 vertices of an edge are what
+// that fit a CTA: 47 instructions a warp for 32 vertices of an edge are what
 // bounds it.  Whatever is no flag complex in runs, vertices first, or does
 // not fit (`refused`; malformed matrices too) is left to the grid-wide kernels.
 //
