@@ -10,8 +10,10 @@
 //     the algorithm has it; a column that holds a low which one to its left
 //     comes to as well gives it up and goes on.  The lows of a reduced matrix
 //     are unique, so they are those of the walk, and twist clears, dimension
-//     by dimension, the columns it would.  So is row where only the lows are
-//     asked for.
+//     by dimension, the columns it would.
+//   * row: the lows are the same ones.  The CPU form's running essential
+//     estimate follows from every column's own additions, replayed side by
+//     side once the pairs are known (k_row_exact).
 //   * standard / twist with trackers, which follow the walk itself, and twist
 //     on matrices whose dimensions do not separate, where the clearing depends
 //     on the order: one launch in which a single warp walks the columns in
@@ -20,7 +22,7 @@
 //     so that columns needing no addition are retired 32 at a time; a column
 //     that needs additions is reduced by the whole warp with the column kept
 //     in shared memory across its chain of additions.
-//   * row with the running essential estimate or trackers: one CTA walks the
+//   * row with trackers, or where the replay finds no room: one CTA walks the
 //     rows from the bottom; a warp finds the next row with two or more columns
 //     on it (per-row buckets), and the CTA's 32 warps add the row's pivot into
 //     all of that row's other columns in parallel (mark_neighbours /
@@ -628,6 +630,182 @@ __global__ void k_claim_clear(ClaimArgs a) {
         if (a.dim[j] == a.want_dim && a.low[j] >= 0) a.low[a.low[j]] = -1;
 }
 
+// ------------------------------------- the row form's running estimate
+// The row algorithm adds the first column with low i into the others with that
+// low, so each column goes through the lows that it meets when it adds the
+// reduced columns to its left one by one, whatever the order of the rows; the
+// running estimate (ph_row.cu:2-31) follows from who met which low, and over
+// which row.  With the pairs known (k_claim), k_row_exact takes the columns in
+// order, a warp each, and waits for the reduced columns it adds: all to its
+// left, so the first unfinished one never waits.  Every low met is an event;
+// k_row_marks finds, for a low, the columns that were the first ever to hold
+// it when they came to it.
+// Bound by the longest chain of columns that wait for one another.  One CTA
+// walking the rows takes a few microseconds a row: 6.6 ms for an image of some
+// 40 x 40, now 0.32 to the call's end; 205 ms of device time on 128 x 128, now
+// 3.5 (1.2 of it k_claim).
+struct RowArgs {
+    int64_t m;
+    const int64_t *colptr;
+    const Holder *holder;     // final
+    unsigned long long *done; // a reduced column: segment / 4 << 32 | rows; 0: not yet
+    int32_t *ess;
+    int *first;               // the first column to start with each low
+    int *count, *place;       // events of each low, and where they go
+    int *ev_low;              // the events: low met, from which row, by which column
+    int2 *ev;
+    int2 *sorted;
+    unsigned *n_ev;
+    unsigned cap;
+    int *quit;                // no room, or a wait that did not end: the walk does it
+    ClaimArgs c;              // for the columns' additions
+};
+
+constexpr int ROW_WAIT = 1 << 22;  // looks at a column to the left, a few seconds
+template <class Column>
+__global__ void __launch_bounds__(CL_THREADS) k_row_exact(RowArgs a) {
+    extern __shared__ __align__(16) int smem[];  // a.c.words a warp
+    const Tile32 tile = cg::tiled_partition<32>(cg::this_thread_block());
+    const int lane = tile.thread_rank();
+    __shared__ int s_pick[CL_WARPS][32];
+    Column c;
+    c.init(tile, a.c, smem + (size_t)(threadIdx.x >> 5) * a.c.words, s_pick[threadIdx.x >> 5]);
+    long long adds = 0, slots = 0;
+    int *const pool = a.c.pool;
+    bool quit = false;
+    while (!quit) {
+        long long idx = 0;
+        if (lane == 0) idx = *(volatile int *)a.quit ? a.m : (long long)atomicAdd(&a.c.count->next, 1ull);
+        idx = tile.shfl(idx, 0);
+        if (idx >= a.m) break;
+        const int j = (int)idx;
+        const int64_t c0 = a.colptr[j];
+        const int n = (int)(a.colptr[j + 1] - c0);
+        if (n == 0) continue;
+        long long seg = 8ll * j + 4 * ((c0 + 3) >> 2);  // as k_setup_columns put it
+        const int *R = pool + seg + SEG_HDR;
+        int l = R[n - 1];
+        if (lane == 0) atomicMin(a.first + l, j);
+        int q = a.holder[l].col, rows = n;
+        c.start();
+        if (q != j && !c.add(tile, a.c, lane < n ? R[lane] : 0, R, n)) quit = true;
+        while (!quit && l >= 0 && q != j) {
+            // the reduced column with this low, to the left
+            unsigned long long d = 0;
+            if (lane == 0 && q >= 0 && q < j)
+                for (int tries = 0; tries < ROW_WAIT; tries++) {
+                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(d) : "l"(a.done + q) : "memory");
+                    if (d || ((tries & 255) == 255 && *(volatile int *)a.quit)) break;
+                    if (tries > 16) __nanosleep(100);
+                }
+            d = tile.shfl(d, 0);
+            tile.sync();
+            const int np = (int)(unsigned)d, before = c.n;
+            const int *P = pool + (long long)(d >> 32 << 2) + SEG_HDR;
+            if (!d || !c.add(tile, a.c, lane < np ? P[lane] : 0, P, np)) {
+                quit = true;
+                break;
+            }
+            adds++;
+            slots += before + np + c.n;
+            const int nl = c.low;
+            if (lane == 0) {
+                a.ess[l] = 0;
+                a.ess[q] = 0;
+                if (nl >= 0) {
+                    const unsigned e = atomicAdd(a.n_ev, 1u);
+                    if (e < a.cap) {
+                        a.ev_low[e] = nl;
+                        a.ev[e] = make_int2(l, j);
+                        atomicAdd(a.count + nl, 1);
+                    }
+                    quit = e >= a.cap;
+                }
+            }
+            quit = tile.any(quit);
+            l = nl;
+            if (l >= 0) q = a.holder[l].col;
+            rows = c.n;
+        }
+        if (!quit && l >= 0) {  // a pivot: its reduced rows for those to its right
+            if (c.n) {
+                if (lane == 0) seg = pool_alloc(a.c.st, SEG_HDR + round4(rows));
+                seg = tile.shfl(seg, 0);
+                if (seg < 0) quit = true;
+                else c.write(tile, pool + seg + SEG_HDR);
+            }
+            tile.sync();
+            if (!quit && lane == 0)
+                asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(a.done + j),
+                             "l"((unsigned long long)(seg >> 2) << 32 | (unsigned)rows)
+                             : "memory");
+        }
+        c.end(tile);
+    }
+    if (lane == 0) {
+        if (quit) atomicExch(a.quit, 1);
+        if (adds) {
+            atomicAdd(&a.c.st->additions, (unsigned long long)adds);
+            atomicAdd(&a.c.st->slots, (unsigned long long)slots);
+        }
+    }
+}
+
+// place[r] = events of the lows before r.  One CTA.
+__global__ void __launch_bounds__(1024) k_row_places(RowArgs a) {
+    __shared__ int s_sum[32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    int run = 0;
+    for (int64_t r0 = 0; r0 < a.m; r0 += 1024) {
+        const int64_t r = r0 + tid;
+        const int x = r < a.m ? a.count[r] : 0;
+        int incl = x;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) s_sum[wid] = incl;
+        __syncthreads();
+        const int w = s_sum[lane];
+        const int before = __reduce_add_sync(0xffffffffu, lane < wid ? w : 0);
+        if (r < a.m) a.place[r] = run + before + incl - x;
+        run += __reduce_add_sync(0xffffffffu, w);
+        __syncthreads();
+    }
+}
+__global__ void k_row_scatter(RowArgs a) {
+    if (*a.quit) return;
+    const unsigned n = *a.n_ev;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
+        a.sorted[atomicAdd(a.place + a.ev_low[e], 1)] = a.ev[e];
+}
+// A low a warp.  Rows come in descending order, so the columns that are first
+// when they come are found by steps: of those left of the first so far, the
+// ones over the largest row, and the leftmost of them.
+__global__ void __launch_bounds__(256) k_row_marks(RowArgs a) {
+    if (*a.quit) return;
+    const int lane = threadIdx.x & 31;
+    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < a.m;
+         r += (int64_t)gridDim.x * blockDim.x >> 5) {
+        const int n = a.count[r];
+        const int2 *const ev = a.sorted + (a.place[r] - n);  // place: past them, after the scatter
+        for (int first = a.first[r];;) {
+            int row = -1, col = INT_MAX;
+            for (int i = lane; i < n; i += 32) {
+                const int2 e = ev[i];
+                if (e.y < first && (e.x > row || (e.x == row && e.y < col))) row = e.x, col = e.y;
+            }
+            const int top = __reduce_max_sync(0xffffffffu, row);
+            if (top < 0) break;
+            first = __reduce_min_sync(0xffffffffu, row == top ? col : INT_MAX);
+            if (lane == 0) a.ess[first] = a.ess[r] = 0;
+        }
+    }
+}
+__global__ void k_row_ones(int64_t m, int32_t *ess) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) ess[j] = 1;
+}
+
 // Row buckets: every column with a low joins the bucket of that row;
 // pivots[r] = the first column holding low r (ph_row.cu:56-59).
 __global__ void k_row_buckets(SeqArgs a) {
@@ -896,6 +1074,71 @@ static int claim_columns(Context *ctx, Work &w, int top, bool twist, int *regrow
     return claim_columns_as<ListColumn>(ctx, w, 3 * CL_CAP, top, twist, regrows);
 }
 
+// The row form's running estimate in ess[], after claim_columns; *done false
+// (ess as it was) when events or columns find no room.
+template <class Column>
+static int row_estimate(Context *ctx, Work &w, int words, int32_t *ess, bool *done) {
+    cudaStream_t s = ctx->stream;
+    const int64_t m = w.m;
+    *done = false;
+    const int64_t cap = std::min<int64_t>(16 * m + (1 << 16), 1ll << 30);
+    auto r256 = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    const size_t at[] = {r256(256 + sizeof(ClaimCount)), r256(8 * (size_t)m), r256(4 * (size_t)m), r256(4 * (size_t)m),
+                         r256(4 * (size_t)m), r256(4 * (size_t)cap), r256(8 * (size_t)cap), r256(8 * (size_t)cap)};
+    size_t off[9] = {};
+    for (int q = 0; q < 8; q++) off[q + 1] = off[q] + at[q];
+    char *tmp = (char *)ctx_alloc(ctx, S_TMP, off[8]);
+    if (!tmp) return OPH_OK;
+    RowArgs a{};
+    a.m = m; a.colptr = w.colptr; a.ess = ess; a.cap = (unsigned)cap;
+    a.holder = reinterpret_cast<const Holder *>(w.rec);
+    a.n_ev = reinterpret_cast<unsigned *>(tmp);
+    a.quit = reinterpret_cast<int *>(tmp + 64);
+    a.c.count = reinterpret_cast<ClaimCount *>(tmp + 128);
+    a.done = reinterpret_cast<unsigned long long *>(tmp + off[1]);
+    a.count = reinterpret_cast<int *>(tmp + off[2]);
+    a.first = reinterpret_cast<int *>(tmp + off[3]);
+    a.place = reinterpret_cast<int *>(tmp + off[4]);
+    a.ev_low = reinterpret_cast<int *>(tmp + off[5]);
+    a.ev = reinterpret_cast<int2 *>(tmp + off[6]);
+    a.sorted = reinterpret_cast<int2 *>(tmp + off[7]);
+    a.c.m = m; a.c.pool = w.pool; a.c.st = w.st; a.c.words = words;
+    OPH_CUDA_TRY(cudaMemsetAsync(tmp, 0, off[3], s));
+    OPH_CUDA_TRY(cudaMemsetAsync(a.first, 0x7f, 4 * (size_t)m, s));
+    OPH_CUDA_TRY(cudaMemsetAsync(&w.st->additions, 0, 2 * sizeof(unsigned long long), s));  // these are the row form's
+    static bool attr = false;
+    if (!attr) {
+        OPH_CUDA_TRY(cudaFuncSetAttribute(k_row_exact<Column>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(int) * CL_WARPS * CL_BITS));
+        attr = true;
+    }
+    const size_t smem = sizeof(int) * CL_WARPS * (size_t)words;
+    const int64_t per_sm = std::min<int64_t>(2048 / CL_THREADS, (220 << 10) / (smem + 2048));
+    const int grid = (int)std::min<int64_t>((m + CL_WARPS - 1) / CL_WARPS, ctx->sm_count * per_sm);
+    const int grid_m = (int)std::max<int64_t>(1, std::min<int64_t>((m + 255) / 256, (int64_t)ctx->sm_count * 16));
+    k_row_exact<Column><<<grid, CL_THREADS, smem, s>>>(a);
+    k_row_places<<<1, 1024, 0, s>>>(a);
+    k_row_scatter<<<ctx->sm_count * 4, 256, 0, s>>>(a);
+    k_row_marks<<<ctx->sm_count * 8, 256, 0, s>>>(a);
+    ctx->launches += 4;
+    OPH_CUDA_TRY(cudaGetLastError());
+    int *const quit = reinterpret_cast<int *>(ctx->h_status + 1);
+    OPH_CUDA_TRY(cudaMemcpyAsync(quit, a.quit, sizeof(int), cudaMemcpyDeviceToHost, s));
+    OPH_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, w.st, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
+    OPH_CUDA_TRY(cudaStreamSynchronize(s));
+    *done = !*quit;
+    if (*quit) {
+        k_row_ones<<<grid_m, 256, 0, s>>>(m, ess);
+        ctx->launches++;
+    }
+    return OPH_OK;
+}
+static int row_estimate(Context *ctx, Work &w, int32_t *ess, bool *done) {
+    const int64_t words = ((w.m + 31) / 32 + 31) / 32 * 32;
+    if (words <= CL_BITS) return row_estimate<BitColumn>(ctx, w, (int)words, ess, done);
+    return row_estimate<ListColumn>(ctx, w, 3 * CL_CAP, ess, done);
+}
+
 // The columns as they came, for a walk after columns side by side did not fit.
 static int restart_store(Context *ctx, Work &w, SeqArgs &a) {
     const int rc = setup_store(ctx, w, false);
@@ -994,20 +1237,22 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
         a.row_quirk = (algo == OPH_ALGO_PH_ROW) && d_ess != nullptr;
         SeqTracking *tk = ctx->seq_track;
         long long *ev_base = nullptr;
-        // without the running estimate and trackers only the lows are asked
-        // for, which are those of the columns side by side
-        bool side_by_side = !tk && !a.row_quirk;
+        // without trackers: the lows, which are those of the columns side by
+        // side, and the running estimate where it is asked for
+        bool side_by_side = !tk;
         if (side_by_side) {
             int rc = claim_columns(ctx, w, -1, false, &regrows);
-            if (rc == OPH_ERR_OOM || rc == OPH_ERR_OVERFLOW) {
+            bool done = rc == OPH_OK;
+            if (done && a.row_quirk) rc = row_estimate(ctx, w, d_ess, &done);
+            if (rc && rc != OPH_ERR_OOM && rc != OPH_ERR_OVERFLOW) return rc;
+            if (!done) {
                 side_by_side = false;
-                rc = restart_store(ctx, w, a);
-                // claim_columns used this slot
+                if ((rc = restart_store(ctx, w, a))) return rc;
+                // both used this slot
                 a.bhead = (int32_t *)ctx_alloc(ctx, S_TMP, sizeof(int32_t) * (3 * m + 1));
-                if (!rc && !a.bhead) rc = OPH_ERR_OOM;
+                if (!a.bhead) return OPH_ERR_OOM;
                 a.bnext = a.bhead + m; a.bcnt = a.bnext + m;
             }
-            if (rc) return rc;
         }
         if (tk) {
             // the initial lows and a log of the walk's additions for the

@@ -22,6 +22,7 @@ SHAPES = {
     "image": lambda: cx.lower_star_image(60, 71, seed=4, sigma=0.5),
     "smooth": lambda: cx.lower_star_image(45, 90, seed=6, sigma=6.0),
     "large": lambda: cx.lower_star_image(110, 113, seed=4, sigma=2.0),
+    "circle": lambda: cx.rips(cx.points_circle(25, 2), np.inf),
 }
 
 
@@ -72,3 +73,63 @@ def plain(cols, algo):
             if algo == "twist":
                 low[low[j]] = -1
     return np.array(low, np.int32)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("pool", [0, 1])
+def test_row_estimate(cuda_lib, shape, pool):
+    """The CPU row form's running essential estimate, replayed side by side."""
+    bm = SHAPES[shape]()
+    want, want_ess, st = oracle.ph_row(bm)
+    with Context(0) as c:
+        if pool:
+            c.set_limits(initial_pool_bytes=pool)
+        low, ess, info = c.reduce(bm, "ph_row")
+    np.testing.assert_array_equal(low, want)
+    np.testing.assert_array_equal(ess, want_ess)
+    assert info["additions"] == st["additions"]
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_row_estimate_of_any_matrix(ctx, seed):
+    """The same on columns that are no complex's boundaries, among them many
+    with equal lows (the oracle's row form adds within one dimension only, so
+    the walk over all columns is restated here)."""
+    rng = np.random.default_rng(seed)
+    m, rows = 150, (150, 20)[seed % 2]
+    cols = [sorted(rng.choice(min(rows, max(j, 1)), size=min(int(rng.integers(0, 6)), j), replace=False).tolist())
+            for j in range(m)]
+    bm = BoundaryMatrix.from_columns(cols)
+    want, want_ess = plain_row(cols)
+    low, ess, _ = ctx.reduce(bm, "ph_row")
+    np.testing.assert_array_equal(low, want)
+    np.testing.assert_array_equal(ess, want_ess)
+
+
+def plain_row(cols):
+    """Rows from the bottom: the first column with the row as its low into the
+    others; the estimate cleared at the row and the first column, and at a
+    column that is then the first ever to hold its new low, and at that low; at the
+    end at every pair (ph_row.cu:2-121)."""
+    m = len(cols)
+    work = [set(c) for c in cols]
+    low = [max(c, default=-1) for c in work]
+    first = [min((j for j in range(m) if low[j] == r), default=m) for r in range(m)]
+    ess = [1] * m
+    for i in range(m - 1, -1, -1):
+        here = [j for j in range(m) if low[j] == i]
+        if len(here) < 2:
+            continue
+        ess[i] = ess[here[0]] = 0
+        for j in here[1:]:
+            work[j] ^= work[here[0]]
+            low[j] = max(work[j], default=-1)
+            if low[j] >= 0:
+                first[low[j]] = min(first[low[j]], j)
+        for j in here[1:]:
+            if low[j] >= 0 and first[low[j]] == j:
+                ess[j] = ess[low[j]] = 0
+    for j in range(m):
+        if low[j] >= 0:
+            ess[j] = ess[low[j]] = 0
+    return np.array(low, np.int32), np.array(ess, np.int32)
