@@ -1556,8 +1556,13 @@ __device__ bool in_triangles(const int32_t *col, const int32_t *tab, const uint1
 // The outputs of a whole instance, as k_c2_runs_out writes them, by a CTA: a
 // word a thread, from word `first` on and every `step` words, filled with what
 // a positive triangle gets, 16 bytes a store; then the few vertices, edges and
-// paired triangles are corrected.  Bound by the writes.
-template <int THREADS>
+// paired triangles are corrected.  Bound by the writes where there are many
+// instances (157 us for 684 MB), by the chain of a word's edges where there are
+// few: up to 32 at the start of an instance, so there (EACH) the vertices and
+// edges take a thread each.  50 points through openph() 213-226 us -> 205-216, 40
+// of 20 to 60 points from the host 286-291 -> 276-282; 1,024
+// complexes would take 0.7-1.4% longer.
+template <int THREADS, bool EACH>
 __device__ __forceinline__ void in_out(const C2Args &a, const C2Inst &in, int first, int step) {
     const int none = a.one_based ? 0 : -1, tid = threadIdx.x;
     auto fill = [&](int32_t *p, int n, int value) {
@@ -1572,7 +1577,12 @@ __device__ __forceinline__ void in_out(const C2Args &a, const C2Inst &in, int fi
     const int nw = (int)((in.cols + 31) >> 5);
     int32_t *const low = a.low + in.base, *const ess = a.ess ? a.ess + in.base : nullptr;
     for (int c0 = 32 * first; c0 < in.cols; c0 += 32 * step) {
-        const int n = min(32 * THREADS, (int)in.cols - c0);
+        const int n = min(32 * THREADS, (int)in.cols - c0), w_next = (c0 >> 5) + THREADS;
+        int k0 = 0, k1 = 0;  // its edges
+        if (EACH) {
+            k0 = words[c0 >> 5].epre;
+            k1 = w_next < nw ? words[w_next].epre : in.eoff + in.ne;
+        }
         fill(low + c0, n, none);
         if (ess) fill(ess + c0, n, 1);
         __syncthreads();
@@ -1590,21 +1600,38 @@ __device__ __forceinline__ void in_out(const C2Args &a, const C2Inst &in, int fi
                 low[j] = j - 1 + a.one_based;
                 if (ess) ess[j] = 0;
             }
-            if (ess)
-                for (unsigned x = w.v; x; x &= x - 1) {
-                    const int j = 32 * wi + __ffs(x) - 1;
-                    if (a.dead[in.voff + j]) ess[j] = 0;
+            if (!EACH) {
+                if (ess)
+                    for (unsigned x = w.v; x; x &= x - 1) {
+                        const int j = 32 * wi + __ffs(x) - 1;
+                        if (a.dead[in.voff + j]) ess[j] = 0;
+                    }
+                // bit x: the column after x is no triangle, or past the instance's end
+                const unsigned next =
+                    notri >> 1 | (wi + 1 < nw ? (words[wi + 1].v | words[wi + 1].e) << 31 : ~(here >> 1));
+                int k = w.epre;
+                for (unsigned x = w.e; x; x &= x - 1, k++) {
+                    const int bit = __ffs(x) - 1, j = 32 * wi + bit, y = a.neg[k];
+                    const bool run = !((next >> bit) & 1u);
+                    if (y >= 0) low[j] = y + a.one_based;
+                    if (y < 0 && !run) a.res[atomicAdd(&a.st->nres, 1)] = k;
+                    else if (ess) ess[j] = 0;
                 }
-            // bit x: the column after x is no triangle, or past the instance's end
-            const unsigned next = notri >> 1 | (wi + 1 < nw ? (words[wi + 1].v | words[wi + 1].e) << 31 : ~(here >> 1));
-            int k = w.epre;
-            for (unsigned x = w.e; x; x &= x - 1, k++) {
-                const int bit = __ffs(x) - 1, j = 32 * wi + bit, y = a.neg[k];
-                const bool run = !((next >> bit) & 1u);
-                if (y >= 0) low[j] = y + a.one_based;
-                if (y < 0 && !run) a.res[atomicAdd(&a.st->nres, 1)] = k;
-                else if (ess) ess[j] = 0;
             }
+        }
+        if (EACH && ess)
+            for (int v = c0 + tid; v < min(in.nv, c0 + n); v += THREADS)
+                if (a.dead[in.voff + v]) ess[v] = 0;
+        for (int k = k0 + tid; k < k1; k += THREADS) {
+            const int j = a.elist[k], y = a.neg[k];
+            bool run = j + 1 < in.cols;  // a triangle follows
+            if (run) {
+                const C2Word next = words[(j + 1) >> 5];
+                run = !(((next.v | next.e) >> ((j + 1) & 31)) & 1u);
+            }
+            if (y >= 0) low[j] = y + a.one_based;
+            if (y < 0 && !run) a.res[atomicAdd(&a.st->nres, 1)] = k;
+            else if (ess) ess[j] = 0;
         }
         __syncthreads();
     }
@@ -1844,7 +1871,7 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         if (tid == 0 && s_no) a.st->refused = 1;
         // a single small one's outputs at once: 12 points 54 us -> 46-50 in all
         if constexpr (OUT)
-            if (!s_no && !a.st->refused) in_out<IN_THREADS>(a, in, 0, IN_THREADS);
+            if (!s_no && !a.st->refused) in_out<IN_THREADS, true>(a, in, 0, IN_THREADS);
         __syncthreads();
     }
 }
@@ -1915,11 +1942,12 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst_more(C2Args a) {
 
 // The outputs, IO_COLS columns a block.
 constexpr int IO_THREADS = 256, IO_COLS = 32 * IO_THREADS;
+template <bool EACH>
 __global__ void __launch_bounds__(IO_THREADS) k_c2_inst_out(C2Args a, int parts) {
     if (a.st->refused || a.st->no_room) return;
     for (int b = blockIdx.x / parts; b < a.count; b += gridDim.x / parts) {
         const C2Inst in = a.inst[b];
-        in_out<IO_THREADS>(a, in, (int)(blockIdx.x % parts) * IO_THREADS, parts * IO_THREADS);
+        in_out<IO_THREADS, EACH>(a, in, (int)(blockIdx.x % parts) * IO_THREADS, parts * IO_THREADS);
     }
 }
 
@@ -2184,7 +2212,9 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
         // enough blocks for the outputs of one instance as of many
         const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(16, (m / a.count + IO_COLS - 1) / IO_COLS));
         if (!out_here) {
-            k_c2_inst_out<<<parts * std::min(a.count, 65535), IO_THREADS, 0, s>>>(a, parts);
+            const int blocks = parts * std::min(a.count, 65535);
+            if (blocks <= 8 * ctx->sm_count) k_c2_inst_out<true><<<blocks, IO_THREADS, 0, s>>>(a, parts);
+            else k_c2_inst_out<false><<<blocks, IO_THREADS, 0, s>>>(a, parts);
             ctx->launches++;
         }
         if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
