@@ -790,7 +790,7 @@ def run_configs(local, pool):
 # ------------------------------------------------------------ variants
 def run_variants(local, pool):
     """The six other algorithms of the reference (standard, twist, ph_row and
-    their parallel forms, each a single persistent GPU walker here) and pms
+    their parallel forms, their columns side by side here) and pms
     on one lower-star image, one reduction each after a warm-up, device time
     of the call; every low checked against the oracle's twist."""
     from openph_gb300 import api
