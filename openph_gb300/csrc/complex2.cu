@@ -922,7 +922,9 @@ template <bool RUNS>
 __global__ void __launch_bounds__(C2_THREADS) k_c2_triangles(C2Args a, int kruskal_blocks, int sort_blocks, int max_nv) {
     extern __shared__ __align__(16) uint32_t tri_smem[];
     __shared__ int s_parts;
-    if (a.st->bad || (RUNS && a.st->unsorted)) return;
+    // other blocks set these flags meanwhile: a block's threads leave together, or those that stay
+    // would work on components and rows that nobody set up
+    if (__syncthreads_or(a.st->bad || (RUNS && a.st->unsorted))) return;
     const int lane = threadIdx.x & 31;
     if ((int)blockIdx.x < kruskal_blocks) {
         for (int b = blockIdx.x; b < a.count; b += kruskal_blocks) {
@@ -1889,7 +1891,8 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst_more(C2Args a) {
     constexpr int NW = IN_THREADS / 32;
     __shared__ int s_i;
     const int tid = threadIdx.x, wid = tid >> 5;
-    if (a.st->refused || a.st->no_room) return;
+    // other blocks set `refused` meanwhile: a block's threads leave together (thread 0 hands out the items)
+    if (__syncthreads_or(a.st->refused || a.st->no_room)) return;
     const int n_items = a.st->items;
     for (int i = blockIdx.x; i < n_items; i = s_i) {
         const int2 item = a.items[i];
