@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(1024) k_c2_scan(C2Args a, int64_t ntiles) {
                 s.base = o0;
                 s.cols = o1 - o0;
                 atomicMax(&a.st->max_nv, s.nv);
+                if (s.ne == 0 && s.nv != s.cols) a.st->bad = 1;  // triangles, but no edges for their rows
             }
         }
         // coff serves the form tried first (runs); the table's is k_c2_cells'
@@ -447,8 +448,9 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_edges(C2Args a) {
             int32_t *t = a.cells + in.coff;
             const int pitch = c2_pitch(in.nv), x = u - in.voff, y = v - in.voff;
             const C2Word w = a.words[j >> 5];
+            // a second edge on them, a vertex to come, or triangles before the first edge (in no edge's run)
             if (atomicCAS(t + (int64_t)x * pitch + y, -1, k - in.eoff) != -1 ||
-                w.vpre + __popc(w.v & below(j & 31)) != in.voff + in.nv)
+                w.vpre + __popc(w.v & below(j & 31)) != in.voff + in.nv || (k == in.eoff && j - in.base != in.nv))
                 a.st->unsorted = 1;
             t[(int64_t)y * pitch + x] = k - in.eoff;
             int32_t *const c = a.tab + in.coff;
@@ -863,7 +865,9 @@ __device__ void c2_sort_row(const int32_t *src, int32_t *dst, int nv, int pitch,
 // Nothing is looked up: a warp takes an edge, its lanes the vertices; two
 // rows of the table of edge columns (vertices by vertices) say which have a
 // triangle (a ballot is the run's word), and the triangles' rows are compared
-// with what they must be.  A matrix that passes is a complex in such runs.
+// with what they must be.  The first edge must come right after the vertices,
+// so that every column with three rows is in some edge's run.  A matrix that
+// passes is a complex in such runs.
 //
 // One word of 32 vertices: its set bits, the columns of the two edges.
 // VW > 0: that many words (else vw); four words' rows are in flight at a
@@ -1745,7 +1749,8 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         // (bytes) behind; the rest is scratch
         const int ends_at = (max(6 * nw2, 4 * pitch * nv + 4 * ne) + 15) & ~15;
         const int scratch_at = (ends_at + 2 * ne + 15) & ~15, left = IN_SMEM - scratch_at;
-        if (outside || ne > 65535 || nv > IN_MAX_NV || left < max(6 * nv, 4 * pitch)) {
+        // (without edges there are vertices only: a triangle has rows)
+        if (outside || (ne == 0 && nv != cols) || ne > 65535 || nv > IN_MAX_NV || left < max(6 * nv, 4 * pitch)) {
             if (tid == 0) a.st->refused = 1;
             s_no = 1;
         }
@@ -1820,6 +1825,7 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         for (int k = tid; k < ne; k += IN_THREADS) {
             const int j = __ldcg(elist + k), s = 2 * k + 3 * (j - nv - k);
             int r0 = rows[s], r1 = rows[s + 1];
+            if (k == 0 && j != nv) s_no = 1;  // triangles before the first edge are in no edge's run
             if (r0 < 0 || r1 <= r0 || r1 >= nv) {
                 s_no = 1;
                 r0 = r1 = 0;

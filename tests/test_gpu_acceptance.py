@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import oracle
+from openph_gb300 import api
 from openph_gb300 import complexes as cx
 from openph_gb300.complexes import BoundaryMatrix
 
@@ -39,3 +40,98 @@ def test_refused_by_one_block_while_others_start(ctx, n):
         for b in (0, 99, 100, 149):
             np.testing.assert_array_equal(lows[b], want if b >= 100 else small_want)
             np.testing.assert_array_equal(esss[b], want_ess if b >= 100 else small_ess)
+
+
+@pytest.fixture(scope="module")
+def server(cuda_lib):
+    with api.Server(0, budget_bytes=4 << 30, max_active=64) as srv:
+        yield srv
+
+
+def device(bm):
+    import torch
+    return (torch.from_numpy(bm.colptr).cuda(), torch.from_numpy(bm.rows if bm.nnz else np.zeros(1, np.int32)).cuda(),
+            torch.empty(2 * bm.m, dtype=torch.int32, device="cuda"))
+
+
+def check_everywhere(ctx, server, bm, batches=(3, 130)):
+    """Every entry point that tries the forms gives the oracle's lows: single
+    calls with host and device input, with and without ess, 1-based, batches
+    that take whole instances and that do not, and the server."""
+    import torch
+    want, want_ess, _ = oracle.twist(bm)
+
+    def same(low, ess, where):
+        np.testing.assert_array_equal(low, want, err_msg=where)
+        if ess is not None:
+            np.testing.assert_array_equal(ess, want_ess, err_msg=where)
+
+    low, ess, arg, _ = ctx.reduce(bm, "pms", with_arglow=True)
+    same(low, ess, "host")
+    want_arg = np.full(bm.m, -1, np.int32)
+    want_arg[want[want >= 0]] = np.flatnonzero(want >= 0)
+    np.testing.assert_array_equal(arg, want_arg)
+    colptr, rows, out = device(bm)
+    for with_ess in (True, False):
+        torch.cuda.synchronize()
+        ctx.reduce_device(bm.m, colptr.data_ptr(), rows.data_ptr(), out.data_ptr(),
+                          out.data_ptr() + 4 * bm.m if with_ess else None)
+        res = out.cpu().numpy()
+        same(res[:bm.m], res[bm.m:] if with_ess else None, f"device, ess {with_ess}")
+    r, c = bm.to_coo1()
+    low, ess, *_ = api.ph("pms", r, c, bm.m)
+    same(low - 1, ess, "ph")
+    rips = cx.rips_cube(7, seed=2)
+    rips_want, rips_ess, _ = oracle.twist(rips)
+    for count in batches:
+        mats = [rips] * (count - 1)
+        mats.insert(count // 2, bm)
+        lows, esss, _ = ctx.reduce_batch(mats, "pms")
+        same(lows[count // 2], esss[count // 2], f"batch of {count}")
+        for b in {0, count - 1} - {count // 2}:
+            np.testing.assert_array_equal(lows[b], rips_want)
+            np.testing.assert_array_equal(esss[b], rips_ess)
+    low, ess, _ = server.wait(server.submit(bm))
+    same(low, ess, "server")
+
+
+# columns of three rows before the first edge, or without any edge: no run holds them
+NO_EDGE_BEFORE = {
+    "no edges": [[], [], [], [], [0, 1, 2], [0, 1, 3], [1, 2, 3]],
+    "no edges, one": [[], [], [], [0, 1, 2]],
+    "rows to the right": [[], [], [], [4, 5, 6], [0, 1], [0, 2], [1, 2]],
+    "rows of vertices": [[], [], [], [0, 1, 2], [0, 1], [0, 2], [1, 2]],
+    "one edge after": [[], [], [], [0, 1, 2], [0, 1]],
+}
+
+
+@pytest.mark.parametrize("name", NO_EDGE_BEFORE)
+def test_three_rows_before_the_first_edge(ctx, server, name):
+    check_everywhere(ctx, server, BoundaryMatrix.from_columns(NO_EDGE_BEFORE[name]))
+
+
+@pytest.mark.parametrize("kind", ["rows to the right", "rows of vertices"])
+def test_three_rows_before_the_first_edge_grid_wide(ctx, server, kind):
+    """The same past 2^15 columns, where the runs are checked grid-wide."""
+    bm = cx.rips_cube(60, seed=3)
+    cols = [bm.column(j).tolist() for j in range(bm.m)]
+    tri = [x + 1 for x in cols[next(j for j in range(bm.m) if len(cols[j]) == 3)]]
+    cols = [[x + (x >= 60) for x in c] for c in cols]
+    cols.insert(60, tri if kind == "rows to the right" else [0, 1, 2])
+    check_everywhere(ctx, server, BoundaryMatrix.from_columns(cols), batches=(3,))
+
+
+@pytest.mark.parametrize("row", [5, 7, -1])
+def test_malformed_rows_before_the_first_edge(ctx, row):
+    """Rows out of range in such a column are refused as anywhere else."""
+    bm = BoundaryMatrix(np.array([0, 0, 0, 0, 3, 5]), np.array([0, 1, row, 0, 1], np.int32))
+    low = np.empty(5, np.int32)
+    colptr, rows, out = device(bm)
+    import torch
+    torch.cuda.synchronize()
+    L = api.lib()
+    assert L.oph_reduce(ctx.handle, api.algo_id("pms"), 5, bm.colptr, api._ptr(bm.rows), low, None, None,
+                        None) == api.OPH_ERR_BAD_INPUT
+    with pytest.raises(api.OphError) as e:
+        ctx.reduce_device(5, colptr.data_ptr(), rows.data_ptr(), out.data_ptr())
+    assert e.value.status == api.OPH_ERR_BAD_INPUT
