@@ -921,7 +921,8 @@ __device__ __forceinline__ bool flag_run(const int32_t *tu, const int32_t *tv, i
 // RUNS: the next ones sort the vertices' edges (a CTA each), the rest check
 // the runs, a warp per edge; what fails sets `unsorted`, and the edge-vertex
 // table is built instead.  Table: the rest check the triangles, a thread
-// each, and write each at its three entries, bound by those scattered writes.
+// each, which also must come after their edges, and write each at its three
+// entries, bound by those scattered writes.
 template <bool RUNS>
 __global__ void __launch_bounds__(C2_THREADS) k_c2_triangles(C2Args a, int kruskal_blocks, int sort_blocks, int max_nv) {
     extern __shared__ __align__(16) uint32_t tri_smem[];
@@ -985,7 +986,9 @@ __global__ void __launch_bounds__(C2_THREADS) k_c2_triangles(C2Args a, int krusk
         if (j >= a.m || ((w.v | w.e) >> lane) & 1u) continue;
         const C2Inst &in = a.inst[c2_inst_of(a, j)];
         int k[3], o[3];
-        if (!c2_triangle(a, j, w, in, k) ||
+        // a triangle before one of its edges is left to the general path: a residual
+        // column is looked at from its edge on, where its triangles must be
+        if (!c2_triangle(a, j, w, in, k) || k[2] >= w.epre + __popc(w.e & below(lane)) ||
             !c2_opposite(a.erec[k[0]], a.erec[k[1]], a.erec[k[2]], o[0], o[1], o[2])) {
             bad = true;
             continue;

@@ -95,6 +95,13 @@ def check_everywhere(ctx, server, bm, batches=(3, 130)):
     same(low, ess, "server")
 
 
+def faces_late(bm, order):
+    """The columns of bm, its simplices listed as `order` says."""
+    pos = np.empty(bm.m, np.int64)
+    pos[order] = np.arange(bm.m)
+    return BoundaryMatrix.from_columns([sorted(pos[bm.column(j)].tolist()) for j in order])
+
+
 # columns of three rows before the first edge, or without any edge: no run holds them
 NO_EDGE_BEFORE = {
     "no edges": [[], [], [], [], [0, 1, 2], [0, 1, 3], [1, 2, 3]],
@@ -135,3 +142,28 @@ def test_malformed_rows_before_the_first_edge(ctx, row):
     with pytest.raises(api.OphError) as e:
         ctx.reduce_device(5, colptr.data_ptr(), rows.data_ptr(), out.data_ptr())
     assert e.value.status == api.OPH_ERR_BAD_INPUT
+
+
+# simplices of a complete complex (runs refused, edges crowded: the table), of an image (a graph), of three points
+@pytest.mark.parametrize("make", [lambda: cx.rips_cube(30, seed=4), lambda: cx.rips_cube(62, seed=4),
+                                  lambda: cx.lower_star_image(12, 15, seed=4), lambda: cx.rips_cube(3, seed=4)],
+                         ids=["crowded", "crowded, large", "image", "triangle"])
+@pytest.mark.parametrize("kinds", [(3, 0, 2), (0, 3, 2), (2, 0, 3), (3, 2, 0)])
+def test_faces_after_cofaces(ctx, server, make, kinds):
+    """Columns by their number of rows, triangles before edges or edges before
+    vertices: rows above the diagonal are accepted input."""
+    bm = make()
+    size = np.diff(bm.colptr)
+    order = np.concatenate([np.flatnonzero(size == k) for k in kinds])
+    check_everywhere(ctx, server, faces_late(bm, order), batches=(3,) if bm.m > 30_000 else (3, 130))
+
+
+def test_one_triangle_before_an_edge(ctx, server):
+    """A Rips complex with some triangles moved before their last edge."""
+    bm = cx.rips_cube(20, seed=5)
+    size = np.diff(bm.colptr)
+    rng = np.random.default_rng(6)
+    key = np.arange(bm.m, dtype=float)
+    for t in rng.choice(np.flatnonzero(size == 3), 12, replace=False):
+        key[t] = bm.column(t).max() - 0.5 - 20 * rng.random()
+    check_everywhere(ctx, server, faces_late(bm, np.argsort(key, kind="stable")))
