@@ -1994,8 +1994,11 @@ int c2_named_matrix(int64_t m, int64_t nv, int64_t ne, int64_t nt) {
 }
 }  // namespace
 
+// False when the driver refused a launch (its resources): the form is not done,
+// and the general path says what it thinks of the device.
+static bool c2_launched() { return cudaGetLastError() == cudaSuccess; }
+
 static int c2_read_status(Context *ctx, const C2Args &a, C2Status *hs) {
-    OPH_CUDA_TRY(cudaGetLastError());
     OPH_CUDA_TRY(cudaMemcpyAsync(hs, a.st, sizeof(C2Status), cudaMemcpyDeviceToHost, ctx->stream));
     OPH_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return OPH_OK;
@@ -2036,7 +2039,8 @@ static int c2_run_graph(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t 
     // and another thread's context may have half the device's blocks
     static std::mutex alone[64];
     std::unique_lock<std::mutex> turn(alone[ctx->device & 63]);
-    OPH_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_c2_graph, dim3(gg), dim3(C2_THREADS), params, 0, s));
+    cudaLaunchCooperativeKernel((const void *)k_c2_graph, dim3(gg), dim3(C2_THREADS), params, 0, s);
+    if (!c2_launched()) return OPH_OK;
     ctx->launches += 3;
     cudaEventRecord(ctx->ev[1], s);
     int rc = c2_read_status(ctx, a, hs);
@@ -2072,6 +2076,15 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     int gr = small ? c2_residual_grid<RUNS, RS_SMALL, RS_SMALL_WORDS>(ctx)
                    : c2_residual_grid<RUNS, RS_LARGE, RS_LARGE_WORDS>(ctx);
     if (gr == 0) return OPH_OK;
+    // the components of C2_MAX_NV vertices take 48 KB beside the kernel's own shared memory
+    static PerDevice roomy;
+    if (!RUNS && !roomy.get(ctx->device, [] {
+            return cudaFuncSetAttribute(k_c2_triangles<RUNS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        6 * C2_MAX_NV) == cudaSuccess;
+        })) {
+        cudaGetLastError();
+        return OPH_OK;
+    }
     gr = (int)std::min<int64_t>(ne, gr);
     const int nv = hs->nv;
     a.arena_cap = (1 << 20) + 16 * ne;
@@ -2121,6 +2134,7 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
         k_c2_residual<RUNS, RS_SMALL, RS_SMALL_WORDS><<<gr, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
     else
         k_c2_residual<RUNS, RS_LARGE, RS_LARGE_WORDS><<<gr, RS_LARGE, RS_LARGE_WORDS * sizeof(uint32_t), s>>>(a);
+    if (!c2_launched()) return OPH_OK;
     ctx->launches += RUNS ? 4 : 6;
     cudaEventRecord(ctx->ev[1], s);
     int rc = c2_read_status(ctx, a, hs);
@@ -2233,6 +2247,7 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
         // a residual edge or so per vertex
         const int rg = (int)std::min<int64_t>(gr, std::max<int64_t>(1, a.cap_e));
         k_c2_residual<true, RS_SMALL, RS_SMALL_WORDS><<<rg, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
+        if (!c2_launched()) return OPH_OK;
         ctx->launches += 2;
         cudaEventRecord(ctx->ev[1], s);
         int rc = c2_read_status(ctx, a, hs);

@@ -1,5 +1,6 @@
 // Host-side internals shared by the translation units of libopenph_gb300.
 #pragma once
+#include <atomic>
 #include <vector>
 #include <cstdint>
 #include <cstdio>
@@ -223,6 +224,19 @@ struct Context {
     // reduction instead of once per batch of sweeps; loop_key as sweep_key
     cudaGraphExec_t loop_graph = nullptr;
     std::vector<unsigned char> loop_key;
+};
+
+// A positive answer of the driver, asked for once a device (an occupancy, an
+// attribute set); several threads may ask at the same time.
+struct PerDevice {
+    std::atomic<int> known[64] = {};
+    template <class Ask>
+    int get(int device, Ask ask) {
+        std::atomic<int> &k = known[device & 63];
+        int n = k.load(std::memory_order_acquire);
+        if (n <= 0 && (n = ask()) > 0) k.store(n, std::memory_order_release);
+        return n;
+    }
 };
 
 // buffer slots of Context::bufs

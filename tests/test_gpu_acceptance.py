@@ -167,3 +167,17 @@ def test_one_triangle_before_an_edge(ctx, server):
     for t in rng.choice(np.flatnonzero(size == 3), 12, replace=False):
         key[t] = bm.column(t).max() - 0.5 - 20 * rng.random()
     check_everywhere(ctx, server, faces_late(bm, np.argsort(key, kind="stable")))
+
+
+def sparse(nv, cluster):
+    """A complete complex on a few of nv vertices, the others alone."""
+    bm = cx.rips_cube(cluster, seed=9)
+    colptr = np.concatenate([np.zeros(nv - cluster, np.int64), bm.colptr])
+    return BoundaryMatrix(colptr, bm.rows + np.int32(nv - cluster))
+
+
+@pytest.mark.parametrize("nv", [1024, 1025, 8189, 8190, 8192, 8193])
+@pytest.mark.parametrize("cluster", [5, 20])
+def test_many_vertices(ctx, server, nv, cluster):
+    """Either side of the forms' limits on vertices."""
+    check_everywhere(ctx, server, sparse(nv, cluster), batches=(3,))
