@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 #include <vector>
 
@@ -22,29 +23,37 @@ using namespace oph;
 
 namespace oph {
 
+void ctx_release(Context *ctx, int slot) {
+    DevBuf &b = ctx->bufs[slot];
+    if (!b.ptr) return;
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(b.ptr);
+    b.ptr = nullptr;
+    b.bytes = 0;
+}
+
 void *ctx_alloc(Context *ctx, int slot, size_t bytes) {
     DevBuf &b = ctx->bufs[slot];
     if (bytes == 0) bytes = 16;
     bytes = (bytes + 255) & ~(size_t)255;
     if (b.bytes >= bytes) return b.ptr;
-    if (ctx->budget > 0) {
-        size_t total = 0;
-        for (int i = 0; i < S_NSLOTS; i++) total += (i == slot) ? 0 : ctx->bufs[i].bytes;
-        if ((int64_t)(total + bytes) > ctx->budget) return nullptr;
+    constexpr int spare[] = {S_C2_TAB, S_C2_WORK, S_C2_MODE, S_C2_CELLS, S_GEN, S_ROWEST};
+    const bool is_spare = std::find(std::begin(spare), std::end(spare), slot) != std::end(spare);
+    for (bool last = is_spare;; last = true) {
+        size_t total = bytes;
+        for (int i = 0; i < S_NSLOTS; i++) total += i == slot ? 0 : ctx->bufs[i].bytes;
+        if (ctx->budget <= 0 || (int64_t)total <= ctx->budget) {
+            ctx_release(ctx, slot);
+            if (cudaMalloc(&b.ptr, bytes) == cudaSuccess) {
+                b.bytes = bytes;
+                return b.ptr;
+            }
+            cudaGetLastError();
+            b.ptr = nullptr;
+        }
+        if (last) return nullptr;
+        for (int q : spare) ctx_release(ctx, q);
     }
-    if (b.ptr) {
-        cudaStreamSynchronize(ctx->stream);
-        cudaFree(b.ptr);
-        b.ptr = nullptr;
-        b.bytes = 0;
-    }
-    if (cudaMalloc(&b.ptr, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        b.ptr = nullptr;
-        return nullptr;
-    }
-    b.bytes = bytes;
-    return b.ptr;
 }
 
 // --------------------------------------------------------------- kernels

@@ -511,8 +511,9 @@ int grid_of(Context *ctx, int64_t n) {
 
 // Scratch of one generator call: first from the context's own buffer, kept
 // from call to call (pool allocations are given back to the driver at every
-// synchronisation, and cost more than the kernels on small complexes), then
-// from the stream's memory pool, released on every exit.
+// synchronisation, and cost more than the kernels on small complexes) up to
+// KEEP_MOST bytes a slot, then from the stream's memory pool, released on every
+// exit.
 struct Scratch {
     cudaStream_t s;
     std::vector<void *> ptrs;
@@ -522,8 +523,9 @@ struct Scratch {
     // the context's buffer `slot`, of at least `bytes` where its budget
     // allows, for what is taken from here on (S_GEN, and those of the
     // reduction, which nothing uses now)
+    static constexpr size_t KEEP_MOST = 256 << 20;
     void keep(Context *ctx, int slot, size_t bytes) {
-        kept = (char *)ctx_alloc(ctx, slot, bytes);
+        kept = bytes <= KEEP_MOST ? (char *)ctx_alloc(ctx, slot, bytes) : nullptr;
         room = kept ? ctx->bufs[slot].bytes : 0;
         used = 0;
     }

@@ -154,7 +154,12 @@ int dual_build_store(cudaStream_t s, int sm_count, const int64_t *colptr, const 
 int dual_lows(Context *ctx, const Work &wd, int32_t **low);
 
 // capi.cu
+// A slot's buffer of at least `bytes`, kept for later calls; nullptr past the
+// context's budget or the device's memory.  The spare slots' buffers (S_C2_*,
+// S_GEN, S_ROWEST) hold nothing once the step that asked for them is over,
+// and whoever asks for another slot then gets their room before it is refused.
 void *ctx_alloc(Context *ctx, int slot, size_t bytes);
+void ctx_release(Context *ctx, int slot);
 int ctx_sync_status(Context *ctx, Work &w, DevStatus *out);
 
 // Per-sweep progress trackers of a pms reduction (the reference's track(),
@@ -243,7 +248,7 @@ struct PerDevice {
 enum Slot {
     S_STATUS, S_COLPTR, S_ROWS, S_LOW, S_CLASSES, S_CLEAR, S_DIM, S_FIRST, S_LEFT, S_BETA, S_WORK, S_WIDE, S_SEG,
     S_ROWPIV, S_AGG, S_POOL, S_POOL2, S_ESS, S_ARGLOW, S_COO_R, S_COO_C, S_LOWTRUE, S_TRACK, S_INSTOFF, S_TMP,
-    S_ULIST, S_KAGG, S_ESSHAT, S_SLIST, S_DGRADE, S_DCOLPTR, S_DSORT, S_DTEMP, S_DLOW, S_BITMAP, S_CHECK, S_IASC, S_IBUCKET, S_IOPEN, S_RANGES, S_SEQNS, S_PRECLEAR, S_C2_TAB, S_C2_WORK, S_C2_MODE, S_C2_CELLS, S_GEN, S_NSLOTS
+    S_ULIST, S_KAGG, S_ESSHAT, S_SLIST, S_DGRADE, S_DCOLPTR, S_DSORT, S_DTEMP, S_DLOW, S_BITMAP, S_CHECK, S_IASC, S_IBUCKET, S_IOPEN, S_RANGES, S_SEQNS, S_PRECLEAR, S_C2_TAB, S_C2_WORK, S_C2_MODE, S_C2_CELLS, S_GEN, S_ROWEST, S_NSLOTS
 };
 
 }  // namespace oph

@@ -1087,7 +1087,7 @@ static int row_estimate(Context *ctx, Work &w, int words, int32_t *ess, bool *do
                          r256(4 * (size_t)m), r256(4 * (size_t)cap), r256(8 * (size_t)cap), r256(8 * (size_t)cap)};
     size_t off[9] = {};
     for (int q = 0; q < 8; q++) off[q + 1] = off[q] + at[q];
-    char *tmp = (char *)ctx_alloc(ctx, S_TMP, off[8]);
+    char *tmp = (char *)ctx_alloc(ctx, S_ROWEST, off[8]);
     if (!tmp) return OPH_OK;
     RowArgs a{};
     a.m = m; a.colptr = w.colptr; a.ess = ess; a.cap = (unsigned)cap;
@@ -1179,6 +1179,7 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
             int rc = claim_columns(ctx, w, a.twist ? maxdim : -1, a.twist != 0, &regrows);
             if (rc == OPH_ERR_OOM || rc == OPH_ERR_OVERFLOW) {  // the walk writes less: it may still fit
                 side_by_side = false;
+                ctx_release(ctx, S_TMP);
                 rc = restart_store(ctx, w, a);
             }
             if (rc) return rc;
@@ -1247,8 +1248,9 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
             if (rc && rc != OPH_ERR_OOM && rc != OPH_ERR_OVERFLOW) return rc;
             if (!done) {
                 side_by_side = false;
+                ctx_release(ctx, S_ROWEST);
                 if ((rc = restart_store(ctx, w, a))) return rc;
-                // both used this slot
+                // the columns side by side used this slot
                 a.bhead = (int32_t *)ctx_alloc(ctx, S_TMP, sizeof(int32_t) * (3 * m + 1));
                 if (!a.bhead) return OPH_ERR_OOM;
                 a.bnext = a.bhead + m; a.bcnt = a.bnext + m;
