@@ -2020,11 +2020,13 @@ static int c2_run_graph(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t 
         if (!p) return OPH_OK;
     }
     // a grid that is resident as a whole, no larger than the first round's work
-    static int per_sm[64];
-    int &nb = per_sm[ctx->device & 63];
-    if (!nb && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_c2_graph, C2_THREADS, 0) != cudaSuccess) {
+    static PerDevice per_sm;
+    const int nb = per_sm.get(ctx->device, [] {
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_c2_graph, C2_THREADS, 0) == cudaSuccess ? n : 0;
+    });
+    if (nb <= 0) {
         cudaGetLastError();
-        nb = 0;
         return OPH_OK;
     }
     const int gg = c2_grid(ctx, ne, std::min(nb, 4));
@@ -2051,15 +2053,20 @@ static int c2_run_graph(Context *ctx, C2Args a, int64_t nv, int64_t ne, int64_t 
 
 template <bool RUNS, int THREADS, int WORDS>
 static int c2_residual_grid(Context *ctx) {
-    static int per_sm[64];
-    int &nb = per_sm[ctx->device & 63];
+    static PerDevice per_sm;
     constexpr int SMEM = WORDS * (int)sizeof(uint32_t);
-    if (!nb && (cudaFuncSetAttribute(k_c2_residual<RUNS, THREADS, WORDS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     SMEM) != cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_c2_residual<RUNS, THREADS, WORDS>, THREADS,
-                                                              SMEM) != cudaSuccess)) {
+    static PerDevice attr;
+    if (!allow_shared(attr, ctx->device, k_c2_residual<RUNS, THREADS, WORDS>, SMEM)) return 0;
+    const int nb = per_sm.get(ctx->device, [] {
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_c2_residual<RUNS, THREADS, WORDS>, THREADS, SMEM) ==
+                       cudaSuccess
+                   ? n
+                   : 0;
+    });
+    if (nb <= 0) {
         cudaGetLastError();
-        nb = 0;
+        return 0;
     }
     return nb * ctx->sm_count;
 }
@@ -2078,13 +2085,7 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     if (gr == 0) return OPH_OK;
     // the components of C2_MAX_NV vertices take 48 KB beside the kernel's own shared memory
     static PerDevice roomy;
-    if (!RUNS && !roomy.get(ctx->device, [] {
-            return cudaFuncSetAttribute(k_c2_triangles<RUNS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        6 * C2_MAX_NV) == cudaSuccess;
-        })) {
-        cudaGetLastError();
-        return OPH_OK;
-    }
+    if (!RUNS && !allow_shared(roomy, ctx->device, k_c2_triangles<RUNS>, 6 * C2_MAX_NV)) return OPH_OK;
     gr = (int)std::min<int64_t>(ne, gr);
     const int nv = hs->nv;
     a.arena_cap = (1 << 20) + 16 * ne;
@@ -2154,17 +2155,11 @@ constexpr int IN_MIN_COUNT = 128;
 static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
     *done = false;
     cudaStream_t s = ctx->stream;
-    static int ready[64];
-    int &ok = ready[ctx->device & 63];
-    if (!ok) {
-        if (cudaFuncSetAttribute(k_c2_inst<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_c2_inst<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_c2_inst_more, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM) != cudaSuccess) {
-            cudaGetLastError();
-            return OPH_OK;
-        }
-        ok = 1;
-    }
+    static PerDevice one, each, more;
+    if (!allow_shared(one, ctx->device, k_c2_inst<true>, IN_SMEM) ||
+        !allow_shared(each, ctx->device, k_c2_inst<false>, IN_SMEM) ||
+        !allow_shared(more, ctx->device, k_c2_inst_more, IN_SMEM))
+        return OPH_OK;
     int gr = c2_residual_grid<true, RS_SMALL, RS_SMALL_WORDS>(ctx);
     if (gr == 0) return OPH_OK;
     // bounds for the tables: guesses from the columns, or what an earlier call needed

@@ -244,6 +244,18 @@ struct PerDevice {
     }
 };
 
+// A kernel's dynamic shared memory allowed up to `bytes` on a device (the
+// attribute belongs to the device, not to the process).
+template <class Kernel>
+bool allow_shared(PerDevice &asked, int device, Kernel kernel, size_t bytes) {
+    return asked.get(device, [&] {
+        const bool ok =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }) > 0;
+}
+
 // buffer slots of Context::bufs
 enum Slot {
     S_STATUS, S_COLPTR, S_ROWS, S_LOW, S_CLASSES, S_CLEAR, S_DIM, S_FIRST, S_LEFT, S_BETA, S_WORK, S_WIDE, S_SEG,

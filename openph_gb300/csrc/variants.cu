@@ -1009,12 +1009,8 @@ template <class Column>
 static int claim_columns_as(Context *ctx, Work &w, int words, int top, bool twist, int *regrows) {
     cudaStream_t s = ctx->stream;
     const int64_t m = w.m;
-    static bool attr = false;
-    if (!attr) {
-        OPH_CUDA_TRY(cudaFuncSetAttribute(k_claim<Column>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)sizeof(int) * CL_WARPS * CL_BITS));
-        attr = true;
-    }
+    static PerDevice attr;
+    if (!allow_shared(attr, ctx->device, k_claim<Column>, sizeof(int) * CL_WARPS * CL_BITS)) return OPH_ERR_CUDA;
     const size_t smem = sizeof(int) * CL_WARPS * (size_t)words;
     ClaimArgs a{};
     a.m = m; a.low = w.low; a.dim = w.dim; a.pool = w.pool; a.st = w.st; a.seg = w.seg; a.words = words;
@@ -1106,12 +1102,8 @@ static int row_estimate(Context *ctx, Work &w, int words, int32_t *ess, bool *do
     OPH_CUDA_TRY(cudaMemsetAsync(tmp, 0, off[3], s));
     OPH_CUDA_TRY(cudaMemsetAsync(a.first, 0x7f, 4 * (size_t)m, s));
     OPH_CUDA_TRY(cudaMemsetAsync(&w.st->additions, 0, 2 * sizeof(unsigned long long), s));  // these are the row form's
-    static bool attr = false;
-    if (!attr) {
-        OPH_CUDA_TRY(cudaFuncSetAttribute(k_row_exact<Column>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)sizeof(int) * CL_WARPS * CL_BITS));
-        attr = true;
-    }
+    static PerDevice attr;
+    if (!allow_shared(attr, ctx->device, k_row_exact<Column>, sizeof(int) * CL_WARPS * CL_BITS)) return OPH_ERR_CUDA;
     const size_t smem = sizeof(int) * CL_WARPS * (size_t)words;
     const int64_t per_sm = std::min<int64_t>(2048 / CL_THREADS, (220 << 10) / (smem + 2048));
     const int grid = (int)std::min<int64_t>((m + CL_WARPS - 1) / CL_WARPS, ctx->sm_count * per_sm);
@@ -1197,12 +1189,9 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
             OPH_CUDA_TRY(cudaStreamSynchronize(s));
         }
         if (!side_by_side) OPH_CUDA_TRY(cudaMemsetAsync(a.arglow, 0xff, sizeof(int32_t) * m, s));
-        static bool attr = false;
+        static PerDevice attr;
         const size_t smem = 3 * SEQ_CAP * sizeof(int);
-        if (!attr) {
-            OPH_CUDA_TRY(cudaFuncSetAttribute(k_seq_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            attr = true;
-        }
+        if (!allow_shared(attr, ctx->device, k_seq_walk, smem)) return OPH_ERR_CUDA;
         if (!side_by_side && !(a.twist && maxdim < 1)) {
             for (;;) {
                 k_seq_walk<<<1, 32, smem, s>>>(a);
@@ -1268,12 +1257,9 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
             OPH_CUDA_TRY(cudaMemsetAsync(ev_base, 0, 16, s));
             a.ev = reinterpret_cast<int *>(ev_base + 2);
         }
-        static bool attr = false;
+        static PerDevice attr;
         const size_t smem = (size_t)(ROW_THREADS / 32) * 3 * ROW_CAP * sizeof(int);
-        if (!attr) {
-            OPH_CUDA_TRY(cudaFuncSetAttribute(k_row_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            attr = true;
-        }
+        if (!allow_shared(attr, ctx->device, k_row_walk, smem)) return OPH_ERR_CUDA;
         while (!side_by_side) {
             OPH_CUDA_TRY(cudaMemsetAsync(a.bhead, 0xff, sizeof(int32_t) * m, s));
             OPH_CUDA_TRY(cudaMemsetAsync(a.bcnt, 0, sizeof(int32_t) * m, s));
