@@ -39,7 +39,9 @@
 // Which form (reduce_complex2): a single matrix of at most 2^15 columns, or a
 // batch of at least 128 or of that size on average, as whole instances; else,
 // or where one of them does not fit, the graph when three triangles come to
-// at most two edges, the runs, the table.
+// at most two edges, the runs (unless the whole instances were found not to
+// come in runs), the table.  A column of other width, found by the first kernel
+// that looks, ends the attempt at once.
 //
 // What is accepted is checked on the device before it is reported: every
 // column has 0, 2 or 3 rows, ascending and in range, the rows of an edge are
@@ -1526,8 +1528,10 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
 // Against a launch per step over all columns this saves the launches, which
 // are all that the smallest complexes cost, and the trips to L2 for tables
 // that fit a CTA: 47 instructions a warp for 32 vertices of an edge are what
-// bounds it.  Whatever is no flag complex in runs, vertices first, or does
-// not fit (`refused`; malformed matrices too) is left to the grid-wide kernels.
+// bounds it.  Whatever is no flag complex in runs, vertices first (`unsorted`),
+// or does not fit (`refused`, as the others) is left to the grid-wide kernels;
+// columns that none of the forms takes (`bad`) to the general path at once.
+// The CTAs stop where one instance is refused.
 //
 // The tables that the residual columns read later are carved from common
 // arrays by counters; when those turn out too small the host makes them
@@ -1689,11 +1693,12 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         a.st->nnz = a.colptr[a.m];
         if (a.colptr[0] != 0 || (a.nnz >= 0 && a.st->nnz != a.nnz) ||
             (a.inst_off && (a.inst_off[0] != 0 || a.inst_off[a.count] != a.m)))
-            a.st->refused = 1;
+            a.st->bad = a.st->refused = 1;
     }
     for (;;) {
         if (tid == 0) {
-            s_b = atomicAdd(&a.st->next, 1);
+            const int stop = *(volatile int *)&a.st->refused, next = atomicAdd(&a.st->next, 1);
+            s_b = stop ? a.count : next;
             s_nv = s_ne = 0;
             s_no = 0;
         }
@@ -1780,6 +1785,12 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         __syncthreads();
         if (s_no) {
             if (no) a.st->refused = 1;
+            // (why: a column that no form takes, or a vertex after other columns)
+            for (int j = tid; j < cols; j += IN_THREADS) {
+                const int64_t n = cp[j + 1] - cp[j];
+                if (n != 0 && n != 2 && n != 3) a.st->bad = 1;
+                if (n == 0 && cp[j] != c_first) a.st->unsorted = 1;
+            }
             __syncthreads();
             continue;
         }
@@ -1828,7 +1839,7 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
         for (int k = tid; k < ne; k += IN_THREADS) {
             const int j = __ldcg(elist + k), s = 2 * k + 3 * (j - nv - k);
             int r0 = rows[s], r1 = rows[s + 1];
-            if (k == 0 && j != nv) s_no = 1;  // triangles before the first edge are in no edge's run
+            if (k == 0 && j != nv) s_no = a.st->unsorted = 1;  // triangles before the first edge are in no edge's run
             if (r0 < 0 || r1 <= r0 || r1 >= nv) {
                 s_no = 1;
                 r0 = r1 = 0;
@@ -1877,7 +1888,7 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst(C2Args a) {
             case 4: wrong = in_triangles<4>(col, tab, ends, rows, runs, 0, ne, ne, nv, cols); break;
             default: wrong = in_triangles<0>(col, tab, ends, rows, runs, 0, ne, ne, nv, cols); break;
         }
-        if (wrong) s_no = 1;
+        if (wrong) s_no = a.st->unsorted = 1;
         __syncthreads();
         if (tid == 0 && s_no) a.st->refused = 1;
         // a single small one's outputs at once: 12 points 54 us -> 46-50 in all
@@ -1939,7 +1950,7 @@ __global__ void __launch_bounds__(IN_THREADS, 2) k_c2_inst_more(C2Args a) {
             case 4: check(std::integral_constant<int, 4>()); break;
             default: check(std::integral_constant<int, 0>()); break;
         }
-        if (wrong) a.st->refused = 1;
+        if (wrong) a.st->unsorted = a.st->refused = 1;
         const int pieces = (ne + a.chunk - 1) / a.chunk;
         // as many warps as there is room for rows (one at least: k_c2_inst had it beside 6 ne > 12 chunk bytes)
         int32_t *const row = reinterpret_cast<int32_t *>(ends + a.chunk);
@@ -2152,8 +2163,8 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
 constexpr int64_t IN_MAX_COLS = 1 << 15;
 constexpr int IN_MIN_COUNT = 128;
 
-static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
-    *done = false;
+static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done, bool *looked) {
+    *done = *looked = false;
     cudaStream_t s = ctx->stream;
     static PerDevice one, each, more;
     if (!allow_shared(one, ctx->device, k_c2_inst<true>, IN_SMEM) ||
@@ -2247,6 +2258,7 @@ static int c2_run_inst(Context *ctx, C2Args a, C2Status *hs, bool *done) {
         cudaEventRecord(ctx->ev[1], s);
         int rc = c2_read_status(ctx, a, hs);
         if (rc) return rc;
+        *looked = true;
         if (hs->refused || !hs->no_room) break;
         const long long used[4] = {hs->ne, hs->nv, hs->pairs, hs->run_words};
         for (int q = 0; q < 4; q++)
@@ -2292,17 +2304,21 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
     DevStatus *hb = ctx->h_status + 1;
     int rc;
     bool done = false;
+    bool runs = true, counted = false;  // whether the run form may apply; whether hs holds the counts
     int64_t nv, ne, nt;
     cudaEventRecord(ctx->ev[0], s);
     if (job.rows && (!batch || job.want_nnz >= 0) && (batch ? a.count >= IN_MIN_COUNT || m / a.count <= IN_MAX_COLS : m <= IN_MAX_COLS)) {
         if (job.before) OPH_CUDA_TRY(cudaMemcpyAsync(hb, job.before, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
-        if ((rc = c2_run_inst(ctx, a, hs, &done))) return rc;
-        if (done) {
+        bool looked = false;
+        if ((rc = c2_run_inst(ctx, a, hs, &done, &looked))) return rc;
+        if (looked) {
             job.nnz = hs->nnz;
             job.nnz_read = true;
             job.before_error = job.before ? hb->error : 0;
-            if (job.before_error) return OPH_OK;
-            done = job.want_nnz < 0 || hs->nnz == job.want_nnz;
+            if (job.before_error || hs->bad) return OPH_OK;
+            done = done && (job.want_nnz < 0 || hs->nnz == job.want_nnz);
+            runs = !hs->unsorted;
+            counted = !batch;
         }
     }
     if (!done) {
@@ -2322,12 +2338,23 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
     k_c2_scan<<<1, 1024, 0, s>>>(a, ntiles);
     OPH_CUDA_TRY(cudaGetLastError());
     ctx->launches += 2;
-    if (job.before) OPH_CUDA_TRY(cudaMemcpyAsync(hb, job.before, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
-    if ((rc = c2_read_status(ctx, a, hs))) return rc;
-    job.nnz = hs->nnz;
-    job.nnz_read = true;
-    job.before_error = job.before ? hb->error : 0;
-    if (job.before_error) return OPH_OK;
+    if (counted) {  // one matrix, whose columns a CTA has counted
+        C2Status st{};
+        st.nnz = hs->nnz;
+        st.nv = st.max_nv = hs->nv;
+        st.ne = hs->ne;
+        st.cells = (long long)c2_pitch(st.nv) * st.ne;
+        st.pairs = (long long)c2_pitch(st.nv) * st.nv;
+        st.run_words = (long long)((st.nv + 31) >> 5) * st.ne;
+        *hs = st;
+    } else {
+        if (job.before) OPH_CUDA_TRY(cudaMemcpyAsync(hb, job.before, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
+        if ((rc = c2_read_status(ctx, a, hs))) return rc;
+        job.nnz = hs->nnz;
+        job.nnz_read = true;
+        job.before_error = job.before ? hb->error : 0;
+        if (job.before_error) return OPH_OK;
+    }
     nv = hs->nv;
     ne = hs->ne;
     nt = m - nv - ne;
@@ -2348,7 +2375,7 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
     // every edge with at most two triangles: a graph (an edge found to have
     // more leaves it to the dense form)
     if (3 * nt <= 2 * ne && (rc = c2_run_graph(ctx, a, nv, ne, nt, hs, &done))) return rc;
-    if (!done && !hs->bad && (rc = c2_run_dense<true>(ctx, a, ne, nt, hs, &done))) return rc;
+    if (!done && !hs->bad && runs && (rc = c2_run_dense<true>(ctx, a, ne, nt, hs, &done))) return rc;
     if (!done && !hs->bad && !hs->overflow) {
         // not in runs: the same with the table (the status as before the try)
         if (hs->unsorted) {

@@ -54,12 +54,21 @@ def device(bm):
             torch.empty(2 * bm.m, dtype=torch.int32, device="cuda"))
 
 
-def check_everywhere(ctx, server, bm, batches=(3, 130)):
+def general(ctx, bm):
+    """What the sweeps on D give, for matrices that are no complexes (twist
+    leaves columns of one row alone, and clears by dimension)."""
+    ctx.set_dual("never")
+    low, ess, _ = ctx.reduce(bm, "pms")
+    ctx.set_dual("auto")
+    return low, ess
+
+
+def check_everywhere(ctx, server, bm, batches=(3, 130), want=None):
     """Every entry point that tries the forms gives the oracle's lows: single
     calls with host and device input, with and without ess, 1-based, batches
     that take whole instances and that do not, and the server."""
     import torch
-    want, want_ess, _ = oracle.twist(bm)
+    want, want_ess = want or oracle.twist(bm)[:2]
 
     def same(low, ess, where):
         np.testing.assert_array_equal(low, want, err_msg=where)
@@ -181,3 +190,37 @@ def sparse(nv, cluster):
 def test_many_vertices(ctx, server, nv, cluster):
     """Either side of the forms' limits on vertices."""
     check_everywhere(ctx, server, sparse(nv, cluster), batches=(3,))
+
+
+def test_batches_with_one_that_no_form_takes(ctx):
+    """First, in the middle and last in a batch: the CTAs stop at it, and the
+    general path reduces the whole batch."""
+    from cases import lower_star_volume, simplex_skeleton
+    rips = [cx.rips_cube(20 + 7 * s % 40, seed=s) for s in range(140)]
+    for odd in (lower_star_volume(3, seed=1), simplex_skeleton(7, seed=2),
+                BoundaryMatrix.from_columns([[], [0], [], [0, 2]])):
+        for at in (0, 70, 140):
+            mats = rips[:at] + [odd] + rips[at:]
+            lows, esss, _ = ctx.reduce_batch(mats, "pms")
+            for b in {0, 1, at, 139, 140}:
+                want, want_ess = general(ctx, odd) if b == at else oracle.twist(mats[b])[:2]
+                np.testing.assert_array_equal(lows[b], want)
+                np.testing.assert_array_equal(esss[b], want_ess)
+
+
+@pytest.mark.parametrize("last", [0, 1, 2, 3, 4])
+def test_last_columns_of_any_width(ctx, server, last):
+    """The look at a host matrix's last columns: widths of other complexes at
+    the end, before the last 64 columns, and at their edge."""
+    bm = cx.rips_cube(9, seed=last)
+    cols = [bm.column(j).tolist() for j in range(bm.m)]
+    if last == 4:  # the triangles of four points
+        points = []
+        for j, c in enumerate(cols):
+            points.append({j} if not c else set().union(*(points[x] for x in c)))
+        rows = [j for j in range(bm.m) if len(cols[j]) == 3 and points[j] <= {0, 2, 3, 7}]
+    else:
+        rows = list(range(last))
+    for gap in (0, 62, 63, 64, 200):
+        m = BoundaryMatrix.from_columns(cols + [rows] + [[]] * gap)
+        check_everywhere(ctx, server, m, batches=(3,), want=general(ctx, m))
