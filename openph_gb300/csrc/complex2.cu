@@ -113,7 +113,11 @@ __host__ __device__ constexpr int rs_wave(int threads) { return threads >= 1024 
 __host__ __device__ constexpr int rs_list(int threads) { return threads >= 1024 ? 16384 : 4096; }
 constexpr int RS_FLAG = 1 << 30;
 // Many vertices: long rows and few, long residual columns, so large CTAs and
-// windows; below, more CTAs.
+// windows; below, more CTAs.  The table form takes large ones always: its
+// columns, of random orders above all, are long sums of one another, which
+// published windows add at once (a random order of all simplices on 40 points
+// 1,905 us with small CTAs and 452 with large; where all lists are short, on a
+// grid of 125 points, 303 and 325).
 constexpr int RS_MAPS = 512;  // windows of published columns kept, 16 MB
 constexpr int RS_SMALL_NV = 160, RS_SMALL = 256, RS_SMALL_WORDS = 4096, RS_LARGE = 1024, RS_LARGE_WORDS = 8192;
 
@@ -1223,6 +1227,9 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
 // 8,192: 356 us, 16,384: 272); batches of small ones as many CTAs as fit: six
 // an SM, at 40 registers with some spills, took 1,556-1,581 us for 1,024
 // complexes, five 1,607-1,628, four 1,618-1,644.
+// Table: lists run out (`overflow`) where columns are sums of sums, in random
+// orders on 50 points and more; all CTAs then stop, for the general path's time
+// comes on top: 1,390 us of 1,720 on 50 points, 1,690 of 2,150 on 60.
 template <bool RUNS, int THREADS, int WORDS>
 __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_residual(C2Args a) {
     if (a.st->bad || (RUNS && (a.st->unsorted || a.st->refused || a.st->no_room))) return;
@@ -1232,7 +1239,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
     constexpr int WAVE = rs_wave(THREADS);
     constexpr int HEAD = MAPS ? 4 : 0;  // of a published list: its window's place (-1: none), start, and what lies past it
     __shared__ int s_low[NW], s_cnt[NW], s_wave[WAVE];
-    __shared__ int s_i, s_later, s_act, s_other;
+    __shared__ int s_i, s_later, s_act, s_other, s_stop;
     __shared__ unsigned long long s_sum, s_sums[WAVE];
     enum { ACT_DONE, ACT_ADD, ACT_STEAL, ACT_FAIL };
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1242,11 +1249,12 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
     for (;;) {
         if (tid == 0) {
             s_i = atomicAdd(&a.st->cursor, 1);
+            if (!RUNS) s_stop = *(volatile int *)&a.st->overflow;
             s_later = INT_MAX;
         }
         __syncthreads();
         const int i = s_i;
-        if (i >= nres) break;
+        if (i >= nres || (!RUNS && s_stop)) break;
         int k = a.res[i];
         const C2Inst in = a.inst[a.erec[k].z];
         // columns here are relative to in.wbase; an owner's value in low[] is col - shift
@@ -1365,6 +1373,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
             const bool have = cnt > 0 && (s_wave[0] & ~RS_FLAG) == low;
             wave = min(2 * wave, WAVE);
             __syncthreads();
+            if (!RUNS && tid == 0) s_stop = *(volatile int *)&a.st->overflow;
             if (tid < cnt) {  // the owners, all at once
                 const int t = s_wave[tid] & ~RS_FLAG, fl = s_wave[tid] & RS_FLAG;
                 int o;
@@ -1374,7 +1383,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
             }
             __syncthreads();
             const int p0 = have ? s_wave[0] : -1;
-            if (n + WAVE > RS_LIST) {
+            if (n + WAVE > RS_LIST || (!RUNS && s_stop)) {
                 if (tid == 0) a.st->overflow = 1;
                 break;
             }
@@ -2090,8 +2099,8 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     const long long cells = RUNS ? hs->pairs : hs->cells, run_words = RUNS ? hs->run_words : 0;
     if (hs->max_nv > (RUNS ? 1 << ADJ_SHIFT : C2_MAX_NV) || 3 * cells > room || 2 * run_words > room) return OPH_OK;
     cudaStream_t s = ctx->stream;
-    const bool small = hs->max_nv <= RS_SMALL_NV;
-    int gr = small ? c2_residual_grid<RUNS, RS_SMALL, RS_SMALL_WORDS>(ctx)
+    const bool small = RUNS && hs->max_nv <= RS_SMALL_NV;
+    int gr = small ? c2_residual_grid<true, RS_SMALL, RS_SMALL_WORDS>(ctx)
                    : c2_residual_grid<RUNS, RS_LARGE, RS_LARGE_WORDS>(ctx);
     if (gr == 0) return OPH_OK;
     // the components of C2_MAX_NV vertices take 48 KB beside the kernel's own shared memory
@@ -2143,7 +2152,7 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     }
     if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
     if (small)
-        k_c2_residual<RUNS, RS_SMALL, RS_SMALL_WORDS><<<gr, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
+        k_c2_residual<true, RS_SMALL, RS_SMALL_WORDS><<<gr, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
     else
         k_c2_residual<RUNS, RS_LARGE, RS_LARGE_WORDS><<<gr, RS_LARGE, RS_LARGE_WORDS * sizeof(uint32_t), s>>>(a);
     if (!c2_launched()) return OPH_OK;

@@ -192,6 +192,29 @@ def test_many_vertices(ctx, server, nv, cluster):
     check_everywhere(ctx, server, sparse(nv, cluster), batches=(3,))
 
 
+def reordered(bm, seed, only=None):
+    """The complex in a random filtration order, or one in which the simplices
+    of `only` rows take random values and the others their faces'."""
+    rng = np.random.default_rng(seed)
+    size = np.diff(bm.colptr)
+    val = rng.random(bm.m)
+    if only is not None:
+        val[size != only] = 0
+    for j in range(bm.m):
+        col = bm.column(j)
+        if len(col):
+            val[j] = max(val[j], val[col].max() + (1e-9 if only in (None, len(col)) else 0))
+    return faces_late(bm, np.argsort(val, kind="stable"))
+
+
+@pytest.mark.parametrize("n,only", [(20, None), (36, None), (40, 2), (50, None), (62, None), (62, 2), (90, None)])
+def test_orders_whose_lists_run_out(ctx, server, n, only):
+    """Random orders: columns that are sums of sums, whose lists fit, or fill
+    up on one CTA while the others are at work (up to and past the sizes of
+    whole instances)."""
+    check_everywhere(ctx, server, reordered(cx.rips_cube(n, seed=n), n, only), batches=(3,) if n > 50 else (3, 130))
+
+
 def test_batches_with_one_that_no_form_takes(ctx):
     """First, in the middle and last in a batch: the CTAs stop at it, and the
     general path reduces the whole batch."""
