@@ -156,7 +156,8 @@ int oph_reduce_batch_device(oph_context *ctx, int algo, int32_t count, const int
  * one block-diagonal column space, admits queued requests between sweeps
  * while they fit in the device arena (budget_bytes of HBM, allocated up
  * front), and releases each request as soon as it has converged.  At most
- * max_active requests are on the device at once.  Simplicial 2-complexes need
+ * max_active requests are on the device at once, those in the lanes included.
+ * Simplicial 2-complexes need
  * no sweeps: four lanes beside the worker, each with a context of its own,
  * reduce them as they come; the others, and those the lanes cannot take, join
  * the sweeps (OPH_SERVE_CHAIN_CAP set: all of them).  There each request is reduced on

@@ -366,6 +366,7 @@ struct Server {
     std::vector<Context *> lane_ctx;
     std::deque<Request *> direct;       // requests for the lanes
     int in_lanes = 0;                   // of them and in a lane
+    int on_sweeps = 0;                  // slots taken, or about to be
     std::condition_variable cv_lane;
     cudaMemPool_t mem = nullptr;        // submitted matrices (kept between requests, up to the rest of that share)
     cudaStream_t sub_stream = nullptr;  // submissions: copy, check, grade
@@ -408,6 +409,14 @@ struct Server {
     int64_t region_ints(int64_t m, int64_t nnz) const { return packed_ints(m, nnz) * 4 + 4096; }
     // staging regions of admitted requests, released after the next sync
     std::vector<std::pair<int64_t, int64_t>> staged;
+
+    // Requests in the lanes and in the sweeps' slots come to max_slots at most.  A
+    // lane leaves a place to the sweeps while they have requests waiting and none
+    // at work; after a failure of the worker there is nobody to leave it to.
+    int at_work() const { return on_sweeps + in_lanes - (int)direct.size(); }
+    bool lane_room() const {
+        return error || at_work() + (on_sweeps == 0 && !pending.empty() ? 1 : 0) < max_slots;
+    }
 
     int grid(int64_t n) const {
         int64_t gsz = (n + 255) / 256, cap = (int64_t)ctx->sm_count * 16;
@@ -581,6 +590,7 @@ struct Server {
                 pool.release(r->reg, r->reg_ints);
                 slots[r->slot] = nullptr;
                 r->slot = -1;
+                on_sweeps--;
                 if (r->split && !r->user) r->part_done = true;
             }
             for (Request *r : users) {
@@ -595,6 +605,7 @@ struct Server {
             }
         }
         cv_done.notify_all();
+        cv_lane.notify_all();
     }
 
     // After a sweep: the D part of every split request whose D' part has
@@ -644,6 +655,7 @@ struct Server {
     void fail_all(int rc) {
         std::lock_guard<std::mutex> lk(mu);
         error = rc;
+        cv_lane.notify_all();
         for (auto &kv : all)
             if (!kv.second->done && !kv.second->in_lane) {  // the lanes finish or fail theirs
                 kv.second->status = rc;
@@ -732,7 +744,7 @@ struct Server {
             Request *r = nullptr;
             {
                 std::unique_lock<std::mutex> lk(mu);
-                cv_lane.wait(lk, [&] { return stop || !direct.empty(); });
+                cv_lane.wait(lk, [&] { return direct.empty() ? stop : lane_room(); });
                 if (direct.empty()) return;
                 r = direct.front();
                 direct.pop_front();
@@ -763,6 +775,7 @@ struct Server {
             }
             cv_done.notify_all();
             cv_work.notify_one();
+            cv_lane.notify_all();
         }
     }
 
@@ -774,18 +787,25 @@ struct Server {
             Request *r = nullptr;
             {
                 std::unique_lock<std::mutex> lk(mu);
-                if (wait_for_work && active == 0) cv_work.wait(lk, [&] { return (stop && in_lanes == 0) || !pending.empty(); });
-                if (pending.empty()) break;
+                if (wait_for_work && active == 0)
+                    cv_work.wait(lk, [&] {
+                        return pending.empty() ? stop && in_lanes == 0 : at_work() < max_slots;
+                    });
+                if (pending.empty() || at_work() >= max_slots) break;
                 r = pending.front();
+                on_sweeps++;
             }
             int b = -1;
             for (int k = 0; k < max_slots; k++)
                 if (!slots[k]) { b = k; break; }
-            if (b < 0 || admit(r, b, s) != 0) break;  // no room now: retry after the next sweep
+            const bool ok = b >= 0 && admit(r, b, s) == 0;
             {
                 std::lock_guard<std::mutex> lk(mu);
-                pending.pop_front();
+                if (ok) pending.pop_front();
+                else on_sweeps--;
             }
+            cv_lane.notify_all();
+            if (!ok) break;  // no room now: retry after the next sweep
             active++;
             n++;
         }
@@ -823,9 +843,9 @@ struct Server {
                     if (stop && in_lanes == 0 && pending.empty() && active == 0) return;
                 }
                 if (active == 0) {
+                    std::lock_guard<std::mutex> lk(mu);
                     if (!pending.empty()) {
                         // the head request cannot fit even in an empty arena
-                        std::lock_guard<std::mutex> lk(mu);
                         Request *r = pending.front();
                         pending.pop_front();
                         if (r->user) {  // a split request's D part: the request fails
@@ -838,6 +858,7 @@ struct Server {
                         r->status = OPH_ERR_OOM;
                         r->done = true;
                         cv_done.notify_all();
+                        cv_lane.notify_all();
                     }
                     continue;
                 }
