@@ -157,14 +157,15 @@ int oph_reduce_batch_device(oph_context *ctx, int algo, int32_t count, const int
  * while they fit in the device arena (budget_bytes of HBM, allocated up
  * front), and releases each request as soon as it has converged.  At most
  * max_active requests are on the device at once, those in the lanes included.
- * Simplicial 2-complexes need
- * no sweeps: four lanes beside the worker, each with a context of its own,
- * reduce them as they come; the others, and those the lanes cannot take, join
- * the sweeps (OPH_SERVE_CHAIN_CAP set: all of them).  There each request is reduced on
- * the matrix a single-matrix pms reduction would choose for it (OPH_DUAL_AUTO
- * below: a Rips-like request through its anti-transpose, built at
- * admission; a request split by block as two parts side by side, the D part
- * joining after the D' part's first sweep), and the results are identical to
+ * Simplicial 2-complexes need no sweeps: four lanes beside the worker, each
+ * with a context of its own, reduce them as they come; the others, and those
+ * the lanes cannot take, join the sweeps (all of them when OPH_SERVE_CHAIN_CAP,
+ * or one of OPH_NO_CLUSTER, OPH_NO_INST_TRANSPOSE, OPH_HOST_LOOP and OPH_TRACE,
+ * is set at creation).  There each request is reduced on the matrix a
+ * single-matrix pms reduction would choose for it (OPH_DUAL_AUTO below: a
+ * Rips-like request through its anti-transpose, built at admission; a request
+ * split by block as two parts side by side, the D part joining after the D'
+ * part's first sweep), and the results are identical to
  * that reduction's.  A chain of additions in the bitmap tiers stops after 128
  * additions a sweep (environment variable OPH_SERVE_CHAIN_CAP, read at
  * creation; 0 for no limit) and goes on in the next sweep, so no sweep of

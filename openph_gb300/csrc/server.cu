@@ -1086,8 +1086,9 @@ __attribute__((visibility("default"))) int oph_server_create(int device, int64_t
     sv->pool.init(sv->pool_ints);
     sv->slots.assign(max_active, nullptr);
     sv->worker = std::thread([sv] { sv->run(); });
-    // the chain cap is the sweeps': who sets it means them
-    if (!getenv("OPH_SERVE_CHAIN_CAP"))
+    // the chain cap and the switches of the general path (complex2_applies) are the
+    // sweeps': who sets one means them
+    if (!getenv("OPH_SERVE_CHAIN_CAP") && complex2_applies(ctx, OPH_ALGO_PMS))
         for (int q = 0; q < SERVE_LANES; q++) {
             oph_context *c = nullptr;
             if (oph_context_create(device, &c) != OPH_OK) break;  // the sweeps take every request

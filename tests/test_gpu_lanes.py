@@ -50,3 +50,17 @@ def test_max_active(cuda_lib, mix, max_active):
         th.join()
         assert srv.stats()["completed"] == 2 * len(reqs)
     assert 1 <= max(seen) <= max_active
+
+
+@pytest.mark.parametrize("switch", [None, "OPH_SERVE_CHAIN_CAP", "OPH_NO_CLUSTER", "OPH_NO_INST_TRANSPOSE",
+                                    "OPH_HOST_LOOP", "OPH_TRACE"])
+def test_switches_of_the_general_path(cuda_lib, monkeypatch, mix, switch):
+    """Without one, 2-complexes take no sweep; with one set at creation, every
+    request goes through the sweeps."""
+    if switch:
+        monkeypatch.setenv(switch, "0" if switch == "OPH_TRACE" else "1")
+    reqs, want = mix
+    lanes = [k for k in range(len(reqs)) if k % 4]
+    with Server(0, budget_bytes=8 << 30, max_active=8) as srv:
+        check(srv, [srv.submit(reqs[k]) for k in lanes], [want[k] for k in lanes])
+        assert (srv.stats()["sweeps"] > 0) == bool(switch)
