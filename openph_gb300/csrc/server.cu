@@ -754,8 +754,10 @@ struct Server {
             bool taken = false;
             int rc = reduce_in_lane(c, r, &info, &taken);
             if (rc == OPH_OK && !taken) rc = grade(r, c->stream);
+            bool tight;  // another lane may have waited for this one's place
             {
                 std::lock_guard<std::mutex> lk(mu);
+                tight = at_work() + 1 >= max_slots;
                 in_lanes--;
                 r->in_lane = false;
                 if (error && !taken) rc = error;  // the worker is gone
@@ -775,7 +777,7 @@ struct Server {
             }
             cv_done.notify_all();
             cv_work.notify_one();
-            cv_lane.notify_all();
+            if (tight) cv_lane.notify_all();
         }
     }
 
