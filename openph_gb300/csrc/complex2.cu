@@ -50,6 +50,7 @@
 // included, is left to the general path and its own checks.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 
@@ -2286,6 +2287,16 @@ bool complex2_applies(const Context *ctx, int algo) {
         if (getenv(name)) return false;
     return algo == OPH_ALGO_PMS && !ctx->track && ctx->dual == OPH_DUAL_AUTO && ctx->tier0 == 0 &&
            ctx->max_sweeps == 0 && ctx->initial_pool_bytes == 0 && !ctx->count_slots;
+}
+
+size_t complex2_least(const Context *ctx, int64_t m, int64_t nnz) {
+    const double columns = 8.0 * m + 0.5 * m;  // outputs, words
+    // a graph: three triangles to two edges at most, so the edges hold a quarter of the entries at least
+    const double graph_ne = nnz / 4.0, graph = columns + 56 * graph_ne + 12 * std::max(0.0, m - nnz / 2.0);
+    // dense: ne edges span at most sqrt(2)/3 ne^1.5 triangles; the arena, and a list a CTA
+    const double ne = std::pow(nnz / 3.42, 2.0 / 3.0), lists = std::min(ne, 6.0 * ctx->sm_count);
+    const double dense = columns + 0.25 * m + 24 * ne + sizeof(int32_t) * ((1 << 20) + lists * rs_list(RS_SMALL));
+    return (size_t)(5 * nnz > 12 * m ? dense : std::min(graph, dense));
 }
 
 int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {

@@ -97,6 +97,9 @@ struct C2Job {
     int before_error = 0;
 };
 bool complex2_applies(const Context *ctx, int algo);
+// The least that any form takes of the context's buffers for a matrix of m
+// columns and nnz entries, low and ess included: with less it is not worth a try.
+size_t complex2_least(const Context *ctx, int64_t m, int64_t nnz);
 int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken);
 
 // variants.cu

@@ -1144,7 +1144,10 @@ int submit_copy(oph_server *sv, int64_t m, int64_t nnz, const int64_t *colptr, c
     r->nnz = nnz;
     r->d_buf = buf;
     r->t_submit = now_ms();
-    const bool lane = m > 0 && !sv->lanes.empty();
+    // what a lane's share of the budget cannot hold joins the sweeps at once, not
+    // behind the requests that came while a lane tried
+    const bool lane =
+        m > 0 && !sv->lanes.empty() && (int64_t)complex2_least(sv->lane_ctx[0], m, nnz) <= sv->lane_ctx[0]->budget;
     if (!lane) {
         const int rc = sv->grade(r, s);
         if (rc) {

@@ -64,3 +64,14 @@ def test_switches_of_the_general_path(cuda_lib, monkeypatch, mix, switch):
     with Server(0, budget_bytes=8 << 30, max_active=8) as srv:
         check(srv, [srv.submit(reqs[k]) for k in lanes], [want[k] for k in lanes])
         assert (srv.stats()["sweeps"] > 0) == bool(switch)
+
+
+@pytest.mark.parametrize("budget", [64 << 20, 256 << 20, 2 << 30])
+def test_requests_beyond_a_lane(cuda_lib, mix, budget):
+    """Budgets whose lanes hold some of the requests, or next to none: those go
+    to the sweeps, beside the lanes."""
+    reqs, want = mix
+    with Server(0, budget_bytes=budget, max_active=16) as srv:
+        for _ in range(2):
+            check(srv, [srv.submit(bm) for bm in reqs], want)
+        assert srv.stats()["sweeps"] > 0 and srv.stats()["completed"] == 2 * len(reqs)
