@@ -345,9 +345,13 @@ __global__ void k_srv_set_region(unsigned long long *ipool, int *ireps, int *iov
     iover[b] = 0;
 }
 
-__global__ void k_srv_sweep_reset(DevStatus *st) {
+// Before a sweep that compacts into list `next`: one that finds no repeated low
+// writes no list, and what an earlier sweep left there would be merged with
+// the requests admitted meanwhile, which may hold the same columns by now.
+__global__ void k_srv_sweep_reset(DevStatus *st, int next) {
     st->converged = 0;
     st->overflow = 0;
+    st->ucount[next] = 0;
 }
 
 // ------------------------------------------------------------------ server
@@ -900,7 +904,7 @@ struct Server {
             gg.m = grid(hi);
             gg.t = (int)std::max<int64_t>(1, std::min<int64_t>(sa.ntiles, (int64_t)ctx->sm_count * 8));
             cudaMemsetAsync(a.ireps, 0, sizeof(int) * max_slots, s);
-            k_srv_sweep_reset<<<1, 1, 0, s>>>(a.st);
+            k_srv_sweep_reset<<<1, 1, 0, s>>>(a.st, lp ^ 1);
             launch_sweep(sa, gg, s, lp, trace > 1 ? tev : nullptr);  // compacts list lp into the other one
             lp ^= 1;
             cudaMemcpyAsync(h_ireps, a.ireps, sizeof(int) * max_slots, cudaMemcpyDeviceToHost, s);

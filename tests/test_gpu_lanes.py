@@ -43,11 +43,13 @@ def test_max_active(cuda_lib, mix, max_active):
                 seen.append(srv.stats()["active"])
         th = threading.Thread(target=watch)
         th.start()
-        for order in (range(len(reqs)), reversed(range(len(reqs)))):
-            order = list(order)
-            check(srv, [srv.submit(reqs[k]) for k in order], [want[k] for k in order])
-        stop.set()
-        th.join()
+        try:
+            for order in (range(len(reqs)), reversed(range(len(reqs)))):
+                order = list(order)
+                check(srv, [srv.submit(reqs[k]) for k in order], [want[k] for k in order])
+        finally:
+            stop.set()
+            th.join()
         assert srv.stats()["completed"] == 2 * len(reqs)
     assert 1 <= max(seen) <= max_active
 
@@ -75,3 +77,14 @@ def test_requests_beyond_a_lane(cuda_lib, mix, budget):
         for _ in range(2):
             check(srv, [srv.submit(bm) for bm in reqs], want)
         assert srv.stats()["sweeps"] > 0 and srv.stats()["completed"] == 2 * len(reqs)
+
+
+@pytest.mark.parametrize("max_active", [2, 3, 4])
+def test_admissions_beside_a_last_sweep(cuda_lib, mix, max_active):
+    """Few places: a sweep often finds every listed request reduced while others
+    are being admitted, into columns that earlier ones have left."""
+    reqs, want = mix
+    order = [k for k in range(len(reqs)) if k % 4 == 0] * 3  # the volumes, which need sweeps
+    for _ in range(25):
+        with Server(0, budget_bytes=1 << 30, max_active=max_active) as srv:
+            check(srv, [srv.submit(reqs[k]) for k in order], [want[k] for k in order])
