@@ -187,7 +187,8 @@ typedef struct {
     int64_t completed, pending, active, sweeps, regrows;
     int64_t pool_bytes_in_use, columns_in_use, arena_bytes;
     int64_t dual_admitted;  /* requests with a part reduced through their
-                               anti-transpose (split by block or whole)   */
+                               anti-transpose (split by block or whole; in a
+                               lane: for which OPH_DUAL_AUTO names it)    */
 } oph_server_counters;
 
 int oph_server_create(int device, int64_t budget_bytes, int32_t max_active, oph_server **out);

@@ -46,8 +46,11 @@
 // What is accepted is checked on the device before it is reported: every
 // column has 0, 2 or 3 rows, ascending and in range, the rows of an edge are
 // vertices, the rows of a triangle are the three edges of a triangle (so
-// D D = 0, which clearing relies on).  Anything else, malformed input
-// included, is left to the general path and its own checks.
+// D D = 0, which clearing relies on).  A column may come before its rows'
+// columns (rows above the diagonal are accepted input): the graph takes any
+// order, the runs know theirs, vertices first and every triangle in its last
+// edge's run, and the table wants triangles after their edges.  Anything else,
+// malformed input included, is left to the general path and its own checks.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -640,8 +643,8 @@ __device__ __forceinline__ bool c2_meet(unsigned *arrived, unsigned goal) {
 // pixels and more), so they are shortened for all nodes at once before roots
 // are looked for edge by edge.  A round is two passes over the live edges,
 // each followed by a meeting of the grid.  Bound by the latency of its
-// dependent loads and the meetings (2-3 us): 10 rounds on the 512 x 512
-// lower-star image (1.57M slots, then 320K, 76K, ...), 19 on white noise of
+// dependent loads and the meetings (2-3 us): 11 rounds on a smooth 512 x 512
+// lower-star image (1.57M slots, then 320K, 76K, ...), 17 on white noise of
 // that size.
 __global__ void __launch_bounds__(C2_THREADS) k_c2_graph(C2Args a, int max_rounds) {
     if (a.st->bad || a.st->crowded) return;  // written by earlier kernels: the same for every block
@@ -1204,8 +1207,9 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
 // * Waves: not only the low's pivot is added but those of the first rs_wave()
 //   set bits that have one.  Every column added comes before k in D' (a row
 //   of the sum lies in a column of the sum, and its owner is the first column
-//   that can hold it), so this is a reduction like any other, and the chain
-//   of 970 additions on the torus takes 35 waves of 32.
+//   that can hold it), so this is a reduction like any other, and the longest
+//   column of the 5M-column torus (some 1,200 additions) takes 17 waves of up
+//   to 128.
 // * Owners: low[t] names the owner of triangle t.  A residual column claims
 //   its low by compare-and-swap once its list is published.  Found claimed by
 //   an earlier column, that column is added; by a later one, the claim is
@@ -1217,8 +1221,8 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
 //   adder's (the windows lie on a common grid, and nothing comes before a
 //   low), instead of the 25 columns or so of the list one by one.
 //
-// Bound by the longest column, on one SM: of 14K cycles a wave on the torus
-// 9.7K went into some 77 columns, 126 cycles each (240 instructions a warp),
+// Bound by the longest column, on one SM: of 14K cycles a wave (of 32) on the
+// torus 9.7K went into some 77 columns, 126 cycles each (240 instructions a warp),
 // 2.7K into the search of the window and 1.5K into the owners.  With published
 // windows 28 columns are left to a wave: 250 us -> 190, with wider waves 165
 // (a device call on 200K columns 337 -> 278 -> 252).  Flattening the lists of
