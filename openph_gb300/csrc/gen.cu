@@ -65,7 +65,7 @@ __device__ __forceinline__ unsigned long long lexkey(int dim, unsigned a, unsign
 // What the host reads of a Rips complex, and the longest edge (its bits).
 struct RipsTotals {
     unsigned long long edges, triangles, longest;
-    int tied, crowded;  // equally long edges; too many of one coarse length
+    int tied, crowded;  // equally long edges; ranks not settled: too many of one coarse length, or tied
 };
 __global__ void __launch_bounds__(256) k_rips_dist(const double *__restrict__ pts, int n, int d, double thr,
                                                    double *__restrict__ D, unsigned *__restrict__ adj, int words,
@@ -309,18 +309,18 @@ __global__ void k_rips_rank(const unsigned *__restrict__ coarse, const unsigned 
             const unsigned c = coarse[k];
             int same = 0;
             bool tied = false;
-            for (long long q = k - 1; q >= 0 && coarse[q] == c && same < RIPS_SAME; q--, same++) {
+            for (long long q = k - 1; q >= 0 && coarse[q] == c && same < RIPS_SAME && !tied; q--, same++) {
                 const unsigned long long x = key[place[q]];
                 at -= x > mine;
-                tied |= x == mine;
+                tied = x == mine;
             }
-            for (long long q = k + 1; q < E && coarse[q] == c && same < RIPS_SAME; q++, same++) {
+            for (long long q = k + 1; q < E && coarse[q] == c && same < RIPS_SAME && !tied; q++, same++) {
                 const unsigned long long x = key[place[q]];
                 at += x < mine;
-                tied |= x == mine;
+                tied = x == mine;
             }
             if (tied) totals->tied = 1;
-            if (same == RIPS_SAME) totals->crowded = 1;
+            if (tied || same == RIPS_SAME) totals->crowded = 1;  // (nothing more is read from these ranks)
         } else if (k > 0 && key[place[k - 1]] == mine) {
             totals->tied = 1;
         }
@@ -687,12 +687,20 @@ __attribute__((visibility("default"))) int oph_rips_device(oph_context *ctx, con
         OPH_CUDA_TRY(cudaGetLastError());
         OPH_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, s));
         OPH_CUDA_TRY(cudaStreamSynchronize(s));
-        if (t.crowded && !exact) continue;
-        // (with equally long edges the triangles by last edge add up to the same)
-        m = n + E + (int64_t)t.triangles;
-        nnz = 2 * E + 3 * (int64_t)t.triangles;
+        if (t.crowded && !t.tied && !exact) continue;
         break;
     }
+    if (t.tied) {  // the triangles above every edge
+        OPH_CUDA_TRY(cudaMemsetAsync(tcnt, 0, 8 * e1, s));
+        k_rips_tri_count<<<wgrid, 256, 0, s>>>(adj, n, words, eoff, tcnt);
+        OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(st2, sb2, tcnt, toff, E + 1, s));
+        if (t.crowded) {  // (else those by last edge have been counted, as many)
+            OPH_CUDA_TRY(cudaMemcpyAsync(&t.triangles, toff + E, sizeof(long long), cudaMemcpyDeviceToHost, s));
+            OPH_CUDA_TRY(cudaStreamSynchronize(s));
+        }
+    }
+    m = n + E + (int64_t)t.triangles;
+    nnz = 2 * E + 3 * (int64_t)t.triangles;
     if (m >= (1ll << 31)) return OPH_ERR_BAD_INPUT;
     if (m_out) *m_out = m;
     if (nnz_out) *nnz_out = nnz;
@@ -702,9 +710,6 @@ __attribute__((visibility("default"))) int oph_rips_device(oph_context *ctx, con
     SKey *k0 = (SKey *)sc.get(sizeof(SKey) * (size_t)m), *k1 = (SKey *)sc.get(sizeof(SKey) * (size_t)m);
     int32_t *vpos = (int32_t *)sc.get(sizeof(int32_t) * (size_t)n);
     if (!k0 || !k1 || !vpos) return OPH_ERR_OOM;
-    OPH_CUDA_TRY(cudaMemsetAsync(tcnt, 0, 8 * e1, s));
-    k_rips_tri_count<<<wgrid, 256, 0, s>>>(adj, n, words, eoff, tcnt);
-    OPH_CUDA_TRY(cub::DeviceScan::ExclusiveSum(st2, sb2, tcnt, toff, E + 1, s));
     k_rips_keys<<<wgrid, 256, 0, s>>>(adj, D, n, words, eoff, toff, E, k0);
     SKey *sorted = nullptr;
     int rc = sort_and_colptr(ctx, sc, k0, k1, m, d_colptr, d_value, &sorted);

@@ -110,3 +110,12 @@ def test_lower_star_odd_sides_equal_host(cuda_lib, h, w):
     img[h // 2:, w // 2:] *= -1
     img[0, 0], img[1, 1], img[0, 1] = 0.0, -0.0, 0.0
     assert_same(cx.lower_star_device(img), cx.lower_star(img))
+
+
+def test_rips_many_equal_lengths(cuda_lib):
+    """Hundreds of edges of one length, all of them in one coarse class or in
+    each of many: the order by full keys at once."""
+    g = np.stack(np.meshgrid(*[np.arange(6.0)] * 3), -1).reshape(-1, 3)
+    for pts, thr in ((g, 1.0), (g, 1.8), (g[:120], np.inf), (np.zeros((70, 3)), np.inf),
+                     (np.concatenate([g[:50], cx.points_cube(60, 2) + 9]), 2.0)):
+        assert_same(cx.rips_device(pts, thr), cx.rips(pts, thr))
