@@ -2310,6 +2310,7 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
     ctx->prof = oph_profile{};
     const int64_t m = job.m;
     if (m < 1 || m >= (1 << 29)) return OPH_OK;
+    if (!job.rows && job.want_nnz == 0) return OPH_OK;  // vertices only: one sweep finds nothing to do
     cudaStream_t s = ctx->stream;
     const int64_t nwords = (m + 31) / 32, ntiles = (m + C2_TILE - 1) / C2_TILE;
     const bool batch = job.inst_off != nullptr;

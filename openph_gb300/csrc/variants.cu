@@ -1233,7 +1233,7 @@ int run_sequential(Context *ctx, Work &w, int algo, int32_t *d_ess, oph_info *in
         if (side_by_side) {
             int rc = claim_columns(ctx, w, -1, false, &regrows);
             bool done = rc == OPH_OK;
-            if (done && a.row_quirk) rc = row_estimate(ctx, w, d_ess, &done);
+            if (done && a.row_quirk && w.nnz > 0) rc = row_estimate(ctx, w, d_ess, &done);
             if (rc && rc != OPH_ERR_OOM && rc != OPH_ERR_OVERFLOW) return rc;
             if (!done) {
                 side_by_side = false;

@@ -247,3 +247,13 @@ def test_last_columns_of_any_width(ctx, server, last):
     for gap in (0, 62, 63, 64, 200):
         m = BoundaryMatrix.from_columns(cols + [rows] + [[]] * gap)
         check_everywhere(ctx, server, m, batches=(3,), want=general(ctx, m))
+
+
+@pytest.mark.parametrize("m", [1, 2, 3000, 70_000])
+def test_vertices_only(ctx, server, m):
+    """Nothing to reduce, through every entry point and algorithm."""
+    bm = BoundaryMatrix(np.zeros(m + 1, np.int64), np.zeros(0, np.int32))
+    check_everywhere(ctx, server, bm, batches=(3,))
+    for algo in api.ALGORITHMS:
+        low, ess, _ = ctx.reduce(bm, algo)
+        assert (low == -1).all() and (ess == 1).all()
