@@ -2019,7 +2019,7 @@ int c2_named_matrix(int64_t m, int64_t nv, int64_t ne, int64_t nt) {
 }
 }  // namespace
 
-// False when the driver refused a launch (its resources): the form is not done,
+// False when CUDA refused a launch (its resources): the form is not done,
 // and the general path says what it thinks of the device.
 static bool c2_launched() { return cudaGetLastError() == cudaSuccess; }
 

@@ -234,7 +234,7 @@ struct Context {
     std::vector<unsigned char> loop_key;
 };
 
-// A positive answer of the driver, asked for once a device (an occupancy, an
+// A positive answer of CUDA, asked for once a device (an occupancy, an
 // attribute set); several threads may ask at the same time.
 struct PerDevice {
     std::atomic<int> known[64] = {};

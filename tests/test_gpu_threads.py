@@ -1,5 +1,5 @@
 """Several threads, a context each, in a process whose first calls they make:
-what is asked of the driver once a device is asked by all of them at the same
+what is asked of CUDA once a device is asked by all of them at the same
 time, and graph reductions take turns."""
 import subprocess
 import sys
