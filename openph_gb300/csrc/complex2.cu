@@ -89,7 +89,7 @@ struct C2Status {
     int live[3];     // edges left, by round modulo three
     unsigned arrived;  // blocks at the graph's meetings
     unsigned long long joins;
-    int max_nv;      // the largest instance's vertices
+    int max_nv, max_cols;  // the largest instance's vertices, columns
     int unsorted;    // the triangles do not come in runs
     int next;        // whole instances: the CTAs' queue
     int refused;     //   an instance is too large, or no complex in runs
@@ -118,12 +118,15 @@ __host__ __device__ constexpr int rs_list(int threads) { return threads >= 1024 
 constexpr int RS_FLAG = 1 << 30;
 // Many vertices: long rows and few, long residual columns, so large CTAs and
 // windows; below, more CTAs.  The table form takes large ones always: its
-// columns, of random orders above all, are long sums of one another, which
-// published windows add at once (a random order of all simplices on 40 points
-// 1,905 us with small CTAs and 452 with large; where all lists are short, on a
-// grid of 125 points, 303 and 325).
+// columns, of random orders above all, are sums of sums, whose lists grow with
+// every addition, while published windows add at once.  Up to 2^18 columns an
+// instance (RS_XL_WORDS: 1.3M) one window holds them all and no list is kept.  A
+// random order of all simplices on 40 points took 1,905 us with small CTAs, 452
+// with large ones, 388 without lists; on 60 points the lists ran out after 430
+// us (and the column store took 1,700), now 615.  Where all columns are short, on
+// a grid of 125 points, small CTAs took 303 us, large ones take 325.
 constexpr int RS_MAPS = 512;  // windows of published columns kept, 16 MB
-constexpr int RS_SMALL_NV = 160, RS_SMALL = 256, RS_SMALL_WORDS = 4096, RS_LARGE = 1024, RS_LARGE_WORDS = 8192;
+constexpr int RS_SMALL_NV = 160, RS_SMALL = 256, RS_SMALL_WORDS = 4096, RS_LARGE = 1024, RS_LARGE_WORDS = 8192, RS_XL_WORDS = 40960;
 
 struct C2Args {
     int64_t m;
@@ -166,8 +169,9 @@ struct C2Args {
     int32_t *arena;
     long long arena_cap;
     int32_t *lists;           // per CTA: rs_list() edges
-    uint32_t *maps;           // large CTAs: windows of published columns, map_cap of RS_LARGE_WORDS
-    int map_cap;
+    uint32_t *maps;           // large CTAs: windows of published columns, map_cap of map_words
+    int map_cap, map_words;
+    int whole;                // table: a window holds every column of an instance, and no list is kept
     // whole instances: what the tables hold (edges, vertices, table entries, run words)
     long long cap_e, cap_v, cap_c, cap_r;
     long long nnz;            //   and the entries rows[] holds (-1: colptr[m], one matrix)
@@ -324,6 +328,7 @@ __global__ void __launch_bounds__(1024) k_c2_scan(C2Args a, int64_t ntiles) {
             s.cols = a.m;
             a.inst[0] = s;
             a.st->max_nv = s.nv;
+            a.st->max_cols = (int)a.m;
             a.st->cells = (long long)c2_pitch(s.nv) * s.ne;
             a.st->pairs = (long long)c2_pitch(s.nv) * s.nv;
             a.st->run_words = (long long)((s.nv + 31) >> 5) * s.ne;
@@ -348,6 +353,7 @@ __global__ void __launch_bounds__(1024) k_c2_scan(C2Args a, int64_t ntiles) {
                 s.base = o0;
                 s.cols = o1 - o0;
                 atomicMax(&a.st->max_nv, s.nv);
+                atomicMax(&a.st->max_cols, (int)s.cols);
                 if (s.ne == 0 && s.nv != s.cols) a.st->bad = 1;  // triangles, but no edges for their rows
             }
         }
@@ -1232,9 +1238,8 @@ __device__ __forceinline__ void rs_toggle(const C2Args &a, const C2Inst &in, int
 // 8,192: 356 us, 16,384: 272); batches of small ones as many CTAs as fit: six
 // an SM, at 40 registers with some spills, took 1,556-1,581 us for 1,024
 // complexes, five 1,607-1,628, four 1,618-1,644.
-// Table: lists run out (`overflow`) where columns are sums of sums, in random
-// orders on 50 points and more; all CTAs then stop, for the general path's time
-// comes on top: 1,390 us of 1,720 on 50 points, 1,690 of 2,150 on 60.
+// Table: where lists run out (`overflow`; past RS_XL_WORDS), or windows, all
+// CTAs stop: the general path's time comes on top.
 template <bool RUNS, int THREADS, int WORDS>
 __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_residual(C2Args a) {
     if (a.st->bad || (RUNS && (a.st->unsorted || a.st->refused || a.st->no_room))) return;
@@ -1249,6 +1254,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
     enum { ACT_DONE, ACT_ADD, ACT_STEAL, ACT_FAIL };
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nres = a.st->nres, none = a.one_based ? 0 : -1;
+    const bool whole = !RUNS && MAPS && a.whole;
+    const int map_words = whole ? a.map_words : WORDS;
     int32_t *list = a.lists + (size_t)blockIdx.x * RS_LIST;
     unsigned long long adds = 0, slots = 0;
     for (;;) {
@@ -1277,9 +1284,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
             const int32_t *const from = a.arena + (sum >> 24) + HEAD;
             if (n + len > RS_LIST) return false;
             if (MAPS && head.x >= 0 && head.y >= w0) {
-                const uint32_t *const map = a.maps + (size_t)head.x * WORDS;
+                const uint32_t *const map = a.maps + (size_t)head.x * map_words;
                 const int off = (head.y - w0) >> 5;
-                for (int q = off + 4 * tid; q < WORDS; q += 4 * THREADS) {
+                for (int q = off + 4 * tid; q < map_words; q += 4 * THREADS) {
                     const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(map + (q - off)));
                     if (x.x) rs_xor(bits + q, x.x);
                     if (x.y) rs_xor(bits + q + 1, x.y);
@@ -1301,7 +1308,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
         for (;;) {
             if (fresh) {
                 // on a grid of half windows, so that published ones fit each other
-                w0 = MAPS ? pos & ~(16 * WORDS - 1) : pos & ~127;
+                w0 = whole ? (int)(in.base - in.wbase) & ~127 : MAPS ? pos & ~(16 * WORDS - 1) : pos & ~127;
                 if (RUNS)
                     hi = (w0 + 32ll * WORDS >= cols ? in.eoff + in.ne : c2_edge_rank(a, in, w0 + 32 * WORDS)) - in.eoff;
                 for (int q = 4 * tid; q < WORDS; q += 4 * THREADS)
@@ -1388,18 +1395,19 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
             }
             __syncthreads();
             const int p0 = have ? s_wave[0] : -1;
-            if (n + WAVE > RS_LIST || (!RUNS && s_stop)) {
+            if ((!whole && n + WAVE > RS_LIST) || (!RUNS && s_stop)) {
                 if (tid == 0) a.st->overflow = 1;
                 break;
             }
             if (!have || ((p0 & RS_FLAG) && (p0 & ~RS_FLAG) < k)) {
                 // claim the low: the list first, then the owner
                 if (tid == 0) {
-                    const int room = (HEAD + n + 3) & ~3;
+                    const int room = (HEAD + (whole ? 0 : n) + 3) & ~3;
                     const unsigned long long off = atomicAdd(&a.st->arena, (unsigned long long)room);
                     s_sum = off;
                     s_act = off + room > (unsigned long long)a.arena_cap ? ACT_FAIL : ACT_DONE;
                     if (MAPS) s_other = atomicAdd(&a.st->maps, 1);
+                    if (whole && s_other >= a.map_cap) s_act = ACT_FAIL;
                 }
                 if (MAPS && later != INT_MAX) atomicMin(&s_later, later);
                 __syncthreads();
@@ -1411,16 +1419,16 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
                 if (MAPS) {
                     const int place = s_other < a.map_cap ? s_other : -1;
                     if (place >= 0)
-                        for (int q = 4 * tid; q < WORDS; q += 4 * THREADS)
-                            __stcg(reinterpret_cast<uint4 *>(a.maps + (size_t)place * WORDS + q),
+                        for (int q = 4 * tid; q < map_words; q += 4 * THREADS)
+                            __stcg(reinterpret_cast<uint4 *>(a.maps + (size_t)place * map_words + q),
                                    *reinterpret_cast<const uint4 *>(bits + q));
                     if (tid == 0) __stcg(reinterpret_cast<int4 *>(a.arena + off), make_int4(place, w0, s_later, 0));
                 }
-                for (int v = tid; v < n; v += THREADS) __stcg(a.arena + off + HEAD + v, __ldcg(list + v));
+                for (int v = tid; !whole && v < n; v += THREADS) __stcg(a.arena + off + HEAD + v, __ldcg(list + v));
                 __threadfence();
                 __syncthreads();
                 if (tid == 0) {
-                    *(volatile unsigned long long *)(a.sum + k) = (off << 24) | (unsigned)n;
+                    *(volatile unsigned long long *)(a.sum + k) = (off << 24) | (unsigned)(whole ? 0 : n);
                     const int e = a.elist[k];
                     if (out_ess) {
                         out_ess[low] = 0;
@@ -1492,14 +1500,14 @@ __global__ void __launch_bounds__(THREADS, THREADS == RS_SMALL ? 6 : 1) k_c2_res
                 const unsigned m_app = __ballot_sync(0xffffffffu, p >= 0 && !(p & RS_FLAG));
                 nres_w += __popc(__ballot_sync(0xffffffffu, res));
                 if (wid == h / 32) {
-                    if ((m_app >> lane) & 1u) __stcg(list + n + app + __popc(m_app & below(lane)), p);
+                    if (!whole && ((m_app >> lane) & 1u)) __stcg(list + n + app + __popc(m_app & below(lane)), p);
                     if (res) s_sums[h + lane] = *(volatile unsigned long long *)(a.sum + (p & ~RS_FLAG));
                 }
                 app += __popc(m_app);
             }
             for (int q = wid; q < cnt; q += NW)
                 if (!(s_wave[q] & RS_FLAG)) rs_toggle<RUNS, WORDS>(a, in, s_wave[q], w0, hi, bits, later);
-            n += app;
+            if (!whole) n += app;
             adds += app + nres_w;
             slots += (unsigned long long)app * in.nv;
             bool full = false;
@@ -2105,7 +2113,10 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     if (hs->max_nv > (RUNS ? 1 << ADJ_SHIFT : C2_MAX_NV) || 3 * cells > room || 2 * run_words > room) return OPH_OK;
     cudaStream_t s = ctx->stream;
     const bool small = RUNS && hs->max_nv <= RS_SMALL_NV;
+    // (a window starts at a multiple of 128 columns)
+    const bool xl = !RUNS && hs->max_cols > 32 * RS_LARGE_WORDS - 128 && hs->max_cols <= 32 * RS_XL_WORDS - 128;
     int gr = small ? c2_residual_grid<true, RS_SMALL, RS_SMALL_WORDS>(ctx)
+             : xl  ? c2_residual_grid<false, RS_LARGE, RS_XL_WORDS>(ctx)
                    : c2_residual_grid<RUNS, RS_LARGE, RS_LARGE_WORDS>(ctx);
     if (gr == 0) return OPH_OK;
     // the components of C2_MAX_NV vertices take 48 KB beside the kernel's own shared memory
@@ -2126,8 +2137,12 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
         a.sum = c.take<unsigned long long>(ne);
         a.arena = c.take<int32_t>(a.arena_cap);
         a.lists = c.take<int32_t>((size_t)gr * rs_list(small ? RS_SMALL : RS_LARGE));
-        a.map_cap = small ? 0 : (int)std::min<int64_t>(ne, RS_MAPS);
-        a.maps = c.take<uint32_t>((size_t)a.map_cap * RS_LARGE_WORDS);
+        a.whole = !RUNS && hs->max_cols <= 32 * (xl ? RS_XL_WORDS : RS_LARGE_WORDS) - 128;
+        a.map_words = a.whole ? ((hs->max_cols + 127) / 32 + 4) & ~3 : RS_LARGE_WORDS;
+        a.map_cap = small ? 0
+                          : (int)std::min<int64_t>(a.whole ? 2 * ne : ne,
+                                                   (xl ? 4ll : 1ll) * RS_MAPS * RS_LARGE_WORDS / a.map_words);
+        a.maps = c.take<uint32_t>((size_t)a.map_cap * a.map_words);
         if (p) break;
         p = (char *)ctx_alloc(ctx, S_C2_MODE, c.off);
         if (!p) return OPH_OK;
@@ -2158,6 +2173,8 @@ static int c2_run_dense(Context *ctx, C2Args a, int64_t ne, int64_t nt, C2Status
     if (ctx->profile) cudaEventRecord(ctx->ev[2], s);
     if (small)
         k_c2_residual<true, RS_SMALL, RS_SMALL_WORDS><<<gr, RS_SMALL, RS_SMALL_WORDS * sizeof(uint32_t), s>>>(a);
+    else if (xl)
+        k_c2_residual<false, RS_LARGE, RS_XL_WORDS><<<gr, RS_LARGE, RS_XL_WORDS * sizeof(uint32_t), s>>>(a);
     else
         k_c2_residual<RUNS, RS_LARGE, RS_LARGE_WORDS><<<gr, RS_LARGE, RS_LARGE_WORDS * sizeof(uint32_t), s>>>(a);
     if (!c2_launched()) return OPH_OK;
@@ -2367,6 +2384,7 @@ int reduce_complex2(Context *ctx, C2Job &job, oph_info *info, bool *taken) {
         C2Status st{};
         st.nnz = hs->nnz;
         st.nv = st.max_nv = hs->nv;
+        st.max_cols = (int)m;
         st.ne = hs->ne;
         st.cells = (long long)c2_pitch(st.nv) * st.ne;
         st.pairs = (long long)c2_pitch(st.nv) * st.nv;

@@ -208,10 +208,9 @@ def reordered(bm, seed, only=None):
 
 
 @pytest.mark.parametrize("n,only", [(20, None), (36, None), (40, 2), (50, None), (62, None), (62, 2), (90, None)])
-def test_orders_whose_lists_run_out(ctx, server, n, only):
-    """Random orders: columns that are sums of sums, whose lists fit, or fill
-    up on one CTA while the others are at work (up to and past the sizes of
-    whole instances)."""
+def test_random_orders(ctx, server, n, only):
+    """Columns that are sums of sums, many claimed and taken over at the same
+    time (up to and past the sizes of whole instances)."""
     check_everywhere(ctx, server, reordered(cx.rips_cube(n, seed=n), n, only), batches=(3,) if n > 50 else (3, 130))
 
 
@@ -257,3 +256,32 @@ def test_vertices_only(ctx, server, m):
     for algo in api.ALGORITHMS:
         low, ess, _ = ctx.reduce(bm, algo)
         assert (low == -1).all() and (ess == 1).all()
+
+
+@pytest.mark.parametrize("points,cut", [(125, 262_015), (125, 262_016), (125, 262_017), (125, 325_625),
+                                        (201, 1_310_592), (201, 1_310_593)])
+def test_window_of_a_whole_instance(ctx, points, cut):
+    """A grid's complex (ties: the table) cut off at the sizes of the residual
+    columns' windows, alone and behind another in a batch."""
+    g = np.stack(np.meshgrid(*[np.arange(6.0 if points > 125 else 5.0)] * 3), -1).reshape(-1, 3)[:points]
+    bm = cx.rips(g)
+    bm = BoundaryMatrix(bm.colptr[:cut + 1], bm.rows[:bm.colptr[cut]])
+    want, want_ess, _ = oracle.twist(bm)
+    low, ess, _ = ctx.reduce(bm, "pms")
+    np.testing.assert_array_equal(low, want)
+    np.testing.assert_array_equal(ess, want_ess)
+    lows, esss, _ = ctx.reduce_batch([cx.rips_cube(9, seed=1), bm, cx.rips_cube(11, seed=1)], "pms")
+    np.testing.assert_array_equal(lows[1], want)
+    np.testing.assert_array_equal(esss[1], want_ess)
+    np.testing.assert_array_equal(lows[2], oracle.twist(cx.rips_cube(11, seed=1))[0])
+
+
+@pytest.mark.parametrize("n,only,copies", [(25, None, 6), (40, 2, 3), (60, None, 2), (30, 2, 50)])
+def test_batches_in_random_order(ctx, n, only, copies):
+    mats = [reordered(cx.rips_cube(n - k % 3, seed=k), 50 + k, only) for k in range(min(copies, 5))]
+    want = [oracle.twist(bm)[:2] for bm in mats]
+    order = [k % len(mats) for k in range(copies)]
+    lows, esss, _ = ctx.reduce_batch([mats[k] for k in order], "pms")
+    for k, low, ess in zip(order, lows, esss):
+        np.testing.assert_array_equal(low, want[k][0])
+        np.testing.assert_array_equal(ess, want[k][1])
